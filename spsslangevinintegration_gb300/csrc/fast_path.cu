@@ -56,6 +56,7 @@ struct FastControl
                             // device launch of the rebuild graph was refused
   int uses_verlet;
   int tile_next;            // work counter of the persistent tile kernel
+  unsigned ticket;          // blocks of the running reduction that are done (its last block puts it back to 0)
   int triggered;            // the last step's displacement trigger fired (its rebuild may already be done)
   long long sample_every;   // order-parameter samples after steps that are multiples of this (0: none)
   long long sample_from;    // ... and not before this step
@@ -131,7 +132,7 @@ struct FastBuffers
   short *vl;
   int *vl_cnt;
   float *nu;             // natural frequencies (global field), slot = original index
-  double *field;         // Z = <e^{i phi}>, W = <omega e^{i phi}> and derived values (global field)
+  float *field;          // Z = <e^{i phi}>, W = <omega e^{i phi}> and derived values (global field)
   double *field_partial; // block partials of the field sums
   const SysParams *sys;  // system table
   const int *sys_of;     // system of each slot (equivalently of each original index)
@@ -224,7 +225,12 @@ struct FastPath
   DeviceArray<int> sys_of, tile_sys;
   DeviceArray<SysControl> sysctl;
   DeviceArray<float> nu;
-  DeviceArray<double> field, field_partial;
+  DeviceArray<float> field;
+  DeviceArray<double> field_partial;
+  // order parameters of the whole context (fast_order_parameters)
+  DeviceArray<double2> turn_table;     // unit vectors of the phase's bit groups, made at first use
+  DeviceArray<double> observe_partial;
+  double *h_order = nullptr;           // pinned: the four sums, written by the reduction's last block
   std::vector<SysParams> h_sys;
   int nsys = 1;
   int total_cells = 1;
@@ -488,6 +494,21 @@ __device__ __forceinline__ void rows_from_shared(double *__restrict__ g, const d
   }
 }
 
+// A block's rows of floats to global (possibly host) memory, 16 bytes at a time
+// where the array allows it.
+__device__ __forceinline__ void rows_from_shared(float *__restrict__ g, const float *sh, int count)
+{
+  int done = 0;
+  if (((uintptr_t) g & 15) == 0)
+  {
+    float4 *g4 = reinterpret_cast<float4 *>(g);
+    const float4 *s4 = reinterpret_cast<const float4 *>(sh);
+    for (int i = threadIdx.x; i < count / 4; i += blockDim.x) g4[i] = s4[i];
+    done = count & ~3;
+  }
+  for (int i = done + threadIdx.x; i < count; i += blockDim.x) g[i] = sh[i];
+}
+
 // Upload from reference AoS, one thread per original index p (its block's
 // rows read as one coalesced chunk), scattered to the particle's slot inv[p]
 // (identity when no slot order exists yet).
@@ -567,6 +588,54 @@ __global__ void fast_download_kernel(double *__restrict__ x, int n, int s, int m
   }
   __syncthreads();
   rows_from_shared(x + (long) s * p0, rows, count);
+}
+
+// Trajectory frame: the float conversion of the downloaded state (and, WRAP,
+// the observers' wraps), one thread per original index, without the FP64 copy
+// of the state in between; `out` may be host memory, which the rows then reach
+// over the host link as whole lines.  N = 4,194,304 to page-locked memory:
+// FP64 download, frame kernel and copy took 0.79 ms, this takes 0.535, of
+// which the link needs 0.52 (100.7 MB).
+template<bool WRAP>
+__global__ void __launch_bounds__(256) fast_frame_kernel(float *__restrict__ out, int n, int s, int model, FastBuffers B)
+{
+  extern __shared__ __align__(16) float frame_rows[];
+  const int p0 = blockIdx.x * blockDim.x;
+  const int count = min((int) blockDim.x, n - p0) * s;
+  const int p = p0 + threadIdx.x;
+  if (p < n)
+  {
+    const int par = B.ctrl->parity;
+    const unsigned q = B.inv[p];
+    const uint4 r = (par ? B.rec1 : B.rec0)[q];
+    const uint4 a = (par ? B.aux1 : B.aux0)[q];
+    const int2 im = B.img[p];
+    const int turns = B.turns[p];
+    float *st = frame_rows + s * threadIdx.x;
+    // the expressions of fast_download_kernel
+    float x = __double2float_rn((double) im.x + (double) join64(r.x, a.x) * 5.421010862427522e-20);
+    float y = __double2float_rn((double) im.y + (double) join64(r.y, a.y) * 5.421010862427522e-20);
+    float ph = __double2float_rn(6.283185307179586 * ((double) turns + (double) a.z * 2.3283064365386963e-10));
+    if (WRAP)
+    {
+      x = frame_wrap_position(x);
+      y = frame_wrap_position(y);
+      ph = frame_wrap_phase(ph);
+    }
+    st[0] = x;
+    st[1] = y;
+    const int ip = model == 1 ? 2 : 4;
+    st[ip] = ph;
+    st[ip + 1] = __uint_as_float(a.w);
+    if (model == 2)
+    {
+      const float2 v = B.vel[q];
+      st[2] = v.x;
+      st[3] = v.y;
+    }
+  }
+  __syncthreads();
+  rows_from_shared(out + (long) s * p0, frame_rows, count);
 }
 
 // ---------------------------------------------------------------- rebuild
@@ -1973,6 +2042,31 @@ __device__ __forceinline__ double warp_sum(double v)
   return v;
 }
 
+// v / |v| in FP64, added to (sx, sy); nothing for v = 0.  The reciprocal square
+// root starts from the FP32 one (relative error below 2^-22) and takes one
+// third-order step, y (1 + e/2 + 3 e^2/8) with e = 1 - |v|^2 y^2, whose
+// remainder 5 e^3 / 16 is below 1e-19: 12 FP64 instructions against about 70
+// for the square root and the two divisions (GB300 runs FP64 at 1/69 of its
+// FP32 rate, so the FP64 count is what these reductions cost).
+__device__ __forceinline__ void add_direction(float2 v, double &sx, double &sy)
+{
+  // powers of two that bring the larger component near 1: no overflow or
+  // underflow of the FP32 square for any finite v
+  const float big = fmaxf(fabsf(v.x), fabsf(v.y));
+  if (!(big > 0.0f)) return;
+  const int ex = max(-120, min(120, 127 - (int) (__float_as_uint(big) >> 23)));
+  const float scale = __uint_as_float((uint32_t) (ex + 127) << 23);
+  const float fx = __fmul_rn(v.x, scale), fy = __fmul_rn(v.y, scale);
+  const double x = fx, y = fy;
+  const double m2 = fma(x, x, y * y);
+  if (!(m2 > 0.0)) return;  // a NaN component: left out, as a comparison |v| > 0 leaves it out
+  const double r = rsqrtf(fmaf(fx, fx, __fmul_rn(fy, fy)));
+  const double e = fma(-m2 * r, r, 1.0);
+  const double c = fma(r * e, fma(e, 0.375, 0.5), r);
+  sx = fma(x, c, sx);
+  sy = fma(y, c, sy);
+}
+
 // partial[k] = sums over chunk k (at most kOrderChunk slots of one system);
 // a small grid walks all chunks, so the gated launch that finds no sampling
 // step costs a few hundred CTAs.
@@ -1996,14 +2090,7 @@ __global__ void fast_order_partials_kernel(FastParams P, FastBuffers B, OrderSum
       a1 += (double) __uint_as_float(r.w);
       if (P.model == 2)
       {
-        const float2 v = B.vel[q];
-        const double vx = v.x, vy = v.y;
-        const double m = sqrt(vx * vx + vy * vy);
-        if (m > 0.0)
-        {
-          a2 += vx / m;
-          a3 += vy / m;
-        }
+        add_direction(B.vel[q], a2, a3);
       }
     }
     a0 = warp_sum(a0);
@@ -2082,63 +2169,181 @@ __global__ void fast_order_finish_kernel(FastParams P, FastBuffers B, const Orde
 // of the SRK stepper, to W = <omega e^{i phi}>), both summed in FP64 over the
 // stage state; no lists.
 
-constexpr int kFieldBlocks = 304;
+constexpr int kFieldBlocks = 2 * 152;
 
-__global__ void fast_field_partials_kernel(FastParams P, FastBuffers B)
+// Error-free running sum hi + lo of floats (Knuth's TwoSum): the rounding
+// error of every addition is kept in lo.
+__device__ __forceinline__ void two_sum_add(float &hi, float &lo, float x)
+{
+  const float s = __fadd_rn(hi, x);
+  const float b = __fsub_rn(s, hi);
+  lo = __fadd_rn(lo, __fadd_rn(__fsub_rn(hi, __fsub_rn(s, b)), __fsub_rn(x, b)));
+  hi = s;
+}
+
+// Whether this block is the last of the launch to get here (its partials are
+// written); all threads of the block get the answer.
+__device__ __forceinline__ bool last_block(FastControl *ctrl)
+{
+  __shared__ unsigned mine;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0)
+  {
+    mine = atomicAdd(&ctrl->ticket, 1u);
+    if (mine == gridDim.x - 1) ctrl->ticket = 0u;
+    __threadfence();
+  }
+  __syncthreads();
+  return mine == gridDim.x - 1;
+}
+
+// Sums of cos phi, sin phi, omega cos phi, omega sin phi over the particles,
+// and from them field = {Re Z, Im Z, |Z|, Re W, Im W, |W|, cos arg W, sin arg W}
+// by the last block.  A thread's few terms are summed in FP32 with every
+// rounding error kept (products too), which no FP64 sum of them would better
+// by more than 1e-14 of a term; FP64 takes over at the thread sums.  FP64
+// conversions and additions for every particle (seven on a 1/69-rate pipe)
+// and one thread adding 304 partials in turn made these two kernels 21.3 and
+// 71.5 us at N = 999,983 (cold); one launch of 28 us now.
+__global__ void __launch_bounds__(256) fast_field_partials_kernel(FastParams P, FastBuffers B)
 {
   __shared__ double sh[4][8];
   const int par = B.ctrl->parity;
   const uint4 *rec = par ? B.rec1 : B.rec0;
   const uint4 *aux = par ? B.aux1 : B.aux0;
-  double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
+  float hi[4] = {0.f, 0.f, 0.f, 0.f}, lo[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < P.n; q += gridDim.x * blockDim.x)
   {
-    const double c = (double) __uint_as_float(rec[q].z), sn = (double) __uint_as_float(rec[q].w);
-    const double w = (double) __uint_as_float(aux[q].w);
-    a0 += c;
-    a1 += sn;
-    a2 += w * c;
-    a3 += w * sn;
+    const uint2 cs = __ldg(reinterpret_cast<const uint2 *>(&rec[q].z));
+    const float c = __uint_as_float(cs.x), sn = __uint_as_float(cs.y);
+    const float w = __uint_as_float(__ldg(&aux[q].w));
+    const float wc = __fmul_rn(w, c), ws = __fmul_rn(w, sn);
+    two_sum_add(hi[0], lo[0], c);
+    two_sum_add(hi[1], lo[1], sn);
+    two_sum_add(hi[2], lo[2], wc);
+    two_sum_add(hi[3], lo[3], ws);
+    lo[2] = __fadd_rn(lo[2], fmaf(w, c, -wc));
+    lo[3] = __fadd_rn(lo[3], fmaf(w, sn, -ws));
   }
-  a0 = warp_sum(a0);
-  a1 = warp_sum(a1);
-  a2 = warp_sum(a2);
-  a3 = warp_sum(a3);
-  const int wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  if ((threadIdx.x & 31) == 0)
+  const int wid = threadIdx.x >> 5;
+#pragma unroll
+  for (int c = 0; c < 4; ++c)
   {
-    sh[0][wid] = a0;
-    sh[1][wid] = a1;
-    sh[2][wid] = a2;
-    sh[3][wid] = a3;
+    const double a = warp_sum((double) hi[c] + (double) lo[c]);
+    if ((threadIdx.x & 31) == 0) sh[c][wid] = a;
   }
   __syncthreads();
-  if (threadIdx.x == 0)
+  if (threadIdx.x < 4)
   {
-    double t[4] = {0.0, 0.0, 0.0, 0.0};
-    for (int k = 0; k < nw; ++k)
-      for (int c = 0; c < 4; ++c) t[c] += sh[c][k];
-    for (int c = 0; c < 4; ++c) B.field_partial[4 * blockIdx.x + c] = t[c];
+    double t = 0.0;
+    for (int k = 0; k < 8; ++k) t += sh[threadIdx.x][k];
+    B.field_partial[4 * blockIdx.x + threadIdx.x] = t;
   }
+  if (!last_block(B.ctrl)) return;
+  double t[4];
+  block_sum_partials(B.field_partial, gridDim.x, t);
+  if (threadIdx.x != 0) return;
+  const double zr = t[0] / P.n, zi = t[1] / P.n, wr = t[2] / P.n, wi = t[3] / P.n;
+  const double aw = sqrt(wr * wr + wi * wi);
+  B.field[0] = (float) zr;
+  B.field[1] = (float) zi;
+  B.field[2] = (float) sqrt(zr * zr + zi * zi);
+  B.field[3] = (float) wr;
+  B.field[4] = (float) wi;
+  B.field[5] = (float) aw;
+  B.field[6] = aw > 0.0 ? (float) (wr / aw) : 1.0f;  // arg 0 = 0, as std::arg
+  B.field[7] = aw > 0.0 ? (float) (wi / aw) : 0.0f;
 }
 
-// field = {Re Z, Im Z, |Z|, Re W, Im W, |W|, cos arg W, sin arg W}
-__global__ void fast_field_finish_kernel(FastParams P, FastBuffers B)
+// ---------------------------------------------------------------- order parameters of the context
+//
+// The observers' reduction over every particle of the context
+// (BinaryObserverFirstOrder.cpp:125-142, BinaryObserverSecondOrder.cpp:121-138)
+// from the 32-bit phases and the velocities, in FP64.
+
+// e^{i 2 pi P / 2^32} = T1[P >> 21] T2[(P >> 10) & 2047] T3[P & 1023].
+constexpr int kTurn1 = 2048, kTurn2 = 2048, kTurn3 = 1024, kTurnAll = kTurn1 + kTurn2 + kTurn3;
+// Contexts of at least this many particles take e^{i phi} from the tables (80
+// KB of shared memory a block, so at most two blocks an SM), smaller ones
+// evaluate sincospi.  A whole order-parameter call, tables / sincospi: 31.3 /
+// 31.9 us at 50,000 particles, 33.0 / 35.2 at 100,000, 66.6 / 105.2 at
+// 1,000,000; below 50,000 the two do not differ.
+constexpr int kTurnTableMin = 50000;
+
+__global__ void fast_turn_table_kernel(double2 *__restrict__ table)
 {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  double t[4] = {0.0, 0.0, 0.0, 0.0};
-  for (int b = 0; b < kFieldBlocks; ++b)
-    for (int c = 0; c < 4; ++c) t[c] += B.field_partial[4 * b + c];
-  const double zr = t[0] / P.n, zi = t[1] / P.n, wr = t[2] / P.n, wi = t[3] / P.n;
-  const double aw = atan2(wi, wr);  // arg 0 = 0, as std::arg
-  B.field[0] = zr;
-  B.field[1] = zi;
-  B.field[2] = sqrt(zr * zr + zi * zi);
-  B.field[3] = wr;
-  B.field[4] = wi;
-  B.field[5] = sqrt(wr * wr + wi * wi);
-  B.field[6] = cos(aw);
-  B.field[7] = sin(aw);
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= kTurnAll) return;
+  double turns;  // exact: a power of two times an integer
+  if (i < kTurn1) turns = (double) i / 2048.0;
+  else if (i < kTurn1 + kTurn2) turns = (double) (i - kTurn1) / 4194304.0;
+  else turns = (double) (i - kTurn1 - kTurn2) / 4294967296.0;
+  double s, c;
+  sincospi(2.0 * turns, &s, &c);
+  table[i] = make_double2(c, s);
+}
+
+// FP64 instructions bound this kernel (4,194,304 particles: 8 a phase with the
+// tables, 12 a velocity, 8.4 us for each of them at the measured 0.50 T/s).
+// Through an FP64 copy of the state, sincos, square roots and divisions it was
+// three kernels of 181 + 436 + 204 us; this one takes 179 us.
+template<bool TABLE>
+__global__ void __launch_bounds__(256) fast_observe_kernel(FastParams P, FastBuffers B, const double2 *__restrict__ table,
+                                                           double *__restrict__ partial, double *__restrict__ sums)
+{
+  extern __shared__ __align__(16) double2 turn[];
+  __shared__ double sh[4][8];
+  if (TABLE)
+  {
+    for (int i = threadIdx.x; i < kTurnAll; i += blockDim.x) turn[i] = table[i];
+    __syncthreads();
+  }
+  const uint4 *aux = B.ctrl->parity ? B.aux1 : B.aux0;
+  double a[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll 2
+  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < P.n; q += gridDim.x * blockDim.x)
+  {
+    const uint32_t ph = __ldg(&aux[q].z);
+    const float2 v = P.model == 2 ? B.vel[q] : make_float2(0.f, 0.f);
+    if (TABLE)
+    {
+      const double2 x = turn[ph >> 21], y = turn[kTurn1 + ((ph >> 10) & 2047u)];
+      const double2 z = turn[kTurn1 + kTurn2 + (ph & 1023u)];
+      const double yc = fma(y.x, z.x, -(y.y * z.y)), ys = fma(y.x, z.y, y.y * z.x);
+      a[0] = fma(x.x, yc, a[0]);
+      a[0] = fma(-x.y, ys, a[0]);
+      a[1] = fma(x.y, yc, a[1]);
+      a[1] = fma(x.x, ys, a[1]);
+    } else
+    {
+      double sn, cs;
+      sincospi((double) ph * 4.6566128730773926e-10, &sn, &cs);  // 2 / 2^32, exact
+      a[0] += cs;
+      a[1] += sn;
+    }
+    if (P.model == 2) add_direction(v, a[2], a[3]);
+  }
+  const int wid = threadIdx.x >> 5;
+#pragma unroll
+  for (int c = 0; c < 4; ++c)
+  {
+    const double t = warp_sum(a[c]);
+    if ((threadIdx.x & 31) == 0) sh[c][wid] = t;
+  }
+  __syncthreads();
+  if (threadIdx.x < 4)
+  {
+    double t = 0.0;
+    for (int k = 0; k < 8; ++k) t += sh[threadIdx.x][k];
+    partial[4 * blockIdx.x + threadIdx.x] = t;
+  }
+  if (!last_block(B.ctrl)) return;
+  double t[4];
+  block_sum_partials(partial, gridDim.x, t);
+  if (threadIdx.x == 0)
+    for (int c = 0; c < 4; ++c) sums[c] = t[c];
 }
 
 // One SE or SRK step of the first-order model in the global field:
@@ -2164,9 +2369,9 @@ __global__ void __launch_bounds__(kTB, 4) fast_global_step_kernel(FastParams P, 
     const uint4 ai = ain[q];
     float z[6];
     draw_noise<1, STEPPER>(P, ctrl->step, p, z);
-    const float zr = (float) B.field[0], zi = (float) B.field[1], az = (float) B.field[2];
-    const float wr = (float) B.field[3], wim = (float) B.field[4], aw = (float) B.field[5];
-    const float cw = (float) B.field[6], sw = (float) B.field[7];
+    const float zr = B.field[0], zi = B.field[1], az = B.field[2];
+    const float wr = B.field[3], wim = B.field[4], aw = B.field[5];
+    const float cw = B.field[6], sw = B.field[7];
     const float cphi = __uint_as_float(ri.z), sphi = __uint_as_float(ri.w), wi = __uint_as_float(ai.w);
     const float SZ = fmaf(zi, cphi, -__fmul_rn(zr, sphi));  // |Z| sin(arg Z - phi)
     const float KZ = fmaf(zr, cphi, __fmul_rn(zi, sphi));   // |Z| cos(arg Z - phi)
@@ -2547,6 +2752,9 @@ void fast_destroy(spss_ctx *ctx)
   f->nu.release();
   f->field.release();
   f->field_partial.release();
+  f->turn_table.release();
+  f->observe_partial.release();
+  if (f->h_order) cudaFreeHost(f->h_order);
   f->order_partial.release();
   f->order_items.release();
   f->order_first.release();
@@ -2633,9 +2841,8 @@ static void launch_step_kind(spss_ctx *ctx, const FastParams &P, const FastBuffe
     if (MODEL == 1)
     {
       fast_field_partials_kernel<<<kFieldBlocks, 256, 0, ctx->stream>>>(P, B);
-      fast_field_finish_kernel<<<1, 32, 0, ctx->stream>>>(P, B);
       fast_global_step_kernel<STEPPER><<<grid, kTB, 0, ctx->stream>>>(P, B);
-      ctx->launches += 2;
+      ctx->launches += 1;
     }
   } else if (ctx->fast->kind == KIND_ALL_PAIRS)
   {
@@ -3042,6 +3249,50 @@ int fast_system_order_parameters(spss_ctx *ctx, double *h_out)
                                 ctx->stream));
   SPSS_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
   return SPSS_OK;
+}
+
+// |<e^{i phi}>|, its argument and the velocity-direction pair over the context.
+int fast_order_parameters(spss_ctx *ctx, double *out4)
+{
+  FastPath *f = ctx->fast;
+  const bool table = ctx->p.n >= kTurnTableMin;
+  const int blocks = std::min(2 * 152, blocks_for(ctx->p.n, 256));
+  const int smem = table ? kTurnAll * (int) sizeof(double2) : 0;
+  SPSS_TRY(f->observe_partial.reserve(4 * 2 * 152));
+  if (!f->h_order) SPSS_CUDA_TRY(cudaMallocHost((void **) &f->h_order, 4 * sizeof(double)));
+  if (table && !f->turn_table.ptr)
+  {
+    SPSS_TRY(f->turn_table.reserve(kTurnAll));
+    SPSS_CUDA_TRY(cudaFuncSetAttribute(fast_observe_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    fast_turn_table_kernel<<<blocks_for(kTurnAll, 256), 256, 0, ctx->stream>>>(f->turn_table.ptr);
+    ++ctx->launches;
+    SPSS_TRY(check_launch("fast_turn_table_kernel"));
+  }
+  const FastParams P = params(ctx, 0.0);
+  const FastBuffers B = buffers(ctx);
+  if (table)
+    fast_observe_kernel<true><<<blocks, 256, smem, ctx->stream>>>(P, B, f->turn_table.ptr, f->observe_partial.ptr,
+                                                                  f->h_order);
+  else
+    fast_observe_kernel<false><<<blocks, 256, 0, ctx->stream>>>(P, B, nullptr, f->observe_partial.ptr, f->h_order);
+  ++ctx->launches;
+  SPSS_TRY(check_launch("fast_observe_kernel"));
+  SPSS_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+  // two square roots and two arguments: a chain of FP64 latencies on the device, nothing here
+  order_from_sums(f->h_order, (double) ctx->p.n, ctx->p.model, out4);
+  return SPSS_OK;
+}
+
+// The state as a float frame at `d_out` (device memory, or host memory the GPU addresses).
+int fast_frame(spss_ctx *ctx, int wrap, float *d_out)
+{
+  const int smem = (int) sizeof(float) * 256 * ctx->s, blocks = blocks_for(ctx->p.n, 256);
+  if (wrap)
+    fast_frame_kernel<true><<<blocks, 256, smem, ctx->stream>>>(d_out, ctx->p.n, ctx->s, ctx->p.model, buffers(ctx));
+  else
+    fast_frame_kernel<false><<<blocks, 256, smem, ctx->stream>>>(d_out, ctx->p.n, ctx->s, ctx->p.model, buffers(ctx));
+  ++ctx->launches;
+  return check_launch("fast_frame_kernel");
 }
 
 int fast_rebuild_count(spss_ctx *ctx, unsigned long long *count)

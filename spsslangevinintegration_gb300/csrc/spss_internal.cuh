@@ -210,6 +210,76 @@ __device__ __forceinline__ void normals4_f64(const NoiseKey &nk, uint32_t partic
   box_muller_f64(u.z, u.w, z[2], z[3]);
 }
 
+// ------------------------------------------------------------------ reductions
+
+// Sums of `nparts` partials of four values each, in a fixed order, by one
+// block of 256 threads (the result is valid in thread 0): thread t adds
+// partials t, t + 256, ..., the warps' lanes combine by a shuffle tree, thread
+// 0 adds the warps.
+__device__ __forceinline__ void block_sum_partials(const double *__restrict__ partials, int nparts, double t[4])
+{
+  __shared__ double sh[8][4];
+#pragma unroll
+  for (int c = 0; c < 4; ++c) t[c] = 0.0;
+  for (int b = threadIdx.x; b < nparts; b += 256)
+  {
+    // __ldcg: the partials may have been written by other blocks of the same launch
+    const double2 lo = __ldcg(reinterpret_cast<const double2 *>(partials + 4 * (long) b));
+    const double2 hi = __ldcg(reinterpret_cast<const double2 *>(partials + 4 * (long) b + 2));
+    t[0] += lo.x;
+    t[1] += lo.y;
+    t[2] += hi.x;
+    t[3] += hi.y;
+  }
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) t[c] += __shfl_xor_sync(0xffffffffu, t[c], off);
+  if ((threadIdx.x & 31) == 0)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) sh[threadIdx.x >> 5][c] = t[c];
+  __syncthreads();
+  if (threadIdx.x == 0)
+    for (int w = 1; w < 8; ++w)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) t[c] += sh[w][c];
+}
+
+// {|R|, arg R, |R_v|, arg R_v} from the sums of cos phi, sin phi, v_x/|v|, v_y/|v|.
+__host__ __device__ __forceinline__ void order_from_sums(const double t[4], double n, int model, double *out)
+{
+  const double re = t[0] / n, im = t[1] / n;
+  out[0] = sqrt(re * re + im * im);
+  out[1] = atan2(im, re);
+  if (model == 2)
+  {
+    const double vre = t[2] / n, vim = t[3] / n;
+    out[2] = sqrt(vre * vre + vim * vim);
+    out[3] = atan2(vim, vre);
+  } else
+  {
+    out[2] = out[0];
+    out[3] = out[1];
+  }
+}
+
+// The reference's observer wraps of a frame value, computed in double on the
+// float value and rounded back (BinaryObserverFirstOrder.cpp:112-117,
+// PeriodicBoundaryConditions.cpp:137-145): `x -= floor(x * 1) * 1` and
+// `phi -= floor(phi / 2 pi) * 2 pi`.
+__device__ __forceinline__ float frame_wrap_position(float v)
+{
+  const double d = (double) v;
+  return __double2float_rn(__dsub_rn(d, floor(d)));
+}
+
+__device__ __forceinline__ float frame_wrap_phase(float v)
+{
+  const double two_pi = 6.283185307179586;
+  const double d = (double) v;
+  return __double2float_rn(__dsub_rn(d, __dmul_rn(floor(__ddiv_rn(d, two_pi)), two_pi)));
+}
+
 inline int normals_per_particle(int model, int stepper)
 {
   if (stepper == SPSS_STEPPER_RK4) return 0;
@@ -326,8 +396,7 @@ struct spss_ctx
   int average_count = 0;
   // AoS staging buffers for host-array entry points
   spss::DeviceArray<double> scratch_a, scratch_b, scratch_c;
-  // trajectory frames (spss_frame_async): the AoS state of a fast context and the float frame
-  spss::DeviceArray<double> frame_state;
+  // trajectory frames (spss_frame_async) on their way to memory the GPU cannot address
   spss::DeviceArray<float> frame;
 };
 
@@ -374,6 +443,8 @@ int fast_system_order_parameters(spss_ctx *ctx, double *h_out);
 int fast_batch_run(spss_ctx *ctx, int stepper, double dt, long nsteps, long sample_every, long sample_from);
 int fast_batch_stats(spss_ctx *ctx, double *h_out);
 int fast_batch_reset_stats(spss_ctx *ctx);
+int fast_order_parameters(spss_ctx *ctx, double *out4);
+int fast_frame(spss_ctx *ctx, int wrap, float *d_out);
 int fast_num_systems(const spss_ctx *ctx);
 int fast_system_first(const spss_ctx *ctx, int r);
 
