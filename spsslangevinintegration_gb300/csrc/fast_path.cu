@@ -1086,13 +1086,6 @@ __device__ __forceinline__ void gather_sums(const FastParams &P, const FastBuffe
     // list unusable: the stencil of the rebuild-time cell holds every particle
     // the list would (displacements since the rebuild < skin / 2)
   }
-  if (KIND == KIND_ALL_PAIRS)
-  {
-    const int end = P.first + P.sub_n;
-    for (int j = P.first; j < end; ++j)
-      if (j != q) candidate<OMEGA, KIND == KIND_CELLS>(P, ri, Xi, Yi, rec, aux, j, a);
-    return;
-  }
   const int *coff = B.cell_off + P.cell0;
   const int c = B.cell_sorted[q] - P.cell0;
   const int cx = c % P.nc, cy = c / P.nc;
@@ -1438,35 +1431,242 @@ __device__ __forceinline__ void publish_max(FastControl *ctrl, SysControl *sysct
   if ((threadIdx.x & 31) == 0 && err) atomicOr(&ctrl->error, 1);
 }
 
-// One SE or SRK step of one particle per thread, neighbours gathered from
-// global memory (all pairs; also usable for every kind).
-template<int MODEL, int STEPPER, int KIND, bool MULTI>
-__global__ void __launch_bounds__(kTB, 4) fast_step_kernel(FastParams P, FastBuffers B)
+// ---------------------------------------------------------------- all pairs
+//
+// A block steps 32 particles, one per lane, and its 16 warps share the scan:
+// warp w takes the w-th sixteenth of the system's slots, so all lanes of a warp
+// test the same candidate (one record load for the warp) and a system of a few
+// thousand particles fills the chip.  The slices are summed in order, so a
+// particle's sums depend on its system alone (a system of a batch has the
+// bits it has by itself).  One thread per particle scanning everything left
+// most SMs idle (N = 4,000: 16 blocks): 625 us, this 18 us; the
+// instructions of a pair bound it from about N = 4,000 on.
+constexpr int kPairWarps = 16;
+
+// Running sums over a slice, the (cos, sin) and omega (cos, sin) pairs packed.
+// The count is kept as a float (exact below 2^24, more than a slice can be
+// scanned through): the integer pipe is what bounds the loop.
+struct PairAcc
 {
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  float2 cs, w;
+  float card;
+};
+
+// Both components of a packed FP32 pair in one instruction (each rounded as
+// the scalar addition and fma).
+__device__ __forceinline__ float2 add2(float2 a, float2 b)
+{
+  float2 r;
+  asm("{\n .reg .b64 x, y, z;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n add.rn.f32x2 z, x, y;\n"
+      " mov.b64 {%0, %1}, z;\n}"
+      : "=f"(r.x), "=f"(r.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return r;
+}
+
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c)
+{
+  float2 r;
+  asm("{\n .reg .b64 x, y, z, u;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n mov.b64 z, {%6, %7};\n"
+      " fma.rn.f32x2 u, x, y, z;\n mov.b64 {%0, %1}, u;\n}"
+      : "=f"(r.x), "=f"(r.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return r;
+}
+
+// U staged candidates, decided in FP32; `nearest` keeps the smallest distance
+// of any d2 to rho^2, so the caller sees whether one lay inside the guard band.
+// SELF: candidate `self` (an index into the staged rows) is the particle.
+template<bool OMEGA, bool SELF, int U>
+__device__ __forceinline__ void pair_group(const uint4 *srec, const float *sw, int k0, int self, uint32_t xi, uint32_t yi,
+                                           float rho2, float &nearest, PairAcc &a)
+{
+  uint4 r[U];
+  float w[U], d2[U];
+#pragma unroll
+  for (int k = 0; k < U; ++k)
+  {
+    r[k] = srec[k0 + k];
+    w[k] = OMEGA ? sw[k0 + k] : 0.0f;
+  }
+#pragma unroll
+  for (int k = 0; k < U; ++k)
+  {
+    const float dx = (float) (int) (r[k].x - xi);
+    const float dy = (float) (int) (r[k].y - yi);
+    d2[k] = fmaf(dx, dx, dy * dy);
+    if (SELF && k0 + k == self) d2[k] = 3.0e38f;
+    nearest = fminf(nearest, fabsf(d2[k] - rho2));
+  }
+#pragma unroll
+  for (int k = 0; k < U; ++k)
+    if (d2[k] <= rho2)
+    {
+      const float2 cs = make_float2(__uint_as_float(r[k].z), __uint_as_float(r[k].w));
+      a.cs = add2(a.cs, cs);
+      if (OMEGA) a.w = fma2(make_float2(w[k], w[k]), cs, a.w);
+      a.card += 1.0f;
+    }
+}
+
+// The same candidates again (one of them lies inside the guard band), each
+// decided by in_range.
+template<bool OMEGA>
+__device__ __noinline__ void pair_batch_exact(const uint4 *srec, const float *sw,
+                                              const uint4 *__restrict__ aux, int j0, int m, int q, const uint4 ri,
+                                              float rho2, float band, double rho2_d, PairAcc *acc)
+{
+  const uint4 ai = aux[q];
+  const uint64_t Xi = join64(ri.x, ai.x), Yi = join64(ri.y, ai.y);
+  PairAcc a = *acc;
+  for (int k = 0; k < m; ++k)
+  {
+    if (j0 + k == q) continue;
+    const uint4 rj = srec[k];
+    const float dx = (float) (int) (rj.x - ri.x), dy = (float) (int) (rj.y - ri.y);
+    const float d2 = fmaf(dx, dx, dy * dy);
+    bool in = d2 <= rho2;
+    if (fabsf(d2 - rho2) <= band)
+    {
+      const uint2 l = __ldg(reinterpret_cast<const uint2 *>(&aux[j0 + k]));
+      in = exact_within_inline(rj.x, rj.y, l.x, l.y, Xi, Yi, rho2_d);
+    }
+    if (!in) continue;
+    const float2 cs = make_float2(__uint_as_float(rj.z), __uint_as_float(rj.w));
+    a.cs = add2(a.cs, cs);
+    if (OMEGA) a.w = fma2(make_float2(sw[k], sw[k]), cs, a.w);
+    a.card += 1.0f;
+  }
+  *acc = a;
+}
+
+// Candidates [j0, j1) of particle q by one warp: 32 records at a time, one per
+// lane, go through the warp's own shared rows while the next 32 are on their
+// way (read straight from global memory, one candidate for the whole warp at a
+// time, every eighth record waited for L2: 27.0 us at N = 4,000 against
+// 18.4).  A batch with a candidate inside the guard band is done again
+// with the FP64 decisions (about one in 3,000), so the common path has one
+// comparison a candidate: the integer pipe (differences, conversions,
+// comparisons) bounds it.
+template<bool OMEGA, bool SELF>
+__device__ __forceinline__ void pair_slice(const uint4 *__restrict__ rec, const uint4 *__restrict__ aux, uint4 *srec,
+                                           float *sw, int j0, int j1, int q, const uint4 &ri, float rho2, float band,
+                                           const double *rho2_d, PairAcc &a)
+{
+  const int lane = threadIdx.x & 31;
+  uint4 next = make_uint4(0u, 0u, 0u, 0u);
+  float next_w = 0.0f;
+  if (j0 + lane < j1)
+  {
+    next = __ldg(&rec[j0 + lane]);
+    if (OMEGA) next_w = __uint_as_float(__ldg(&aux[j0 + lane].w));
+  }
+  for (; j0 < j1; j0 += 32)
+  {
+    srec[lane] = next;
+    if (OMEGA) sw[lane] = next_w;
+    __syncwarp();
+    if (j0 + 32 + lane < j1)
+    {
+      next = __ldg(&rec[j0 + 32 + lane]);
+      if (OMEGA) next_w = __uint_as_float(__ldg(&aux[j0 + 32 + lane].w));
+    }
+    const int m = min(32, j1 - j0);
+    const PairAcc before = a;
+    float nearest = 3.0e38f;
+    int k = 0;
+#pragma unroll 1
+    for (; k + 8 <= m; k += 8) pair_group<OMEGA, SELF, 8>(srec, sw, k, q - j0, ri.x, ri.y, rho2, nearest, a);
+#pragma unroll 1
+    for (; k < m; ++k) pair_group<OMEGA, SELF, 1>(srec, sw, k, q - j0, ri.x, ri.y, rho2, nearest, a);
+    if (nearest <= band)
+    {
+      PairAcc again = before;
+      pair_batch_exact<OMEGA>(srec, sw, aux, j0, m, q, ri, rho2, band, *rho2_d, &again);
+      a = again;
+    }
+    __syncwarp();
+  }
+}
+
+template<int MODEL, int STEPPER, bool MULTI>
+__global__ void __launch_bounds__(32 * kPairWarps, 2) fast_allpairs_kernel(FastParams P, FastBuffers B)
+{
+  __shared__ float sums[5][kPairWarps][32];
+  __shared__ __align__(16) uint4 srec[kPairWarps][32];
+  __shared__ float sw[kPairWarps][STEPPER == 2 ? 32 : 1];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int begin = 32 * blockIdx.x;
+  const int q = begin + lane;
   FastControl *ctrl = B.ctrl;
   const int par = ctrl->parity;
   const uint4 *rin = par ? B.rec1 : B.rec0;
   const uint4 *ain = par ? B.aux1 : B.aux0;
   uint4 *rout = par ? B.rec0 : B.rec1;
   uint4 *aout = par ? B.aux0 : B.aux1;
+  const bool live = q < P.n;
+  const int qc = live ? q : P.n - 1;
+  const uint4 ri = rin[qc];
+  const int sys = MULTI ? B.sys_of[qc] : 0;
+  // a block of a batch may hold the end of one system and the next ones: each
+  // is scanned in turn by the lanes it owns
+  const int sys_end = MULTI ? B.sys_of[min(begin + 31, P.n - 1)] : 0;
+  PairAcc a{make_float2(0.f, 0.f), make_float2(0.f, 0.f), 0.f};
+  for (int s = MULTI ? B.sys_of[begin] : 0; s <= sys_end; ++s)
+  {
+    const int first = MULTI ? B.sys[s].first : P.first, n = MULTI ? B.sys[s].n : P.sub_n;
+    const double *rho2_d = MULTI ? &B.sys[s].rho2_d : &P.rho2_d;
+    // a lane of another system takes nothing
+    const float rho2 = sys != s ? -1.0f : (MULTI ? B.sys[s].rho2_f : P.rho2_f);
+    const float band = sys != s ? -1.0f : (MULTI ? B.sys[s].band_f : P.band_f);
+    const int j0 = first + (int) ((long long) n * warp / kPairWarps);
+    const int j1 = first + (int) ((long long) n * (warp + 1) / kPairWarps);
+    if (j0 < begin + 32 && j1 > begin)
+      pair_slice<STEPPER == 2, true>(rin, ain, srec[warp], sw[warp], j0, j1, qc, ri, rho2, band, rho2_d, a);
+    else
+      pair_slice<STEPPER == 2, false>(rin, ain, srec[warp], sw[warp], j0, j1, qc, ri, rho2, band, rho2_d, a);
+  }
+  sums[0][warp][lane] = a.cs.x;
+  sums[1][warp][lane] = a.cs.y;
+  sums[2][warp][lane] = a.card;
+  if (STEPPER == 2)
+  {
+    sums[3][warp][lane] = a.w.x;
+    sums[4][warp][lane] = a.w.y;
+  }
+  __syncthreads();
+  // warp c adds the slices of sum c in order
+  if (warp < (STEPPER == 2 ? 5 : 3))
+  {
+    if (warp == 2)
+    {
+      int card = 0;
+      for (int w = 0; w < kPairWarps; ++w) card += (int) sums[2][w][lane];
+      sums[2][0][lane] = __int_as_float(card);
+    } else
+    {
+      float t = sums[warp][0][lane];
+      for (int w = 1; w < kPairWarps; ++w) t = __fadd_rn(t, sums[warp][w][lane]);
+      sums[warp][0][lane] = t;
+    }
+  }
+  __syncthreads();
+  if (warp != 0) return;
   float d2max = 0.0f;
   int err = 0;
-  int sys = 0;
-  if (q < P.n)
+  if (live)
   {
-    sys = MULTI ? B.sys_of[q] : 0;
     const FastParams Q = MULTI ? with_system(P, B.sys[sys]) : P;
-    const unsigned p = B.pid[q];
-    const uint4 ri = rin[q];
-    const uint4 ai = ain[q];
     const float2 v = MODEL == 2 ? B.vel[q] : make_float2(0.f, 0.f);
     float z[6];
-    draw_noise<MODEL, STEPPER>(Q, ctrl->step, p, z);  // overlaps the loads above
-    Acc a{0.f, 0.f, 0.f, 0.f, 0};
-    gather_sums<KIND, STEPPER == 2>(Q, B, rin, ain, q, KIND == KIND_VERLET ? -1 : 0, nullptr, 0, ri,
-                                    join64(ri.x, ai.x), join64(ri.y, ai.y), a);
-    d2max = update_particle<MODEL, STEPPER>(Q, B, q, ri, ai, v, a, z, rout, aout, err);
+    draw_noise<MODEL, STEPPER>(Q, ctrl->step, B.pid[q], z);
+    Acc t{sums[1][0][lane], sums[0][0][lane], 0.f, 0.f, __float_as_int(sums[2][0][lane])};
+    if (STEPPER == 2)
+    {
+      t.ws = sums[4][0][lane];
+      t.wc = sums[3][0][lane];
+    }
+    d2max = update_particle<MODEL, STEPPER>(Q, B, q, ri, ain[q], v, t, z, rout, aout, err);
   }
   publish_max(ctrl, B.sysctl, sys, d2max, err);
 }
@@ -2846,8 +3046,9 @@ static void launch_step_kind(spss_ctx *ctx, const FastParams &P, const FastBuffe
     }
   } else if (ctx->fast->kind == KIND_ALL_PAIRS)
   {
-    if (P.nsys > 1) fast_step_kernel<MODEL, STEPPER, KIND_ALL_PAIRS, true><<<grid, kTB, 0, ctx->stream>>>(P, B);
-    else fast_step_kernel<MODEL, STEPPER, KIND_ALL_PAIRS, false><<<grid, kTB, 0, ctx->stream>>>(P, B);
+    const int blocks = blocks_for(P.n, 32);
+    if (P.nsys > 1) fast_allpairs_kernel<MODEL, STEPPER, true><<<blocks, 32 * kPairWarps, 0, ctx->stream>>>(P, B);
+    else fast_allpairs_kernel<MODEL, STEPPER, false><<<blocks, 32 * kPairWarps, 0, ctx->stream>>>(P, B);
   } else if (ctx->fast->kind == KIND_CELLS)
   {
     launch_tiles<MODEL, STEPPER, KIND_CELLS>(ctx, P, B, tiles);
@@ -2871,7 +3072,7 @@ static int launch_step(spss_ctx *ctx, int stepper, const FastParams &P, cudaGrap
     else launch_step_kind<2, 2>(ctx, P, B);
   }
   ++ctx->launches;
-  SPSS_TRY(check_launch("fast_step_kernel"));
+  SPSS_TRY(check_launch("step kernel"));
   if (ctx->timing) SPSS_CUDA_TRY(cudaEventRecord(ctx->ev1, ctx->stream));
   FastPath *f = ctx->fast;
   if (rebuild_exec)
