@@ -53,6 +53,7 @@ struct K64
   double v0, xi, xi_r, xi_phi, sigma, alpha, rho2, rmax2, ca, sa;
   int higher_order;
   float rho_excl;  // a pair whose float minimum-image distance bound exceeds this is out of range
+  float rho_incl, rmax_excl, rmax_incl;  // the cutoffs less (plus) two margins
 };
 
 // Margin of the all-pairs range pre-test, in box units: covers the float
@@ -80,6 +81,9 @@ static K64 make_k64(const spss_ctx *ctx)
   k.sa = std::sin(p.alpha);
   k.higher_order = ctx->higher_order;
   k.rho_excl = (float) (p.rho + 2.0 * kPretestMargin);
+  k.rho_incl = (float) std::max(0.0, p.rho - 2.0 * kPretestMargin);
+  k.rmax_excl = (float) (ctx->r_max + 2.0 * kPretestMargin);
+  k.rmax_incl = (float) std::max(0.0, ctx->r_max - 2.0 * kPretestMargin);
   return k;
 }
 
@@ -198,29 +202,40 @@ __device__ __forceinline__ void write_k(const K64 &k, int i, const double *st, S
                                         const double2 *cs = nullptr)
 {
   const long ii = (long) k.s * i;
+  double c, s;
+  if (cs)
+  {
+    c = cs->x;
+    s = cs->y;
+  } else
+  {
+    sincos(st[k.model == 1 ? 2 : 4], &s, &c);
+  }
+  double *tail = k_next + ii + (k.model == 1 ? 2 : 4);  // {omega, torque}
   if (k.model == 1)
   {
-    const double phi_i = st[2], omega_i = st[3];
-    k_next[ii] = k.v0 * (cs ? cs->x : cos(phi_i));
-    k_next[ii + 1] = k.v0 * (cs ? cs->y : sin(phi_i));
-    k_next[ii + 2] = omega_i;
+    *reinterpret_cast<double2 *>(k_next + ii) = make_double2(k.v0 * c, k.v0 * s);
+    const double omega_i = st[3];
     if (a.card != 0.0)
     {
-      k_next[ii + 3] = -k.xi * omega_i + k.sigma * a.af / a.card;
+      *reinterpret_cast<double2 *>(tail) = make_double2(omega_i, -k.xi * omega_i + k.sigma * a.af / a.card);
       if (k.higher_order) a.caf *= k.sigma / a.card;
+    } else
+    {
+      tail[0] = omega_i;
     }
   } else
   {
-    const double v_x_i = st[2], v_y_i = st[3], phi_i = st[4], omega_i = st[5];
-    k_next[ii] = v_x_i;
-    k_next[ii + 1] = v_y_i;
-    k_next[ii + 2] = -k.xi_r * v_x_i + k.v0 * (cs ? cs->x : cos(phi_i));
-    k_next[ii + 3] = -k.xi_r * v_y_i + k.v0 * (cs ? cs->y : sin(phi_i));
-    k_next[ii + 4] = omega_i;
+    const double v_x_i = st[2], v_y_i = st[3], omega_i = st[5];
+    *reinterpret_cast<double2 *>(k_next + ii) = make_double2(v_x_i, v_y_i);
+    *reinterpret_cast<double2 *>(k_next + ii + 2) = make_double2(-k.xi_r * v_x_i + k.v0 * c, -k.xi_r * v_y_i + k.v0 * s);
     if (a.card != 0.0)
     {
-      k_next[ii + 5] = -k.xi_phi * omega_i + k.sigma * a.af / a.card;
+      *reinterpret_cast<double2 *>(tail) = make_double2(omega_i, -k.xi_phi * omega_i + k.sigma * a.af / a.card);
       if (k.higher_order) a.caf *= k.sigma / a.card;
+    } else
+    {
+      tail[0] = omega_i;
     }
   }
   if (k.higher_order) caf[i] = a.caf;
@@ -228,12 +243,24 @@ __device__ __forceinline__ void write_k(const K64 &k, int i, const double *st, S
 
 // ------------------------------------------------------------ kernels
 
-// rk_system_state = system_state + k_coef * dt * k_prev (ParticleSystemFirstOrder.cpp:175-184).
-__global__ void f64_stage_kernel(const double *__restrict__ st, const double *__restrict__ kp,
-                                 double *__restrict__ rk, long len, double k_coef, double dt)
+// rk_system_state = system_state + k_coef * dt * k_prev (ParticleSystemFirstOrder.cpp:175-184),
+// and (posf not null) the stage positions wrapped into the unit box as floats
+// for the range pre-test; one particle per thread.
+__global__ void f64_stage_kernel(K64 k, const double *__restrict__ st, const double *__restrict__ kp,
+                                 double *__restrict__ rk, float2 *__restrict__ posf, double k_coef, double dt)
 {
-  const long q = (long) blockIdx.x * blockDim.x + threadIdx.x;
-  if (q < len) rk[q] = st[q] + k_coef * dt * kp[q];
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= k.n) return;
+  const double2 *s2 = reinterpret_cast<const double2 *>(st + (long) k.s * i);
+  const double2 *k2 = reinterpret_cast<const double2 *>(kp + (long) k.s * i);
+  double2 *r2 = reinterpret_cast<double2 *>(rk + (long) k.s * i);
+  for (int q = 0; q < k.s / 2; ++q)
+  {
+    const double2 a = s2[q], b = k2[q];
+    const double2 r = make_double2(a.x + k_coef * dt * b.x, a.y + k_coef * dt * b.y);
+    r2[q] = r;
+    if (q == 0 && posf) posf[i] = make_float2((float) (r.x - floor(r.x)), (float) (r.y - floor(r.y)));
+  }
 }
 
 __global__ void f64_cell_kernel(K64 k, const double *__restrict__ rk, int nc, int *__restrict__ cell_of)
@@ -275,6 +302,25 @@ __device__ __forceinline__ bool pretest_out(const K64 &k, float2 a, float2 b)
   dx = fmaxf(fminf(dx, 1.0f - dx) - kPretestMargin, 0.0f);
   dy = fmaxf(fminf(dy, 1.0f - dy) - kPretestMargin, 0.0f);
   return dx > k.rho_excl || dy > k.rho_excl || dx * dx + dy * dy > k.rho_excl * k.rho_excl;
+}
+
+// Where a pair stands to a cutoff by its float wrapped positions alone: 0 out of
+// range, 1 in range, 2 too near the cutoff to tell.  The exact minimum image of
+// the float positions is within the margin of the FP64 distance whenever the
+// reference's distance function picks the minimum image: the first-order
+// classes always do; the second-order one does for coordinate differences
+// below 1, so a float difference within the margin of 1 is left to the FP64
+// expression, and its all-pairs routine, whose x_j is not wrapped, may not use
+// the answer 1.  `incl` and `excl` are the cutoff less and plus 2 margins.
+__device__ __forceinline__ int pretest(float2 a, float2 b, float incl, float excl)
+{
+  const float rx = fabsf(b.x - a.x), ry = fabsf(b.y - a.y);
+  const float dx = fminf(rx, 1.0f - rx), dy = fminf(ry, 1.0f - ry);
+  const float lx = fmaxf(dx - kPretestMargin, 0.0f), ly = fmaxf(dy - kPretestMargin, 0.0f);
+  if (fmaf(lx, lx, ly * ly) > excl * excl) return 0;
+  const float ux = fabsf(dx) + kPretestMargin, uy = fabsf(dy) + kPretestMargin;
+  if (fmaf(ux, ux, uy * uy) < incl * incl && fmaxf(rx, ry) < 1.0f - kPretestMargin) return 1;
+  return 2;
 }
 
 // The next RK4 stage, written by the pair kernel of this one (null rk: none):
@@ -374,60 +420,224 @@ __global__ void f64_allpairs_kernel(K64 k, const double *__restrict__ rk, const 
   }
 }
 
-// Linked list (ParticleSystemFirstOrder.cpp:231-353, ParticleSystemSecondOrder.cpp:276-409).
-__global__ void f64_linked_list_kernel(K64 k, const double *__restrict__ rk, int nc, const int *__restrict__ off,
-                                       const int *__restrict__ mem, double *__restrict__ k_next,
-                                       double *__restrict__ caf)
+// ------------------------------------------------------------ neighbour sums
+//
+// One particle per lane finds its neighbours; the pair terms are then evaluated
+// by the whole warp.  GB300 executes an FP64 instruction for a warp in the time
+// of about 69 FP32 ones whether one lane needs it or 32, so the FP64 sines of
+// the few candidates in range (6 of 18 at density 2, each lane's at its own
+// place in the scan) cost as much as if every candidate were in range.  The
+// scan uses the float pre-test (FP64 only for a pair within the margins of the
+// cutoff) and queues the neighbours per lane; the queues are laid end to end
+// and 32 pair terms are evaluated at a time; each lane then adds its own terms
+// in the order it found them, so the sums are the reference's, bit for bit.
+// N = 65,536, density 2: linked list 313 -> 67 us; Verlet pairs at N = 20,011
+// 87 -> 37 us.
+constexpr int kQueue = 16;       // queued neighbours a lane
+constexpr int kScan = 4;         // candidates a lane looks at together (their loads are in flight at once)
+constexpr int kPairThreads = 32;  // one warp a block: 20,011 particles in blocks of 64 left SMs with 3 blocks beside SMs with 2
+
+struct PairBuffers
 {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= k.n) return;
+  double af[kQueue * 32], caf[kQueue * 32];
+  int j[kQueue * 32];
+  unsigned short flat[kQueue * 32];
+};
+
+// Pair terms: first order ParticleSystemFirstOrderPtr.cpp:404-415; second order
+// ParticleSystemSecondOrder.cpp:160-161 (see add_pair).
+__device__ __forceinline__ void pair_terms(const K64 &k, double phi_i, double omega_i, double phi_j, double omega_j,
+                                           double &af, double &caf)
+{
+  const double d = k.model == 1 ? phi_j - phi_i : phi_j - phi_i - k.alpha;
+  double s, c = 0.0;
+  if (k.higher_order || (k.model == 1 && k.sa != 0.0)) sincos(d, &s, &c);
+  else s = sin(d);
+  caf = 0.0;
+  if (k.model == 1)
+  {
+    af = s * k.ca - c * k.sa;
+    if (k.higher_order) caf = (omega_j - omega_i) * (c * k.ca + s * k.sa);
+  } else
+  {
+    af = s;
+    if (k.higher_order) caf = (omega_j - omega_i) * c;
+  }
+}
+
+// Evaluates the queued pairs of the warp's lanes (cnt of this lane's, in rows
+// j[m * 32 + lane]) and adds each lane's terms to its sums in order.
+__device__ __forceinline__ void add_queued(const K64 &k, PairBuffers &Q, const double *__restrict__ rk, int cnt,
+                                           double phi_i, double omega_i, Sums &a)
+{
+  const int lane = threadIdx.x & 31;
+  int end = cnt;
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1)
+  {
+    const int y = __shfl_up_sync(0xffffffffu, end, off);
+    if (lane >= off) end += y;
+  }
+  const int total = __shfl_sync(0xffffffffu, end, 31);
+  for (int m = 0; m < cnt; ++m) Q.flat[end - cnt + m] = (unsigned short) (m * 32 + lane);
+  __syncwarp();
+  const int ip = k.model == 1 ? 2 : 4;
+  for (int base = 0; base < total; base += 32)
+  {
+    const int p = base + lane;
+    const int f = p < total ? Q.flat[p] : lane;
+    const double phi_o = __shfl_sync(0xffffffffu, phi_i, f & 31), omega_o = __shfl_sync(0xffffffffu, omega_i, f & 31);
+    if (p < total)
+    {
+      const double2 pj = *reinterpret_cast<const double2 *>(rk + (long) k.s * Q.j[f] + ip);
+      double af, caf;
+      pair_terms(k, phi_o, omega_o, pj.x, pj.y, af, caf);
+      Q.af[f] = af;
+      if (k.higher_order) Q.caf[f] = caf;
+    }
+  }
+  __syncwarp();
+  for (int m = 0; m < cnt; ++m)
+  {
+    a.af += Q.af[m * 32 + lane];
+    if (k.higher_order) a.caf += Q.caf[m * 32 + lane];
+  }
+  a.card += (double) cnt;
+  __syncwarp();
+}
+
+// Candidates list[m .. m + kScan) (below e) of the lane's particle i: those in
+// range go to the lane's queue, in order.
+__device__ __forceinline__ void scan_candidates(const K64 &k, PairBuffers &Q, const double *__restrict__ rk,
+                                                const float2 *__restrict__ posf, const int *__restrict__ list, int m,
+                                                int e, int i, float2 p_i, double x_i, double y_i, int &cnt)
+{
+  int j[kScan];
+  float2 p[kScan];
+#pragma unroll
+  for (int u = 0; u < kScan; ++u) j[u] = m + u < e ? __ldg(list + m + u) : i;
+#pragma unroll
+  for (int u = 0; u < kScan; ++u) p[u] = __ldg(posf + j[u]);
+#pragma unroll
+  for (int u = 0; u < kScan; ++u)
+  {
+    int in = j[u] == i ? 0 : pretest(p_i, p[u], k.rho_incl, k.rho_excl);
+    if (in == 2)
+    {
+      const double *sj = rk + (long) k.s * j[u];
+      in = pair_dr2<true>(k, x_i, y_i, sj[0], sj[1]) <= k.rho2;
+    }
+    if (in) Q.j[32 * cnt++ + (threadIdx.x & 31)] = j[u];
+  }
+}
+
+// The stencil of a cell as runs of the cell list, in the reference's order: a
+// row of three cells away from the grid's edge is one run, cells at the edge
+// are runs of their own.  `c` counts the stencil's cells done.
+__device__ __forceinline__ void next_run(int cx, int cy, int nc, const int *__restrict__ off, int &c, int &m, int &e)
+{
+  const int row = adjust_cell(cy + c_stencil[c][1], nc) * nc;
+  if (cx > 0 && cx + 1 < nc)
+  {
+    m = off[row + cx - 1];
+    e = off[row + cx + 2];
+    c += 3;
+    return;
+  }
+  const int jc = row + adjust_cell(cx + c_stencil[c][0], nc);
+  m = off[jc];
+  e = off[jc + 1];
+  ++c;
+}
+
+// Linked list (ParticleSystemFirstOrder.cpp:231-353, ParticleSystemSecondOrder.cpp:276-409).
+// Particles are taken in cell order, so a warp's lanes scan neighbouring cells.
+__global__ void __launch_bounds__(kPairThreads) f64_linked_list_kernel(K64 k, const double *__restrict__ rk,
+                                                                       const float2 *__restrict__ posf, int nc,
+                                                                       const int *__restrict__ off,
+                                                                       const int *__restrict__ mem,
+                                                                       double *__restrict__ k_next,
+                                                                       double *__restrict__ caf)
+{
+  __shared__ PairBuffers buf[kPairThreads / 32];
+  PairBuffers &Q = buf[threadIdx.x >> 5];
+  const int t = blockIdx.x * kPairThreads + threadIdx.x;
+  const bool live = t < k.n;
+  const int i = mem[live ? t : k.n - 1];
   const int ip = k.model == 1 ? 2 : 4;
   const double *st = rk + (long) k.s * i;
   double x_i, y_i;
   pos_for_cells(k, rk, i, x_i, y_i);
   const double phi_i = st[ip], omega_i = st[ip + 1];
+  const float2 p_i = posf[i];
   const int cx = cell_coord(x_i, nc), cy = cell_coord(y_i, nc);
   Sums a{0.0, 0.0, 0.0};
-  for (int c = 0; c < 9; ++c)
+  int c = live ? 0 : 9, m = 0, e = 0, cnt = 0;
+  while (true)
   {
-    const int jc = adjust_cell(cy + c_stencil[c][1], nc) * nc + adjust_cell(cx + c_stencil[c][0], nc);
-    for (int m = off[jc]; m < off[jc + 1]; ++m)
+    while (cnt <= kQueue - kScan)
     {
-      const int j = mem[m];
-      if (j == i) continue;
-      const double *sj = rk + (long) k.s * j;
-      if (pair_dr2<true>(k, x_i, y_i, sj[0], sj[1]) <= k.rho2) add_pair(k, a, phi_i, omega_i, sj[ip], sj[ip + 1]);
+      if (m >= e)
+      {
+        if (c >= 9) break;
+        next_run(cx, cy, nc, off, c, m, e);
+        continue;
+      }
+      scan_candidates(k, Q, rk, posf, mem, m, e, i, p_i, x_i, y_i, cnt);
+      m += kScan;
     }
+    add_queued(k, Q, rk, cnt, phi_i, omega_i, a);
+    cnt = 0;
+    if (!__any_sync(0xffffffffu, c < 9 || m < e)) break;
   }
-  write_k(k, i, st, a, k_next, caf);
+  if (live) write_k(k, i, st, a, k_next, caf);
 }
 
 // Verlet list from the cell list (ParticleSystemFirstOrder.cpp:536-589): first
-// pass counts, second pass fills in the reference's push_back order.
+// pass counts, second pass fills in the reference's push_back order.  Almost
+// every pair is decided by the float pre-test (N = 20,011: 97 + 83 us with the
+// FP64 distance for every candidate, 22 + 24 us with it).
 template<bool FILL>
-__global__ void f64_verlet_cells_kernel(K64 k, const double *__restrict__ rk, int nc, const int *__restrict__ off,
-                                        const int *__restrict__ mem, int *__restrict__ count,
-                                        const int *__restrict__ vl_off, int *__restrict__ vl_ent)
+__global__ void f64_verlet_cells_kernel(K64 k, const double *__restrict__ rk, const float2 *__restrict__ posf, int nc,
+                                        const int *__restrict__ off, const int *__restrict__ mem,
+                                        int *__restrict__ count, const int *__restrict__ vl_off,
+                                        int *__restrict__ vl_ent)
 {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= k.n) return;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= k.n) return;
+  const int i = mem[t];
   double x_i, y_i;
   pos_for_cells(k, rk, i, x_i, y_i);
+  const float2 p_i = posf[i];
   const int cx = cell_coord(x_i, nc), cy = cell_coord(y_i, nc);
   int cnt = 0;
-  int base = FILL ? vl_off[i] : 0;
-  for (int c = 0; c < 9; ++c)
+  const int base = FILL ? vl_off[i] : 0;
+  for (int c = 0; c < 9;)
   {
-    const int jc = adjust_cell(cy + c_stencil[c][1], nc) * nc + adjust_cell(cx + c_stencil[c][0], nc);
-    for (int m = off[jc]; m < off[jc + 1]; ++m)
+    int m, e;
+    next_run(cx, cy, nc, off, c, m, e);
+    for (; m < e; m += kScan)
     {
-      const int j = mem[m];
-      if (j == i) continue;
-      const double *sj = rk + (long) k.s * j;
-      if (pair_dr2<true>(k, x_i, y_i, sj[0], sj[1]) <= k.rmax2)
+      int j[kScan];
+      float2 p[kScan];
+#pragma unroll
+      for (int u = 0; u < kScan; ++u) j[u] = m + u < e ? __ldg(mem + m + u) : i;
+#pragma unroll
+      for (int u = 0; u < kScan; ++u) p[u] = __ldg(posf + j[u]);
+#pragma unroll
+      for (int u = 0; u < kScan; ++u)
       {
-        if (FILL) vl_ent[base + cnt] = j;
-        ++cnt;
+        int in = j[u] == i ? 0 : pretest(p_i, p[u], k.rmax_incl, k.rmax_excl);
+        if (in == 2)
+        {
+          const double *sj = rk + (long) k.s * j[u];
+          in = pair_dr2<true>(k, x_i, y_i, sj[0], sj[1]) <= k.rmax2;
+        }
+        if (in)
+        {
+          if (FILL) vl_ent[base + cnt] = j[u];
+          ++cnt;
+        }
       }
     }
   }
@@ -458,26 +668,42 @@ __global__ void f64_verlet_all_kernel(K64 k, const double *__restrict__ rk, int 
 }
 
 // Pair loop over the Verlet list (ParticleSystemFirstOrder.cpp:594-648, ParticleSystemFirstOrderPtr.cpp:861-930).
-__global__ void f64_verlet_pairs_kernel(K64 k, const double *__restrict__ rk, const int *__restrict__ vl_off,
-                                        const int *__restrict__ vl_ent, double *__restrict__ k_next,
-                                        double *__restrict__ caf)
+// `order` (not null): particles in the cell order of the last build, so a
+// warp's lanes read neighbouring particles.
+__global__ void __launch_bounds__(kPairThreads) f64_verlet_pairs_kernel(K64 k, const double *__restrict__ rk,
+                                                                        const float2 *__restrict__ posf,
+                                                                        const int *__restrict__ order,
+                                                                        const int *__restrict__ vl_off,
+                                                                        const int *__restrict__ vl_ent,
+                                                                        double *__restrict__ k_next,
+                                                                        double *__restrict__ caf)
 {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= k.n) return;
+  __shared__ PairBuffers buf[kPairThreads / 32];
+  PairBuffers &Q = buf[threadIdx.x >> 5];
+  const int t = blockIdx.x * kPairThreads + threadIdx.x;
+  const bool live = t < k.n;
+  const int i = order ? order[live ? t : k.n - 1] : (live ? t : k.n - 1);
   const int ip = k.model == 1 ? 2 : 4;
   const double *st = rk + (long) k.s * i;
   double x_i = st[0], y_i = st[1];
   if (k.model == 2) wrap_if_outside(x_i, y_i);
   const double phi_i = st[ip], omega_i = st[ip + 1];
+  const float2 p_i = posf[i];
   Sums a{0.0, 0.0, 0.0};
-  for (int m = vl_off[i]; m < vl_off[i + 1]; ++m)
+  int m = vl_off[i], cnt = 0;
+  const int e = live ? vl_off[i + 1] : m;
+  while (true)
   {
-    const int j = vl_ent[m];
-    if (j == i) continue;
-    const double *sj = rk + (long) k.s * j;
-    if (pair_dr2<true>(k, x_i, y_i, sj[0], sj[1]) <= k.rho2) add_pair(k, a, phi_i, omega_i, sj[ip], sj[ip + 1]);
+    while (cnt <= kQueue - kScan && m < e)
+    {
+      scan_candidates(k, Q, rk, posf, vl_ent, m, e, i, p_i, x_i, y_i, cnt);
+      m += kScan;
+    }
+    add_queued(k, Q, rk, cnt, phi_i, omega_i, a);
+    cnt = 0;
+    if (!__any_sync(0xffffffffu, m < e)) break;
   }
-  write_k(k, i, st, a, k_next, caf);
+  if (live) write_k(k, i, st, a, k_next, caf);
 }
 
 // Global polar order field, first order (ParticleSystemFirstOrder.cpp:122-159,
@@ -785,7 +1011,7 @@ static int build_verlet(spss_ctx *ctx, const K64 &k, bool from_cells)
   {
     SPSS_TRY(build_cells(ctx, k, ctx->nc_verlet));
     f64_verlet_cells_kernel<false><<<blocks_for(k.n, tb), tb, 0, ctx->stream>>>(
-        k, f->rk.ptr, ctx->nc_verlet, f->binner.offsets.ptr, f->binner.members.ptr, f->vl_count.ptr, nullptr,
+        k, f->rk.ptr, f->posf.ptr, ctx->nc_verlet, f->binner.offsets.ptr, f->binner.members.ptr, f->vl_count.ptr, nullptr,
         nullptr);
   } else
   {
@@ -802,7 +1028,7 @@ static int build_verlet(spss_ctx *ctx, const K64 &k, bool from_cells)
   if (from_cells)
   {
     f64_verlet_cells_kernel<true><<<blocks_for(k.n, tb), tb, 0, ctx->stream>>>(
-        k, f->rk.ptr, ctx->nc_verlet, f->binner.offsets.ptr, f->binner.members.ptr, nullptr, f->vl_off.ptr,
+        k, f->rk.ptr, f->posf.ptr, ctx->nc_verlet, f->binner.offsets.ptr, f->binner.members.ptr, nullptr, f->vl_off.ptr,
         f->vl_ent.ptr);
   } else
   {
@@ -824,13 +1050,13 @@ int f64_evaluate(spss_ctx *ctx, int variant, const double *d_state, const double
   if (variant < SPSS_VARIANT_ALL_PAIRS || variant > SPSS_VARIANT_GLOBAL_FIELD) return SPSS_ERR_INVALID_ARGUMENT;
   if (variant == SPSS_VARIANT_GLOBAL_FIELD && ctx->p.model != 1) return SPSS_ERR_NOT_SUPPORTED;
   const K64 k = make_k64(ctx);
-  const long len = (long) k.n * k.s;
   const int tb = 256;
   if (variant == SPSS_VARIANT_ALL_PAIRS)
     f64_stage_posf_kernel<<<blocks_for(k.n, tb), tb, 0, ctx->stream>>>(k, d_state, d_kprev, f->rk.ptr, f->posf.ptr,
                                                                        f->csphi.ptr, k_coef, dt);
   else
-    f64_stage_kernel<<<blocks_for(len, tb), tb, 0, ctx->stream>>>(d_state, d_kprev, f->rk.ptr, len, k_coef, dt);
+    f64_stage_kernel<<<blocks_for(k.n, tb), tb, 0, ctx->stream>>>(
+        k, d_state, d_kprev, f->rk.ptr, variant == SPSS_VARIANT_GLOBAL_FIELD ? nullptr : f->posf.ptr, k_coef, dt);
   ++ctx->launches;
   SPSS_TRY(check_launch("f64_stage_kernel"));
   if (k.higher_order) SPSS_CUDA_TRY(cudaMemsetAsync(f->caf.ptr, 0, sizeof(double) * k.n, ctx->stream));
@@ -843,8 +1069,8 @@ int f64_evaluate(spss_ctx *ctx, int variant, const double *d_state, const double
       return check_launch("f64_allpairs_kernel");
     case SPSS_VARIANT_LINKED_LIST:
       SPSS_TRY(build_cells(ctx, k, ctx->nc));
-      f64_linked_list_kernel<<<blocks_for(k.n, 128), 128, 0, ctx->stream>>>(
-          k, f->rk.ptr, ctx->nc, f->binner.offsets.ptr, f->binner.members.ptr, d_knext, f->caf.ptr);
+      f64_linked_list_kernel<<<blocks_for(k.n, kPairThreads), kPairThreads, 0, ctx->stream>>>(
+          k, f->rk.ptr, f->posf.ptr, ctx->nc, f->binner.offsets.ptr, f->binner.members.ptr, d_knext, f->caf.ptr);
       ++ctx->launches;
       return check_launch("f64_linked_list_kernel");
     case SPSS_VARIANT_VERLET:
@@ -856,8 +1082,9 @@ int f64_evaluate(spss_ctx *ctx, int variant, const double *d_state, const double
         ++ctx->list_builds;
       }
       ctx->uses_verlet_list = 1;
-      f64_verlet_pairs_kernel<<<blocks_for(k.n, 128), 128, 0, ctx->stream>>>(k, f->rk.ptr, f->vl_off.ptr,
-                                                                             f->vl_ent.ptr, d_knext, f->caf.ptr);
+      f64_verlet_pairs_kernel<<<blocks_for(k.n, kPairThreads), kPairThreads, 0, ctx->stream>>>(
+          k, f->rk.ptr, f->posf.ptr, f->cells_nc ? f->binner.members.ptr : nullptr, f->vl_off.ptr, f->vl_ent.ptr,
+          d_knext, f->caf.ptr);
       ++ctx->launches;
       return check_launch("f64_verlet_pairs_kernel");
     case SPSS_VARIANT_GLOBAL_FIELD:
