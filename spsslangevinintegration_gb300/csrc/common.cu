@@ -31,6 +31,33 @@ const char *last_error_text()
   return g_last_error;
 }
 
+// ------------------------------------------------------------------ tables of the FP64 functions
+
+__global__ void f64_tables_kernel(double2 *__restrict__ table)
+{
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= kTableEntries) return;
+  if (i < kTrigTable)
+  {
+    double s, c;
+    sincospi((double) i / 128.0, &s, &c);
+    table[i] = make_double2(c, s);
+    return;
+  }
+  const int j = i - kTrigTable + kLogFirst;
+  const double inv = 128.0 / (double) j;
+  // -log(inv) of the rounded inv, from the exact j / 128: log(j / 128) - log1p(delta), inv = (1 + delta) 128 / j
+  const double delta = fma(inv, (double) j / 128.0, -1.0);
+  table[i] = make_double2(inv, log((double) j / 128.0) - delta);
+}
+
+int make_f64_tables(DeviceArray<double2> &table, cudaStream_t stream)
+{
+  SPSS_TRY(table.reserve(kTableEntries));
+  f64_tables_kernel<<<(kTableEntries + 127) / 128, 128, 0, stream>>>(table.ptr);
+  return check_launch("f64_tables_kernel");
+}
+
 // ------------------------------------------------------------------ scan
 
 constexpr int kScanThreads = 256;

@@ -25,6 +25,7 @@ struct F64Path
       scratch_knext;
   DeviceArray<int> cell_of;
   DeviceArray<float2> posf;  // stage positions wrapped into the box, float (all-pairs range pre-test)
+  DeviceArray<double2> table;  // of the FP64 functions
   DeviceArray<double2> csphi;  // cos and sin of the stage phase (all pairs: written with the stage)
   // the other stage buffers of an all-pairs RK4 step, whose pair kernels
   // write the next stage's state while they read this one's
@@ -51,15 +52,19 @@ struct K64
 {
   int model, flavor, n, s;
   double v0, xi, xi_r, xi_phi, sigma, alpha, rho2, rmax2, ca, sa;
+  const double2 *table;  // of the FP64 functions (make_f64_tables)
   int higher_order;
   float rho_excl;  // a pair whose float minimum-image distance bound exceeds this is out of range
   float rho_incl, rmax_excl, rmax_incl;  // the cutoffs less (plus) two margins
 };
 
-// Margin of the all-pairs range pre-test, in box units: covers the float
-// rounding of the wrapped positions and of the bound (a few 1e-8) and the
-// FP64 wrap of positions up to 1e4 boxes away (1e-12), many times over.
-constexpr float kPretestMargin = 2e-5f;
+// Margin of the range pre-test, in box units: six times what the float rounding
+// of the wrapped positions (6e-8 a difference), of the minimum image and of
+// the squares (1e-7 together) and the FP64 wrap of positions up to 1e4 boxes
+// away (1e-12) amount to.  A pair nearer to the cutoff than this is decided in
+// FP64, for the whole warp's time: at N = 65,536 a margin of 2e-5 left 0.27
+// such pairs a particle and the linked-list kernel took 64 us, now 44.
+constexpr float kPretestMargin = 1e-6f;
 
 static K64 make_k64(const spss_ctx *ctx)
 {
@@ -80,6 +85,7 @@ static K64 make_k64(const spss_ctx *ctx)
   k.ca = std::cos(p.alpha);  // host libm, as the reference's constructor
   k.sa = std::sin(p.alpha);
   k.higher_order = ctx->higher_order;
+  k.table = ctx->f64->table.ptr;
   k.rho_excl = (float) (p.rho + 2.0 * kPretestMargin);
   k.rho_incl = (float) std::max(0.0, p.rho - 2.0 * kPretestMargin);
   k.rmax_excl = (float) (ctx->r_max + 2.0 * kPretestMargin);
@@ -178,65 +184,55 @@ struct Sums
 // Pair terms: first order ParticleSystemFirstOrderPtr.cpp:404-415; second
 // order ParticleSystemSecondOrder.cpp:160-161 (its complementary force is the
 // first-order term in the second-order sin(phi_j - phi_i - alpha) convention).
-__device__ __forceinline__ void add_pair(const K64 &k, Sums &a, double phi_i, double omega_i, double phi_j,
-                                         double omega_j)
+__device__ __forceinline__ void pair_terms(const K64 &k, double phi_i, double omega_i, double phi_j, double omega_j,
+                                           double &af, double &caf)
 {
+  const double d = k.model == 1 ? phi_j - phi_i : phi_j - phi_i - k.alpha;
+  double s, c = 0.0;
+  if (k.higher_order || (k.model == 1 && k.sa != 0.0)) fast_sincos(k.table, d, s, c);
+  else s = fast_sin(k.table, d);
+  caf = 0.0;
   if (k.model == 1)
   {
-    a.af += sin(phi_j - phi_i) * k.ca - cos(phi_j - phi_i) * k.sa;
-    a.card += 1.0;
-    if (k.higher_order) a.caf += (omega_j - omega_i) * (cos(phi_j - phi_i) * k.ca + sin(phi_j - phi_i) * k.sa);
+    af = s * k.ca - c * k.sa;
+    if (k.higher_order) caf = (omega_j - omega_i) * (c * k.ca + s * k.sa);
   } else
   {
-    a.af += sin(phi_j - phi_i - k.alpha);
-    a.card += 1.0;
-    if (k.higher_order) a.caf += (omega_j - omega_i) * cos(phi_j - phi_i - k.alpha);
+    af = s;
+    if (k.higher_order) caf = (omega_j - omega_i) * c;
   }
 }
 
 // Output of one particle (ParticleSystemFirstOrder.cpp:220-226, ParticleSystemSecondOrder.cpp:166-175);
 // the torque component is left untouched when the particle has no neighbour.
-// `cs`: cos and sin of the particle's phase computed beforehand (the same
-// functions of the same value), or null.
-__device__ __forceinline__ void write_k(const K64 &k, int i, const double *st, Sums a, double *k_next, double *caf,
-                                        const double2 *cs = nullptr)
+// In two parts: what needs the pair sums (the torque component and the
+// complementary force) and what does not (c, s: cos and sin of the phase).
+__device__ __forceinline__ void write_k_but_torque(const K64 &k, int i, const double *st, double *k_next, double c,
+                                                   double s)
 {
-  const long ii = (long) k.s * i;
-  double c, s;
-  if (cs)
-  {
-    c = cs->x;
-    s = cs->y;
-  } else
-  {
-    sincos(st[k.model == 1 ? 2 : 4], &s, &c);
-  }
-  double *tail = k_next + ii + (k.model == 1 ? 2 : 4);  // {omega, torque}
+  double *out = k_next + (long) k.s * i;
   if (k.model == 1)
   {
-    *reinterpret_cast<double2 *>(k_next + ii) = make_double2(k.v0 * c, k.v0 * s);
-    const double omega_i = st[3];
-    if (a.card != 0.0)
-    {
-      *reinterpret_cast<double2 *>(tail) = make_double2(omega_i, -k.xi * omega_i + k.sigma * a.af / a.card);
-      if (k.higher_order) a.caf *= k.sigma / a.card;
-    } else
-    {
-      tail[0] = omega_i;
-    }
+    *reinterpret_cast<double2 *>(out) = make_double2(k.v0 * c, k.v0 * s);
+    out[2] = st[3];
   } else
   {
-    const double v_x_i = st[2], v_y_i = st[3], omega_i = st[5];
-    *reinterpret_cast<double2 *>(k_next + ii) = make_double2(v_x_i, v_y_i);
-    *reinterpret_cast<double2 *>(k_next + ii + 2) = make_double2(-k.xi_r * v_x_i + k.v0 * c, -k.xi_r * v_y_i + k.v0 * s);
-    if (a.card != 0.0)
-    {
-      *reinterpret_cast<double2 *>(tail) = make_double2(omega_i, -k.xi_phi * omega_i + k.sigma * a.af / a.card);
-      if (k.higher_order) a.caf *= k.sigma / a.card;
-    } else
-    {
-      tail[0] = omega_i;
-    }
+    const double v_x_i = st[2], v_y_i = st[3];
+    *reinterpret_cast<double2 *>(out) = make_double2(v_x_i, v_y_i);
+    *reinterpret_cast<double2 *>(out + 2) = make_double2(-k.xi_r * v_x_i + k.v0 * c, -k.xi_r * v_y_i + k.v0 * s);
+    out[4] = st[5];
+  }
+}
+
+__device__ __forceinline__ void write_k(const K64 &k, int i, const double *st, Sums a, double *k_next, double *caf)
+{
+  double c, s;
+  fast_sincos(k.table, st[k.model == 1 ? 2 : 4], s, c);
+  write_k_but_torque(k, i, st, k_next, c, s);
+  if (a.card != 0.0)
+  {
+    k_next[(long) k.s * i + k.s - 1] = -(k.model == 1 ? k.xi : k.xi_phi) * st[k.s - 1] + k.sigma * a.af / a.card;
+    if (k.higher_order) a.caf *= k.sigma / a.card;
   }
   if (k.higher_order) caf[i] = a.caf;
 }
@@ -288,20 +284,9 @@ __global__ void f64_stage_posf_kernel(K64 k, const double *__restrict__ st, cons
   const double x = rk[ii], y = rk[ii + 1];
   posf[i] = make_float2((float) (x - floor(x)), (float) (y - floor(y)));
   const double phi = rk[ii + (k.model == 1 ? 2 : 4)];
-  csphi[i] = make_double2(cos(phi), sin(phi));
-}
-
-// A lower bound of the minimum-image distance of two particles from their
-// float wrapped positions (exact minimum image of the wrapped coordinates,
-// less the margin): every periodic image the reference's distance functions
-// may pick is at least this far, so a pair whose bound exceeds rho is out of
-// range for the FP64 test as well.
-__device__ __forceinline__ bool pretest_out(const K64 &k, float2 a, float2 b)
-{
-  float dx = fabsf(b.x - a.x), dy = fabsf(b.y - a.y);
-  dx = fmaxf(fminf(dx, 1.0f - dx) - kPretestMargin, 0.0f);
-  dy = fmaxf(fminf(dy, 1.0f - dy) - kPretestMargin, 0.0f);
-  return dx > k.rho_excl || dy > k.rho_excl || dx * dx + dy * dy > k.rho_excl * k.rho_excl;
+  double c, sn;
+  fast_sincos(k.table, phi, sn, c);
+  csphi[i] = make_double2(c, sn);
 }
 
 // Where a pair stands to a cutoff by its float wrapped positions alone: 0 out of
@@ -311,113 +296,271 @@ __device__ __forceinline__ bool pretest_out(const K64 &k, float2 a, float2 b)
 // classes always do; the second-order one does for coordinate differences
 // below 1, so a float difference within the margin of 1 is left to the FP64
 // expression, and its all-pairs routine, whose x_j is not wrapped, may not use
-// the answer 1.  `incl` and `excl` are the cutoff less and plus 2 margins.
+// the answer 1.  Out of range holds for every image the reference may pick.
+// `incl` and `excl` are the cutoff less and plus 2 margins.
 __device__ __forceinline__ int pretest(float2 a, float2 b, float incl, float excl)
 {
   const float rx = fabsf(b.x - a.x), ry = fabsf(b.y - a.y);
   const float dx = fminf(rx, 1.0f - rx), dy = fminf(ry, 1.0f - ry);
   const float lx = fmaxf(dx - kPretestMargin, 0.0f), ly = fmaxf(dy - kPretestMargin, 0.0f);
-  if (fmaf(lx, lx, ly * ly) > excl * excl) return 0;
   const float ux = fabsf(dx) + kPretestMargin, uy = fabsf(dy) + kPretestMargin;
-  if (fmaf(ux, ux, uy * uy) < incl * incl && fmaxf(rx, ry) < 1.0f - kPretestMargin) return 1;
-  return 2;
+  // without branches: several pairs are tested at once
+  const bool out = fmaf(lx, lx, ly * ly) > excl * excl;
+  const bool sure = fmaf(ux, ux, uy * uy) < incl * incl && fmaxf(rx, ry) < 1.0f - kPretestMargin;
+  return out ? 0 : (sure ? 1 : 2);
 }
 
-// The next RK4 stage, written by the pair kernel of this one (null rk: none):
-// rk = x + coef * dt * k_next, its wrapped float position and the cos and sin
-// of its phase, the expressions of f64_stage_posf_kernel.
+// What the pair kernel of an RK4 stage does after its derivative: the next
+// stage rk = x + coef * dt * k_next (COMBINE: first the step's result
+// x += (k1 + 2 k2 + 2 k3 + k4) dt / 6, RungeKutta4Stepper.cpp:56-59, which is
+// the first stage of the next step), its wrapped float position and the cos
+// and sin of its phase, the expressions of f64_stage_posf_kernel.
 struct NextStage
 {
-  const double *x;
+  double *x;
   double coef, dt;
   double *rk;
   float2 *posf;
   double2 *csphi;
+  const double *k1, *k2, *k3;  // COMBINE
+  double *td;
 };
 
-// All pairs (ParticleSystemFirstOrder.cpp:162-228, ParticleSystemFirstOrderPtr.cpp:225-316,
-// ParticleSystemSecondOrder.cpp:116-177): one warp per particle, lanes stride
-// over j, partial sums combined by a fixed shuffle tree.  A float pre-test
-// on the wrapped positions excludes the pairs that are certainly out of
-// range; every other pair is decided by the reference's FP64 expression, so
-// the neighbour sets are the FP64 ones.
-__global__ void f64_allpairs_kernel(K64 k, const double *__restrict__ rk, const float2 *__restrict__ posf,
-                                    const double2 *__restrict__ csphi, double *__restrict__ k_next,
-                                    double *__restrict__ caf, NextStage next)
+enum
 {
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (warp >= k.n) return;
-  const int i = warp;
-  const int ip = k.model == 1 ? 2 : 4;
-  const double *st = rk + (long) k.s * i;
-  double x_i = st[0], y_i = st[1];
-  const double phi_i = st[ip], omega_i = st[ip + 1];
-  if (k.model == 1 && k.flavor == 1)
+  AFTER_NOTHING = 0,
+  AFTER_STAGE = 1,
+  AFTER_COMBINE = 2
+};
+
+// Component q of the next stage of a particle from its derivative kq (at
+// `at`, its place in the state): k1, k2, k3 and x as stored there.
+struct StageWords
+{
+  double x, k1, k2, k3;
+};
+
+template<int AFTER>
+__device__ __forceinline__ StageWords load_stage(const NextStage &next, long at)
+{
+  if (AFTER == AFTER_COMBINE) return StageWords{next.x[at], next.k1[at], next.k2[at], next.k3[at]};
+  return StageWords{AFTER == AFTER_STAGE ? next.x[at] : 0.0, 0.0, 0.0, 0.0};
+}
+
+template<int AFTER>
+__device__ __forceinline__ double advance_component(const NextStage &next, long at, const StageWords &w, double kq)
+{
+  double r;
+  if (AFTER == AFTER_COMBINE)
   {
-    x_i = wrap1(x_i);
-    y_i = wrap1(y_i);
+    const double d = (w.k1 + 2.0 * w.k2 + 2.0 * w.k3 + kq) * next.dt / 6.0;
+    next.td[at] = d;
+    r = w.x + d;
+    next.x[at] = r;
+  } else
+  {
+    r = w.x + next.coef * next.dt * kq;
   }
-  const float2 pi = posf[i];
+  next.rk[at] = r;
+  return r;
+}
+
+// The next stage but omega, whose derivative needs the pair sums, with the
+// float position and the cos and sin of the phase.
+template<int AFTER>
+__device__ __forceinline__ void advance_but_omega(const K64 &k, int i, const double *k_next, const NextStage &next)
+{
+  const long ii = (long) k.s * i;
+  double row[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+  for (int q = 0; q < 5; ++q)
+    if (q < k.s - 1) row[q] = advance_component<AFTER>(next, ii + q, load_stage<AFTER>(next, ii + q), k_next[ii + q]);
+  next.posf[i] = make_float2((float) (row[0] - floor(row[0])), (float) (row[1] - floor(row[1])));
+  double c, sn;
+  fast_sincos(k.table, k.model == 1 ? row[2] : row[4], sn, c);
+  next.csphi[i] = make_double2(c, sn);
+}
+
+// All pairs (ParticleSystemFirstOrder.cpp:162-228, ParticleSystemFirstOrderPtr.cpp:225-316,
+// ParticleSystemSecondOrder.cpp:116-177): eight particles a block, two warps
+// scanning half the system each for one of them by the float pre-test (FP64
+// within the margins of the cutoff, and for every second-order pair not
+// certainly out of range); the neighbours' phases, in ascending order, wait in
+// the warp's queue.  After the scan the block evaluates all its pair terms
+// together, so an FP64 instruction runs for many lanes (see "neighbour sums"),
+// while another warp does what does not need them: everything of the
+// derivative and of the next stage but the torque and omega.  A warp whose
+// queue fills up (many neighbours) evaluates it on the spot.
+// At N = 1,000 the block is a chain of latencies (an FP64 instruction's result
+// takes some 50 cycles): 11 us an evaluation in a graph of steps; with one
+// warp a particle doing all of its own FP64 work it was 24.
+constexpr int kAllParticles = 8;
+constexpr int kAllWarps = 2 * kAllParticles;
+constexpr int kAllQueue = 64;
+
+template<int AFTER>
+__global__ void __launch_bounds__(32 * kAllWarps) f64_allpairs_kernel(K64 k, const double *__restrict__ rk,
+                                                                      const float2 *__restrict__ posf,
+                                                                      const double2 *__restrict__ csphi,
+                                                                      double *__restrict__ k_next,
+                                                                      double *__restrict__ caf, NextStage next)
+{
+  __shared__ double2 queue[kAllWarps][kAllQueue];  // phase and omega of the neighbours
+  __shared__ double term[kAllWarps * kAllQueue], cterm[kAllWarps * kAllQueue];
+  __shared__ double2 own[kAllParticles];
+  __shared__ double early[kAllWarps][3];  // sums of the queues evaluated during the scan
+  __shared__ int count[kAllWarps];
+  pdl_enter();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int i0 = blockIdx.x * kAllParticles;
+  const int i = i0 + (warp >> 1);
+  const int ip = k.model == 1 ? 2 : 4;
+  int cnt = 0;
   Sums a{0.0, 0.0, 0.0};
-  // the lane's candidates j = lane, lane + 32, ... in that order; the float
-  // positions of four of them are loaded together.  The pair terms (FP64 sin
-  // and cos, a warp's full FP64 pipe time whatever the lanes) wait until the
-  // scan is over, so the few neighbours of a particle, found by different
-  // lanes in different iterations, are summed in one pass; each lane still
-  // adds its own neighbours in ascending j, so the sums are unchanged.
-  int pend[4], np = 0;
-  for (int j0 = lane; j0 < k.n; j0 += 128)
+  if (i < k.n)
   {
-    float2 pj[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) pj[u] = j0 + 32 * u < k.n ? posf[j0 + 32 * u] : pi;
-#pragma unroll
-    for (int u = 0; u < 4; ++u)
+    const double *st = rk + (long) k.s * i;
+    const double2 mine = *reinterpret_cast<const double2 *>(st + ip);
+    if (lane == 0) own[warp >> 1] = mine;
+    const float2 p_i = posf[i];
+    const int half = (k.n + 1) / 2;
+    const int begin = (warp & 1) ? half : 0, end = (warp & 1) ? k.n : half;
+    constexpr int U = 8;
+    for (int j0 = begin + lane; j0 - lane < end; j0 += 32 * U)
     {
-      const int j = j0 + 32 * u;
-      if (j >= k.n || j == i || pretest_out(k, pi, pj[u])) continue;
-      const double *sj = rk + (long) k.s * j;
-      if (pair_dr2<false>(k, x_i, y_i, sj[0], sj[1]) <= k.rho2)
+      float2 p[U];
+      int in[U];
+      bool unsure = false;
+#pragma unroll
+      for (int u = 0; u < U; ++u) p[u] = posf[min(j0 + 32 * u, k.n - 1)];
+#pragma unroll
+      for (int u = 0; u < U; ++u)
       {
-        if (np == 4)
+        const int j = j0 + 32 * u;
+        in[u] = pretest(p_i, p[u], k.rho_incl, k.rho_excl);
+        if (j >= end || j == i) in[u] = 0;
+        if (in[u] == 1 && k.model == 2) in[u] = 2;
+        unsure |= in[u] == 2;
+      }
+      if (unsure)
+      {
+        double x_i = st[0], y_i = st[1];
+        if (k.model == 1 && k.flavor == 1)
         {
-          for (int t = 0; t < 4; ++t)
-          {
-            const double *sp = rk + (long) k.s * pend[t];
-            add_pair(k, a, phi_i, omega_i, sp[ip], sp[ip + 1]);
-          }
-          np = 0;
+          x_i = wrap1(x_i);
+          y_i = wrap1(y_i);
         }
-        pend[np++] = j;
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          if (in[u] == 2)
+          {
+            const double *sj = rk + (long) k.s * (j0 + 32 * u);
+            in[u] = pair_dr2<false>(k, x_i, y_i, sj[0], sj[1]) <= k.rho2;
+          }
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+      {
+        const unsigned found = __ballot_sync(0xffffffffu, in[u]);
+        if (!found) continue;
+        if (in[u])
+          queue[warp][cnt + __popc(found & ((1u << lane) - 1u))] =
+              *reinterpret_cast<const double2 *>(rk + (long) k.s * (j0 + 32 * u) + ip);
+        cnt += __popc(found);
+        if (cnt > kAllQueue - 32)
+        {
+          __syncwarp();
+          for (int q = lane; q < cnt; q += 32)
+          {
+            const double2 pj = queue[warp][q];
+            double af, cf;
+            pair_terms(k, mine.x, mine.y, pj.x, pj.y, af, cf);
+            a.af += af;
+            a.caf += cf;
+          }
+          a.card += (double) cnt;
+          cnt = 0;
+          __syncwarp();
+        }
       }
     }
   }
-  for (int t = 0; t < np; ++t)
-  {
-    const double *sp = rk + (long) k.s * pend[t];
-    add_pair(k, a, phi_i, omega_i, sp[ip], sp[ip + 1]);
-  }
+  if (__any_sync(0xffffffffu, a.card != 0.0))
 #pragma unroll
-  for (int off = 16; off > 0; off >>= 1)
+    for (int off = 16; off > 0; off >>= 1)
+    {
+      a.af += __shfl_xor_sync(0xffffffffu, a.af, off);
+      a.caf += __shfl_xor_sync(0xffffffffu, a.caf, off);
+    }
+  if (lane == 0)
   {
-    a.af += __shfl_xor_sync(0xffffffffu, a.af, off);
-    a.card += __shfl_xor_sync(0xffffffffu, a.card, off);
-    a.caf += __shfl_xor_sync(0xffffffffu, a.caf, off);
+    count[warp] = cnt;
+    early[warp][0] = a.af;
+    early[warp][1] = a.card;
+    early[warp][2] = a.caf;
   }
-  if (lane != 0) return;
-  write_k(k, i, st, a, k_next, caf, csphi + i);
-  if (next.rk)
+  __syncthreads();
+  // warp 0 (as many more as there are pairs): the block's queued pairs, end to
+  // end; the last warp: the rest of the derivative and of the next stage
+  int total = 0;
+#pragma unroll
+  for (int w = 0; w < kAllWarps; ++w) total += count[w];
+  const int g = i0 + lane;
+  if (warp == kAllWarps - 1 && lane < kAllParticles && g < k.n)
   {
-    // this particle's derivative is complete (an entry write_k left untouched
-    // keeps the value it had, as the stage kernel would read it)
-    const long ii = (long) k.s * i;
-    for (int q = 0; q < k.s; ++q) next.rk[ii + q] = next.x[ii + q] + next.coef * next.dt * k_next[ii + q];
-    const double x = next.rk[ii], y = next.rk[ii + 1];
-    next.posf[i] = make_float2((float) (x - floor(x)), (float) (y - floor(y)));
-    const double phi = next.rk[ii + (k.model == 1 ? 2 : 4)];
-    next.csphi[i] = make_double2(cos(phi), sin(phi));
+    const double2 cs = csphi[g];
+    write_k_but_torque(k, g, rk + (long) k.s * g, k_next, cs.x, cs.y);
+    if (AFTER != AFTER_NOTHING) advance_but_omega<AFTER>(k, g, k_next, next);
   }
+  // what the finishing lanes need from memory, asked for before the pair terms
+  const bool finisher = warp == 0 && lane < kAllParticles && g < k.n;
+  const long at = (long) k.s * (finisher ? g : i0) + k.s - 1;
+  StageWords words{0.0, 0.0, 0.0, 0.0};
+  double torque = 0.0;
+  if (finisher && AFTER != AFTER_NOTHING)
+  {
+    words = load_stage<AFTER>(next, at);
+    torque = k_next[at];  // kept where the particle has no neighbour
+  }
+  const int workers = 32 * (kAllWarps - 1);
+  if (threadIdx.x < workers)
+    for (int p = threadIdx.x; p < total; p += workers)
+    {
+      int w = 0, q = p;
+      while (q >= count[w]) q -= count[w++];
+      const double2 pj = queue[w][q], me = own[w >> 1];
+      double af, cf;
+      pair_terms(k, me.x, me.y, pj.x, pj.y, af, cf);
+      term[p] = af;
+      if (k.higher_order) cterm[p] = cf;
+    }
+  __syncthreads();
+  if (!finisher) return;
+  a = Sums{0.0, 0.0, 0.0};
+  const int w = 2 * lane;
+  int p = 0;
+#pragma unroll
+  for (int v = 0; v < kAllWarps; ++v) p += v < w ? count[v] : 0;
+  const int c0 = count[w], c1 = count[w + 1];
+  a.card = early[w][1] + early[w + 1][1] + (double) (c0 + c1);
+  if (early[w][1] != 0.0 || early[w + 1][1] != 0.0)
+  {
+    a.af = early[w][0] + early[w + 1][0];
+    a.caf = early[w][2] + early[w + 1][2];
+  }
+  for (const int e = p + c0 + c1; p < e; ++p)
+  {
+    a.af += term[p];
+    if (k.higher_order) a.caf += cterm[p];
+  }
+  if (a.card != 0.0)
+  {
+    torque = -(k.model == 1 ? k.xi : k.xi_phi) * own[lane].y + k.sigma * a.af / a.card;
+    k_next[at] = torque;
+    if (k.higher_order) a.caf *= k.sigma / a.card;
+  }
+  if (k.higher_order) caf[g] = a.caf;
+  if (AFTER != AFTER_NOTHING) advance_component<AFTER>(next, at, words, torque);
 }
 
 // ------------------------------------------------------------ neighbour sums
@@ -432,7 +575,8 @@ __global__ void f64_allpairs_kernel(K64 k, const double *__restrict__ rk, const 
 // and 32 pair terms are evaluated at a time; each lane then adds its own terms
 // in the order it found them, so the sums are the reference's, bit for bit.
 // N = 65,536, density 2: linked list 313 -> 67 us; Verlet pairs at N = 20,011
-// 87 -> 37 us.
+// 87 -> 37 us (44 and 29 us with the table-driven functions and the narrow
+// pre-test margin).
 constexpr int kQueue = 16;       // queued neighbours a lane
 constexpr int kScan = 4;         // candidates a lane looks at together (their loads are in flight at once)
 constexpr int kPairThreads = 32;  // one warp a block: 20,011 particles in blocks of 64 left SMs with 3 blocks beside SMs with 2
@@ -443,27 +587,6 @@ struct PairBuffers
   int j[kQueue * 32];
   unsigned short flat[kQueue * 32];
 };
-
-// Pair terms: first order ParticleSystemFirstOrderPtr.cpp:404-415; second order
-// ParticleSystemSecondOrder.cpp:160-161 (see add_pair).
-__device__ __forceinline__ void pair_terms(const K64 &k, double phi_i, double omega_i, double phi_j, double omega_j,
-                                           double &af, double &caf)
-{
-  const double d = k.model == 1 ? phi_j - phi_i : phi_j - phi_i - k.alpha;
-  double s, c = 0.0;
-  if (k.higher_order || (k.model == 1 && k.sa != 0.0)) sincos(d, &s, &c);
-  else s = sin(d);
-  caf = 0.0;
-  if (k.model == 1)
-  {
-    af = s * k.ca - c * k.sa;
-    if (k.higher_order) caf = (omega_j - omega_i) * (c * k.ca + s * k.sa);
-  } else
-  {
-    af = s;
-    if (k.higher_order) caf = (omega_j - omega_i) * c;
-  }
-}
 
 // Evaluates the queued pairs of the warp's lanes (cnt of this lane's, in rows
 // j[m * 32 + lane]) and adds each lane's terms to its sums in order.
@@ -779,30 +902,40 @@ __global__ void f64_rk4_combine_kernel(double *__restrict__ x, const double *__r
 // ParticleSystemSecondOrder::AddNoise, ParticleSystemSecondOrder.cpp:439-451).
 __global__ void f64_se2_kernel(double *__restrict__ x, const double *__restrict__ det, double *__restrict__ td,
                                int n, double dt, double sqrt_dt, double intensity_r, double intensity_phi,
-                               NoiseKey nk)
+                               NoiseKey nk, const double2 *__restrict__ table)
 {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  double z[4];
-  normals4_f64(nk, (uint32_t) i, 0, z);
-  double stoch[6] = {0.0, 0.0, intensity_r * z[0], intensity_r * z[1], 0.0, intensity_phi * z[2]};
-  const long ii = 6L * i;
-  for (int s = 0; s < 6; ++s)
-  {
-    const double d = dt * det[ii + s] + sqrt_dt * stoch[s];
-    td[ii + s] = d;
-    x[ii + s] += d;
-  }
+  const uint4 u = philox_block(nk, (uint32_t) i, 0);
+  // without translational noise (intensity_r = 0) its two normals multiply 0
+  double z[4] = {0.0, 0.0, 0.0, 0.0};
+  if (intensity_r != 0.0) box_muller_f64(table, u.x, u.y, z[0], z[1]);
+  box_muller_f64(table, u.z, u.w, z[2], z[3]);
+  double2 *t2 = reinterpret_cast<double2 *>(td + 6L * i);
+  double2 *x2 = reinterpret_cast<double2 *>(x + 6L * i);
+  const double2 *d2 = reinterpret_cast<const double2 *>(det + 6L * i);
+  const double2 dr = d2[0], dv = d2[1], dp = d2[2];
+  const double2 tr = make_double2(dt * dr.x, dt * dr.y);
+  const double2 tv = make_double2(dt * dv.x + sqrt_dt * (intensity_r * z[0]), dt * dv.y + sqrt_dt * (intensity_r * z[1]));
+  const double2 tp = make_double2(dt * dp.x, dt * dp.y + sqrt_dt * (intensity_phi * z[2]));
+  t2[0] = tr;
+  t2[1] = tv;
+  t2[2] = tp;
+  const double2 a = x2[0], b = x2[1], c = x2[2];
+  x2[0] = make_double2(a.x + tr.x, a.y + tr.y);
+  x2[1] = make_double2(b.x + tv.x, b.y + tv.y);
+  x2[2] = make_double2(c.x + tp.x, c.y + tp.y);
 }
 
 // First-order stochastic Euler (StochasticEulerStepperPtr.hpp:40-73).
 __global__ void f64_se1_kernel(double *__restrict__ x, const double *__restrict__ d, double *__restrict__ td, int n,
-                               double dt, double sqrt_dt, double intensity_phi, NoiseKey nk)
+                               double dt, double sqrt_dt, double intensity_phi, NoiseKey nk,
+                               const double2 *__restrict__ table)
 {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  double z[4];
-  normals4_f64(nk, (uint32_t) i, 0, z);
+  double z[2];
+  normals_f64<1>(table, nk, (uint32_t) i, 0, z);
   const double delta_W_phi = sqrt_dt * z[0];
   const long ii = 4L * i;
   td[ii] = d[ii] * dt;
@@ -815,12 +948,13 @@ __global__ void f64_se1_kernel(double *__restrict__ x, const double *__restrict_
 // First-order strong order 1.5 Taylor scheme (StochasticRungeKuttaStepperPtr.hpp:40-76).
 __global__ void f64_srk1_kernel(double *__restrict__ x, const double *__restrict__ d, const double *__restrict__ caf,
                                 double *__restrict__ td, int n, double dt, double sqrt_dt, double dt15,
-                                double inv_sqrt3, double sqrt_2noise, double friction, NoiseKey nk)
+                                double inv_sqrt3, double sqrt_2noise, double friction, NoiseKey nk,
+                                const double2 *__restrict__ table)
 {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  double z[4];
-  normals4_f64(nk, (uint32_t) i, 0, z);
+  double z[2];
+  normals_f64<1>(table, nk, (uint32_t) i, 0, z);
   const double U_1 = z[0], U_2 = z[1];
   const double delta_W_i = U_1 * sqrt_dt;
   const double delta_Z_i = 0.5 * dt15 * (U_1 + inv_sqrt3 * U_2);
@@ -838,19 +972,20 @@ __global__ void f64_srk1_kernel(double *__restrict__ x, const double *__restrict
 // additive noise on v_x, v_y (b_r) and omega (b_phi); see spss_oracle.c.
 __global__ void f64_srk2_kernel(double *__restrict__ x, const double *__restrict__ d, const double *__restrict__ caf,
                                 double *__restrict__ td, int n, double dt, double sqdt, double dt15, double inv_sqrt3,
-                                double b_r, double b_phi, double xi_r, double xi_phi, double v0, NoiseKey nk)
+                                double b_r, double b_phi, double xi_r, double xi_phi, double v0, NoiseKey nk,
+                                const double2 *__restrict__ table)
 {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  double u[8];
-  normals4_f64(nk, (uint32_t) i, 0, u);
-  normals4_f64(nk, (uint32_t) i, 1, u + 4);
+  double u[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+  if (b_r != 0.0) normals_f64<2>(table, nk, (uint32_t) i, 0, u);  // b_r = 0 multiplies them
+  normals_f64<1>(table, nk, (uint32_t) i, 1, u + 4);
   const double dWx = u[0] * sqdt, dZx = 0.5 * dt15 * (u[0] + inv_sqrt3 * u[1]);
   const double dWy = u[2] * sqdt, dZy = 0.5 * dt15 * (u[2] + inv_sqrt3 * u[3]);
   const double dWw = u[4] * sqdt, dZw = 0.5 * dt15 * (u[4] + inv_sqrt3 * u[5]);
   const long ii = 6L * i;
-  const double phi = x[ii + 4];
-  const double cphi = cos(phi), sphi = sin(phi);
+  double cphi, sphi;
+  fast_sincos(table, x[ii + 4], sphi, cphi);
   td[ii] = d[ii] * dt + 0.5 * d[ii + 2] * dt * dt + b_r * dZx;
   td[ii + 1] = d[ii + 1] * dt + 0.5 * d[ii + 3] * dt * dt + b_r * dZy;
   td[ii + 2] = d[ii + 2] * dt + 0.5 * (-xi_r * d[ii + 2] - v0 * sphi * d[ii + 4]) * dt * dt + b_r * (dWx - xi_r * dZx);
@@ -882,13 +1017,14 @@ __global__ void f64_max2_kernel(const double *__restrict__ td, int n, int s, uns
   if (threadIdx.x == 0) atomicMax(out, (unsigned long long) __double_as_longlong(sh[0]));
 }
 
-__global__ void f64_noise_kernel(double *__restrict__ out, int n, int per, NoiseKey nk)
+__global__ void f64_noise_kernel(double *__restrict__ out, int n, int per, NoiseKey nk,
+                                 const double2 *__restrict__ table)
 {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  double u[8];
-  normals4_f64(nk, (uint32_t) i, 0, u);
-  if (per > 4) normals4_f64(nk, (uint32_t) i, 1, u + 4);
+  double u[6];
+  normals_f64<2>(table, nk, (uint32_t) i, 0, u);
+  if (per > 4) normals_f64<1>(table, nk, (uint32_t) i, 1, u + 4);
   for (int d = 0; d < per; ++d) out[(long) per * i + d] = u[d];
 }
 
@@ -928,6 +1064,7 @@ int f64_create(spss_ctx *ctx)
   SPSS_TRY(f->vl_off.reserve(ctx->p.n + 1));
   SPSS_TRY(f->max2.reserve(1));
   SPSS_TRY(f->partials.reserve(4 * 1024));
+  SPSS_TRY(make_f64_tables(f->table, ctx->stream));
   SPSS_CUDA_TRY(cudaMallocHost((void **) &f->h_max2, sizeof(unsigned long long)));
   SPSS_CUDA_TRY(cudaMemsetAsync(f->state.ptr, 0, sizeof(double) * len, ctx->stream));
   for (auto &kb : f->k) SPSS_CUDA_TRY(cudaMemsetAsync(kb.ptr, 0, sizeof(double) * len, ctx->stream));
@@ -954,6 +1091,7 @@ void f64_destroy(spss_ctx *ctx)
   f->cell_of.release();
   f->posf.release();
   f->csphi.release();
+  f->table.release();
   f->rk2.release();
   f->posf2.release();
   f->csphi2.release();
@@ -1063,7 +1201,7 @@ int f64_evaluate(spss_ctx *ctx, int variant, const double *d_state, const double
   switch (variant)
   {
     case SPSS_VARIANT_ALL_PAIRS:
-      f64_allpairs_kernel<<<blocks_for(32L * k.n, 128), 128, 0, ctx->stream>>>(
+      f64_allpairs_kernel<AFTER_NOTHING><<<blocks_for(k.n, kAllParticles), 32 * kAllWarps, 0, ctx->stream>>>(
           k, f->rk.ptr, f->posf.ptr, f->csphi.ptr, d_knext, f->caf.ptr, NextStage{});
       ++ctx->launches;
       return check_launch("f64_allpairs_kernel");
@@ -1127,6 +1265,36 @@ static NoiseKey noise_key(const spss_ctx *ctx, unsigned long long step)
   return nk;
 }
 
+// The four evaluations of an all-pairs RK4 step whose first stage stands in the
+// first stage buffers; the last one leaves the next step's first stage there.
+static int allpairs_rk4_stages(spss_ctx *ctx, const K64 &k, double dt, bool chained)
+{
+  F64Path *f = ctx->f64;
+  double *rk[2] = {f->rk.ptr, f->rk2.ptr};
+  float2 *pf[2] = {f->posf.ptr, f->posf2.ptr};
+  double2 *cs[2] = {f->csphi.ptr, f->csphi2.ptr};
+  const double coef[4] = {0.5, 0.5, 1.0, 0.0};
+  for (int e = 0; e < 4; ++e)
+  {
+    const int a = e & 1, b = a ^ 1;
+    const NextStage next{f->state.ptr, coef[e],     dt,          rk[b],       pf[b],
+                         cs[b],        f->k[0].ptr, f->k[1].ptr, f->k[2].ptr, f->td.ptr};
+    const int blocks = blocks_for(k.n, kAllParticles), threads = 32 * kAllWarps;
+    const double *in = rk[a];
+    const float2 *pin = pf[a];
+    const double2 *cin = cs[a];
+    if (e < 3)
+      SPSS_CUDA_TRY(launch_chained(chained && e > 0, f64_allpairs_kernel<AFTER_STAGE>, blocks, threads, 0, ctx->stream,
+                                   k, in, pin, cin, f->k[e].ptr, f->caf.ptr, next));
+    else
+      SPSS_CUDA_TRY(launch_chained(chained, f64_allpairs_kernel<AFTER_COMBINE>, blocks, threads, 0, ctx->stream, k, in,
+                                   pin, cin, f->k[e].ptr, f->caf.ptr, next));
+    ++ctx->launches;
+    SPSS_TRY(check_launch("f64_allpairs_kernel"));
+  }
+  return SPSS_OK;
+}
+
 int f64_step(spss_ctx *ctx, int stepper, double t, double dt)
 {
   (void) t;
@@ -1137,35 +1305,19 @@ int f64_step(spss_ctx *ctx, int stepper, double t, double dt)
   const int tb = 256;
   if (stepper == SPSS_STEPPER_RK4 && variant_for(ctx, variant) == SPSS_VARIANT_ALL_PAIRS && !ctx->higher_order)
   {
-    // four all-pairs evaluations, each pair kernel also writing the next
-    // stage (x + 0.5 dt k1, x + 0.5 dt k2, x + dt k3) into the other stage
-    // buffers: six kernels instead of nine, the same arithmetic
-    double *x = f->state.ptr;
+    // the first stage, then four all-pairs evaluations, each also writing the
+    // next stage (x + 0.5 dt k1, x + 0.5 dt k2, x + dt k3, and the step's
+    // result, which is the next step's first stage) into the other stage
+    // buffers
     const K64 k = make_k64(ctx);
     SPSS_TRY(f->rk2.reserve(len));
     SPSS_TRY(f->posf2.reserve(n));
     SPSS_TRY(f->csphi2.reserve(n));
-    f64_stage_posf_kernel<<<blocks_for(n, tb), tb, 0, ctx->stream>>>(k, x, f->k[0].ptr, f->rk.ptr, f->posf.ptr,
-                                                                     f->csphi.ptr, 0.0, dt);
+    f64_stage_posf_kernel<<<blocks_for(n, tb), tb, 0, ctx->stream>>>(k, f->state.ptr, f->k[0].ptr, f->rk.ptr,
+                                                                     f->posf.ptr, f->csphi.ptr, 0.0, dt);
     ++ctx->launches;
     SPSS_TRY(check_launch("f64_stage_posf_kernel"));
-    double *rk[2] = {f->rk.ptr, f->rk2.ptr};
-    float2 *pf[2] = {f->posf.ptr, f->posf2.ptr};
-    double2 *cs[2] = {f->csphi.ptr, f->csphi2.ptr};
-    const double coef[3] = {0.5, 0.5, 1.0};
-    for (int e = 0; e < 4; ++e)
-    {
-      const int a = e & 1, b = a ^ 1;
-      const NextStage next = e < 3 ? NextStage{x, coef[e], dt, rk[b], pf[b], cs[b]} : NextStage{};
-      f64_allpairs_kernel<<<blocks_for(32L * n, 128), 128, 0, ctx->stream>>>(k, rk[a], pf[a], cs[a], f->k[e].ptr,
-                                                                            f->caf.ptr, next);
-      ++ctx->launches;
-      SPSS_TRY(check_launch("f64_allpairs_kernel"));
-    }
-    f64_rk4_combine_kernel<<<blocks_for(len, tb), tb, 0, ctx->stream>>>(x, f->k[0].ptr, f->k[1].ptr, f->k[2].ptr,
-                                                                        f->k[3].ptr, f->td.ptr, len, dt);
-    ++ctx->launches;
-    SPSS_TRY(check_launch("f64_rk4_combine_kernel"));
+    SPSS_TRY(allpairs_rk4_stages(ctx, k, dt, false));
   } else if (stepper == SPSS_STEPPER_RK4)
   {
     double *x = f->state.ptr;
@@ -1189,21 +1341,23 @@ int f64_step(spss_ctx *ctx, int stepper, double t, double dt)
       if (ctx->p.model == 2)
         f64_se2_kernel<<<blocks_for(n, tb), tb, 0, ctx->stream>>>(f->state.ptr, f->det.ptr, f->td.ptr, n, dt,
                                                                   sqrt_dt, std::sqrt(2.0 * ctx->p.D_r),
-                                                                  std::sqrt(2.0 * ctx->p.D_phi), nk);
+                                                                  std::sqrt(2.0 * ctx->p.D_phi), nk, f->table.ptr);
       else
         f64_se1_kernel<<<blocks_for(n, tb), tb, 0, ctx->stream>>>(f->state.ptr, f->det.ptr, f->td.ptr, n, dt,
-                                                                  sqrt_dt, std::sqrt(2.0 * ctx->p.D_phi), nk);
+                                                                  sqrt_dt, std::sqrt(2.0 * ctx->p.D_phi), nk, f->table.ptr);
     } else if (stepper == SPSS_STEPPER_STOCHASTIC_RUNGE_KUTTA)
     {
       const double dt15 = std::pow(dt, 1.5), inv_sqrt3 = 1.0 / std::sqrt(3.0);
       if (ctx->p.model == 1)
         f64_srk1_kernel<<<blocks_for(n, tb), tb, 0, ctx->stream>>>(f->state.ptr, f->det.ptr, f->caf.ptr, f->td.ptr,
                                                                    n, dt, sqrt_dt, dt15, inv_sqrt3,
-                                                                   std::sqrt(2.0 * ctx->p.D_phi), ctx->p.xi, nk);
+                                                                   std::sqrt(2.0 * ctx->p.D_phi), ctx->p.xi, nk,
+                                                                   f->table.ptr);
       else
         f64_srk2_kernel<<<blocks_for(n, tb), tb, 0, ctx->stream>>>(
             f->state.ptr, f->det.ptr, f->caf.ptr, f->td.ptr, n, dt, sqrt_dt, dt15, inv_sqrt3,
-            std::sqrt(2.0 * ctx->p.D_r), std::sqrt(2.0 * ctx->p.D_phi), ctx->p.xi_r, ctx->p.xi_phi, ctx->p.v0, nk);
+            std::sqrt(2.0 * ctx->p.D_r), std::sqrt(2.0 * ctx->p.D_phi), ctx->p.xi_r, ctx->p.xi_phi, ctx->p.v0, nk,
+            f->table.ptr);
     } else
     {
       return SPSS_ERR_INVALID_ARGUMENT;
@@ -1244,6 +1398,7 @@ int f64_steps(spss_ctx *ctx, int stepper, double t0, double dt, int nsteps)
   }
   t += dt;
   SPSS_TRY(f64_step(ctx, stepper, t, dt));
+  const bool stages_only = variant_for(ctx, ctx->p.variant) == SPSS_VARIANT_ALL_PAIRS && !ctx->higher_order;
   if (!f->rk4_exec || f->rk4_dt != dt || f->rk4_higher_order != ctx->higher_order)
   {
     if (f->rk4_exec) cudaGraphExecDestroy(f->rk4_exec);
@@ -1256,7 +1411,9 @@ int f64_steps(spss_ctx *ctx, int stepper, double t0, double dt, int nsteps)
     SPSS_CUDA_TRY(cudaStreamSynchronize(work));
     int rc = SPSS_OK;
     if (cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) rc = SPSS_ERR_CUDA;
-    if (rc == SPSS_OK) rc = f64_step(ctx, stepper, t + dt, dt);
+    // an all-pairs step leaves the next step's first stage behind: without the stage kernel
+    if (rc == SPSS_OK)
+      rc = stages_only ? allpairs_rk4_stages(ctx, make_k64(ctx), dt, true) : f64_step(ctx, stepper, t + dt, dt);
     cudaGraph_t g = nullptr;
     const cudaError_t e = cudaStreamEndCapture(ctx->stream, &g);
     ctx->stream = work;
@@ -1284,7 +1441,8 @@ int f64_noise(spss_ctx *ctx, int stepper, unsigned long long step, double *d_out
 {
   const int per = normals_per_particle(ctx->p.model, stepper);
   if (per == 0) return SPSS_OK;
-  f64_noise_kernel<<<blocks_for(ctx->p.n, 256), 256, 0, ctx->stream>>>(d_out, ctx->p.n, per, noise_key(ctx, step));
+  f64_noise_kernel<<<blocks_for(ctx->p.n, 256), 256, 0, ctx->stream>>>(d_out, ctx->p.n, per, noise_key(ctx, step),
+                                                                     ctx->f64->table.ptr);
   ++ctx->launches;
   return check_launch("f64_noise_kernel");
 }

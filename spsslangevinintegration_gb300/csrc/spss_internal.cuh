@@ -72,6 +72,38 @@ inline cudaError_t launch_chained(bool chained, void (*kernel)(Params...), dim3 
   return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
+// ------------------------------------------------------------------ device memory
+
+template<class T>
+struct DeviceArray
+{
+  T *ptr = nullptr;
+  size_t count = 0;
+  int reserve(size_t n)
+  {
+    if (n <= count && ptr) return SPSS_OK;
+    release();
+    if (n == 0) n = 1;
+    cudaError_t e = cudaMalloc((void **) &ptr, n * sizeof(T));
+    if (e != cudaSuccess)
+    {
+      ptr = nullptr;
+      count = 0;
+      cudaGetLastError();
+      return SPSS_ERR_OUT_OF_MEMORY;
+    }
+    count = n;
+    return SPSS_OK;
+  }
+  void release()
+  {
+    if (ptr) cudaFree(ptr);
+    ptr = nullptr;
+    count = 0;
+  }
+  size_t bytes() const { return count * sizeof(T); }
+};
+
 // ------------------------------------------------------------------ Philox
 
 // Philox4x32-10 (Salmon, Moraes, Dror & Shaw, "Parallel random numbers: as
@@ -139,15 +171,118 @@ __device__ __forceinline__ uint4 philox_block(const NoiseKey &nk, uint32_t parti
   return Philox::generate(c, make_uint2((uint32_t) nk.seed, (uint32_t) (nk.seed >> 32)));
 }
 
+// ------------------------------------------------------------------ FP64 functions
+//
+// GB300 has one FP64 instruction for about 69 FP32 ones, and the FP64 kernels
+// are bound by their count: the general-purpose functions spend about 40
+// (sin), 30 (log) and 15 (sqrt) of them.  Table-driven evaluation (the method
+// of P. T. P. Tang, "Table-driven implementation of the logarithm function in
+// IEEE floating-point arithmetic", ACM TOMS 16, 1990, and of his sine of the
+// same kind) needs 14 for a sine, 16 with the cosine, 13 for the logarithm and
+// 8 for the square root, at the same accuracy (about 1 ulp; measured against
+// the CUDA functions in tests/test_gpu_f64_functions.py).
+
+constexpr int kTrigTable = 256;      // cos and sin of 2 pi k / 256
+constexpr int kLogFirst = 88, kLogLast = 184;  // j / 128 covers [sqrt(1/2), sqrt(2)] with room
+constexpr int kTableEntries = kTrigTable + (kLogLast - kLogFirst + 1);
+
+// 1.5 * 2^52: adding it rounds to an integer, which then stands in the low word.
+#define SPSS_ROUND_MAGIC 6755399441055744.0
+
+// sin and cos of 2 pi k / 256 + r, 0 <= |r| <= 2 pi / 256: Taylor polynomials
+// (remainders below 1e-20 and 4e-18) and the angle sum.
+__device__ __forceinline__ void sincos_at(const double2 *__restrict__ table, int k, double r, double &s, double &c)
+{
+  const double2 T = __ldg(table + (k & (kTrigTable - 1)));
+  const double p = r * r;
+  const double sr = fma(r * p, fma(p, fma(p, -1.0 / 5040.0, 1.0 / 120.0), -1.0 / 6.0), r);
+  const double cm = p * fma(p, fma(p, -1.0 / 720.0, 1.0 / 24.0), -0.5);
+  s = fma(T.x, sr, fma(T.y, cm, T.y));
+  c = fma(-T.y, sr, fma(T.x, cm, T.x));
+}
+
+// Largest |x| that the two-part reduction takes: k < 2^19 keeps k * (upper
+// part, 33 bits) exact.  Beyond it (and for infinities and NaN) the CUDA
+// functions.
+constexpr double kTrigMax = 4096.0;
+
+__device__ __forceinline__ void reduce_turn(double x, int &k, double &r)
+{
+  const double t = fma(x, 40.743665431525205957, SPSS_ROUND_MAGIC);  // 128 / pi
+  k = __double2loint(t);
+  const double kd = t - SPSS_ROUND_MAGIC;
+  // pi / 128 = 0x1.921fb544p-6 (33 bits) + 0x1.0b4611a626331p-40
+  r = fma(kd, -0x1.921fb544p-6, x);
+  r = fma(kd, -0x1.0b4611a626331p-40, r);
+}
+
+__device__ __forceinline__ void fast_sincos(const double2 *__restrict__ table, double x, double &s, double &c)
+{
+  if (!(fabs(x) <= kTrigMax))
+  {
+    sincos(x, &s, &c);
+    return;
+  }
+  int k;
+  double r;
+  reduce_turn(x, k, r);
+  sincos_at(table, k, r, s, c);
+}
+
+__device__ __forceinline__ double fast_sin(const double2 *__restrict__ table, double x)
+{
+  double s, c;
+  fast_sincos(table, x, s, c);  // the cosine is not computed where it is not used
+  return s;
+}
+
+// log((a + 0.5) 2^-32) for a 32-bit a: the mantissa m in [sqrt(1/2), sqrt(2)),
+// c = j / 128 the nearest table point (c = 1 around 1, where the result is
+// small), log(m / c) by its series to r^7 (|r| <= 1 / 180).
+__device__ __forceinline__ double log_uniform(const double2 *__restrict__ table, uint32_t a)
+{
+  const double u = __hiloint2double(0x43300000, (int) a) - 4503599627370495.5;  // a + 0.5, exact
+  int hi = __double2hiint(u);
+  const int shift = (hi - 0x3fe6a09f) >> 20;  // 0x3fe6a09f: sqrt(1/2), rounded up
+  hi -= shift << 20;
+  const double m = __hiloint2double(hi, __double2loint(u));
+  const float mf = __uint_as_float((((uint32_t) hi - 0x38000000u) << 3));  // the leading 21 bits
+  const int j = __float2int_rn(mf * 128.0f);
+  const double2 T = __ldg(table + kTrigTable + (j - kLogFirst));  // 128 / j (rounded), minus the log of that
+  const double r = fma(m, T.x, -1.0);
+  double q = fma(r, 1.0 / 7.0, -1.0 / 6.0);
+  q = fma(r, q, 1.0 / 5.0);
+  q = fma(r, q, -1.0 / 4.0);
+  q = fma(r, q, 1.0 / 3.0);
+  q = fma(r, q, -0.5);
+  const double e = __hiloint2double(0x43300000, (shift - 32) ^ 0x80000000) - 4503601774854144.0;  // (double) (shift - 32)
+  return fma(e, 0.693147180559945309417, T.y) + fma(r * r, q, r);
+}
+
+// Square root of a positive double in the range of float normals: the FP32
+// reciprocal square root and one third-order step.
+__device__ __forceinline__ double sqrt_positive(double v)
+{
+  const double y = (double) rsqrtf((float) v);
+  const double g = v * y;
+  const double e = fma(-g, y, 1.0);
+  return fma(g * e, fma(e, 0.375, 0.5), g);
+}
+
+// The tables of the functions above: cos, sin of 2 pi k / 256, then 128 / j and
+// -log(128 / j as rounded).
+int make_f64_tables(DeviceArray<double2> &table, cudaStream_t stream);
+
 // Box-Muller on two 32-bit uniforms in (0, 1): FP64 variant for the
 // reference-arithmetic path, FP32 variant for the fast path.
-__device__ __forceinline__ void box_muller_f64(uint32_t a, uint32_t b, double &z0, double &z1)
+__device__ __forceinline__ void box_muller_f64(const double2 *__restrict__ table, uint32_t a, uint32_t b, double &z0,
+                                               double &z1)
 {
-  const double u1 = ((double) a + 0.5) * 2.3283064365386963e-10;
-  const double u2 = ((double) b + 0.5) * 2.3283064365386963e-10;
-  const double r = sqrt(-2.0 * log(u1));
+  const double r = sqrt_positive(-2.0 * log_uniform(table, a));
+  // angle 2 pi (b + 0.5) 2^-32: the 256th of a turn and the rest
+  const double rest = __hiloint2double(0x43300000, (int) (b & 0xffffffu)) - 4503599627370495.5;  // + 0.5, exact
   double s, c;
-  sincospi(2.0 * u2, &s, &c);
+  sincos_at(table, (int) (b >> 24), rest * 1.46291807926715968e-9, s, c);  // 2 pi / 2^32
   z0 = r * c;
   z1 = r * s;
 }
@@ -203,11 +338,14 @@ __device__ __forceinline__ void normals4_f32(const NoiseKey &nk, uint32_t partic
   box_muller_f32(u.z, u.w, z[2], z[3]);
 }
 
-__device__ __forceinline__ void normals4_f64(const NoiseKey &nk, uint32_t particle, uint32_t block, double z[4])
+// The first `pairs` Box-Muller pairs of a block of four uniforms.
+template<int PAIRS>
+__device__ __forceinline__ void normals_f64(const double2 *__restrict__ table, const NoiseKey &nk, uint32_t particle,
+                                            uint32_t block, double *z)
 {
   const uint4 u = philox_block(nk, particle, block);
-  box_muller_f64(u.x, u.y, z[0], z[1]);
-  box_muller_f64(u.z, u.w, z[2], z[3]);
+  box_muller_f64(table, u.x, u.y, z[0], z[1]);
+  if (PAIRS > 1) box_muller_f64(table, u.z, u.w, z[2], z[3]);
 }
 
 // ------------------------------------------------------------------ reductions
@@ -286,38 +424,6 @@ inline int normals_per_particle(int model, int stepper)
   if (stepper == SPSS_STEPPER_STOCHASTIC_EULER) return model == 1 ? 1 : 3;
   return model == 1 ? 2 : 6;
 }
-
-// ------------------------------------------------------------------ device memory
-
-template<class T>
-struct DeviceArray
-{
-  T *ptr = nullptr;
-  size_t count = 0;
-  int reserve(size_t n)
-  {
-    if (n <= count && ptr) return SPSS_OK;
-    release();
-    if (n == 0) n = 1;
-    cudaError_t e = cudaMalloc((void **) &ptr, n * sizeof(T));
-    if (e != cudaSuccess)
-    {
-      ptr = nullptr;
-      count = 0;
-      cudaGetLastError();
-      return SPSS_ERR_OUT_OF_MEMORY;
-    }
-    count = n;
-    return SPSS_OK;
-  }
-  void release()
-  {
-    if (ptr) cudaFree(ptr);
-    ptr = nullptr;
-    count = 0;
-  }
-  size_t bytes() const { return count * sizeof(T); }
-};
 
 // Exclusive prefix sum of `n` int32 counts into offsets[0..n] (offsets[n] =
 // total), three-phase with recursion on the block sums.
