@@ -1,22 +1,25 @@
 // Learned surrogate: the 5 -> 128 -> 128 -> 128 -> 4 GELU network of
 // spss_surrogate.h, trained and evaluated by hand-written tcgen05 kernels.
 //
-// Tensor-core scheme (one CTA = 128 rows of a batch, 4 warps):
+// Tensor-core scheme (one CTA = 128 rows of a batch, 16 warps):
 //   * operands live in shared memory in the K-major, no-swizzle canonical
 //     layout: core matrices of 8 rows x 16 bytes (8 BF16), adjacent along K at
 //     128 bytes (leading byte offset), row groups at K/8 * 128 bytes (stride
-//     byte offset);
+//     byte offset); the weight copies and the input tiles are kept in that
+//     layout in global memory, so a tile or a set of weights is one bulk copy;
 //   * one thread issues tcgen05.mma.cta_group::1.kind::f16 (BF16 x BF16 ->
-//     FP32, M = 128, N = 128 or 16, K = 16 per instruction) into a 128-column
-//     tensor-memory accumulator and commits to an mbarrier (bounded wait);
-//   * after the wait every thread reads its own row of the accumulator with
-//     tcgen05.ld (warp w owns lanes 32w .. 32w + 31), applies bias and GELU in
-//     FP32 and writes the BF16 activation back into shared memory as the next
-//     layer's A operand.
-// Backward: dZ_l = dA_l * GELU'(Z_l) with dA_{l-1} = dZ_l W_l (tensor cores,
-// W_l^T staged as the K-major B operand), and dW_l = dZ_l^T A_{l-1} over
-// 128-row batch chunks (both operands staged transposed, accumulated in tensor
-// memory), reduced over CTAs in a fixed order; Adam on FP32 master weights.
+//     FP32, M = 128, N = 128 or 16, K = 16 per instruction) into tensor memory
+//     and commits to an mbarrier (bounded wait);
+//   * after the wait every thread reads 32 columns of a row of the accumulator
+//     with tcgen05.ld (warp w: lanes 32 (w mod 4) .. + 31, columns 32 (w / 4) ..
+//     + 31), applies bias and GELU in FP32 and writes the BF16 activation into
+//     shared memory as the next layer's A operand.
+// Training: one kernel runs forward, loss, dZ_l = dA_l * GELU'(Z_l) with
+// dA_{l-1} = dZ_l W_l, and dW_l = dZ_l^T A_{l-1} for its 128 rows.  The weight
+// gradients read the same row-major tiles as MN-major operands (a core matrix
+// of 8 rows x 8 columns serves either way; only the strides change names), so
+// nothing is transposed.  Partial gradients are summed over CTAs in a fixed
+// order; Adam on FP32 master weights.
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -68,21 +71,39 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint3
 }
 
 // Instruction descriptor of kind::f16: FP32 accumulator, BF16 A and B, both
-// K-major, N >> 3 and M >> 4.
-__device__ __forceinline__ uint32_t instr_desc(int M, int N)
+// K-major (or, `mn`, both MN-major), N >> 3 and M >> 4.
+__device__ __forceinline__ constexpr uint32_t instr_desc(int M, int N, bool mn = false)
 {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t) (N >> 3) << 17) | ((uint32_t) (M >> 4) << 24);
+  return (1u << 4) | (1u << 7) | (1u << 10) | (mn ? (1u << 15) | (1u << 16) : 0u) | ((uint32_t) (N >> 3) << 17) |
+         ((uint32_t) (M >> 4) << 24);
 }
 
-// D[128 x N] (+)= A[128 x K] B[N x K]^T, both operands K-major in shared memory.
-__device__ __forceinline__ void mma_issue(uint32_t tmem, const void *a, const void *b, int K, int N, bool accumulate)
+// An operand in shared memory: `lbo` and `sbo` of its descriptor, and the bytes
+// from one K = 16 step to the next.  K-major: the tile is [rows of M or N][K
+// columns]; MN-major: the same layout read as [K rows][columns of M or N].
+struct Operand
 {
-  const uint32_t idesc = instr_desc(TR, N);
-  const uint32_t sbo = (uint32_t) (K >> 3) * 128u;
-  for (int kk = 0; kk < K / 16; ++kk)
+  uint32_t addr, lbo, sbo, step;
+};
+
+__device__ __forceinline__ Operand k_major(const void *p, int K)
+{
+  return Operand{smem_addr(p), 128u, (uint32_t) (K >> 3) * 128u, 256u};
+}
+
+__device__ __forceinline__ Operand mn_major(const void *p, int columns)
+{
+  const uint32_t group = (uint32_t) (columns >> 3) * 128u;  // eight rows
+  return Operand{smem_addr(p), group, 128u, 2u * group};
+}
+
+// D[128 x N] (+)= A B, K = 16 * steps.
+__device__ __forceinline__ void mma_issue(uint32_t tmem, Operand a, Operand b, int steps, uint32_t idesc, bool accumulate)
+{
+  for (int kk = 0; kk < steps; ++kk)
   {
-    const uint64_t ad = smem_desc(smem_addr(a) + kk * 256, 128, sbo);
-    const uint64_t bd = smem_desc(smem_addr(b) + kk * 256, 128, sbo);
+    const uint64_t ad = smem_desc(a.addr + kk * a.step, a.lbo, a.sbo);
+    const uint64_t bd = smem_desc(b.addr + kk * b.step, b.lbo, b.sbo);
     const uint32_t acc = (accumulate || kk > 0) ? 1u : 0u;
     asm volatile(
         "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(
@@ -128,7 +149,7 @@ __device__ __forceinline__ void publish_operands()
   fence_after_sync();
 }
 
-// 32 (or 16) consecutive accumulator columns of this thread's row.
+// 32 (16, 8) consecutive accumulator columns of this thread's row.
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float v[32])
 {
   uint32_t r[32];
@@ -158,38 +179,47 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float v[16])
   for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]);
 }
 
-// Tensor memory: 128 columns (FP32 128 x 128 accumulator), one warp.
-__device__ __forceinline__ void tmem_alloc(uint32_t *dst)
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float v[8])
 {
-  asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(dst)), "r"(128));
+  uint32_t r[8];
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr));
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+  for (int j = 0; j < 8; ++j) v[j] = __uint_as_float(r[j]);
+}
+
+// Tensor memory columns (a power of two), by one warp.
+__device__ __forceinline__ void tmem_alloc(uint32_t *dst, uint32_t columns)
+{
+  asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(dst)), "r"(columns));
   asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
 }
 
-__device__ __forceinline__ void tmem_dealloc(uint32_t tmem)
+__device__ __forceinline__ void tmem_dealloc(uint32_t tmem, uint32_t columns)
 {
-  asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(128));
+  asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(columns));
+}
+
+// Bulk copy global -> shared (both 16-byte aligned), completing on the mbarrier.
+__device__ __forceinline__ void bulk_copy(void *dst, const void *src, uint32_t bytes, const unsigned long long *mbar)
+{
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                   smem_addr(dst)),
+               "l"(src), "r"(bytes), "r"(smem_addr(mbar))
+               : "memory");
+}
+
+__device__ __forceinline__ void expect_bytes(const unsigned long long *mbar, uint32_t bytes)
+{
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(mbar)), "r"(bytes) : "memory");
 }
 
 __device__ __forceinline__ void mbar_init(unsigned long long *mbar)
 {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(mbar)));
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-}
-
-// ---------------------------------------------------------------- staging
-
-// rows x K BF16 matrix (row-major, `valid` rows present, the rest zero) into
-// the canonical layout, 16 bytes at a time.
-__device__ __forceinline__ void stage_rows(unsigned char *dst, const bf16 *src, int rows, int valid, int K)
-{
-  const int chunks = rows * (K / 8);
-  for (int c = threadIdx.x; c < chunks; c += blockDim.x)
-  {
-    const int r = c / (K / 8), k = (c - r * (K / 8)) * 8;
-    uint4 v = make_uint4(0u, 0u, 0u, 0u);
-    if (r < valid) v = *reinterpret_cast<const uint4 *>(src + (long) r * K + k);
-    *reinterpret_cast<uint4 *>(dst + canon(r, k, K)) = v;
-  }
 }
 
 // Eight consecutive columns c8 .. c8 + 7 of row r of a K-major operand.
@@ -201,316 +231,394 @@ __device__ __forceinline__ void put8(unsigned char *dst, int r, int c8, int K, c
   *reinterpret_cast<uint4 *>(dst + canon(r, c8, K)) = *reinterpret_cast<const uint4 *>(h);
 }
 
+// GELU (exact, erf form) and its derivative.
 __device__ __forceinline__ float gelu(float x)
 {
   return 0.5f * x * (1.0f + erff(x * 0.70710678118654752f));
 }
 
-__device__ __forceinline__ float gelu_grad(float x)
+__device__ __forceinline__ void gelu_both(float x, float &g, float &dg)
 {
-  return 0.5f * (1.0f + erff(x * 0.70710678118654752f)) + x * 0.39894228040143268f * expf(-0.5f * x * x);
+  const float e = 1.0f + erff(x * 0.70710678118654752f);
+  g = 0.5f * x * e;
+  dg = 0.5f * e + x * 0.39894228040143268f * expf(-0.5f * x * x);
 }
+
+// BF16 weights in the canonical layout: forward B operands W1 [128][16], W2, W3
+// [128][128], W4 [16][128]; backward B operands (transposes) W4t [128][16], W3t,
+// W2t.  Offsets in elements.
+constexpr int kF1 = 0, kF2 = kF1 + H * INP, kF3 = kF2 + H * H, kF4 = kF3 + H * H, kForward = kF4 + OUTP * H;
+constexpr int kB4 = 0, kB3 = kB4 + H * OUTP, kB2 = kB3 + H * H, kBackward = kB2 + H * H;
 
 struct Weights
 {
-  const float *p;                     // FP32 master parameters (flat order)
-  const bf16 *w1, *w2, *w3, *w4;      // forward B operands: [128][16], [128][128], [128][128], [16][128]
-  const bf16 *w4t, *w3t, *w2t;        // backward B operands (transposes): [128][16], [128][128], [128][128]
+  const float *p;        // FP32 master parameters (flat order)
+  const bf16 *fwd, *bwd;
 };
 
-struct Acts
+constexpr int kThreads = 512;
+constexpr int kTileX = TR * INP * 2;  // bytes of an input tile
+constexpr int kTileA = TR * H * 2;    // bytes of an activation tile
+constexpr int kFwdSmem = kTileX + kTileA + kForward * 2;                                   // 108 KiB: two CTAs an SM
+constexpr int kTrainSmem = kTileX + 4 * kTileA + TR * OUTP * 2 + kForward * 2;             // 208 KiB
+
+// Accumulator columns c .. c + 7 of this thread's row plus their biases.
+__device__ __forceinline__ void biased8(uint32_t trow, const float *b, int c, float v[8])
 {
-  bf16 *a[3];   // GELU outputs of the hidden layers, [rows][128]
-  float *z[3];  // pre-activations, [rows][128]
-};
-
-constexpr int kFwdSmem = TR * H * 2 + H * INP * 2 + 2 * H * H * 2 + OUTP * H * 2;   // 104 KiB
-constexpr int kBwdSmem = TR * H * 2 + H * OUTP * 2 + 2 * H * H * 2;                // 100 KiB
-constexpr int kGradSmem = TR * TR * 2 + H * TR * 2;                                 // 64 KiB
+  const float4 b0 = __ldg(reinterpret_cast<const float4 *>(b + c)), b1 = __ldg(reinterpret_cast<const float4 *>(b + c + 4));
+  tmem_ld8(trow + c, v);
+  v[0] += b0.x;
+  v[1] += b0.y;
+  v[2] += b0.z;
+  v[3] += b0.w;
+  v[4] += b1.x;
+  v[5] += b1.y;
+  v[6] += b1.z;
+  v[7] += b1.w;
+}
 
 // ---------------------------------------------------------------- forward
 
-// Rows [128 b, 128 b + 128) of x (BF16 [n][16], inputs zero-padded): output
-// y [n][4] (FP32); with `acts`, the hidden activations and pre-activations.
-__global__ void __launch_bounds__(TR, 1) mlp_forward_kernel(Weights W, const bf16 *__restrict__ x, int n,
-                                                            float *__restrict__ y, Acts acts, int save, int *status)
+// Network outputs y [n][4] of the input tiles x (128 rows of BF16 [16] each, in
+// the canonical layout; rows beyond n zero).  A CTA keeps the weights and takes
+// tiles blockIdx.x, blockIdx.x + gridDim.x, ...  Bound by the GELUs (25 million
+// at 65,536 rows, some 35 instructions each): with one thread a row and the
+// weights staged by the threads for every tile 70 us there, now 37.
+__global__ void __launch_bounds__(kThreads, 2) mlp_forward_kernel(Weights W, const bf16 *__restrict__ x, int n,
+                                                                  float *__restrict__ y, int *status)
 {
   extern __shared__ __align__(128) unsigned char smem[];
-  unsigned char *sA = smem;
-  unsigned char *sW1 = sA + TR * H * 2;
-  unsigned char *sW2 = sW1 + H * INP * 2;
-  unsigned char *sW3 = sW2 + H * H * 2;
-  unsigned char *sW4 = sW3 + H * H * 2;
-  __shared__ __align__(8) unsigned long long mbar;
+  unsigned char *sX = smem;
+  unsigned char *sA = sX + kTileX;
+  const bf16 *sW = reinterpret_cast<const bf16 *>(sA + kTileA);
+  __shared__ __align__(8) unsigned long long mload, mmath;
   __shared__ uint32_t tmem_base;
   const int tid = threadIdx.x, warp = tid >> 5;
-  const int row0 = blockIdx.x * TR;
-  const int valid = min(TR, n - row0);
-  const int row = row0 + tid;
-  stage_rows(sA, x + (long) row0 * INP, TR, valid, INP);
-  stage_rows(sW1, W.w1, H, H, INP);
-  stage_rows(sW2, W.w2, H, H, H);
-  stage_rows(sW3, W.w3, H, H, H);
-  stage_rows(sW4, W.w4, OUTP, OUTP, H);
-  if (warp == 0) tmem_alloc(&tmem_base);
-  if (tid == 0) mbar_init(&mbar);
+  const int tiles = (n + TR - 1) / TR;
+  const int r = 32 * (warp & 3) + (tid & 31), c0 = 32 * (warp >> 2);
+  if (warp == 0) tmem_alloc(&tmem_base, 128);
+  if (tid == 0)
+  {
+    mbar_init(&mload);
+    mbar_init(&mmath);
+    expect_bytes(&mload, kForward * 2 + kTileX);
+    bulk_copy((void *) sW, W.fwd, kForward * 2, &mload);
+    bulk_copy(sX, x + (long) blockIdx.x * TR * INP, kTileX, &mload);
+  }
   publish_operands();
   const uint32_t tmem = tmem_base;
-  const uint32_t trow = tmem + ((uint32_t) (warp * 32) << 16);
-  uint32_t phase = 0;
+  const uint32_t trow = tmem + ((uint32_t) (32 * (warp & 3)) << 16);
+  uint32_t phase = 0, lphase = 0;
   bool ok = true;
-  for (int l = 0; l < 4 && ok; ++l)
+  for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x)
   {
-    const unsigned char *sB = l == 0 ? sW1 : (l == 1 ? sW2 : (l == 2 ? sW3 : sW4));
+    ok = __syncthreads_and(wait_phase(&mload, lphase));
+    if (!ok) break;
+    lphase ^= 1u;
+    for (int l = 0; l < 4 && ok; ++l)
+    {
+      if (tid == 0)
+      {
+        const bf16 *w = sW + (l == 0 ? kF1 : (l == 1 ? kF2 : (l == 2 ? kF3 : kF4)));
+        const int K = l == 0 ? INP : H;
+        mma_issue(tmem, k_major(l == 0 ? sX : sA, K), k_major(w, K), K / 16, instr_desc(TR, l == 3 ? OUTP : H), false);
+        mma_commit(&mmath);
+      }
+      ok = __syncthreads_and(wait_phase(&mmath, phase));
+      if (!ok) break;
+      phase ^= 1u;
+      fence_after_sync();
+      if (l < 3)
+      {
+        if (l == 0 && tid == 0 && tile + (int) gridDim.x < tiles)
+        {
+          // the input tile has been read: fetch the next one
+          expect_bytes(&mload, kTileX);
+          bulk_copy(sX, x + (long) (tile + gridDim.x) * TR * INP, kTileX, &mload);
+        }
+        const float *b = W.p + (l == 0 ? ob1 : (l == 1 ? ob2 : ob3));
+#pragma unroll 1
+        for (int c = c0; c < c0 + 32; c += 8)
+        {
+          float v[8];
+          biased8(trow, b, c, v);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) v[j] = gelu(v[j]);
+          put8(sA, r, c, H, v);
+        }
+        publish_operands();
+      } else
+      {
+        const int row = tile * TR + r;
+        if (warp < 4)
+        {
+          float v[16];
+          tmem_ld16(trow, v);
+          const float *b = W.p + ob4;
+          if (row < n)
+            *reinterpret_cast<float4 *>(y + (long) row * OUT) =
+                make_float4(v[0] + __ldg(b), v[1] + __ldg(b + 1), v[2] + __ldg(b + 2), v[3] + __ldg(b + 3));
+        }
+        fence_before_sync();
+        __syncthreads();  // the accumulator has been read
+        fence_after_sync();
+      }
+    }
+  }
+  if (!ok)
+  {
+    // a copy or an accumulator did not complete in time: report and give what
+    // is in flight a second bounded wait before the memory is released
+    if (tid == 0) atomicOr(status, 1);
+    wait_phase(&mload, lphase);
+    wait_phase(&mmath, phase);
+  }
+  fence_before_sync();
+  __syncthreads();
+  if (warp == 0) tmem_dealloc(tmem, 128);
+}
+
+// ---------------------------------------------------------------- training
+
+struct Partials
+{
+  float *w[4];  // [cta][128][kin] per layer (layer 4: rows 0 .. 3)
+  float *b[4];  // [cta][128]
+};
+
+// Sum over the 128 rows of column m of a tile with K columns, added to `s` in
+// row order.
+__device__ __forceinline__ float add_column(const unsigned char *tile, int m, int K, float s)
+{
+#pragma unroll 16
+  for (int k = 0; k < TR; ++k) s += __bfloat162float(*reinterpret_cast<const bf16 *>(tile + canon(k, m, K)));
+  return s;
+}
+
+// Loss and gradient partials of the rows of tiles blockIdx.x, blockIdx.x +
+// gridDim.x, ... of a batch: forward, dZ4 = 2 w (y - t) / n_batch, dZ3, dZ2, dZ1
+// and the weight gradients, each accumulated in its own tensor-memory columns.
+// `dgelu`: scratch, 3 * 32 * 512 floats a CTA (GELU' of a thread's own
+// elements, written and read back by the same thread).
+// A minibatch of 1,024 rows is eight CTAs, each a chain of eleven MMA-epilogue
+// stages, so latency is all there is: with a kernel each for forward, backward
+// and the four weight gradients, one thread a row and the gradients' operands
+// transposed by 2-byte stores, 69 + 89 + 4 * 16.5 us; this one 34 us.
+__global__ void __launch_bounds__(kThreads, 1) mlp_train_kernel(Weights W, const bf16 *__restrict__ x,
+                                                                const float *__restrict__ t, float4 wl, float scale,
+                                                                int n, float *__restrict__ dgelu, Partials out,
+                                                                float *__restrict__ loss_partial, int *status)
+{
+  extern __shared__ __align__(128) unsigned char smem[];
+  unsigned char *sX = smem;
+  unsigned char *sA1 = sX + kTileX;
+  unsigned char *sA2 = sA1 + kTileA;  // later dZ1
+  unsigned char *sA3 = sA2 + kTileA;  // later dZ2
+  unsigned char *sD = sA3 + kTileA;   // dZ3
+  unsigned char *sZ4 = sD + kTileA;   // dZ4 [128][16]
+  const bf16 *sW = reinterpret_cast<const bf16 *>(sZ4 + TR * OUTP * 2);
+  __shared__ __align__(8) unsigned long long mload, mmath;
+  __shared__ uint32_t tmem_base;
+  __shared__ float red[4];
+  const int tid = threadIdx.x, warp = tid >> 5;
+  const int tiles = (n + TR - 1) / TR;
+  const int r = 32 * (warp & 3) + (tid & 31), c0 = 32 * (warp >> 2);
+  // tensor-memory columns: the chain's accumulator and the weight gradients
+  constexpr uint32_t kChain = 0, kG2 = 128, kG3 = 256, kG4 = 384, kG1 = 416;
+  if (warp == 0) tmem_alloc(&tmem_base, 512);
+  if (tid == 0)
+  {
+    mbar_init(&mload);
+    mbar_init(&mmath);
+  }
+  publish_operands();
+  const uint32_t tmem = tmem_base;
+  const uint32_t trow = tmem + ((uint32_t) (32 * (warp & 3)) << 16);
+  uint32_t phase = 0, lphase = 0;
+  bool ok = true, any = false;
+  float db[4] = {0.f, 0.f, 0.f, 0.f};  // bias gradients of column tid (tid < 128)
+  float *const dg = dgelu + (long) blockIdx.x * 3 * 32 * kThreads + tid;
+  auto done = [&]() -> bool {  // every thread: the committed MMAs are complete
+    const bool all = __syncthreads_and(wait_phase(&mmath, phase));
+    phase ^= all ? 1u : 0u;
+    fence_after_sync();
+    return all;
+  };
+  auto loaded = [&]() -> bool {
+    const bool all = __syncthreads_and(wait_phase(&mload, lphase));
+    lphase ^= all ? 1u : 0u;
+    return all;
+  };
+  for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x)
+  {
+    const int row = tile * TR + r;
+    const bool live = row < n;
     if (tid == 0)
     {
-      mma_issue(tmem, sA, sB, l == 0 ? INP : H, l == 3 ? OUTP : H, false);
-      mma_commit(&mbar);
+      expect_bytes(&mload, kForward * 2 + kTileX);
+      bulk_copy(sX, x + (long) tile * TR * INP, kTileX, &mload);
+      bulk_copy((void *) sW, W.fwd, kForward * 2, &mload);
     }
-    ok = __syncthreads_and(wait_phase(&mbar, phase));
-    if (!ok) break;
-    phase ^= 1u;
-    fence_after_sync();
-    if (l < 3)
+    if (!(ok = loaded())) break;
+    // forward
+    for (int l = 0; l < 3 && ok; ++l)
     {
-      const float *b = W.p + (l == 0 ? ob1 : (l == 1 ? ob2 : ob3));
-      for (int c0 = 0; c0 < H; c0 += 32)
+      unsigned char *in = l == 0 ? sX : (l == 1 ? sA1 : sA2), *to = l == 0 ? sA1 : (l == 1 ? sA2 : sA3);
+      if (tid == 0)
       {
-        float v[32];
-        tmem_ld32(trow + c0, v);
+        const int K = l == 0 ? INP : H;
+        mma_issue(tmem + kChain, k_major(in, K), k_major(sW + (l == 0 ? kF1 : (l == 1 ? kF2 : kF3)), K), K / 16,
+                  instr_desc(TR, H), false);
+        mma_commit(&mmath);
+      }
+      if (!(ok = done())) break;
+      const float *b = W.p + (l == 0 ? ob1 : (l == 1 ? ob2 : ob3));
+#pragma unroll 1
+      for (int c = 0; c < 32; c += 8)
+      {
+        float v[8];
+        biased8(trow + kChain, b, c0 + c, v);
 #pragma unroll
-        for (int j = 0; j < 32; ++j)
+        for (int j = 0; j < 8; ++j)
         {
-          const float z = v[j] + __ldg(b + c0 + j);
-          if (save && tid < valid) acts.z[l][(long) row * H + c0 + j] = z;
-          v[j] = gelu(z);
+          float g, d;
+          gelu_both(v[j], g, d);
+          v[j] = g;
+          dg[(l * 32 + c + j) * kThreads] = d;
         }
-#pragma unroll
-        for (int j = 0; j < 32; j += 8)
-        {
-          put8(sA, tid, c0 + j, H, v + j);
-          if (save && tid < valid)
-          {
-            __nv_bfloat162 h[4];
-            for (int u = 0; u < 4; ++u) h[u] = __floats2bfloat162_rn(v[j + 2 * u], v[j + 2 * u + 1]);
-            *reinterpret_cast<uint4 *>(acts.a[l] + (long) row * H + c0 + j) = *reinterpret_cast<const uint4 *>(h);
-          }
-        }
+        put8(to, r, c0 + c, H, v);
       }
       publish_operands();
-    } else
-    {
-      float v[16];
-      tmem_ld16(trow, v);
-      if (tid < valid)
-        for (int o = 0; o < OUT; ++o) y[(long) row * OUT + o] = v[o] + __ldg(W.p + ob4 + o);
     }
-  }
-  if (!ok)
-  {
-    // the accumulator did not complete in time: report and give the MMAs a
-    // second bounded wait before the tensor memory is released
-    if (tid == 0) atomicOr(status, 1);
-    wait_phase(&mbar, phase);
-  }
-  fence_before_sync();
-  __syncthreads();
-  if (warp == 0) tmem_dealloc(tmem);
-}
-
-// ---------------------------------------------------------------- backward
-
-// Loss gradient dZ4 = 2 w (y - t) / n_batch and the back-propagated dZ3, dZ2,
-// dZ1 (BF16, the operands of the weight gradients); loss partial per CTA.
-__global__ void __launch_bounds__(TR, 1) mlp_backward_kernel(Weights W, const float *__restrict__ y,
-                                                             const float *__restrict__ t, float4 wl, float scale,
-                                                             int n, Acts acts, bf16 *__restrict__ dz4,
-                                                             bf16 *dz3, bf16 *dz2, bf16 *dz1,
-                                                             float *__restrict__ loss_partial, int *status)
-{
-  extern __shared__ __align__(128) unsigned char smem[];
-  unsigned char *sA = smem;
-  unsigned char *sW4t = sA + TR * H * 2;
-  unsigned char *sW3t = sW4t + H * OUTP * 2;
-  unsigned char *sW2t = sW3t + H * H * 2;
-  __shared__ __align__(8) unsigned long long mbar;
-  __shared__ uint32_t tmem_base;
-  __shared__ float red[TR / 32];
-  const int tid = threadIdx.x, warp = tid >> 5;
-  const int row0 = blockIdx.x * TR;
-  const int valid = min(TR, n - row0);
-  const int row = row0 + tid;
-  const bool live = tid < valid;
-  stage_rows(sW4t, W.w4t, H, H, OUTP);
-  stage_rows(sW3t, W.w3t, H, H, H);
-  stage_rows(sW2t, W.w2t, H, H, H);
-  // output layer
-  {
-    const float w4[4] = {wl.x, wl.y, wl.z, wl.w};
-    float g[16], loss = 0.0f;
-#pragma unroll
-    for (int o = 0; o < 16; ++o) g[o] = 0.0f;
-    if (live)
-      for (int o = 0; o < OUT; ++o)
-      {
-        const float d = y[(long) row * OUT + o] - t[(long) row * OUT + o];
-        loss += w4[o] * d * d;
-        g[o] = 2.0f * w4[o] * d * scale;
-      }
-    put8(sA, tid, 0, OUTP, g);
-    put8(sA, tid, 8, OUTP, g + 8);
-    if (live)
-    {
-      __nv_bfloat162 h[8];
-      for (int u = 0; u < 8; ++u) h[u] = __floats2bfloat162_rn(g[2 * u], g[2 * u + 1]);
-      *reinterpret_cast<uint4 *>(dz4 + (long) row * OUTP) = *reinterpret_cast<const uint4 *>(h);
-      *reinterpret_cast<uint4 *>(dz4 + (long) row * OUTP + 8) = *reinterpret_cast<const uint4 *>(h + 4);
-    }
-    for (int off = 16; off > 0; off >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, off);
-    if ((tid & 31) == 0) red[warp] = loss;
-  }
-  if (warp == 0) tmem_alloc(&tmem_base);
-  if (tid == 0) mbar_init(&mbar);
-  publish_operands();
-  if (tid == 0) loss_partial[blockIdx.x] = red[0] + red[1] + red[2] + red[3];
-  const uint32_t tmem = tmem_base;
-  const uint32_t trow = tmem + ((uint32_t) (warp * 32) << 16);
-  uint32_t phase = 0;
-  bool ok = true;
-  // dA_{l} = dZ_{l+1} W_{l+1}, l = 2, 1, 0 (hidden layers 3, 2, 1)
-  for (int l = 2; l >= 0 && ok; --l)
-  {
-    const unsigned char *sB = l == 2 ? sW4t : (l == 1 ? sW3t : sW2t);
-    if (tid == 0)
-    {
-      mma_issue(tmem, sA, sB, l == 2 ? OUTP : H, H, false);
-      mma_commit(&mbar);
-    }
-    ok = __syncthreads_and(wait_phase(&mbar, phase));
     if (!ok) break;
-    phase ^= 1u;
-    fence_after_sync();
-    bf16 *dz = l == 2 ? dz3 : (l == 1 ? dz2 : dz1);
-    for (int c0 = 0; c0 < H; c0 += 32)
-    {
-      float v[32];
-      tmem_ld32(trow + c0, v);
-#pragma unroll
-      for (int j = 0; j < 32; ++j)
-        v[j] = live ? v[j] * gelu_grad(acts.z[l][(long) row * H + c0 + j]) : 0.0f;
-#pragma unroll
-      for (int j = 0; j < 32; j += 8)
-      {
-        put8(sA, tid, c0 + j, H, v + j);
-        if (live)
-        {
-          __nv_bfloat162 h[4];
-          for (int u = 0; u < 4; ++u) h[u] = __floats2bfloat162_rn(v[j + 2 * u], v[j + 2 * u + 1]);
-          *reinterpret_cast<uint4 *>(dz + (long) row * H + c0 + j) = *reinterpret_cast<const uint4 *>(h);
-        }
-      }
-    }
-    publish_operands();
-  }
-  if (!ok)
-  {
-    if (tid == 0) atomicOr(status, 1);
-    wait_phase(&mbar, phase);
-  }
-  fence_before_sync();
-  __syncthreads();
-  if (warp == 0) tmem_dealloc(tmem);
-}
-
-// dW = dZ^T A_prev over 128-row chunks of the batch (CTA c takes chunks c,
-// c + gridDim.x, ...), accumulated in tensor memory: A operand [m = out][k =
-// row] and B operand [n = in][k = row] staged transposed.  dz: [n][zp] (zp
-// outputs, zero rows above), ap: [n][kin].  Partials: pw[cta][128][kin],
-// pb[cta][128].
-__global__ void __launch_bounds__(TR, 1) mlp_weight_grad_kernel(const bf16 *__restrict__ dz, int zp,
-                                                                const bf16 *__restrict__ ap, int kin, int n,
-                                                                float *__restrict__ pw, float *__restrict__ pb,
-                                                                int *status)
-{
-  extern __shared__ __align__(128) unsigned char smem[];
-  unsigned char *sA = smem;               // [128 out][128 rows]
-  unsigned char *sB = sA + TR * TR * 2;   // [kin][128 rows]
-  __shared__ __align__(8) unsigned long long mbar;
-  __shared__ uint32_t tmem_base;
-  const int tid = threadIdx.x, warp = tid >> 5;
-  const int chunks = (n + TR - 1) / TR;
-  // rows of the A operand beyond the layer's outputs stay zero
-  for (int c = tid; c < TR * TR / 8; c += TR)
-  {
-    const int r = c / (TR / 8), k = (c - r * (TR / 8)) * 8;
-    if (r >= zp) *reinterpret_cast<uint4 *>(sA + canon(r, k, TR)) = make_uint4(0u, 0u, 0u, 0u);
-  }
-  if (warp == 0) tmem_alloc(&tmem_base);
-  if (tid == 0) mbar_init(&mbar);
-  fence_before_sync();
-  __syncthreads();
-  fence_after_sync();
-  const uint32_t tmem = tmem_base;
-  uint32_t phase = 0;
-  bool ok = true, any = false;
-  float db = 0.0f;
-  for (int c = blockIdx.x; c < chunks && ok; c += gridDim.x)
-  {
-    // thread = row of the chunk
-    const int r = c * TR + tid;
-    const bool live = r < n;
-    for (int m8 = 0; m8 < zp; m8 += 8)
-    {
-      uint4 raw = make_uint4(0u, 0u, 0u, 0u);
-      if (live) raw = *reinterpret_cast<const uint4 *>(dz + (long) r * zp + m8);
-      const bf16 *h = reinterpret_cast<const bf16 *>(&raw);
-      for (int u = 0; u < 8; ++u) *reinterpret_cast<bf16 *>(sA + canon(m8 + u, tid, TR)) = h[u];
-    }
-    for (int k8 = 0; k8 < kin; k8 += 8)
-    {
-      uint4 raw = make_uint4(0u, 0u, 0u, 0u);
-      if (live) raw = *reinterpret_cast<const uint4 *>(ap + (long) r * kin + k8);
-      const bf16 *h = reinterpret_cast<const bf16 *>(&raw);
-      for (int u = 0; u < 8; ++u) *reinterpret_cast<bf16 *>(sB + canon(k8 + u, tid, TR)) = h[u];
-    }
-    publish_operands();
-    // bias gradient: thread m sums row m of the staged dZ^T
-    if (tid < zp)
-      for (int k = 0; k < TR; ++k) db += __bfloat162float(*reinterpret_cast<const bf16 *>(sA + canon(tid, k, TR)));
+    // output layer and loss
     if (tid == 0)
     {
-      mma_issue(tmem, sA, sB, TR, kin, any);
-      mma_commit(&mbar);
+      mma_issue(tmem + kChain, k_major(sA3, H), k_major(sW + kF4, H), H / 16, instr_desc(TR, OUTP), false);
+      mma_commit(&mmath);
     }
-    ok = __syncthreads_and(wait_phase(&mbar, phase));
-    phase ^= 1u;
-    any = true;
-    fence_after_sync();
-  }
-  const int m = tid;
-  float *out = pw + ((long) blockIdx.x * TR + m) * kin;
-  if (ok && any)
-  {
-    const uint32_t trow = tmem + ((uint32_t) (warp * 32) << 16);
-    for (int c0 = 0; c0 < kin; c0 += 16)
+    if (!(ok = done())) break;
+    if (tid == 0)
     {
-      float v[16];
-      tmem_ld16(trow + c0, v);
-      for (int j = 0; j < 16; ++j) out[c0 + j] = v[j];
+      // the forward weights have been read: the backward ones take their place
+      expect_bytes(&mload, kBackward * 2);
+      bulk_copy((void *) sW, W.bwd, kBackward * 2, &mload);
     }
+    if (warp < 4)
+    {
+      float v[16], g[16], loss = 0.0f;
+      tmem_ld16(trow + kChain, v);
+      const float w4[4] = {wl.x, wl.y, wl.z, wl.w};
+      float4 target = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (live) target = *reinterpret_cast<const float4 *>(t + (long) row * OUT);
+      const float tt[4] = {target.x, target.y, target.z, target.w};
+#pragma unroll
+      for (int o = 0; o < 16; ++o) g[o] = 0.0f;
+      if (live)
+#pragma unroll
+        for (int o = 0; o < OUT; ++o)
+        {
+          const float d = v[o] + __ldg(W.p + ob4 + o) - tt[o];
+          loss += w4[o] * d * d;
+          g[o] = 2.0f * w4[o] * d * scale;
+        }
+      put8(sZ4, r, 0, OUTP, g);
+      put8(sZ4, r, 8, OUTP, g + 8);
+      for (int off = 16; off > 0; off >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, off);
+      if ((tid & 31) == 0) red[warp] = loss;
+    }
+    publish_operands();
+    if (tid == 0) loss_partial[tile] = red[0] + red[1] + red[2] + red[3];
+    if (!(ok = loaded())) break;
+    // dA_l = dZ_{l+1} W_{l+1} for hidden layers 3, 2, 1, each followed by the
+    // weight gradient that its input completes; MMAs run in order, so the wait
+    // for the next chain product also covers that gradient, whose operands may
+    // be overwritten from then on
+    for (int l = 2; l >= 0 && ok; --l)
+    {
+      unsigned char *dz = l == 2 ? sZ4 : (l == 1 ? sD : sA3), *to = l == 2 ? sD : (l == 1 ? sA3 : sA2);
+      if (tid == 0)
+      {
+        const int K = l == 2 ? OUTP : H;
+        mma_issue(tmem + kChain, k_major(dz, K), k_major(sW + (l == 2 ? kB4 : (l == 1 ? kB3 : kB2)), K), K / 16,
+                  instr_desc(TR, H), false);
+        mma_commit(&mmath);
+        if (l == 2)  // dW4^T = A3^T dZ4
+          mma_issue(tmem + kG4, mn_major(sA3, H), mn_major(sZ4, OUTP), TR / 16, instr_desc(TR, OUTP, true), any);
+        else  // dW3 = dZ3^T A2, dW2 = dZ2^T A1
+          mma_issue(tmem + (l == 1 ? kG3 : kG2), mn_major(dz, H), mn_major(l == 1 ? sA2 : sA1, H), TR / 16,
+                    instr_desc(TR, H, true), any);
+      }
+      float d[32], v[32];
+#pragma unroll
+      for (int j = 0; j < 32; ++j) d[j] = dg[(l * 32 + j) * kThreads];
+      if (l == 2)
+      {
+        if (tid < OUTP) db[3] = add_column(sZ4, tid, OUTP, db[3]);
+      } else if (tid < H)
+      {
+        db[l + 1] = add_column(dz, tid, H, db[l + 1]);
+      }
+      if (!(ok = done())) break;
+      tmem_ld32(trow + kChain + c0, v);
+#pragma unroll
+      for (int j = 0; j < 32; ++j) v[j] = live ? v[j] * d[j] : 0.0f;
+#pragma unroll
+      for (int j = 0; j < 32; j += 8) put8(to, r, c0 + j, H, v + j);
+      publish_operands();
+    }
+    if (!ok) break;
+    if (tid == 0)  // dW1 = dZ1^T X
+    {
+      mma_issue(tmem + kG1, mn_major(sA2, H), mn_major(sX, INP), TR / 16, instr_desc(TR, INP, true), any);
+      mma_commit(&mmath);
+    }
+    if (tid < H) db[0] = add_column(sA2, tid, H, db[0]);
+    if (!(ok = done())) break;
+    any = true;
+  }
+  const long cta = blockIdx.x;
+  if (ok)
+  {
+    float v[32], g[16];
+#pragma unroll
+    for (int l = 1; l < 3; ++l)
+    {
+      tmem_ld32(trow + (l == 1 ? kG2 : kG3) + c0, v);
+      float *o = out.w[l] + (cta * TR + r) * H + c0;
+#pragma unroll
+      for (int j = 0; j < 32; j += 4) *reinterpret_cast<float4 *>(o + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+    }
+    if (warp < 4)
+    {
+      tmem_ld16(trow + kG1, g);
+      float *o = out.w[0] + (cta * TR + r) * INP;
+#pragma unroll
+      for (int j = 0; j < 16; j += 4) *reinterpret_cast<float4 *>(o + j) = make_float4(g[j], g[j + 1], g[j + 2], g[j + 3]);
+      tmem_ld16(trow + kG4, g);
+#pragma unroll
+      for (int j = 0; j < OUT; ++j) out.w[3][(cta * TR + j) * H + r] = g[j];
+    }
+    if (tid < H)
+#pragma unroll
+      for (int l = 0; l < 4; ++l) out.b[l][cta * TR + tid] = db[l];
   } else
   {
-    for (int j = 0; j < kin; ++j) out[j] = 0.0f;
-  }
-  pb[(long) blockIdx.x * TR + m] = db;
-  if (!ok)
-  {
+    // report, and give what is in flight a second bounded wait before the
+    // memory is released; the gradient of this batch is zero
     if (tid == 0) atomicOr(status, 1);
-    wait_phase(&mbar, phase ^ 1u);
+    wait_phase(&mload, lphase);
+    wait_phase(&mmath, phase);
+    for (int l = 0; l < 4; ++l)
+    {
+      const int kin = l == 0 ? INP : H;
+      for (int i = tid; i < TR * kin; i += kThreads) out.w[l][cta * TR * kin + i] = 0.0f;
+      if (tid < H) out.b[l][cta * TR + tid] = 0.0f;
+    }
   }
   fence_before_sync();
   __syncthreads();
-  if (warp == 0) tmem_dealloc(tmem);
+  if (warp == 0) tmem_dealloc(tmem, 512);
 }
 
 // ---------------------------------------------------------------- optimiser
@@ -524,7 +632,7 @@ struct Grads
 struct Adam
 {
   float *p, *m1, *m2;
-  bf16 *w1, *w2, *w3, *w4, *w4t, *w3t, *w2t;
+  bf16 *fwd, *bwd;
   float lr, c1, c2;  // learning rate, 1 - beta1^t, 1 - beta2^t
 };
 
@@ -601,35 +709,39 @@ __global__ void mlp_update_kernel(Adam A, Grads G, int update, float *__restrict
   const bf16 h = __float2bfloat16_rn(p);
   switch (layer)
   {
-    case 0: A.w1[m * INP + c] = h; break;
+    case 0: A.fwd[kF1 + canon(m, c, INP) / 2] = h; break;
     case 1:
-      A.w2[m * H + c] = h;
-      A.w2t[c * H + m] = h;
+      A.fwd[kF2 + canon(m, c, H) / 2] = h;
+      A.bwd[kB2 + canon(c, m, H) / 2] = h;
       break;
     case 2:
-      A.w3[m * H + c] = h;
-      A.w3t[c * H + m] = h;
+      A.fwd[kF3 + canon(m, c, H) / 2] = h;
+      A.bwd[kB3 + canon(c, m, H) / 2] = h;
       break;
     default:
-      A.w4[m * H + c] = h;
-      A.w4t[c * OUTP + m] = h;
+      A.fwd[kF4 + canon(m, c, H) / 2] = h;
+      A.bwd[kB4 + canon(c, m, OUTP) / 2] = h;
       break;
   }
 }
 
-// FP32 inputs [n][5] -> BF16 [n][16] (zero padding), optionally gathered
-// through a permutation; targets [n][4] gathered alongside.
+// FP32 inputs [n][5] -> tiles of 128 rows of BF16 [16] in the canonical layout
+// (zero columns, and zero rows up to the end of the last tile), optionally
+// gathered through a permutation; targets [n][4] gathered alongside.
 __global__ void mlp_pack_kernel(const float *__restrict__ x, const float *__restrict__ t, const int *__restrict__ perm,
                                 long n, bf16 *__restrict__ xb, float *__restrict__ tout)
 {
   const long i = (long) blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const long s = perm ? perm[i] : i;
+  if (i >= (n + TR - 1) / TR * TR) return;
   bf16 v[INP];
-  for (int k = 0; k < INP; ++k) v[k] = __float2bfloat16_rn(k < IN ? x[s * IN + k] : 0.0f);
-  *reinterpret_cast<uint4 *>(xb + i * INP) = *reinterpret_cast<const uint4 *>(v);
-  *reinterpret_cast<uint4 *>(xb + i * INP + 8) = *reinterpret_cast<const uint4 *>(v + 8);
-  if (t && tout)
+  const long s = i < n ? (perm ? perm[i] : i) : 0;
+#pragma unroll
+  for (int k = 0; k < INP; ++k) v[k] = __float2bfloat16_rn(k < IN && i < n ? x[s * IN + k] : 0.0f);
+  unsigned char *tile = reinterpret_cast<unsigned char *>(xb) + (i / TR) * kTileX;
+  const int r = (int) (i % TR);
+  *reinterpret_cast<uint4 *>(tile + canon(r, 0, INP)) = *reinterpret_cast<const uint4 *>(v);
+  *reinterpret_cast<uint4 *>(tile + canon(r, 8, INP)) = *reinterpret_cast<const uint4 *>(v + 8);
+  if (t && tout && i < n)
     for (int o = 0; o < OUT; ++o) tout[i * OUT + o] = t[s * OUT + o];
 }
 
@@ -643,17 +755,16 @@ struct spss_mlp
 {
   cudaStream_t stream = nullptr;
   DeviceArray<float> p, m1, m2, grad;
-  DeviceArray<bf16> w1, w2, w3, w4, w4t, w3t, w2t;
+  DeviceArray<bf16> fwd, bwd;
   // resident training set and its shuffled copy
   DeviceArray<float> x_raw, t_raw, t_shuf;
   DeviceArray<bf16> x_shuf;
   DeviceArray<int> perm;
   long n_data = 0;
   // batch workspace
-  DeviceArray<bf16> xb, a[3], dz4, dz[3];
-  DeviceArray<float> xin, tin, y, z[3], pw[4], pb[4], loss_partial;
+  DeviceArray<bf16> xb;
+  DeviceArray<float> xin, tin, y, dgelu, pw[4], pb[4], loss_partial;
   DeviceArray<int> status;
-  long rows_cap = 0;
   long step = 0;
   unsigned long long launches = 0;
 };
@@ -661,33 +772,14 @@ struct spss_mlp
 namespace
 {
 
-int reserve_rows(spss_mlp *m, long rows)
+long padded(long rows)
 {
-  rows = (rows + TR - 1) / TR * TR;
-  if (rows <= m->rows_cap) return SPSS_OK;
-  SPSS_TRY(m->xb.reserve((size_t) rows * INP));
-  SPSS_TRY(m->y.reserve((size_t) rows * OUT));
-  SPSS_TRY(m->tin.reserve((size_t) rows * OUT));
-  SPSS_TRY(m->dz4.reserve((size_t) rows * OUTP));
-  for (int l = 0; l < 3; ++l)
-  {
-    SPSS_TRY(m->a[l].reserve((size_t) rows * H));
-    SPSS_TRY(m->dz[l].reserve((size_t) rows * H));
-    SPSS_TRY(m->z[l].reserve((size_t) rows * H));
-  }
-  SPSS_TRY(m->loss_partial.reserve((size_t) rows / TR));
-  m->rows_cap = rows;
-  return SPSS_OK;
+  return (rows + TR - 1) / TR * TR;
 }
 
 Weights weights(spss_mlp *m)
 {
-  return Weights{m->p.ptr, m->w1.ptr, m->w2.ptr, m->w3.ptr, m->w4.ptr, m->w4t.ptr, m->w3t.ptr, m->w2t.ptr};
-}
-
-Acts acts(spss_mlp *m)
-{
-  return Acts{{m->a[0].ptr, m->a[1].ptr, m->a[2].ptr}, {m->z[0].ptr, m->z[1].ptr, m->z[2].ptr}};
+  return Weights{m->p.ptr, m->fwd.ptr, m->bwd.ptr};
 }
 
 int check_status(spss_mlp *m)
@@ -698,54 +790,42 @@ int check_status(spss_mlp *m)
   return st ? SPSS_ERR_CUDA : SPSS_OK;
 }
 
-int forward_rows(spss_mlp *m, const bf16 *xb, long rows, float *y, int save)
+int forward_rows(spss_mlp *m, const bf16 *xb, long rows, float *y)
 {
-  const int blocks = (int) ((rows + TR - 1) / TR);
-  mlp_forward_kernel<<<blocks, TR, kFwdSmem, m->stream>>>(weights(m), xb, (int) rows, y, acts(m), save,
-                                                          m->status.ptr);
+  const int blocks = (int) std::min<long>(padded(rows) / TR, 2 * 152);
+  mlp_forward_kernel<<<blocks, kThreads, kFwdSmem, m->stream>>>(weights(m), xb, (int) rows, y, m->status.ptr);
   ++m->launches;
   return check_launch("mlp_forward_kernel");
 }
 
-// Gradient of the batch held in xb / tin (rows rows): partials, then the
-// update kernel (with or without an Adam step).
-int backward_rows(spss_mlp *m, long rows, const float w[4], float lr, int update, float *grad_out)
+// Gradient of a batch (input tiles xb, targets tin): partials, then the update
+// kernel (with or without an Adam step); a loss partial per tile.
+int train_rows(spss_mlp *m, const bf16 *xb, const float *tin, long rows, const float w[4], float lr, int update,
+               float *grad_out, float *loss_partial)
 {
-  const int blocks = (int) ((rows + TR - 1) / TR);
+  const int parts = (int) std::min<long>(padded(rows) / TR, kMaxPartials);
   const float4 wl = make_float4(w[0], w[1], w[2], w[3]);
-  mlp_backward_kernel<<<blocks, TR, kBwdSmem, m->stream>>>(weights(m), m->y.ptr, m->tin.ptr, wl,
-                                                           1.0f / (float) rows, (int) rows, acts(m), m->dz4.ptr,
-                                                           m->dz[2].ptr, m->dz[1].ptr, m->dz[0].ptr,
-                                                           m->loss_partial.ptr, m->status.ptr);
-  ++m->launches;
-  SPSS_TRY(check_launch("mlp_backward_kernel"));
-  const int parts = std::min(blocks, kMaxPartials);
+  SPSS_TRY(m->dgelu.reserve((size_t) parts * 3 * 32 * kThreads));
+  Partials out;
   Grads G;
-  // layer l: dZ_l [rows][zp] and its input A_{l-1} [rows][kin]
-  const bf16 *dzs[4] = {m->dz[0].ptr, m->dz[1].ptr, m->dz[2].ptr, m->dz4.ptr};
-  const bf16 *ins[4] = {m->xb.ptr, m->a[0].ptr, m->a[1].ptr, m->a[2].ptr};
   for (int l = 0; l < 4; ++l)
   {
-    const int zp = l == 3 ? OUTP : H, kin = l == 0 ? INP : H;
-    mlp_weight_grad_kernel<<<parts, TR, kGradSmem, m->stream>>>(dzs[l], zp, ins[l], kin, (int) rows, m->pw[l].ptr,
-                                                                m->pb[l].ptr, m->status.ptr);
-    ++m->launches;
-    SPSS_TRY(check_launch("mlp_weight_grad_kernel"));
+    out.w[l] = m->pw[l].ptr;
+    out.b[l] = m->pb[l].ptr;
     G.pw[l] = m->pw[l].ptr;
     G.pb[l] = m->pb[l].ptr;
     G.parts[l] = parts;
   }
+  mlp_train_kernel<<<parts, kThreads, kTrainSmem, m->stream>>>(weights(m), xb, tin, wl, 1.0f / (float) rows, (int) rows,
+                                                               m->dgelu.ptr, out, loss_partial, m->status.ptr);
+  ++m->launches;
+  SPSS_TRY(check_launch("mlp_train_kernel"));
   Adam A;
   A.p = m->p.ptr;
   A.m1 = m->m1.ptr;
   A.m2 = m->m2.ptr;
-  A.w1 = m->w1.ptr;
-  A.w2 = m->w2.ptr;
-  A.w3 = m->w3.ptr;
-  A.w4 = m->w4.ptr;
-  A.w4t = m->w4t.ptr;
-  A.w3t = m->w3t.ptr;
-  A.w2t = m->w2t.ptr;
+  A.fwd = m->fwd.ptr;
+  A.bwd = m->bwd.ptr;
   A.lr = 0.0f;
   A.c1 = A.c2 = 1.0f;
   if (update)
@@ -772,13 +852,8 @@ int refresh_copies(spss_mlp *m)
   Adam A;
   std::memset(&A, 0, sizeof(A));
   A.p = m->p.ptr;
-  A.w1 = m->w1.ptr;
-  A.w2 = m->w2.ptr;
-  A.w3 = m->w3.ptr;
-  A.w4 = m->w4.ptr;
-  A.w4t = m->w4t.ptr;
-  A.w3t = m->w3t.ptr;
-  A.w2t = m->w2t.ptr;
+  A.fwd = m->fwd.ptr;
+  A.bwd = m->bwd.ptr;
   A.c1 = A.c2 = 1.0f;
   mlp_update_kernel<<<(NP + 255) / 256, 256, 0, m->stream>>>(A, G, 0, nullptr);
   return check_launch("mlp_update_kernel");
@@ -786,18 +861,16 @@ int refresh_copies(spss_mlp *m)
 
 int upload_batch(spss_mlp *m, const float *x, const float *t, long n)
 {
-  SPSS_TRY(reserve_rows(m, n));
+  SPSS_TRY(m->xb.reserve((size_t) padded(n) * INP));
   SPSS_TRY(m->xin.reserve((size_t) n * IN));
   SPSS_CUDA_TRY(cudaMemcpyAsync(m->xin.ptr, x, sizeof(float) * n * IN, cudaMemcpyHostToDevice, m->stream));
-  float *traw = nullptr;
   if (t)
   {
-    SPSS_TRY(m->t_raw.reserve((size_t) n * OUT));
-    SPSS_CUDA_TRY(cudaMemcpyAsync(m->t_raw.ptr, t, sizeof(float) * n * OUT, cudaMemcpyHostToDevice, m->stream));
-    traw = m->t_raw.ptr;
+    SPSS_TRY(m->tin.reserve((size_t) n * OUT));
+    SPSS_CUDA_TRY(cudaMemcpyAsync(m->tin.ptr, t, sizeof(float) * n * OUT, cudaMemcpyHostToDevice, m->stream));
   }
-  mlp_pack_kernel<<<(int) ((n + 255) / 256), 256, 0, m->stream>>>(m->xin.ptr, traw, nullptr, n, m->xb.ptr,
-                                                                   t ? m->tin.ptr : nullptr);
+  mlp_pack_kernel<<<(int) ((padded(n) + 255) / 256), 256, 0, m->stream>>>(m->xin.ptr, nullptr, nullptr, n, m->xb.ptr,
+                                                                          nullptr);
   return check_launch("mlp_pack_kernel");
 }
 
@@ -822,9 +895,7 @@ int spss_mlp_create(unsigned long long seed, spss_mlp **out)
     return fail(SPSS_ERR_CUDA);
   }
   if ((rc = m->p.reserve(NP)) || (rc = m->m1.reserve(NP)) || (rc = m->m2.reserve(NP)) || (rc = m->grad.reserve(NP)) ||
-      (rc = m->w1.reserve(H * INP)) || (rc = m->w2.reserve(H * H)) || (rc = m->w3.reserve(H * H)) ||
-      (rc = m->w4.reserve(OUTP * H)) || (rc = m->w4t.reserve(H * OUTP)) || (rc = m->w3t.reserve(H * H)) ||
-      (rc = m->w2t.reserve(H * H)) || (rc = m->status.reserve(1)))
+      (rc = m->fwd.reserve(kForward)) || (rc = m->bwd.reserve(kBackward)) || (rc = m->status.reserve(1)))
     return fail(rc);
   for (int l = 0; l < 4; ++l)
   {
@@ -833,17 +904,14 @@ int spss_mlp_create(unsigned long long seed, spss_mlp **out)
       return fail(rc);
   }
   if (cudaFuncSetAttribute(mlp_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFwdSmem) != cudaSuccess ||
-      cudaFuncSetAttribute(mlp_backward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kBwdSmem) != cudaSuccess ||
-      cudaFuncSetAttribute(mlp_weight_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGradSmem) !=
-          cudaSuccess)
+      cudaFuncSetAttribute(mlp_train_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTrainSmem) != cudaSuccess)
   {
     cudaGetLastError();
     return fail(SPSS_ERR_CUDA);
   }
   // padding of the operand copies stays zero
-  cudaMemsetAsync(m->w1.ptr, 0, sizeof(bf16) * H * INP, m->stream);
-  cudaMemsetAsync(m->w4.ptr, 0, sizeof(bf16) * OUTP * H, m->stream);
-  cudaMemsetAsync(m->w4t.ptr, 0, sizeof(bf16) * H * OUTP, m->stream);
+  cudaMemsetAsync(m->fwd.ptr, 0, sizeof(bf16) * kForward, m->stream);
+  cudaMemsetAsync(m->bwd.ptr, 0, sizeof(bf16) * kBackward, m->stream);
   cudaMemsetAsync(m->m1.ptr, 0, sizeof(float) * NP, m->stream);
   cudaMemsetAsync(m->m2.ptr, 0, sizeof(float) * NP, m->stream);
   cudaMemsetAsync(m->status.ptr, 0, sizeof(int), m->stream);
@@ -875,31 +943,20 @@ int spss_mlp_destroy(spss_mlp *m)
   m->m1.release();
   m->m2.release();
   m->grad.release();
-  m->w1.release();
-  m->w2.release();
-  m->w3.release();
-  m->w4.release();
-  m->w4t.release();
-  m->w3t.release();
-  m->w2t.release();
+  m->fwd.release();
+  m->bwd.release();
   m->x_raw.release();
   m->t_raw.release();
   m->t_shuf.release();
   m->x_shuf.release();
   m->perm.release();
   m->xb.release();
-  m->dz4.release();
   m->xin.release();
   m->tin.release();
   m->y.release();
+  m->dgelu.release();
   m->loss_partial.release();
   m->status.release();
-  for (int l = 0; l < 3; ++l)
-  {
-    m->a[l].release();
-    m->dz[l].release();
-    m->z[l].release();
-  }
   for (int l = 0; l < 4; ++l)
   {
     m->pw[l].release();
@@ -937,8 +994,9 @@ int spss_mlp_forward(spss_mlp *m, const float *x, long n, float *y)
 {
   if (!m || !x || !y || n <= 0) return SPSS_ERR_INVALID_ARGUMENT;
   if (n > 0x7fffff00L) return SPSS_ERR_SIZE;
+  SPSS_TRY(m->y.reserve((size_t) n * OUT));
   SPSS_TRY(upload_batch(m, x, nullptr, n));
-  SPSS_TRY(forward_rows(m, m->xb.ptr, n, m->y.ptr, 0));
+  SPSS_TRY(forward_rows(m, m->xb.ptr, n, m->y.ptr));
   SPSS_CUDA_TRY(cudaMemcpyAsync(y, m->y.ptr, sizeof(float) * n * OUT, cudaMemcpyDeviceToHost, m->stream));
   return check_status(m);
 }
@@ -950,9 +1008,9 @@ int spss_mlp_gradient(spss_mlp *m, const float *x, const float *t, const float *
   const float ones[4] = {1.0f, 1.0f, 1.0f, 1.0f};
   float wl[4];
   std::memcpy(wl, w ? w : ones, 4 * sizeof(float));
+  SPSS_TRY(m->loss_partial.reserve((size_t) padded(n) / TR));
   SPSS_TRY(upload_batch(m, x, t, n));
-  SPSS_TRY(forward_rows(m, m->xb.ptr, n, m->y.ptr, 1));
-  SPSS_TRY(backward_rows(m, n, wl, 0.0f, 0, m->grad.ptr));
+  SPSS_TRY(train_rows(m, m->xb.ptr, m->tin.ptr, n, wl, 0.0f, 0, m->grad.ptr, m->loss_partial.ptr));
   SPSS_CUDA_TRY(cudaMemcpyAsync(grad, m->grad.ptr, sizeof(float) * NP, cudaMemcpyDeviceToHost, m->stream));
   const int blocks = (int) ((n + TR - 1) / TR);
   std::vector<float> lp(blocks);
@@ -974,8 +1032,8 @@ int spss_mlp_set_data(spss_mlp *m, const float *x, const float *t, long n)
   if (n > 0x7fffff00L) return SPSS_ERR_SIZE;
   SPSS_TRY(m->x_raw.reserve((size_t) n * IN));
   SPSS_TRY(m->t_raw.reserve((size_t) n * OUT));
-  SPSS_TRY(m->x_shuf.reserve((size_t) ((n + TR - 1) / TR * TR) * INP));
-  SPSS_TRY(m->t_shuf.reserve((size_t) ((n + TR - 1) / TR * TR) * OUT));
+  SPSS_TRY(m->x_shuf.reserve((size_t) padded(n) * INP));
+  SPSS_TRY(m->t_shuf.reserve((size_t) padded(n) * OUT));
   SPSS_TRY(m->perm.reserve((size_t) n));
   SPSS_CUDA_TRY(cudaMemcpyAsync(m->x_raw.ptr, x, sizeof(float) * n * IN, cudaMemcpyHostToDevice, m->stream));
   SPSS_CUDA_TRY(cudaMemcpyAsync(m->t_raw.ptr, t, sizeof(float) * n * OUT, cudaMemcpyHostToDevice, m->stream));
@@ -990,38 +1048,38 @@ int spss_mlp_train(spss_mlp *m, int epochs, int batch, float lr, const float *w,
   if (!m || epochs < 0 || batch < TR || batch % TR || !(lr > 0.0f)) return SPSS_ERR_INVALID_ARGUMENT;
   if (m->n_data <= 0) return SPSS_ERR_INVALID_ARGUMENT;
   const long n = m->n_data;
-  SPSS_TRY(reserve_rows(m, batch));
   float wl[4] = {1.0f, 1.0f, 1.0f, 1.0f};
   if (w) std::memcpy(wl, w, 4 * sizeof(float));
   std::vector<int> perm((size_t) n);
-  const long nb = (n + batch - 1) / batch;
-  std::vector<float> lp((size_t) nb * (batch / TR));
+  const long nb = (n + batch - 1) / batch, tiles = padded(n) / TR;
+  SPSS_TRY(m->loss_partial.reserve((size_t) tiles));
+  std::vector<float> lp((size_t) tiles);
   for (int e = 0; e < epochs; ++e)
   {
     for (long i = 0; i < n; ++i) perm[i] = (int) i;
     std::mt19937_64 gen(shuffle_seed + (unsigned long long) e);
     std::shuffle(perm.begin(), perm.end(), gen);
     SPSS_CUDA_TRY(cudaMemcpyAsync(m->perm.ptr, perm.data(), sizeof(int) * n, cudaMemcpyHostToDevice, m->stream));
-    mlp_pack_kernel<<<(int) ((n + 255) / 256), 256, 0, m->stream>>>(m->x_raw.ptr, m->t_raw.ptr, m->perm.ptr, n,
-                                                                     m->x_shuf.ptr, m->t_shuf.ptr);
+    mlp_pack_kernel<<<(int) ((padded(n) + 255) / 256), 256, 0, m->stream>>>(m->x_raw.ptr, m->t_raw.ptr, m->perm.ptr, n,
+                                                                            m->x_shuf.ptr, m->t_shuf.ptr);
     SPSS_TRY(check_launch("mlp_pack_kernel"));
+    // the minibatches are runs of whole tiles of the shuffled set, read in
+    // place; their losses are read once, after the epoch
+    for (long b = 0; b < nb; ++b)
+    {
+      const long r0 = b * batch, rows = std::min<long>(batch, n - r0);
+      SPSS_TRY(train_rows(m, m->x_shuf.ptr + r0 * INP, m->t_shuf.ptr + r0 * OUT, rows, wl, lr, 1, nullptr,
+                          m->loss_partial.ptr + r0 / TR));
+    }
+    SPSS_CUDA_TRY(cudaMemcpyAsync(lp.data(), m->loss_partial.ptr, sizeof(float) * tiles, cudaMemcpyDeviceToHost,
+                                  m->stream));
+    SPSS_CUDA_TRY(cudaStreamSynchronize(m->stream));
     double epoch_loss = 0.0;
     for (long b = 0; b < nb; ++b)
     {
       const long r0 = b * batch, rows = std::min<long>(batch, n - r0);
-      // the batch views the shuffled set in place
-      SPSS_CUDA_TRY(cudaMemcpyAsync(m->xb.ptr, m->x_shuf.ptr + r0 * INP, sizeof(bf16) * rows * INP,
-                                    cudaMemcpyDeviceToDevice, m->stream));
-      SPSS_CUDA_TRY(cudaMemcpyAsync(m->tin.ptr, m->t_shuf.ptr + r0 * OUT, sizeof(float) * rows * OUT,
-                                    cudaMemcpyDeviceToDevice, m->stream));
-      SPSS_TRY(forward_rows(m, m->xb.ptr, rows, m->y.ptr, 1));
-      SPSS_TRY(backward_rows(m, rows, wl, lr, 1, nullptr));
-      const int blocks = (int) ((rows + TR - 1) / TR);
-      SPSS_CUDA_TRY(cudaMemcpyAsync(lp.data() + b * (batch / TR), m->loss_partial.ptr, sizeof(float) * blocks,
-                                    cudaMemcpyDeviceToHost, m->stream));
-      SPSS_CUDA_TRY(cudaStreamSynchronize(m->stream));
       double s = 0.0;
-      for (int q = 0; q < blocks; ++q) s += lp[b * (batch / TR) + q];
+      for (long q = r0 / TR; q < (r0 + rows + TR - 1) / TR; ++q) s += lp[q];
       epoch_loss += s / (double) rows;
     }
     if (loss_per_epoch) loss_per_epoch[e] = (float) (epoch_loss / (double) nb);
