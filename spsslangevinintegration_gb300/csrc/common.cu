@@ -61,77 +61,151 @@ int make_f64_tables(DeviceArray<double2> &table, cudaStream_t stream)
 // ------------------------------------------------------------------ scan
 
 constexpr int kScanThreads = 256;
-constexpr int kScanItems = 4;
+constexpr int kScanItems = 16;
 constexpr int kScanTile = kScanThreads * kScanItems;
+// Up to this many tiles every tile adds the sums before its own (its share of
+// at most 32 KiB of L2 reads); beyond it the sums are scanned first.
+constexpr int kScanDirect = 8192;
 
-// Exclusive scan of one tile per block; block totals to `sums`.  When the
-// whole input fits one tile the total is also written to out[n].
-__global__ void scan_tile_kernel(const int *__restrict__ in, int *__restrict__ out, int *__restrict__ sums, int n)
+__device__ __forceinline__ int block_sum(int v, int *warp_tot)
+{
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+  if ((threadIdx.x & 31) == 0) warp_tot[threadIdx.x >> 5] = v;
+  __syncthreads();
+  int t = 0;
+#pragma unroll
+  for (int w = 0; w < kScanThreads / 32; ++w) t += warp_tot[w];
+  __syncthreads();
+  return t;
+}
+
+__device__ __forceinline__ void load_items(const int *__restrict__ in, int base, int n, int v[kScanItems])
+{
+  if (base + kScanItems <= n)
+  {
+#pragma unroll
+    for (int q = 0; q < kScanItems; q += 4) *reinterpret_cast<int4 *>(v + q) = *reinterpret_cast<const int4 *>(in + base + q);
+    return;
+  }
+#pragma unroll
+  for (int q = 0; q < kScanItems; ++q) v[q] = base + q < n ? in[base + q] : 0;
+}
+
+__global__ void __launch_bounds__(kScanThreads) scan_sums_kernel(const int *__restrict__ in, int *__restrict__ sums, int n)
+{
+  __shared__ int warp_tot[kScanThreads / 32];
+  int v[kScanItems], local = 0;
+  load_items(in, blockIdx.x * kScanTile + threadIdx.x * kScanItems, n, v);
+#pragma unroll
+  for (int q = 0; q < kScanItems; ++q) local += v[q];
+  const int t = block_sum(local, warp_tot);
+  if (threadIdx.x == 0) sums[blockIdx.x] = t;
+}
+
+// A cell-list step begins: its re-sort exchanges the vel/pid buffers, its
+// update takes the noise of the step counted here (step - 1), and the next
+// step's cell ids and counts come from it.  What a control kernel after the
+// step would do, without the launch; nothing else in the launch reads these.
+__device__ __forceinline__ void begin_cell_step(FastControl *c)
+{
+  c->step += 1;
+  c->order_parity ^= 1;
+  c->rebuilds += 1;
+  c->cells_fresh = 1;
+  c->rebuild = 1;
+  c->triggered = 1;
+}
+
+// Exclusive scan of one tile per block, after the sum of the tiles before it:
+// `sums` of the tiles (`scanned`: their exclusive prefix), null for one tile.
+__global__ void __launch_bounds__(kScanThreads) scan_tile_kernel(int *__restrict__ in, int *__restrict__ out,
+                                                                 const int *__restrict__ sums, int n, int scanned,
+                                                                 int zero, FastControl *ctrl)
 {
   __shared__ int warp_tot[kScanThreads / 32];
   pdl_enter();
+  if (ctrl && blockIdx.x == 0 && threadIdx.x == 0) begin_cell_step(ctrl);
   const int base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
   int v[kScanItems];
+  load_items(in, base, n, v);
+  int before = 0;
+  if (sums)
+  {
+    if (scanned)
+    {
+      before = sums[blockIdx.x];
+    } else
+    {
+      for (int k = threadIdx.x; k < (int) blockIdx.x; k += kScanThreads) before += sums[k];
+      before = block_sum(before, warp_tot);
+    }
+  }
   int local = 0;
 #pragma unroll
-  for (int q = 0; q < kScanItems; ++q)
-  {
-    v[q] = (base + q < n) ? in[base + q] : 0;
-    local += v[q];
-  }
+  for (int q = 0; q < kScanItems; ++q) local += v[q];
   // inclusive scan of the per-thread totals across the block
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   int x = local;
 #pragma unroll
   for (int off = 1; off < 32; off <<= 1)
   {
-    int y = __shfl_up_sync(0xffffffffu, x, off);
+    const int y = __shfl_up_sync(0xffffffffu, x, off);
     if (lane >= off) x += y;
   }
   if (lane == 31) warp_tot[warp] = x;
   __syncthreads();
-  if (warp == 0)
-  {
-    int w = (lane < kScanThreads / 32) ? warp_tot[lane] : 0;
+  int excl = before + x - local;
 #pragma unroll
-    for (int off = 1; off < 32; off <<= 1)
-    {
-      int y = __shfl_up_sync(0xffffffffu, w, off);
-      if (lane >= off) w += y;
-    }
-    if (lane < kScanThreads / 32) warp_tot[lane] = w;
-  }
-  __syncthreads();
-  int excl = x - local + (warp > 0 ? warp_tot[warp - 1] : 0);
+  for (int w = 0; w < kScanThreads / 32; ++w) excl += w < warp ? warp_tot[w] : 0;
+  int o[kScanItems];
 #pragma unroll
   for (int q = 0; q < kScanItems; ++q)
   {
-    if (base + q < n) out[base + q] = excl;
+    o[q] = excl;
     excl += v[q];
   }
-  if (threadIdx.x == kScanThreads - 1)
+  if (base + kScanItems <= n)
   {
-    const int total = warp_tot[kScanThreads / 32 - 1];
-    if (sums) sums[blockIdx.x] = total;
-    if (gridDim.x == 1) out[n] = total;
+#pragma unroll
+    for (int q = 0; q < kScanItems; q += 4)
+    {
+      *reinterpret_cast<int4 *>(out + base + q) = *reinterpret_cast<const int4 *>(o + q);
+      if (zero) *reinterpret_cast<int4 *>(in + base + q) = make_int4(0, 0, 0, 0);
+    }
+  } else
+  {
+#pragma unroll
+    for (int q = 0; q < kScanItems; ++q)
+      if (base + q < n)
+      {
+        out[base + q] = o[q];
+        if (zero) in[base + q] = 0;
+      }
   }
+  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == kScanThreads - 1) out[n] = excl;
 }
 
-__global__ void scan_add_kernel(int *__restrict__ out, const int *__restrict__ block_off, int n, int nblocks)
+int Scanner::run(int *in, int *out, int n, cudaStream_t stream, unsigned long long &launches, bool chained, bool zero,
+                 FastControl *ctrl)
 {
-  pdl_enter();
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) out[i] += block_off[i / kScanTile];
-  if (i == 0) out[n] = block_off[nblocks];
+  return run_level(in, out, n, 0, stream, launches, chained, zero, ctrl);
 }
 
-int Scanner::run(const int *in, int *out, int n, cudaStream_t stream, unsigned long long &launches, bool chained)
+int Scanner::prepare(int n)
 {
-  return run_level(in, out, n, 0, stream, launches, chained);
+  for (size_t level = 0; n > kScanTile; ++level)
+  {
+    n = (n + kScanTile - 1) / kScanTile;
+    if (levels.size() < 2 * (level + 1)) levels.resize(2 * (level + 1));
+    SPSS_TRY(levels[2 * level].reserve(n));
+    SPSS_TRY(levels[2 * level + 1].reserve(n + 1));
+  }
+  return SPSS_OK;
 }
 
-int Scanner::run_level(const int *in, int *out, int n, size_t level, cudaStream_t stream,
-                       unsigned long long &launches, bool chained)
+int Scanner::run_level(int *in, int *out, int n, size_t level, cudaStream_t stream, unsigned long long &launches,
+                       bool chained, bool zero, FastControl *ctrl)
 {
   if (n <= 0)
   {
@@ -139,25 +213,30 @@ int Scanner::run_level(const int *in, int *out, int n, size_t level, cudaStream_
     return SPSS_OK;
   }
   const int nblocks = (n + kScanTile - 1) / kScanTile;
-  if (nblocks == 1)
+  const int *sums = nullptr;
+  int scanned = 0;
+  if (nblocks > 1)
   {
-    SPSS_CUDA_TRY(launch_chained(chained, scan_tile_kernel, 1, kScanThreads, 0, stream, in, out, (int *) nullptr, n));
+    if (levels.size() < 2 * (level + 1)) levels.resize(2 * (level + 1));
+    SPSS_TRY(levels[2 * level].reserve(nblocks));
+    SPSS_TRY(levels[2 * level + 1].reserve(nblocks + 1));
+    int *s = levels[2 * level].ptr, *off = levels[2 * level + 1].ptr;  // device pointers stay valid if `levels` grows
+    scan_sums_kernel<<<nblocks, kScanThreads, 0, stream>>>(in, s, n);
     ++launches;
-    return check_launch("scan_tile_kernel");
+    SPSS_TRY(check_launch("scan_sums_kernel"));
+    sums = s;
+    if (nblocks > kScanDirect)
+    {
+      SPSS_TRY(run_level(s, off, nblocks, level + 1, stream, launches, chained, false, nullptr));
+      sums = off;
+      scanned = 1;
+    }
   }
-  if (levels.size() < 2 * (level + 1)) levels.resize(2 * (level + 1));
-  SPSS_TRY(levels[2 * level].reserve(nblocks));
-  SPSS_TRY(levels[2 * level + 1].reserve(nblocks + 1));
-  int *sums = levels[2 * level].ptr;       // device pointers stay valid if `levels` grows
-  int *sums_off = levels[2 * level + 1].ptr;
-  SPSS_CUDA_TRY(launch_chained(chained, scan_tile_kernel, nblocks, kScanThreads, 0, stream, in, out, sums, n));
+  // the first launch of a chain is an ordinary one
+  SPSS_CUDA_TRY(launch_chained(chained && nblocks > 1, scan_tile_kernel, nblocks, kScanThreads, 0, stream, in, out, sums, n, scanned,
+                               (int) zero, ctrl));
   ++launches;
-  SPSS_TRY(check_launch("scan_tile_kernel"));
-  SPSS_TRY(run_level(sums, sums_off, nblocks, level + 1, stream, launches, chained));
-  SPSS_CUDA_TRY(launch_chained(chained, scan_add_kernel, (n + 255) / 256, 256, 0, stream, out,
-                               (const int *) sums_off, n, nblocks));
-  ++launches;
-  return check_launch("scan_add_kernel");
+  return check_launch("scan_tile_kernel");
 }
 
 // ------------------------------------------------------------------ binning
@@ -224,27 +303,40 @@ __global__ void bin_sort_kernel(const int *__restrict__ offsets, int ncell, int 
   }
 }
 
-int Binner::run(const int *cell_of, int n, int ncell_in, cudaStream_t stream, unsigned long long &launches,
-                bool chained)
+int Binner::prepare(int n, int ncell_in, cudaStream_t stream)
 {
   ncell = ncell_in;
+  const int *had = count.ptr;
+  const size_t held = count.count;
   SPSS_TRY(count.reserve(ncell));
   SPSS_TRY(offsets.reserve(ncell + 1));
   SPSS_TRY(slot.reserve(n));
   SPSS_TRY(members.reserve(n));
-  SPSS_CUDA_TRY(cudaMemsetAsync(count.ptr, 0, sizeof(int) * ncell, stream));
+  SPSS_TRY(scanner.prepare(ncell));  // nothing is allocated while a step is captured
+  if (count.ptr != had || count.count != held) SPSS_CUDA_TRY(cudaMemsetAsync(count.ptr, 0, sizeof(int) * count.count, stream));
+  return SPSS_OK;
+}
+
+int Binner::place(const int *cell_of, int n, cudaStream_t stream, unsigned long long &launches, bool chained,
+                  FastControl *ctrl)
+{
   const int tb = 256;
-  // the count follows a memset: an ordinary launch
-  bin_count_kernel<<<(n + tb - 1) / tb, tb, 0, stream>>>(cell_of, n, count.ptr, slot.ptr);
-  ++launches;
-  SPSS_TRY(check_launch("bin_count_kernel"));
-  SPSS_TRY(scanner.run(count.ptr, offsets.ptr, ncell, stream, launches, chained));
+  SPSS_TRY(scanner.run(count.ptr, offsets.ptr, ncell, stream, launches, chained, true, ctrl));
   SPSS_CUDA_TRY(launch_chained(chained, bin_scatter_kernel, (n + tb - 1) / tb, tb, 0, stream, cell_of,
                                (const int *) slot.ptr, (const int *) offsets.ptr, n, members.ptr));
   ++launches;
-  SPSS_TRY(check_launch("bin_scatter_kernel"));
-  SPSS_CUDA_TRY(launch_chained(chained, bin_sort_kernel, (ncell + tb - 1) / tb, tb, 0, stream,
-                               (const int *) offsets.ptr, ncell, members.ptr));
+  return check_launch("bin_scatter_kernel");
+}
+
+int Binner::run(const int *cell_of, int n, int ncell_in, cudaStream_t stream, unsigned long long &launches)
+{
+  SPSS_TRY(prepare(n, ncell_in, stream));
+  const int tb = 256;
+  bin_count_kernel<<<(n + tb - 1) / tb, tb, 0, stream>>>(cell_of, n, count.ptr, slot.ptr);
+  ++launches;
+  SPSS_TRY(check_launch("bin_count_kernel"));
+  SPSS_TRY(place(cell_of, n, stream, launches));
+  bin_sort_kernel<<<(ncell + tb - 1) / tb, tb, 0, stream>>>(offsets.ptr, ncell, members.ptr);
   ++launches;
   return check_launch("bin_sort_kernel");
 }

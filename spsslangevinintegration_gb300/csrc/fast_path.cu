@@ -42,26 +42,6 @@ namespace spss
 
 constexpr int kTB = 256;
 
-struct FastControl
-{
-  unsigned long long step;  // Philox step counter of the next stochastic step
-  double acc;               // accumulated displacement of system 0 (FP64)
-  int parity;               // current rec/aux buffer
-  int rebuild;              // lists (and slot order) rebuilt before the next evaluation
-  int cells_fresh;          // cell ids of the current slots were written by the last cell-list step
-  int overflow;             // largest Verlet count seen beyond capacity (0: none)
-  int rebuilds;             // number of rebuilds performed
-  int error;                // bit 0: displacement too large for the fixed-point increment; bit 1: staging
-                            // timeout; bit 2: stencil cell outside the staged segments; bit 3: the
-                            // device launch of the rebuild graph was refused
-  int uses_verlet;
-  int tile_next;            // work counter of the persistent tile kernel
-  unsigned ticket;          // blocks of the running reduction that are done (its last block puts it back to 0)
-  int triggered;            // the last step's displacement trigger fired (its rebuild may already be done)
-  long long sample_every;   // order-parameter samples after steps that are multiples of this (0: none)
-  long long sample_from;    // ... and not before this step
-};
-
 // Per-system Verlet trigger state (CalculateMaxDisplacement of each system).
 struct SysControl
 {
@@ -122,13 +102,15 @@ struct FastBuffers
 {
   uint4 *rec0, *rec1;
   uint4 *aux0, *aux1;
-  float2 *vel, *vel_tmp;
+  float2 *vel, *vel_tmp;  // the current buffer and the other one (buffers_now)
   unsigned *pid, *pid_tmp, *inv;
   int2 *img;   // box crossings, by original index
   int *turns;  // 2 pi turns of the phase, by original index
   int *cell_of, *cell_sorted;
   const int *cell_off;
-  const int *order;
+  const int *order;            // slots in cell order, arrival order inside a cell
+  int *cell_count, *cell_slot; // counts of the next binning, and each slot's arrival number
+  const struct CellTile *cell_tiles;
   short *vl;
   int *vl_cnt;
   float *nu;             // natural frequencies (global field), slot = original index
@@ -139,9 +121,30 @@ struct FastBuffers
   const int *tile_sys;   // system of each tile
   SysControl *sysctl;
   int *tile_maxcnt;  // longest list of each tile (rows to stage)
-  void *tiles;       // TileLayout of every tile, written at rebuild
+  void *tiles;       // TileLayout of every tile (Verlet lists), written at rebuild
   FastControl *ctrl;
 };
+
+// A tile of a cell-list step: rows row0 .. row0 + nrows - 1 and columns col0 ..
+// col0 + ncols - 1 of a system's grid (nc x nc cells from cell0 on); fixed with
+// the tiling, so a step needs only the cell offsets to lay its tiles out.
+struct __align__(16) CellTile
+{
+  int sys, row0, nrows, col0;
+  int ncols, nc, cell0, pad;
+};
+
+// The kernel's view of the buffers with vel and pid the current ones.
+__device__ __forceinline__ void buffers_now(FastBuffers &B, int order_parity)
+{
+  if (!order_parity) return;
+  float2 *v = B.vel;
+  B.vel = B.vel_tmp;
+  B.vel_tmp = v;
+  unsigned *p = B.pid;
+  B.pid = B.pid_tmp;
+  B.pid_tmp = p;
+}
 
 // How a step graph does the list rebuild: under a conditional node at the
 // start of the step (GRAPH_CONDITIONAL), tail-launched as a device graph by the
@@ -161,8 +164,8 @@ enum
 struct Snapshot
 {
   DeviceArray<uint4> rec[2], aux[2];
-  DeviceArray<float2> vel;
-  DeviceArray<unsigned> pid, inv;
+  DeviceArray<float2> vel[2];
+  DeviceArray<unsigned> pid[2], inv;
   DeviceArray<int2> img;
   DeviceArray<int> turns;
   DeviceArray<SysControl> sysctl;
@@ -173,9 +176,9 @@ struct Snapshot
     {
       rec[b].release();
       aux[b].release();
+      vel[b].release();
+      pid[b].release();
     }
-    vel.release();
-    pid.release();
     inv.release();
     img.release();
     turns.release();
@@ -221,6 +224,7 @@ struct FastPath
   DeviceArray<int> turns, cell_of, cell_sorted, vl_cnt, tile_maxcnt;
   DeviceArray<short> vl;
   DeviceArray<unsigned char> tiles;
+  DeviceArray<CellTile> cell_tiles;
   DeviceArray<SysParams> sys;
   DeviceArray<int> sys_of, tile_sys;
   DeviceArray<SysControl> sysctl;
@@ -252,9 +256,6 @@ struct FastPath
   bool perm_valid = false;
   std::map<std::tuple<int, double, int>, GraphEntry> graphs;  // (stepper, dt, with sampling)
   bool device_rebuild = true;  // rebuilds tail-launched as device graphs (cleared if this device refuses)
-  // set while a cell-list step graph is captured: its kernels after the first
-  // are launched as a programmatic-dependent chain (each begins with pdl_enter)
-  bool chain = false;
   // per-system order parameters and their time averages
   DeviceArray<OrderSums> order_partial;
   DeviceArray<int2> order_items;   // (system, first slot) of every chunk, systems in order
@@ -523,6 +524,7 @@ __global__ void fast_upload_kernel(const double *__restrict__ x, int n, int s, i
   const int p = p0 + threadIdx.x;
   if (p >= n) return;
   const int par = B.ctrl->parity;
+  buffers_now(B, B.ctrl->order_parity);
   unsigned q = (unsigned) p;
   if (perm_valid)
   {
@@ -569,6 +571,7 @@ __global__ void fast_download_kernel(double *__restrict__ x, int n, int s, int m
   if (p < n)
   {
     const int par = B.ctrl->parity;
+    buffers_now(B, B.ctrl->order_parity);
     const unsigned q = B.inv[p];
     const uint4 r = (par ? B.rec1 : B.rec0)[q];
     const uint4 a = (par ? B.aux1 : B.aux0)[q];
@@ -606,6 +609,7 @@ __global__ void __launch_bounds__(256) fast_frame_kernel(float *__restrict__ out
   if (p < n)
   {
     const int par = B.ctrl->parity;
+    buffers_now(B, B.ctrl->order_parity);
     const unsigned q = B.inv[p];
     const uint4 r = (par ? B.rec1 : B.rec0)[q];
     const uint4 a = (par ? B.aux1 : B.aux0)[q];
@@ -648,69 +652,83 @@ __device__ __forceinline__ bool rebuilds_system(const FastBuffers &B, int sys)
   return B.ctrl->rebuild != REBUILD_FLAGGED || B.sysctl[sys].rebuild;
 }
 
+// Cell id of every slot, and its arrival number in the cell (the binning's
+// count, in the same pass).
 __global__ void fast_cells_kernel(FastParams P, FastBuffers B)
 {
-  pdl_enter();
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= P.n || B.ctrl->cells_fresh) return;  // the last step wrote every slot's cell id
+  if (q >= P.n) return;
+  int c;
   if (!rebuilds_system(B, B.sys_of[q]))
   {
     // sorted by cell since its last rebuild: the stable counting sort leaves it in place
-    B.cell_of[q] = B.cell_sorted[q];
-    return;
+    c = B.cell_sorted[q];
+  } else
+  {
+    const int par = B.ctrl->parity;
+    const uint4 r = (par ? B.rec1 : B.rec0)[q];
+    const uint4 a = (par ? B.aux1 : B.aux0)[q];
+    const SysParams *S = B.sys + B.sys_of[q];
+    c = S->cell0 + cell_of_fix(join64(r.x, a.x), join64(r.y, a.y), S->nc);
   }
-  const int par = B.ctrl->parity;
-  const uint4 r = (par ? B.rec1 : B.rec0)[q];
-  const uint4 a = (par ? B.aux1 : B.aux0)[q];
-  const SysParams *S = B.sys + B.sys_of[q];
-  B.cell_of[q] = S->cell0 + cell_of_fix(join64(r.x, a.x), join64(r.y, a.y), S->nc);
+  B.cell_of[q] = c;
+  B.cell_slot[q] = atomicAdd(B.cell_count + c, 1);
 }
 
-// New slot q takes the particle of old slot order[q] (cells contiguous,
-// ascending old slot inside a cell).  Writes the other rec/aux buffer.
+// The slots in cell order: the particle at place m of the binning's members
+// (arrival order inside its cell) moves to the place its old slot has among the
+// cell's, ascending: a rank among a handful of members, so the members need
+// no sorting pass of their own.  Writes the other rec/aux and vel/pid buffers.
+// STEP: part of a cell-list step, whose scan already exchanged vel and pid.
+template<bool STEP>
 __global__ void fast_permute_kernel(FastParams P, FastBuffers B)
 {
   pdl_enter();
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= P.n) return;
-  if (!rebuilds_system(B, B.sys_of[q])) return;  // its order is the identity
+  const int m = blockIdx.x * blockDim.x + threadIdx.x;
+  if (m >= P.n) return;
+  if (!STEP && !rebuilds_system(B, B.sys_of[m])) return;  // its order is the identity
   const int par = B.ctrl->parity;
-  const int src = B.order[q];
+  buffers_now(B, B.ctrl->order_parity ^ (STEP ? 1 : 0));
+  const int src = B.order[m];
+  const int c = B.cell_of[src];
+  const int b = B.cell_off[c], e = B.cell_off[c + 1];
+  int q = b;
+  for (int k = b; k < e; ++k) q += B.order[k] < src;
   (par ? B.rec0 : B.rec1)[q] = (par ? B.rec1 : B.rec0)[src];
   (par ? B.aux0 : B.aux1)[q] = (par ? B.aux1 : B.aux0)[src];
   const unsigned p = B.pid[src];
   B.pid_tmp[q] = p;
   B.inv[p] = (unsigned) q;
   if (P.model == 2) B.vel_tmp[q] = B.vel[src];
-  B.cell_sorted[q] = B.cell_of[src];
+  B.cell_sorted[q] = c;
 }
 
-// A rebuild of every system leaves the permuted records in the other buffer
-// (the parity flips); a rebuild of the flagged systems copies theirs back, so
-// the systems left out keep their records where they are.
+// A rebuild of every system leaves the permuted particles in the other buffers
+// (their parities flip); a rebuild of the flagged systems copies theirs back, so
+// the systems left out keep theirs where they are.
 __global__ void fast_copyback_kernel(FastParams P, FastBuffers B)
 {
-  pdl_enter();
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= P.n) return;
+  if (q >= P.n || B.ctrl->rebuild != REBUILD_FLAGGED) return;
   if (!rebuilds_system(B, B.sys_of[q])) return;
-  if (B.ctrl->rebuild == REBUILD_FLAGGED)
-  {
-    const int par = B.ctrl->parity;
-    (par ? B.rec1 : B.rec0)[q] = (par ? B.rec0 : B.rec1)[q];
-    (par ? B.aux1 : B.aux0)[q] = (par ? B.aux0 : B.aux1)[q];
-  }
+  const int par = B.ctrl->parity;
+  buffers_now(B, B.ctrl->order_parity);
+  (par ? B.rec1 : B.rec0)[q] = (par ? B.rec0 : B.rec1)[q];
+  (par ? B.aux1 : B.aux0)[q] = (par ? B.aux0 : B.aux1)[q];
   B.pid[q] = B.pid_tmp[q];
   if (P.model == 2) B.vel[q] = B.vel_tmp[q];
 }
 
-// The permuted records are current: a rebuild of every system flips the
-// buffer parity (the flagged-system form copied its records back).  One
+// The permuted particles are current: a rebuild of every system flips the
+// buffer parities (the flagged-system form copied its particles back).  One
 // thread; runs before the tile layouts and list builds, which read them.
 __global__ void fast_after_permute_kernel(FastControl *ctrl, int permuted)
 {
-  pdl_enter();
-  if (permuted && ctrl->rebuild != REBUILD_FLAGGED) ctrl->parity ^= 1;
+  if (permuted && ctrl->rebuild != REBUILD_FLAGGED)
+  {
+    ctrl->parity ^= 1;
+    ctrl->order_parity ^= 1;
+  }
   ctrl->cells_fresh = 0;  // the slots moved
 }
 
@@ -720,7 +738,6 @@ __global__ void fast_after_permute_kernel(FastControl *ctrl, int permuted)
 // rebuilt at each flagged rebuild).  One block.
 __global__ void fast_after_rebuild_kernel(FastControl *ctrl, SysControl *sysctl, int nsys)
 {
-  pdl_enter();
   for (int r = threadIdx.x; r < nsys; r += blockDim.x) sysctl[r].rebuild = 0;
   if (threadIdx.x == 0)
   {
@@ -731,35 +748,26 @@ __global__ void fast_after_rebuild_kernel(FastControl *ctrl, SysControl *sysctl,
 
 // ---------------------------------------------------------------- tiles
 //
-// A tile is a run of whole cells of one row of a system's rebuild grid; one
-// CTA steps the particles of a tile.  A row holds ceil(nc / tile_cells) tiles.
-// With Verlet lists they split the row's particles into runs of nearly equal
+// Verlet lists: a tile is a run of whole cells of one row of a system's rebuild
+// grid; one CTA steps the particles of a tile.  A row holds ceil(nc /
+// tile_cells) tiles, which split the row's particles into runs of nearly equal
 // count (boundaries at cell edges), so a tile of about 120 particles fills
 // its 128 threads whatever the local density, where runs of equal width leave
 // Poisson counts above 128 to a second pass of a few threads (36-cell tiles
 // at N = 4,194,304: 0.1963 -> 0.1882 ms per launch, same bits); the layout is
-// computed once per rebuild.  Cell lists lay their tiles out every step and
-// keep runs of tile_cells cells: the binary searches of the equal-count
-// boundaries, and widths beyond the run table, cost more there than the fuller
-// warps gain (measured 0.622 -> 0.645 ms per step at N = 4,194,304).  Slots are
-// sorted by cell, so the tile's particles are one slot range and the records
-// of its 3 x (width + 2) neighbour cells are at most six slot segments (three
-// rows, each split in two where the periodic x-wrap crosses the row end).
-// The CTA stages those segments into shared memory with TMA bulk copies; the
-// Verlet list of a particle in a staged tile stores shared-memory indices
-// directly.
+// computed once per rebuild.  Slots are sorted by cell, so the tile's particles
+// are one slot range and the records of its 3 x (width + 2) neighbour cells are
+// at most six slot segments (three rows, each split in two where the periodic
+// x-wrap crosses the row end).  The CTA stages those segments into shared memory
+// with TMA bulk copies; the Verlet list of a particle in a staged tile stores
+// shared-memory indices directly.  (Cell-list tiles: fast_cell_tile_kernel.)
 
 constexpr int kTileCellsDefault = 32;  // cells per tile unless tuned
 constexpr int kTileCap = 512;     // staged neighbour records per CTA (2 x 8 KiB)
 constexpr int kTileThreads = 128;
-// Resident CTAs per SM the Stochastic Euler tile kernels are compiled for.
-// Cell lists: 14 (32 registers, some spilled; the 512-system sweep step ran
-// 1.197 / 1.283 / 1.354 ms at 14 / 12 / 10).  Verlet lists: 10 (48 registers, 4 to 16 bytes spilled); the 512-system
-// sweep at 36-cell tiles ran 0.684 / 0.623 / 0.553 / 0.573 ms per step at
-// 14 / 12 / 10 / 9.
-#ifndef SPSS_SE_TILE_BLOCKS
-#define SPSS_SE_TILE_BLOCKS 14
-#endif
+// Resident CTAs per SM the Stochastic Euler Verlet tile kernel is compiled for:
+// 10 (48 registers, 4 to 16 bytes spilled); the 512-system sweep at 36-cell
+// tiles ran 0.684 / 0.623 / 0.553 / 0.573 ms per step at 14 / 12 / 10 / 9.
 #ifndef SPSS_SE_VERLET_TILE_BLOCKS
 #define SPSS_SE_VERLET_TILE_BLOCKS 10
 #endif
@@ -774,7 +782,7 @@ struct TileLayout
   int row, col0, ncols;  // the tile's cells: row `row`, columns col0 .. col0 + ncols - 1
 };
 
-// Cell-list stencil of one cell of a staged tile: for each stencil row (dy =
+// Stencil of one cell of a staged tile (list build): for each stencil row (dy =
 // -1, 0, 1) the staged records of the three cells (cx - 1, cx, cx + 1, wrapped)
 // as at most three contiguous runs of staged indices, in the reference's
 // stencil order (ParticleSystemFirstOrder.cpp:47-52).
@@ -811,21 +819,13 @@ __device__ __forceinline__ int first_cell_reaching(const int *__restrict__ ro, i
 
 // Deterministic layout of tile t of a system (cell offsets `off` of that
 // system's grid; the list build and the step compute the same).
-__device__ void tile_layout(int t, int nc, int tc, const int *__restrict__ off, bool equal_count, TileLayout &L)
+__device__ void tile_layout(int t, int nc, int tc, const int *__restrict__ off, TileLayout &L)
 {
   const int nbx = tiles_per_row(nc, tc);
   const int cy = t / nbx, bx = t - cy * nbx;
   const int *ro = off + cy * nc;
-  int cx_lo, cx_hi;
-  if (equal_count)
-  {
-    cx_lo = first_cell_reaching(ro, nc, row_target(ro, nc, bx, nbx));
-    cx_hi = bx + 1 == nbx ? nc : first_cell_reaching(ro, nc, row_target(ro, nc, bx + 1, nbx));
-  } else
-  {
-    cx_lo = bx * tc;
-    cx_hi = min(nc, cx_lo + tc);
-  }
+  const int cx_lo = first_cell_reaching(ro, nc, row_target(ro, nc, bx, nbx));
+  const int cx_hi = bx + 1 == nbx ? nc : first_cell_reaching(ro, nc, row_target(ro, nc, bx + 1, nbx));
   L.p_begin = off[cy * nc + cx_lo];
   L.p_end = off[cy * nc + cx_hi];
   L.row = cy;
@@ -890,13 +890,12 @@ __device__ void tile_layout(int t, int nc, int tc, const int *__restrict__ off, 
 // Layout of every tile of every system, once per rebuild.
 __global__ void fast_tile_layout_kernel(FastParams P, FastBuffers B)
 {
-  pdl_enter();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= P.ntiles) return;
   if (!rebuilds_system(B, B.tile_sys[t])) return;
   const SysParams *S = B.sys + B.tile_sys[t];
   TileLayout L;
-  tile_layout(t - S->tile0, S->nc, P.tile_cells, B.cell_off + S->cell0, P.kind == KIND_VERLET, L);
+  tile_layout(t - S->tile0, S->nc, P.tile_cells, B.cell_off + S->cell0, L);
   reinterpret_cast<TileLayout *>(B.tiles)[t] = L;
 }
 
@@ -1158,29 +1157,8 @@ __device__ __forceinline__ void gather_sums_staged(const FastParams &P, const Fa
                                                    const uint4 *saux, const TileLayout &L,
                                                    const uint4 *__restrict__ rec, const uint4 *__restrict__ aux, int q,
                                                    int cnt, const short *lp, int stride, const uint4 &ri, uint64_t Xi,
-                                                   uint64_t Yi, Acc &a, const StencilRuns *runs,
-                                                   const unsigned char *col_of, int self_base)
+                                                   uint64_t Yi, Acc &a)
 {
-  if (KIND == KIND_CELLS && runs)
-  {
-    // cell list from the tile's run table: three rows of contiguous staged
-    // records.  The guard-band decision is inline for Stochastic Euler (no
-    // call in the loop: the batched 512-system sweep step 1.319 -> 1.197 ms,
-    // N = 65,536 0.0638 -> 0.0622 ms, fewer spills at 32 registers) and out of
-    // line for SRK, whose larger kernel ran 0.7 % slower with it inline.
-    const StencilRuns &R = runs[col_of[q - L.p_begin]];
-    const int self = q + self_base;
-#pragma unroll 1
-    for (int r = 0; r < 3; ++r)
-#pragma unroll 1
-      for (int u = 0; u < 3; ++u)
-      {
-        const int e = R.e[r][u];
-        for (int idx = R.s[r][u]; idx < e; ++idx)
-          if (idx != self) candidate_staged<OMEGA, OMEGA>(P, ri, Xi, Yi, srec, saux, L, aux, idx, a);
-      }
-    return;
-  }
   if (KIND == KIND_VERLET && cnt >= 0)
   {
     const long n = stride;
@@ -1228,8 +1206,8 @@ __device__ __forceinline__ void gather_sums_staged(const FastParams &P, const Fa
     }
     return;
   }
-  // cell list, or a Verlet list that did not fit: scan the stencil of the
-  // (rebuild-time) cell; each stencil cell is one contiguous staged range
+  // a Verlet list that did not fit: scan the stencil of the rebuild-time cell;
+  // each stencil cell is one contiguous staged range
   const int *coff = B.cell_off + P.cell0;
   const int c = B.cell_sorted[q] - P.cell0;
   const int cx = c % P.nc, cy = c / P.nc;
@@ -1300,31 +1278,30 @@ __device__ __forceinline__ void sums_forces(const FastParams &P, const Acc &a, f
   }
 }
 
-template<int MODEL, int STEPPER>
+template<int MODEL, int STEPPER, bool CELLS = false>
 __device__ __forceinline__ float advance_particle(const FastParams &P, const FastBuffers &B, int q, const uint4 &ri,
                                                   const uint4 &ai, float2 v, float f_w, float C, const float z[6],
-                                                  uint4 *rout, uint4 *aout, int &err, int *cell_out = nullptr);
+                                                  uint4 *rout, uint4 *aout, int &err);
 
 // Derivative from the neighbour sums, SE or SRK update in fixed point, new
 // record.  Returns |dr|^2 of the step.
-template<int MODEL, int STEPPER>
+template<int MODEL, int STEPPER, bool CELLS = false>
 __device__ __forceinline__ float update_particle(const FastParams &P, const FastBuffers &B, int q, const uint4 &ri,
                                                  const uint4 &ai, float2 v, const Acc &a, const float z[6],
-                                                 uint4 *rout, uint4 *aout, int &err, int *cell_out = nullptr)
+                                                 uint4 *rout, uint4 *aout, int &err)
 {
   float f_w, C;
   sums_forces<STEPPER>(P, a, __uint_as_float(ri.z), __uint_as_float(ri.w), __uint_as_float(ai.w), f_w, C);
-  return advance_particle<MODEL, STEPPER>(P, B, q, ri, ai, v, f_w, C, z, rout, aout, err, cell_out);
+  return advance_particle<MODEL, STEPPER, CELLS>(P, B, q, ri, ai, v, f_w, C, z, rout, aout, err);
 }
 
 // SE or SRK update in fixed point from the forces, new record.  Returns
-// |dr|^2 of the step.  `cell_out` (cell-list steps): the new position's cell
-// id at the slot, which the next step's cell-list rebuild then need not
-// recompute.
-template<int MODEL, int STEPPER>
+// |dr|^2 of the step.  CELLS (cell-list steps): the new position's cell is
+// counted for the next step's binning, which then needs no pass for it.
+template<int MODEL, int STEPPER, bool CELLS>
 __device__ __forceinline__ float advance_particle(const FastParams &P, const FastBuffers &B, int q, const uint4 &ri,
                                                   const uint4 &ai, float2 v, float f_w, float C, const float z[6],
-                                                  uint4 *rout, uint4 *aout, int &err, int *cell_out)
+                                                  uint4 *rout, uint4 *aout, int &err)
 {
   const uint64_t Xi = join64(ri.x, ai.x), Yi = join64(ri.y, ai.y);
   const float cphi = __uint_as_float(ri.z), sphi = __uint_as_float(ri.w);
@@ -1390,7 +1367,12 @@ __device__ __forceinline__ float advance_particle(const FastParams &P, const Fas
   phase_sincos(Pn, sn, cn);
   rout[q] = make_uint4((uint32_t) (Xn >> 32), (uint32_t) (Yn >> 32), __float_as_uint(cn), __float_as_uint(sn));
   aout[q] = make_uint4((uint32_t) Xn, (uint32_t) Yn, Pn, __float_as_uint(__fadd_rn(wi, dw)));
-  if (cell_out) cell_out[q] = P.cell0 + cell_of_fix(Xn, Yn, P.nc);
+  if (CELLS)
+  {
+    const int c = P.cell0 + cell_of_fix(Xn, Yn, P.nc);
+    B.cell_of[q] = c;
+    B.cell_slot[q] = atomicAdd(B.cell_count + c, 1);
+  }
   // box crossings and phase turns are rare: read-modify-write only then (the
   // counts are kept by original index, so the slot re-sort never moves them)
   if (cx | cy | ct)
@@ -1600,6 +1582,7 @@ __global__ void __launch_bounds__(32 * kPairWarps, 2) fast_allpairs_kernel(FastP
   const int q = begin + lane;
   FastControl *ctrl = B.ctrl;
   const int par = ctrl->parity;
+  buffers_now(B, ctrl->order_parity);
   const uint4 *rin = par ? B.rec1 : B.rec0;
   const uint4 *ain = par ? B.aux1 : B.aux0;
   uint4 *rout = par ? B.rec0 : B.rec1;
@@ -1713,8 +1696,7 @@ __device__ __forceinline__ void step_tile(const FastParams &Q, const FastBuffers
                                           OwnParticle o, const uint4 *srec, const uint4 *saux, const short *slist,
                                           const short *glist, int list_staged, int list_stride, bool staged,
                                           const uint4 *rin, const uint4 *ain, uint4 *rout, uint4 *aout, float &d2max,
-                                          int &err, const StencilRuns *runs, const unsigned char *col_of,
-                                          int self_base)
+                                          int &err)
 {
   const int q0 = L.p_begin + threadIdx.x;
   for (int q = q0; q < L.p_end; q += blockDim.x)
@@ -1728,16 +1710,14 @@ __device__ __forceinline__ void step_tile(const FastParams &Q, const FastBuffers
     // entries are read with shared-memory loads
     if (staged && KIND == KIND_VERLET && list_staged)
       gather_sums_staged<KIND, STEPPER == 2>(Q, B, srec, saux, L, rin, ain, q, o.cnt, slist + i, list_stride, o.r,
-                                             Xi, Yi, a, nullptr, col_of, self_base);
+                                             Xi, Yi, a);
     else if (staged)
-      gather_sums_staged<KIND, STEPPER == 2>(Q, B, srec, saux, L, rin, ain, q, o.cnt, lp, list_stride, o.r, Xi, Yi,
-                                             a, runs, col_of, self_base);
+      gather_sums_staged<KIND, STEPPER == 2>(Q, B, srec, saux, L, rin, ain, q, o.cnt, lp, list_stride, o.r, Xi, Yi, a);
     else
       gather_sums<KIND, STEPPER == 2>(Q, B, rin, ain, q, o.cnt, lp, list_stride, o.r, Xi, Yi, a);
     float z[6];
     draw_noise<MODEL, STEPPER>(Q, B.ctrl->step, o.p, z);
-    d2max = fmaxf(d2max, update_particle<MODEL, STEPPER>(Q, B, q, o.r, o.a, o.v, a, z, rout, aout, err,
-                                                         KIND == KIND_CELLS ? B.cell_of : nullptr));
+    d2max = fmaxf(d2max, update_particle<MODEL, STEPPER>(Q, B, q, o.r, o.a, o.v, a, z, rout, aout, err));
   }
 }
 
@@ -1847,13 +1827,10 @@ __device__ __forceinline__ void init_mbarrier(uint32_t mb)
 // memory by TMA bulk copies (cp.async.bulk, completion on an mbarrier).
 // MULTI: several systems, whose parameters come from the system table (one
 // system: from the kernel's parameter space, which costs no registers).
-// Residency: SRK 9 CTAs per SM (56 registers, 24.7 KB of shared memory); SE
-// stages no aux words (11 KB) and runs 14 CTAs per SM on cell lists (faster
-// than 9, 10 or 12 despite a few spilled registers) and 10 on Verlet lists.
+// Verlet lists.  Residency: SRK 9 CTAs per SM (56 registers, 24.7 KB of shared
+// memory); SE stages no aux words and runs 10.
 template<int MODEL, int STEPPER, int KIND, bool MULTI>
-__global__ void __launch_bounds__(kTileThreads, STEPPER == 2 ? 9
-                                                               : (KIND == KIND_VERLET ? SPSS_SE_VERLET_TILE_BLOCKS
-                                                                                      : SPSS_SE_TILE_BLOCKS))
+__global__ void __launch_bounds__(kTileThreads, STEPPER == 2 ? 9 : SPSS_SE_VERLET_TILE_BLOCKS)
     fast_tile_kernel(FastParams P, FastBuffers B)
 {
   __shared__ __align__(16) uint4 srec[kTileCap];
@@ -1861,12 +1838,11 @@ __global__ void __launch_bounds__(kTileThreads, STEPPER == 2 ? 9
   __shared__ __align__(16) short slist[KIND == KIND_VERLET ? kListCap : 8];
   __shared__ __align__(8) unsigned long long mbar;
   __shared__ TileLayout L;
-  __shared__ int list_staged, list_stride, self_base;
-  __shared__ StencilRuns runs[KIND == KIND_CELLS ? kRunCells : 1];
-  __shared__ unsigned char col_of[KIND == KIND_CELLS ? kTileCap : 4];
+  __shared__ int list_staged, list_stride;
   pdl_enter();
   FastControl *ctrl = B.ctrl;
   const int par = ctrl->parity;
+  buffers_now(B, ctrl->order_parity);
   const uint4 *rin = par ? B.rec1 : B.rec0;
   const uint4 *ain = par ? B.aux1 : B.aux0;
   uint4 *rout = par ? B.rec0 : B.rec1;
@@ -1884,9 +1860,6 @@ __global__ void __launch_bounds__(kTileThreads, STEPPER == 2 ? 9
   if (L.p_end <= L.p_begin) return;
   const int sys = MULTI ? B.tile_sys[t] : 0;
   const FastParams Q = MULTI ? with_system(P, B.sys[sys]) : P;
-  // cell lists: the stencil run table, built while the bulk copies land
-  const bool use_runs = KIND == KIND_CELLS && staged && L.ncols <= kRunCells;
-  if (use_runs) build_runs(L, B.cell_off + Q.cell0, Q.nc, runs, col_of, &self_base, &ctrl->error);
   const short *glist = KIND == KIND_VERLET ? B.vl + tile_list_base(P.cap, t, L.p_begin) : nullptr;
   // the thread's first particle is loaded before the wait for the bulk
   // copies, so its global loads are in flight while the tile lands
@@ -1925,16 +1898,14 @@ __global__ void __launch_bounds__(kTileThreads, STEPPER == 2 ? 9
     // entries are read with shared-memory loads
     if (staged && KIND == KIND_VERLET && list_staged)
       gather_sums_staged<KIND, STEPPER == 2>(Q, B, srec, saux, L, rin, ain, q, cnt, slist + i, list_stride, ri, Xi,
-                                             Yi, a, nullptr, col_of, self_base);
+                                             Yi, a);
     else if (staged)
-      gather_sums_staged<KIND, STEPPER == 2>(Q, B, srec, saux, L, rin, ain, q, cnt, lp, list_stride, ri, Xi, Yi, a,
-                                             use_runs ? runs : nullptr, col_of, self_base);
+      gather_sums_staged<KIND, STEPPER == 2>(Q, B, srec, saux, L, rin, ain, q, cnt, lp, list_stride, ri, Xi, Yi, a);
     else
       gather_sums<KIND, STEPPER == 2>(Q, B, rin, ain, q, cnt, lp, list_stride, ri, Xi, Yi, a);
     float z[6];
     draw_noise<MODEL, STEPPER>(Q, ctrl->step, p, z);
-    d2max = fmaxf(d2max, update_particle<MODEL, STEPPER>(Q, B, q, ri, ai, v, a, z, rout, aout, err,
-                                                         KIND == KIND_CELLS ? B.cell_of : nullptr));
+    d2max = fmaxf(d2max, update_particle<MODEL, STEPPER>(Q, B, q, ri, ai, v, a, z, rout, aout, err));
   }
   publish_max(ctrl, B.sysctl, sys, d2max, err);
 }
@@ -1950,13 +1921,12 @@ __global__ void __launch_bounds__(kTileThreads, 8) fast_tile_persistent_kernel(F
   __shared__ __align__(16) short slist[KIND == KIND_VERLET ? kListCap : 8];
   __shared__ __align__(8) unsigned long long mbar;
   __shared__ TileLayout L;
-  __shared__ int list_staged, list_stride, tile_id, self_base;
+  __shared__ int list_staged, list_stride, tile_id;
   __shared__ uint32_t phase;  // mbarrier phase of the next staged tile
-  __shared__ StencilRuns runs[KIND == KIND_CELLS ? kRunCells : 1];
-  __shared__ unsigned char col_of[KIND == KIND_CELLS ? kTileCap : 4];
   pdl_enter();
   FastControl *ctrl = B.ctrl;
   const int par = ctrl->parity;
+  buffers_now(B, ctrl->order_parity);
   const uint4 *rin = par ? B.rec1 : B.rec0;
   const uint4 *ain = par ? B.aux1 : B.aux0;
   uint4 *rout = par ? B.rec0 : B.rec1;
@@ -1983,18 +1953,6 @@ __global__ void __launch_bounds__(kTileThreads, 8) fast_tile_persistent_kernel(F
     if (t >= P.ntiles) break;
     const bool staged = L.staged;
     const int sys = MULTI ? B.tile_sys[t] : 0;
-    const bool use_runs = KIND == KIND_CELLS && staged && L.ncols <= kRunCells && L.p_end > L.p_begin;
-    if (use_runs)
-    {
-      if (MULTI)
-      {
-        const SysParams *S = B.sys + sys;
-        build_runs(L, B.cell_off + S->cell0, S->nc, runs, col_of, &self_base, &ctrl->error);
-      } else
-      {
-        build_runs(L, B.cell_off + P.cell0, P.nc, runs, col_of, &self_base, &ctrl->error);
-      }
-    }
     OwnParticle o;
     if (L.p_begin + (int) threadIdx.x < L.p_end) o = load_own<MODEL, KIND>(B, rin, ain, L.p_begin + threadIdx.x);
     if (staged)
@@ -2015,13 +1973,293 @@ __global__ void __launch_bounds__(kTileThreads, 8) fast_tile_persistent_kernel(F
     int err = 0;
     if (!MULTI)
       step_tile<MODEL, STEPPER, KIND>(P, B, L, o, srec, saux, slist, glist, list_staged, list_stride, staged, rin,
-                                      ain, rout, aout, d2max, err, use_runs ? runs : nullptr, col_of, self_base);
+                                      ain, rout, aout, d2max, err);
     else
       step_tile<MODEL, STEPPER, KIND>(with_system(P, B.sys[sys]), B, L, o, srec, saux, slist, glist, list_staged,
-                                      list_stride, staged, rin, ain, rout, aout, d2max, err,
-                                      use_runs ? runs : nullptr, col_of, self_base);
+                                      list_stride, staged, rin, ain, rout, aout, d2max, err);
     publish_max(ctrl, B.sysctl, sys, d2max, err);
   }
+}
+
+// ---------------------------------------------------------------- cell-list step
+//
+// One SE or SRK step of the particles of a block of cells (nrows x ncols of a
+// system's grid, about 110 particles) per CTA, neighbours from the 3 x 3 stencil
+// of the cells just sorted (ParticleSystemFirstOrder.cpp:231-353).  The nrows +
+// 2 rows of ncols + 2 cells around it are staged in shared memory by bulk
+// copies, column by column in the order of the grid with the periodic halo
+// columns in place, so the stencil of a cell is one contiguous run of staged
+// records per row, in the reference's order (ParticleSystemFirstOrder.cpp:47-52).
+// Tiles of several rows stage (nrows + 2) / nrows records for each of their own
+// and fill the CTA whatever the grid's width, where one row of a small system's
+// 22 cells held 45 particles for 128 threads.  Instructions bound it: 19
+// candidates a particle at density 2, one comparison each; a particle with a
+// candidate inside the guard band is summed again with the FP64 decisions.
+// The layout comes from the cell offsets alone (no pass of its own), and the
+// update counts the new cells for the next step's binning.
+// 512 systems, 8,852,499 particles (SE): one-row tiles, a run table a tile, the
+// layout, cell and count passes of their own 905 + 30 + 24 + 43 us, this
+// MEASURED_CT us.
+constexpr int kCellRows = 4;    // rows of a tile at most
+constexpr int kCellCols = 64;   // columns of a tile at most
+constexpr int kCellTarget = 112;  // mean particles of a tile: 128 threads less 1.5 standard deviations
+
+struct CellRows
+{
+  int base[kCellRows + 2];   // staged index of the row's first record
+  int left[kCellRows + 2], main[kCellRows + 2], right[kCellRows + 2];     // slots of its three pieces
+  int nleft[kCellRows + 2], nmain[kCellRows + 2], nright[kCellRows + 2];  // and their records
+  int total;
+  int own[kCellRows + 1];    // particles of the tile before each of its rows
+};
+
+// Slot of a staged record of row rr.
+__device__ __forceinline__ int cell_slot_of(const CellRows &R, int rr, int idx)
+{
+  int k = idx - R.base[rr];
+  if (k < R.nleft[rr]) return R.left[rr] + k;
+  k -= R.nleft[rr];
+  if (k < R.nmain[rr]) return R.main[rr] + k;
+  return R.right[rr] + (k - R.nmain[rr]);
+}
+
+// Neighbour sums of one particle again, with in_range's decision for every
+// candidate (some candidate lies inside the guard band).
+template<bool OMEGA>
+__device__ __noinline__ void cell_sums_exact(const CellRows &R, const short (*soff)[kCellCols + 4], const uint4 *srec,
+                                             const uint4 *saux, const uint4 *__restrict__ aux, int r, int lc, int self,
+                                             const uint4 ri, const uint4 ai, float rho2, float band, double rho2_d,
+                                             Acc *acc)
+{
+  const uint64_t Xi = join64(ri.x, ai.x), Yi = join64(ri.y, ai.y);
+  Acc a{0.f, 0.f, 0.f, 0.f, 0};
+  for (int rr = r; rr < r + 3; ++rr)
+    for (int idx = soff[rr][lc]; idx < soff[rr][lc + 3]; ++idx)
+    {
+      if (idx == self) continue;
+      const uint4 rj = srec[idx];
+      const float dx = (float) (int) (rj.x - ri.x), dy = (float) (int) (rj.y - ri.y);
+      const float d2 = fmaf(dx, dx, dy * dy);
+      bool in = d2 <= rho2;
+      if (fabsf(d2 - rho2) <= band)
+      {
+        const uint2 l = __ldg(reinterpret_cast<const uint2 *>(&aux[cell_slot_of(R, rr, idx)]));
+        in = exact_within_inline(rj.x, rj.y, l.x, l.y, Xi, Yi, rho2_d);
+      }
+      if (in) accumulate(a, rj, OMEGA ? __uint_as_float(saux[idx].w) : 0.0f);
+    }
+  *acc = a;
+}
+
+#ifndef SPSS_CELL_BLOCKS_SE
+#define SPSS_CELL_BLOCKS_SE 12
+#endif
+#ifndef SPSS_CELL_BLOCKS_SRK
+#define SPSS_CELL_BLOCKS_SRK 9
+#endif
+
+// `fresh`: the slots were just re-sorted (the particles stand in the other
+// rec/aux buffer, the step was counted by the scan); 0: a step on the lists of
+// an earlier binning.
+template<int MODEL, int STEPPER, bool MULTI>
+__global__ void __launch_bounds__(kTileThreads, STEPPER == 2 ? SPSS_CELL_BLOCKS_SRK : SPSS_CELL_BLOCKS_SE)
+    fast_cell_tile_kernel(FastParams P, FastBuffers B, int fresh)
+{
+  __shared__ __align__(16) uint4 srec[kTileCap];
+  __shared__ __align__(16) uint4 saux[STEPPER == 2 ? kTileCap : 1];  // aux words: SRK only (neighbour omega)
+  __shared__ __align__(8) unsigned long long mbar;
+  __shared__ CellRows R;
+  __shared__ short soff[kCellRows + 2][kCellCols + 4];  // staged start of each column, halo columns included
+  __shared__ int staged_all;
+  pdl_enter();
+  FastControl *ctrl = B.ctrl;
+  const int par = ctrl->parity ^ fresh;
+  buffers_now(B, ctrl->order_parity);
+  const uint4 *rin = par ? B.rec1 : B.rec0;
+  const uint4 *ain = par ? B.aux1 : B.aux0;
+  uint4 *rout = par ? B.rec0 : B.rec1;
+  uint4 *aout = par ? B.aux0 : B.aux1;
+  const unsigned long long step = ctrl->step - (unsigned long long) fresh;
+  const CellTile T = B.cell_tiles[blockIdx.x];
+  const int *coff = B.cell_off + T.cell0;
+  const int nc = T.nc, rows = T.nrows + 2;
+  const uint32_t mb = smem_u32(&mbar);
+  if (threadIdx.x < 32)
+  {
+    const int lane = threadIdx.x;
+    int left = 0, main = 0, right = 0, nl = 0, nm = 0, nr = 0;
+    if (lane < rows)
+    {
+      const int row = wrap_cell(T.row0 - 1 + lane, nc) * nc;
+      const int lx = row + wrap_cell(T.col0 - 1, nc), rx = row + wrap_cell(T.col0 + T.ncols, nc);
+      left = coff[lx];
+      main = coff[row + T.col0];
+      right = coff[rx];
+      nl = coff[lx + 1] - left;
+      nm = coff[row + T.col0 + T.ncols] - main;
+      nr = coff[rx + 1] - right;
+    }
+    const int len = nl + nm + nr;
+    int end = len, own = (lane >= 1 && lane <= T.nrows) ? nm : 0;
+#pragma unroll
+    for (int off = 1; off < 8; off <<= 1)
+    {
+      const int y = __shfl_up_sync(0xffffffffu, end, off), z = __shfl_up_sync(0xffffffffu, own, off);
+      if (lane >= off)
+      {
+        end += y;
+        own += z;
+      }
+    }
+    const int total = __shfl_sync(0xffffffffu, end, rows - 1), np = __shfl_sync(0xffffffffu, own, T.nrows);
+    const bool staged = nc >= 3 && total <= kTileCap && np > 0;
+    if (lane < rows)
+    {
+      R.base[lane] = end - len;
+      R.left[lane] = left;
+      R.main[lane] = main;
+      R.right[lane] = right;
+      R.nleft[lane] = nl;
+      R.nmain[lane] = nm;
+      R.nright[lane] = nr;
+      if (lane <= T.nrows) R.own[lane] = own;
+    }
+    if (lane == 0)
+    {
+      R.total = total;
+      staged_all = staged;
+      if (staged)
+      {
+        init_mbarrier(mb);
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mb),
+                     "r"((STEPPER == 2 ? 32u : 16u) * (uint32_t) total)
+                     : "memory");
+      }
+    }
+    __syncwarp();
+    if (staged && lane < rows)
+    {
+      // pieces that follow each other in the slot order are one copy
+      int at = end - len, from[3] = {left, main, right}, n[3] = {nl, nm, nr};
+      if (left + nl == main)
+      {
+        from[1] = left;
+        n[1] += nl;
+        n[0] = 0;
+      }
+      if (from[1] + n[1] == right)
+      {
+        n[1] += nr;
+        n[2] = 0;
+      }
+#pragma unroll
+      for (int k = 0; k < 3; ++k)
+      {
+        if (n[k] == 0) continue;
+        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                         smem_u32(&srec[at])),
+                     "l"(rin + from[k]), "r"(16u * (uint32_t) n[k]), "r"(mb)
+                     : "memory");
+        if (STEPPER == 2)
+          asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                           smem_u32(&saux[at])),
+                       "l"(ain + from[k]), "r"(16u * (uint32_t) n[k]), "r"(mb)
+                       : "memory");
+        at += n[k];
+      }
+    }
+  }
+  __syncthreads();
+  const bool staged = staged_all;
+  const int np = R.own[T.nrows];
+  if (np == 0) return;
+  const SysParams *S = MULTI ? B.sys + T.sys : nullptr;
+  const float rho2 = MULTI ? S->rho2_f : P.rho2_f, band = MULTI ? S->band_f : P.band_f;
+  // the thread's first particle and the column offsets, on their way while the records land
+  int i = threadIdx.x, r = 0, q = 0, lc = 0;
+  OwnParticle o;
+  auto take = [&](int k) {
+    r = 0;
+    while (r + 1 < T.nrows && k >= R.own[r + 1]) ++r;
+    q = R.main[r + 1] + (k - R.own[r]);
+    o = load_own<MODEL, KIND_CELLS>(B, rin, ain, q);
+    lc = B.cell_sorted[q] - T.cell0 - (T.row0 + r) * nc - T.col0;
+  };
+  if (i < np) take(i);
+  if (staged)
+  {
+    for (int w = threadIdx.x; w < rows * (T.ncols + 3); w += kTileThreads)
+    {
+      const int rr = w / (T.ncols + 3), c = w - rr * (T.ncols + 3);
+      int at = R.base[rr];
+      if (c > T.ncols + 1) at += R.nleft[rr] + R.nmain[rr] + R.nright[rr];
+      else if (c > 0) at += R.nleft[rr] + coff[wrap_cell(T.row0 - 1 + rr, nc) * nc + T.col0 + c - 1] - R.main[rr];
+      soff[rr][c] = (short) at;
+    }
+    const uint32_t done = wait_phase(mb, 0);
+    if (!__syncthreads_and(done))
+    {
+      // the copies did not complete in time: report, give them a second
+      // bounded wait so none is in flight when the CTA exits, and stop
+      if (threadIdx.x == 0) atomicOr(&ctrl->error, 2);
+      wait_phase(mb, 0);
+      return;
+    }
+  }
+  int err = 0;
+  for (; i < np; i += kTileThreads)
+  {
+    if (i != (int) threadIdx.x) take(i);
+    Acc a{0.f, 0.f, 0.f, 0.f, 0};
+    if (staged)
+    {
+      const int self = R.base[r + 1] + R.nleft[r + 1] + (q - R.main[r + 1]);
+      float2 cs = make_float2(0.f, 0.f), w = make_float2(0.f, 0.f);
+      int card = 0;
+      float nearest = 3.0e38f;
+#pragma unroll 1
+      for (int rr = r; rr < r + 3; ++rr)
+      {
+        const int e = soff[rr][lc + 3];
+#pragma unroll 2
+        for (int idx = soff[rr][lc]; idx < e; ++idx)
+        {
+          const uint4 rj = srec[idx];
+          const float wj = STEPPER == 2 ? __uint_as_float(saux[idx].w) : 0.0f;
+          const float dx = (float) (int) (rj.x - o.r.x);
+          const float dy = (float) (int) (rj.y - o.r.y);
+          float d2 = fmaf(dx, dx, dy * dy);
+          if (idx == self) d2 = 3.0e38f;
+          nearest = fminf(nearest, fabsf(d2 - rho2));
+          if (d2 <= rho2)
+          {
+            const float2 t = make_float2(__uint_as_float(rj.z), __uint_as_float(rj.w));
+            cs = add2(cs, t);
+            if (STEPPER == 2) w = fma2(make_float2(wj, wj), t, w);
+            card += 1;
+          }
+        }
+      }
+      a = Acc{cs.y, cs.x, w.y, w.x, card};
+      if (nearest <= band)
+      {
+        Acc again;
+        cell_sums_exact<STEPPER == 2>(R, soff, srec, saux, ain, r, lc, self, o.r, o.a, rho2, band,
+                                      MULTI ? S->rho2_d : P.rho2_d, &again);
+        a = again;
+      }
+    } else
+    {
+      const FastParams Q = MULTI ? with_system(P, *S) : P;
+      gather_sums<KIND_CELLS, STEPPER == 2>(Q, B, rin, ain, q, 0, nullptr, 0, o.r, join64(o.r.x, o.a.x),
+                                            join64(o.r.y, o.a.y), a);
+    }
+    const FastParams Q = MULTI ? with_system(P, *S) : P;
+    float z[6];
+    draw_noise<MODEL, STEPPER>(Q, step, o.p, z);
+    update_particle<MODEL, STEPPER, true>(Q, B, q, o.r, o.a, o.v, a, z, rout, aout, err);
+  }
+  if (err) atomicOr(&ctrl->error, 1);
 }
 
 // Verlet lists of one tile per CTA, from the 3x3 stencil of the rebuild grid
@@ -2146,7 +2384,6 @@ __global__ void fast_control_kernel(FastControl *ctrl, SysControl *sysctl, const
                                     cudaGraphExec_t rebuild_exec)
 {
   __shared__ int any;
-  pdl_enter();
   if (threadIdx.x == 0) any = 0;
   __syncthreads();
   for (int r = threadIdx.x; r < nsys; r += blockDim.x)
@@ -2276,6 +2513,7 @@ __global__ void fast_order_partials_kernel(FastParams P, FastBuffers B, OrderSum
   if (gated && !sample_now(B.ctrl)) return;
   __shared__ double sh[4][8];
   const uint4 *rec = B.ctrl->parity ? B.rec1 : B.rec0;
+  buffers_now(B, B.ctrl->order_parity);
   for (int k = blockIdx.x; k < nitems; k += gridDim.x)
   {
     const int2 it = items[k];
@@ -2501,6 +2739,7 @@ __global__ void __launch_bounds__(256) fast_observe_kernel(FastParams P, FastBuf
     __syncthreads();
   }
   const uint4 *aux = B.ctrl->parity ? B.aux1 : B.aux0;
+  buffers_now(B, B.ctrl->order_parity);
   double a[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll 2
   for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < P.n; q += gridDim.x * blockDim.x)
@@ -2556,6 +2795,7 @@ __global__ void __launch_bounds__(kTB, 4) fast_global_step_kernel(FastParams P, 
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   FastControl *ctrl = B.ctrl;
   const int par = ctrl->parity;
+  buffers_now(B, ctrl->order_parity);
   const uint4 *rin = par ? B.rec1 : B.rec0;
   const uint4 *ain = par ? B.aux1 : B.aux0;
   uint4 *rout = par ? B.rec0 : B.rec1;
@@ -2627,6 +2867,9 @@ static FastBuffers buffers(spss_ctx *ctx)
   B.cell_sorted = f->cell_sorted.ptr;
   B.cell_off = f->binner.offsets.ptr;
   B.order = f->binner.members.ptr;
+  B.cell_count = f->binner.count.ptr;
+  B.cell_slot = f->binner.slot.ptr;
+  B.cell_tiles = f->cell_tiles.ptr;
   B.vl = f->vl.ptr;
   B.vl_cnt = f->vl_cnt.ptr;
   B.tile_maxcnt = f->tile_maxcnt.ptr;
@@ -2737,19 +2980,55 @@ static int set_tiling(spss_ctx *ctx, int tile_cells)
   f->tile_cells = tile_cells;
   int ntiles = 0;
   std::vector<int> tile_sys;
+  std::vector<CellTile> cell_tiles;
   for (int r = 0; r < f->nsys; ++r)
   {
     SysParams &S = f->h_sys[r];
     S.tile0 = ntiles;
+    if (f->kind == KIND_CELLS)
+    {
+      // as many whole rows of at most tile_cells cells as fill a CTA, no tile
+      // much smaller than the others
+      const double occupancy = (double) S.n / ((double) S.nc * S.nc);
+      const int widest = std::max(1, std::min({tile_cells, kCellCols, (int) (kCellTarget / occupancy), S.nc}));
+      const int nbx = tiles_per_row(S.nc, widest);
+      const double row = occupancy * S.nc / nbx;  // mean particles of a tile's row
+      const int high = std::max(1, std::min({kCellRows, (int) std::lround(kCellTarget / row), S.nc}));
+      const int nby = tiles_per_row(S.nc, high);
+      for (int y = 0; y < nby; ++y)
+        for (int x = 0; x < nbx; ++x)
+        {
+          CellTile T{};
+          T.sys = r;
+          T.row0 = (int) ((long) S.nc * y / nby);
+          T.nrows = (int) ((long) S.nc * (y + 1) / nby) - T.row0;
+          T.col0 = (int) ((long) S.nc * x / nbx);
+          T.ncols = (int) ((long) S.nc * (x + 1) / nbx) - T.col0;
+          T.nc = S.nc;
+          T.cell0 = S.cell0;
+          cell_tiles.push_back(T);
+        }
+      S.ntiles = nbx * nby;
+      ntiles += S.ntiles;
+      continue;
+    }
     S.ntiles = S.nc * tiles_per_row(S.nc, tile_cells);
     ntiles += S.ntiles;
     tile_sys.insert(tile_sys.end(), (size_t) S.ntiles, r);
   }
   f->ntiles = ntiles;
-  SPSS_TRY(f->tiles.reserve(sizeof(TileLayout) * (size_t) ntiles));
-  SPSS_TRY(f->tile_sys.reserve((size_t) ntiles));
-  SPSS_CUDA_TRY(cudaMemcpyAsync(f->tile_sys.ptr, tile_sys.data(), sizeof(int) * ntiles, cudaMemcpyHostToDevice,
-                                ctx->stream));
+  if (f->kind == KIND_CELLS)
+  {
+    SPSS_TRY(f->cell_tiles.reserve((size_t) ntiles));
+    SPSS_CUDA_TRY(cudaMemcpyAsync(f->cell_tiles.ptr, cell_tiles.data(), sizeof(CellTile) * ntiles,
+                                  cudaMemcpyHostToDevice, ctx->stream));
+  } else
+  {
+    SPSS_TRY(f->tiles.reserve(sizeof(TileLayout) * (size_t) ntiles));
+    SPSS_TRY(f->tile_sys.reserve((size_t) ntiles));
+    SPSS_CUDA_TRY(cudaMemcpyAsync(f->tile_sys.ptr, tile_sys.data(), sizeof(int) * ntiles, cudaMemcpyHostToDevice,
+                                  ctx->stream));
+  }
   SPSS_CUDA_TRY(cudaMemcpyAsync(f->sys.ptr, f->h_sys.data(), sizeof(SysParams) * f->nsys, cudaMemcpyHostToDevice,
                                 ctx->stream));
   if (f->kind == KIND_VERLET)
@@ -2908,6 +3187,7 @@ int fast_create(spss_ctx *ctx)
   f->h_ctrl->uses_verlet = f->kind == KIND_VERLET;
   SPSS_CUDA_TRY(cudaMemcpyAsync(f->ctrl, f->h_ctrl, sizeof(FastControl), cudaMemcpyHostToDevice, ctx->stream));
   SPSS_CUDA_TRY(cudaMemsetAsync(f->vel.ptr, 0, sizeof(float2) * n, ctx->stream));
+  if (has_cells(f->kind)) SPSS_TRY(f->binner.prepare(n, f->total_cells, ctx->stream));
   SPSS_TRY(set_tiling(ctx, kTileCellsDefault));
   // resident CTAs of the persistent tile kernel: one wave
   {
@@ -2945,6 +3225,7 @@ void fast_destroy(spss_ctx *ctx)
   f->vl_cnt.release();
   f->tile_maxcnt.release();
   f->tiles.release();
+  f->cell_tiles.release();
   f->sys.release();
   f->sys_of.release();
   f->tile_sys.release();
@@ -2968,66 +3249,114 @@ void fast_destroy(spss_ctx *ctx)
   ctx->fast = nullptr;
 }
 
-// Cell binning, slot re-sort and (Verlet) list build, as one stream sequence.
+// Cell binning, slot re-sort and list build (Verlet lists), as one stream
+// sequence; kinds without lists only clear the flag.
 static int launch_rebuild(spss_ctx *ctx, const FastParams &P)
 {
   FastPath *f = ctx->fast;
   const FastBuffers B = buffers(ctx);
   const int n = P.n;
-  if (has_cells(f->kind))
+  const bool lists = f->kind == KIND_VERLET;
+  if (lists)
   {
     fast_cells_kernel<<<blocks_for(n, kTB), kTB, 0, ctx->stream>>>(P, B);
     ++ctx->launches;
     SPSS_TRY(check_launch("fast_cells_kernel"));
-    SPSS_TRY(f->binner.run(f->cell_of.ptr, n, f->total_cells, ctx->stream, ctx->launches, f->chain));
-    const FastBuffers B2 = buffers(ctx);  // binner buffers exist now
-    SPSS_CUDA_TRY(launch_chained(f->chain, fast_permute_kernel, blocks_for(n, kTB), kTB, 0, ctx->stream, P, B2));
+    SPSS_TRY(f->binner.place(f->cell_of.ptr, n, ctx->stream, ctx->launches));
+    fast_permute_kernel<false><<<blocks_for(n, kTB), kTB, 0, ctx->stream>>>(P, B);
     ++ctx->launches;
     SPSS_TRY(check_launch("fast_permute_kernel"));
-    SPSS_CUDA_TRY(launch_chained(f->chain, fast_copyback_kernel, blocks_for(n, kTB), kTB, 0, ctx->stream, P, B2));
-    ++ctx->launches;
-    SPSS_TRY(check_launch("fast_copyback_kernel"));
+    if (P.selective)
+    {
+      fast_copyback_kernel<<<blocks_for(n, kTB), kTB, 0, ctx->stream>>>(P, B);
+      ++ctx->launches;
+      SPSS_TRY(check_launch("fast_copyback_kernel"));
+    }
   }
-  SPSS_CUDA_TRY(launch_chained(f->chain, fast_after_permute_kernel, 1, 1, 0, ctx->stream, f->ctrl,
-                               (int) has_cells(f->kind)));
+  fast_after_permute_kernel<<<1, 1, 0, ctx->stream>>>(f->ctrl, (int) lists);
   ++ctx->launches;
   SPSS_TRY(check_launch("fast_after_permute_kernel"));
-  if (has_cells(f->kind))
+  if (lists)
   {
-    SPSS_CUDA_TRY(launch_chained(f->chain, fast_tile_layout_kernel, blocks_for(f->ntiles, 128), 128, 0, ctx->stream,
-                                 P, buffers(ctx)));
+    fast_tile_layout_kernel<<<blocks_for(f->ntiles, 128), 128, 0, ctx->stream>>>(P, B);
     ++ctx->launches;
     SPSS_TRY(check_launch("fast_tile_layout_kernel"));
-  }
-  if (f->kind == KIND_VERLET)
-  {
-    fast_verlet_tile_build_kernel<<<f->ntiles, kTileThreads, 0, ctx->stream>>>(P, buffers(ctx));
+    fast_verlet_tile_build_kernel<<<f->ntiles, kTileThreads, 0, ctx->stream>>>(P, B);
     ++ctx->launches;
     SPSS_TRY(check_launch("fast_verlet_tile_build_kernel"));
   }
-  SPSS_CUDA_TRY(launch_chained(f->chain, fast_after_rebuild_kernel, 1, 256, 0, ctx->stream, f->ctrl, f->sysctl.ptr,
-                               f->nsys));
+  fast_after_rebuild_kernel<<<1, 256, 0, ctx->stream>>>(f->ctrl, f->sysctl.ptr, f->nsys);
   ++ctx->launches;
   return check_launch("fast_after_rebuild_kernel");
 }
 
-template<int MODEL, int STEPPER, int KIND>
-static void launch_tiles(spss_ctx *ctx, const FastParams &P, const FastBuffers &B, int grid)
+// Cell ids and counts of the current slots, where the last cell-list step did
+// not leave them (a new state, a restored snapshot).
+static int ensure_cells(spss_ctx *ctx, const FastParams &P)
 {
-  const bool c = ctx->fast->chain;
-  if (P.persistent)
+  FastPath *f = ctx->fast;
+  if (f->h_ctrl->cells_fresh) return SPSS_OK;
+  SPSS_CUDA_TRY(cudaMemsetAsync(f->binner.count.ptr, 0, sizeof(int) * f->binner.count.count, ctx->stream));
+  fast_cells_kernel<<<blocks_for(P.n, kTB), kTB, 0, ctx->stream>>>(P, buffers(ctx));
+  ++ctx->launches;
+  f->h_ctrl->cells_fresh = 1;
+  return check_launch("fast_cells_kernel");
+}
+
+template<int MODEL, int STEPPER>
+static void launch_cell_tiles(spss_ctx *ctx, const FastParams &P, const FastBuffers &B, int fresh, bool chained)
+{
+  if (P.nsys > 1)
+    launch_chained(chained, fast_cell_tile_kernel<MODEL, STEPPER, true>, P.ntiles, kTileThreads, 0, ctx->stream, P, B, fresh);
+  else
+    launch_chained(chained, fast_cell_tile_kernel<MODEL, STEPPER, false>, P.ntiles, kTileThreads, 0, ctx->stream, P, B, fresh);
+}
+
+static int launch_cell_kernel(spss_ctx *ctx, int stepper, const FastParams &P, int fresh, bool chained)
+{
+  const FastBuffers B = buffers(ctx);
+  if (ctx->timing) SPSS_CUDA_TRY(cudaEventRecord(ctx->ev0, ctx->stream));
+  if (ctx->p.model == 1)
   {
-    if (P.nsys > 1)
-      launch_chained(c, fast_tile_persistent_kernel<MODEL, STEPPER, KIND, true>, grid, kTileThreads, 0, ctx->stream, P, B);
-    else
-      launch_chained(c, fast_tile_persistent_kernel<MODEL, STEPPER, KIND, false>, grid, kTileThreads, 0, ctx->stream, P,
-                     B);
+    if (stepper == SPSS_STEPPER_STOCHASTIC_EULER) launch_cell_tiles<1, 1>(ctx, P, B, fresh, chained);
+    else launch_cell_tiles<1, 2>(ctx, P, B, fresh, chained);
   } else
   {
-    if (P.nsys > 1)
-      launch_chained(c, fast_tile_kernel<MODEL, STEPPER, KIND, true>, grid, kTileThreads, 0, ctx->stream, P, B);
-    else
-      launch_chained(c, fast_tile_kernel<MODEL, STEPPER, KIND, false>, grid, kTileThreads, 0, ctx->stream, P, B);
+    if (stepper == SPSS_STEPPER_STOCHASTIC_EULER) launch_cell_tiles<2, 1>(ctx, P, B, fresh, chained);
+    else launch_cell_tiles<2, 2>(ctx, P, B, fresh, chained);
+  }
+  ++ctx->launches;
+  SPSS_TRY(check_launch("fast_cell_tile_kernel"));
+  if (ctx->timing) SPSS_CUDA_TRY(cudaEventRecord(ctx->ev1, ctx->stream));
+  return SPSS_OK;
+}
+
+// A cell-list step from the counts the last one left: offsets (which also count
+// the step), members, slot re-sort, pair sums and update.  `chained`: captured
+// as a programmatic-dependent chain (each kernel begins with pdl_enter).
+static int launch_cells_step(spss_ctx *ctx, int stepper, const FastParams &P, bool chained)
+{
+  FastPath *f = ctx->fast;
+  SPSS_TRY(f->binner.place(f->cell_of.ptr, P.n, ctx->stream, ctx->launches, chained, f->ctrl));
+  SPSS_CUDA_TRY(launch_chained(chained, fast_permute_kernel<true>, blocks_for(P.n, kTB), kTB, 0, ctx->stream, P,
+                               buffers(ctx)));
+  ++ctx->launches;
+  SPSS_TRY(check_launch("fast_permute_kernel"));
+  return launch_cell_kernel(ctx, stepper, P, 1, chained);
+}
+
+template<int MODEL, int STEPPER>
+static void launch_tiles(spss_ctx *ctx, const FastParams &P, const FastBuffers &B, int grid)
+{
+  constexpr int K = KIND_VERLET;
+  if (P.persistent)
+  {
+    if (P.nsys > 1) launch_chained(false, fast_tile_persistent_kernel<MODEL, STEPPER, K, true>, grid, kTileThreads, 0, ctx->stream, P, B);
+    else launch_chained(false, fast_tile_persistent_kernel<MODEL, STEPPER, K, false>, grid, kTileThreads, 0, ctx->stream, P, B);
+  } else
+  {
+    if (P.nsys > 1) launch_chained(false, fast_tile_kernel<MODEL, STEPPER, K, true>, grid, kTileThreads, 0, ctx->stream, P, B);
+    else launch_chained(false, fast_tile_kernel<MODEL, STEPPER, K, false>, grid, kTileThreads, 0, ctx->stream, P, B);
   }
 }
 
@@ -3049,13 +3378,20 @@ static void launch_step_kind(spss_ctx *ctx, const FastParams &P, const FastBuffe
     const int blocks = blocks_for(P.n, 32);
     if (P.nsys > 1) fast_allpairs_kernel<MODEL, STEPPER, true><<<blocks, 32 * kPairWarps, 0, ctx->stream>>>(P, B);
     else fast_allpairs_kernel<MODEL, STEPPER, false><<<blocks, 32 * kPairWarps, 0, ctx->stream>>>(P, B);
-  } else if (ctx->fast->kind == KIND_CELLS)
-  {
-    launch_tiles<MODEL, STEPPER, KIND_CELLS>(ctx, P, B, tiles);
   } else
   {
-    launch_tiles<MODEL, STEPPER, KIND_VERLET>(ctx, P, B, tiles);
+    launch_tiles<MODEL, STEPPER>(ctx, P, B, tiles);
   }
+}
+
+static int launch_control(spss_ctx *ctx, const FastParams &P, int cells_written)
+{
+  FastPath *f = ctx->fast;
+  fast_control_kernel<false><<<1, 256, 0, ctx->stream>>>(f->ctrl, f->sysctl.ptr, f->sys.ptr, f->nsys, P.always_rebuild,
+                                                         f->kind == KIND_VERLET || f->trigger_only, P.selective,
+                                                         cells_written, nullptr);
+  ++ctx->launches;
+  return check_launch("fast_control_kernel");
 }
 
 static int launch_step(spss_ctx *ctx, int stepper, const FastParams &P, cudaGraphExec_t rebuild_exec = nullptr)
@@ -3078,13 +3414,10 @@ static int launch_step(spss_ctx *ctx, int stepper, const FastParams &P, cudaGrap
   if (rebuild_exec)
     fast_control_kernel<true><<<1, 256, 0, ctx->stream>>>(f->ctrl, f->sysctl.ptr, f->sys.ptr, f->nsys,
                                                           P.always_rebuild, f->kind == KIND_VERLET || f->trigger_only,
-                                                          P.selective, f->kind == KIND_CELLS ? 1 : 0, rebuild_exec);
+                                                          P.selective, 0, rebuild_exec);
   else
-    launch_chained(f->chain, fast_control_kernel<false>, 1, 256, 0, ctx->stream, f->ctrl, f->sysctl.ptr,
-                   (const SysParams *) f->sys.ptr, f->nsys, (int) P.always_rebuild,
-                   (int) (f->kind == KIND_VERLET || f->trigger_only), (int) P.selective,
-                   f->kind == KIND_CELLS ? 1 : 0, (cudaGraphExec_t) nullptr);
-  ++ctx->launches;
+    SPSS_TRY(launch_control(ctx, P, 0));
+  if (rebuild_exec) ++ctx->launches;
   return check_launch("fast_control_kernel");
 }
 
@@ -3182,8 +3515,25 @@ int fast_step(spss_ctx *ctx, int stepper, double t, double dt)
   if (stepper == SPSS_STEPPER_RK4) return SPSS_ERR_NOT_SUPPORTED;
   const FastParams P = params(ctx, dt);
   SPSS_TRY(push_host_control(ctx));
-  if (f->h_ctrl->rebuild) SPSS_TRY(launch_rebuild(ctx, P));
-  SPSS_TRY(launch_step(ctx, stepper, P));
+  if (f->kind == KIND_CELLS)
+  {
+    if (f->h_ctrl->rebuild)
+    {
+      SPSS_TRY(ensure_cells(ctx, P));
+      SPSS_TRY(launch_cells_step(ctx, stepper, P, false));
+    } else
+    {
+      // the caller asked for the lists to stay (spss_set_should_update_lists):
+      // a step on the last binning, which counts the cells anew
+      SPSS_CUDA_TRY(cudaMemsetAsync(f->binner.count.ptr, 0, sizeof(int) * f->binner.count.count, ctx->stream));
+      SPSS_TRY(launch_cell_kernel(ctx, stepper, P, 0, false));
+      SPSS_TRY(launch_control(ctx, P, 1));
+    }
+  } else
+  {
+    if (f->h_ctrl->rebuild) SPSS_TRY(launch_rebuild(ctx, P));
+    SPSS_TRY(launch_step(ctx, stepper, P));
+  }
   const int rc = sync_control(ctx);
   if (ctx->timing)
   {
@@ -3317,19 +3667,14 @@ static int build_graph_on(spss_ctx *ctx, int stepper, const FastParams &P, int s
       ctx->launches = launches0;
     }
   }
-  if (!f->device_rebuild) return build_graph_conditional(ctx, stepper, P, sampling, g, launches0);
+  if (!f->device_rebuild && f->kind != KIND_CELLS)
+    return build_graph_conditional(ctx, stepper, P, sampling, g, launches0);
   const unsigned long long launches_step = ctx->launches;
   cudaGraph_t graph = nullptr;
   SPSS_CUDA_TRY(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeRelaxed));
   int rc = SPSS_OK;
-  if (f->kind == KIND_CELLS)
-  {
-    f->chain = true;  // binning, re-sort, layout, step and control as one dependent chain
-    rc = launch_rebuild(ctx, P);
-    g.per_rebuild = 0;
-  }
-  if (rc == SPSS_OK) rc = launch_step(ctx, stepper, P, trigger ? g.rebuild_exec : nullptr);
-  f->chain = false;
+  if (f->kind == KIND_CELLS) rc = launch_cells_step(ctx, stepper, P, true);
+  else rc = launch_step(ctx, stepper, P, trigger ? g.rebuild_exec : nullptr);
   if (rc == SPSS_OK && sampling) rc = launch_sampling(ctx, P, 1);
   const cudaError_t e = cudaStreamEndCapture(ctx->stream, &graph);
   if (rc != SPSS_OK)
@@ -3346,8 +3691,7 @@ static int build_graph_on(spss_ctx *ctx, int stepper, const FastParams &P, int s
   return SPSS_OK;
 }
 
-// nsteps steps: one graph launch each (the first step of a context runs
-// eagerly so that every lazily sized buffer exists before capture).
+// nsteps steps: one graph launch each.
 static int run_steps(spss_ctx *ctx, int stepper, double dt, long nsteps, int sampling)
 {
   FastPath *f = ctx->fast;
@@ -3364,13 +3708,6 @@ static int run_steps(spss_ctx *ctx, int stepper, double dt, long nsteps, int sam
     return sampling ? sync_control(ctx) : SPSS_OK;
   }
   SPSS_TRY(push_host_control(ctx));
-  if (!f->binner.offsets.ptr && has_cells(f->kind))
-  {
-    SPSS_TRY(fast_step(ctx, stepper, 0.0, dt));
-    if (sampling) SPSS_TRY(launch_sampling(ctx, params(ctx, dt), 1));
-    --nsteps;
-    if (nsteps == 0) return sync_control(ctx);
-  }
   auto key = std::make_tuple(stepper, dt, sampling ? 1 : 0);
   auto it = f->graphs.find(key);
   if (it == f->graphs.end())
@@ -3379,6 +3716,7 @@ static int run_steps(spss_ctx *ctx, int stepper, double dt, long nsteps, int sam
     SPSS_TRY(build_graph(ctx, stepper, dt, sampling, g));
     it = f->graphs.emplace(key, g).first;
   }
+  if (f->kind == KIND_CELLS) SPSS_TRY(ensure_cells(ctx, params(ctx, dt)));
   int rebuilds0 = f->h_ctrl->rebuilds;
   if ((it->second.form == GRAPH_DEVICE || it->second.form == GRAPH_NONE) && f->h_ctrl->rebuild)
   {
@@ -3563,9 +3901,9 @@ static int take_snapshot(spss_ctx *ctx)
   {
     SPSS_TRY(copy_device(S.rec[b], f->rec[b].ptr, n, st));
     SPSS_TRY(copy_device(S.aux[b], f->aux[b].ptr, n, st));
+    SPSS_TRY(copy_device(S.vel[b], b ? f->vel_tmp.ptr : f->vel.ptr, n, st));
+    SPSS_TRY(copy_device(S.pid[b], b ? f->pid_tmp.ptr : f->pid.ptr, n, st));
   }
-  SPSS_TRY(copy_device(S.vel, f->vel.ptr, n, st));
-  SPSS_TRY(copy_device(S.pid, f->pid.ptr, n, st));
   SPSS_TRY(copy_device(S.inv, f->inv.ptr, n, st));
   SPSS_TRY(copy_device(S.img, f->img.ptr, n, st));
   SPSS_TRY(copy_device(S.turns, f->turns.ptr, n, st));
@@ -3587,9 +3925,9 @@ static int restore_snapshot(spss_ctx *ctx, bool keep = false)
   {
     SPSS_TRY(restore_device(f->rec[b].ptr, S.rec[b], n, st));
     SPSS_TRY(restore_device(f->aux[b].ptr, S.aux[b], n, st));
+    SPSS_TRY(restore_device(b ? f->vel_tmp.ptr : f->vel.ptr, S.vel[b], n, st));
+    SPSS_TRY(restore_device(b ? f->pid_tmp.ptr : f->pid.ptr, S.pid[b], n, st));
   }
-  SPSS_TRY(restore_device(f->vel.ptr, S.vel, n, st));
-  SPSS_TRY(restore_device(f->pid.ptr, S.pid, n, st));
   SPSS_TRY(restore_device(f->inv.ptr, S.inv, n, st));
   SPSS_TRY(restore_device(f->img.ptr, S.img, n, st));
   SPSS_TRY(restore_device(f->turns.ptr, S.turns, n, st));
@@ -3629,7 +3967,8 @@ int fast_autotune(spss_ctx *ctx, int stepper, double dt, int steps, double *best
   int best_w = f->tile_cells, best_p = f->persistent;
   int rc = SPSS_OK;
   for (int w : widths)
-    for (int pers = 0; pers <= 1 && rc == SPSS_OK; ++pers)
+    // cell-list steps have one launch form
+    for (int pers = 0; pers <= (f->kind == KIND_CELLS ? 0 : 1) && rc == SPSS_OK; ++pers)
     {
       // every candidate from the same state: a list rebuild that the trigger
       // calls for inside the timed steps falls on the same step for all of

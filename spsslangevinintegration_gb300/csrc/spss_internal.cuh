@@ -425,14 +425,41 @@ inline int normals_per_particle(int model, int stepper)
   return model == 1 ? 2 : 6;
 }
 
+// Control words of a GB300-path context, on the device (fast_path.cu).
+struct FastControl
+{
+  unsigned long long step;  // Philox step counter of the next stochastic step
+  double acc;               // accumulated displacement of system 0 (FP64)
+  int parity;               // current rec/aux buffer
+  int order_parity;         // current vel/pid buffer (they change places only when the slots are re-sorted)
+  int rebuild;              // lists (and slot order) rebuilt before the next evaluation
+  int cells_fresh;          // cell ids and counts of the current slots were written by the last cell-list step
+  int overflow;             // largest Verlet count seen beyond capacity (0: none)
+  int rebuilds;             // number of rebuilds performed
+  int error;                // bit 0: displacement too large for the fixed-point increment; bit 1: staging
+                            // timeout; bit 2: stencil cell outside the staged segments; bit 3: the
+                            // device launch of the rebuild graph was refused
+  int uses_verlet;
+  int tile_next;            // work counter of the persistent tile kernel
+  unsigned ticket;          // blocks of the running reduction that are done (its last block puts it back to 0)
+  int triggered;            // the last step's displacement trigger fired (its rebuild may already be done)
+  long long sample_every;   // order-parameter samples after steps that are multiples of this (0: none)
+  long long sample_from;    // ... and not before this step
+};
+
 // Exclusive prefix sum of `n` int32 counts into offsets[0..n] (offsets[n] =
-// total), three-phase with recursion on the block sums.
+// total): block sums, then every block adds the sums before its own and scans
+// its tile (two launches, one for a single tile).  `zero` clears the counts on
+// the way; `ctrl` (not null): the launch also begins a cell-list step
+// (begin_cell_step).
 struct Scanner
 {
   std::vector<DeviceArray<int>> levels;
-  int run(const int *in, int *out, int n, cudaStream_t stream, unsigned long long &launches, bool chained = false);
-  int run_level(const int *in, int *out, int n, size_t level, cudaStream_t stream, unsigned long long &launches,
-                bool chained);
+  int prepare(int n);  // buffers for n counts
+  int run(int *in, int *out, int n, cudaStream_t stream, unsigned long long &launches, bool chained = false,
+          bool zero = false, FastControl *ctrl = nullptr);
+  int run_level(int *in, int *out, int n, size_t level, cudaStream_t stream, unsigned long long &launches, bool chained,
+                bool zero, FastControl *ctrl);
   void release()
   {
     for (auto &l : levels) l.release();
@@ -448,9 +475,15 @@ struct Binner
   DeviceArray<int> count, offsets, slot, members;
   Scanner scanner;
   int ncell = 0;
-  // chained: launches after the first with the programmatic attribute
-  int run(const int *cell_of, int n, int ncell, cudaStream_t stream, unsigned long long &launches,
-          bool chained = false);
+  // buffers for n elements and ncell cells; newly allocated counts are zero
+  int prepare(int n, int ncell, cudaStream_t stream);
+  // From the counts and each element's arrival number in its cell (slot, both
+  // left by the caller's kernel, counts zero before it): offsets, and members
+  // in arrival order; the counts are zero again.
+  int place(const int *cell_of, int n, cudaStream_t stream, unsigned long long &launches, bool chained = false,
+            FastControl *ctrl = nullptr);
+  // all of it, members in ascending order
+  int run(const int *cell_of, int n, int ncell, cudaStream_t stream, unsigned long long &launches);
   void release()
   {
     count.release();
