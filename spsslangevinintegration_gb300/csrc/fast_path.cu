@@ -2914,8 +2914,13 @@ static SysParams system_params(const spss_params &p, int index, int first, int n
   // i.e. in units of 2^-64 of the box area
   const double area = 18446744073709551616.0;
   S.rho2_f = (float) (rho2 * area);
-  // |d2_f - d2| <= 2 (|dx| + |dy|) 2^-32 + 2^-32 + 4 d2 2^-24 near r = rho; doubled
-  S.band_f = (float) (area * 2.0 * (4.0 * p.rho * 2.3283064365386963e-10 + 2.3283064365386963e-10 + 4.0 * rho2 * 5.9604644775390625e-8));
+  // A difference of the 32-bit high words is off by less than 2^-32 of the box,
+  // so |d2_f - d2| <= 2 (|dx| + |dy|) 2^-32 + 2 * 2^-64 + 5 d2 2^-24 (conversions,
+  // square, fma, rounding of rho2_f), with |dx| + |dy| <= 2 rho near r = rho;
+  // doubled.  (A term 2^-32 in place of 2 * 2^-64 had made the band 300 times
+  // wider at N = 4,194,304: 1.2 % of the particles met it every step.)
+  const double word = 2.3283064365386963e-10;  // 2^-32
+  S.band_f = (float) (area * 2.0 * (4.0 * p.rho * word + 2.0 * word * word + 5.0 * rho2 * 5.9604644775390625e-8));
   const double rmax2 = r_max * r_max;
   S.rmax2_f = (float) (area * (rmax2 + 2.0 * (4.0 * r_max * 2.3283064365386963e-10 + 4.0 * rmax2 * 5.9604644775390625e-8)));
   S.half_skin = 0.5 * (r_max - r_min);
