@@ -110,7 +110,6 @@ struct FastBuffers
   const int *cell_off;
   const int *order;            // slots in cell order, arrival order inside a cell
   int *cell_count, *cell_slot; // counts of the next binning, and each slot's arrival number
-  const struct CellTile *cell_tiles;
   short *vl;
   int *vl_cnt;
   float *nu;             // natural frequencies (global field), slot = original index
@@ -123,15 +122,6 @@ struct FastBuffers
   int *tile_maxcnt;  // longest list of each tile (rows to stage)
   void *tiles;       // TileLayout of every tile (Verlet lists), written at rebuild
   FastControl *ctrl;
-};
-
-// A tile of a cell-list step: rows row0 .. row0 + nrows - 1 and columns col0 ..
-// col0 + ncols - 1 of a system's grid (nc x nc cells from cell0 on); fixed with
-// the tiling, so a step needs only the cell offsets to lay its tiles out.
-struct __align__(16) CellTile
-{
-  int sys, row0, nrows, col0;
-  int ncols, nc, cell0, pad;
 };
 
 // The kernel's view of the buffers with vel and pid the current ones.
@@ -224,7 +214,6 @@ struct FastPath
   DeviceArray<int> turns, cell_of, cell_sorted, vl_cnt, tile_maxcnt;
   DeviceArray<short> vl;
   DeviceArray<unsigned char> tiles;
-  DeviceArray<CellTile> cell_tiles;
   DeviceArray<SysParams> sys;
   DeviceArray<int> sys_of, tile_sys;
   DeviceArray<SysControl> sysctl;
@@ -760,7 +749,7 @@ __global__ void fast_after_rebuild_kernel(FastControl *ctrl, SysControl *sysctl,
 // at most six slot segments (three rows, each split in two where the periodic
 // x-wrap crosses the row end).  The CTA stages those segments into shared memory
 // with TMA bulk copies; the Verlet list of a particle in a staged tile stores
-// shared-memory indices directly.  (Cell-list tiles: fast_cell_tile_kernel.)
+// shared-memory indices directly.  (Cell lists need no tiles: fast_cell_step_kernel.)
 
 constexpr int kTileCellsDefault = 32;  // cells per tile unless tuned
 constexpr int kTileCap = 512;     // staged neighbour records per CTA (2 x 8 KiB)
@@ -1983,95 +1972,90 @@ __global__ void __launch_bounds__(kTileThreads, 8) fast_tile_persistent_kernel(F
 
 // ---------------------------------------------------------------- cell-list step
 //
-// One SE or SRK step of the particles of a block of cells (nrows x ncols of a
-// system's grid, about 110 particles) per CTA, neighbours from the 3 x 3 stencil
-// of the cells just sorted (ParticleSystemFirstOrder.cpp:231-353).  The nrows +
-// 2 rows of ncols + 2 cells around it are staged in shared memory by bulk
-// copies, column by column in the order of the grid with the periodic halo
-// columns in place, so the stencil of a cell is one contiguous run of staged
-// records per row, in the reference's order (ParticleSystemFirstOrder.cpp:47-52).
-// Tiles of several rows stage (nrows + 2) / nrows records for each of their own
-// and fill the CTA whatever the grid's width, where one row of a small system's
-// 22 cells held 45 particles for 128 threads.  Instructions bound it: 19
-// candidates a particle at density 2, one comparison each; a particle with a
-// candidate inside the guard band is summed again with the FP64 decisions.
-// The layout comes from the cell offsets alone (no pass of its own), and the
-// update counts the new cells for the next step's binning.
-// 512 systems, 8,852,499 particles (SE): one-row tiles, a run table a tile, the
-// layout, cell and count passes of their own 905 + 30 + 24 + 43 us, this
-// MEASURED_CT us.
-constexpr int kCellRows = 4;    // rows of a tile at most
-constexpr int kCellCols = 64;   // columns of a tile at most
-constexpr int kCellTarget = 112;  // mean particles of a tile: 128 threads less 1.5 standard deviations
-
-struct CellRows
+// One SE or SRK step of one particle per thread, neighbours from the 3 x 3
+// stencil of the cells just sorted (ParticleSystemFirstOrder.cpp:231-353).  Slots
+// are in cell order, so the stencil of a cell is one run of slots per row (two
+// where the periodic x-wrap crosses the row's end), in the reference's order
+// (ParticleSystemFirstOrder.cpp:47-52), and a warp's runs largely coincide: the
+// records come through L1 without staging, and every warp has 32 particles
+// whatever their density (flocking runs cluster: after 20,000 steps at N = 65,536
+// cells hold up to 100 particles, where tiles of cells took 308 us a step, this
+// 44).  One comparison a candidate; a particle with a candidate inside the guard
+// band is summed again with the FP64 decisions.  Instructions bound it (19
+// candidates a particle at density 2).  512 systems, 8,852,499 particles, SE:
+// staged one-row tiles with a layout pass 905 us, staged tiles of several rows
+// 446, this 392; staging a warp's stretch of records in shared memory instead of
+// leaving it to L1 ran 15 % slower, two candidates at a time everywhere as fast
+// here and 20 % slower in clusters, 6 resident blocks of 256 threads 3 % slower.
+template<bool OMEGA>
+struct CellSums
 {
-  int base[kCellRows + 2];   // staged index of the row's first record
-  int left[kCellRows + 2], main[kCellRows + 2], right[kCellRows + 2];     // slots of its three pieces
-  int nleft[kCellRows + 2], nmain[kCellRows + 2], nright[kCellRows + 2];  // and their records
-  int total;
-  int own[kCellRows + 1];    // particles of the tile before each of its rows
+  float2 cs, w;
+  int card;
+  float nearest;  // smallest distance of a candidate's d2 to rho^2
 };
 
-// Slot of a staged record of row rr.
-__device__ __forceinline__ int cell_slot_of(const CellRows &R, int rr, int idx)
+// U candidates from s on (CLAMP: those at e and beyond left out) but `self`,
+// decided in FP32; their loads are in flight together.
+template<bool OMEGA, int U, bool CLAMP>
+__device__ __forceinline__ void cell_group(const uint4 *__restrict__ rec, const uint4 *__restrict__ aux, int s, int e,
+                                           int self, uint32_t xi, uint32_t yi, float rho2, CellSums<OMEGA> &a)
 {
-  int k = idx - R.base[rr];
-  if (k < R.nleft[rr]) return R.left[rr] + k;
-  k -= R.nleft[rr];
-  if (k < R.nmain[rr]) return R.main[rr] + k;
-  return R.right[rr] + (k - R.nmain[rr]);
-}
-
-// Neighbour sums of one particle again, with in_range's decision for every
-// candidate (some candidate lies inside the guard band).
-template<bool OMEGA>
-__device__ __noinline__ void cell_sums_exact(const CellRows &R, const short (*soff)[kCellCols + 4], const uint4 *srec,
-                                             const uint4 *saux, const uint4 *__restrict__ aux, int r, int lc, int self,
-                                             const uint4 ri, const uint4 ai, float rho2, float band, double rho2_d,
-                                             Acc *acc)
-{
-  const uint64_t Xi = join64(ri.x, ai.x), Yi = join64(ri.y, ai.y);
-  Acc a{0.f, 0.f, 0.f, 0.f, 0};
-  for (int rr = r; rr < r + 3; ++rr)
-    for (int idx = soff[rr][lc]; idx < soff[rr][lc + 3]; ++idx)
+  uint4 r[U];
+  float w[U], d2[U];
+#pragma unroll
+  for (int k = 0; k < U; ++k)
+  {
+    const int t = CLAMP ? min(s + k, e - 1) : s + k;
+    r[k] = __ldg(rec + t);
+    w[k] = OMEGA ? __uint_as_float(__ldg(&aux[t].w)) : 0.0f;
+  }
+#pragma unroll
+  for (int k = 0; k < U; ++k)
+  {
+    const float dx = (float) (int) (r[k].x - xi), dy = (float) (int) (r[k].y - yi);
+    d2[k] = fmaf(dx, dx, dy * dy);
+    if (s + k == self || (CLAMP && s + k >= e)) d2[k] = 3.0e38f;
+    a.nearest = fminf(a.nearest, fabsf(d2[k] - rho2));
+  }
+#pragma unroll
+  for (int k = 0; k < U; ++k)
+    if (d2[k] <= rho2)
     {
-      if (idx == self) continue;
-      const uint4 rj = srec[idx];
-      const float dx = (float) (int) (rj.x - ri.x), dy = (float) (int) (rj.y - ri.y);
-      const float d2 = fmaf(dx, dx, dy * dy);
-      bool in = d2 <= rho2;
-      if (fabsf(d2 - rho2) <= band)
-      {
-        const uint2 l = __ldg(reinterpret_cast<const uint2 *>(&aux[cell_slot_of(R, rr, idx)]));
-        in = exact_within_inline(rj.x, rj.y, l.x, l.y, Xi, Yi, rho2_d);
-      }
-      if (in) accumulate(a, rj, OMEGA ? __uint_as_float(saux[idx].w) : 0.0f);
+      const float2 c = make_float2(__uint_as_float(r[k].z), __uint_as_float(r[k].w));
+      a.cs = add2(a.cs, c);
+      if (OMEGA) a.w = fma2(make_float2(w[k], w[k]), c, a.w);
+      a.card += 1;
     }
-  *acc = a;
 }
 
-#ifndef SPSS_CELL_BLOCKS_SE
-#define SPSS_CELL_BLOCKS_SE 12
+// Candidates [s, e): in fours while they last (the long runs of dense cells),
+// the rest in twos.
+template<bool OMEGA>
+__device__ __forceinline__ void cell_run(const uint4 *__restrict__ rec, const uint4 *__restrict__ aux, int s, int e,
+                                         int self, uint32_t xi, uint32_t yi, float rho2, CellSums<OMEGA> &a)
+{
+#pragma unroll 1
+  for (; s + 4 <= e; s += 4) cell_group<OMEGA, 4, false>(rec, aux, s, e, self, xi, yi, rho2, a);
+#pragma unroll 1
+  for (; s < e; s += 2) cell_group<OMEGA, 2, true>(rec, aux, s, e, self, xi, yi, rho2, a);
+}
+
+#ifndef SPSS_CELL_BLOCKS
+#define SPSS_CELL_BLOCKS 12
 #endif
-#ifndef SPSS_CELL_BLOCKS_SRK
-#define SPSS_CELL_BLOCKS_SRK 9
-#endif
+constexpr int kCellThreads = 128;
 
 // `fresh`: the slots were just re-sorted (the particles stand in the other
 // rec/aux buffer, the step was counted by the scan); 0: a step on the lists of
 // an earlier binning.
 template<int MODEL, int STEPPER, bool MULTI>
-__global__ void __launch_bounds__(kTileThreads, STEPPER == 2 ? SPSS_CELL_BLOCKS_SRK : SPSS_CELL_BLOCKS_SE)
-    fast_cell_tile_kernel(FastParams P, FastBuffers B, int fresh)
+__global__ void __launch_bounds__(kCellThreads, SPSS_CELL_BLOCKS) fast_cell_step_kernel(FastParams P, FastBuffers B, int fresh)
 {
-  __shared__ __align__(16) uint4 srec[kTileCap];
-  __shared__ __align__(16) uint4 saux[STEPPER == 2 ? kTileCap : 1];  // aux words: SRK only (neighbour omega)
-  __shared__ __align__(8) unsigned long long mbar;
-  __shared__ CellRows R;
-  __shared__ short soff[kCellRows + 2][kCellCols + 4];  // staged start of each column, halo columns included
-  __shared__ int staged_all;
   pdl_enter();
+  constexpr bool OMEGA = STEPPER == 2;
+  const int q = blockIdx.x * kCellThreads + threadIdx.x;
+  if (q >= P.n) return;
   FastControl *ctrl = B.ctrl;
   const int par = ctrl->parity ^ fresh;
   buffers_now(B, ctrl->order_parity);
@@ -2079,186 +2063,59 @@ __global__ void __launch_bounds__(kTileThreads, STEPPER == 2 ? SPSS_CELL_BLOCKS_
   const uint4 *ain = par ? B.aux1 : B.aux0;
   uint4 *rout = par ? B.rec0 : B.rec1;
   uint4 *aout = par ? B.aux0 : B.aux1;
-  const unsigned long long step = ctrl->step - (unsigned long long) fresh;
-  const CellTile T = B.cell_tiles[blockIdx.x];
-  const int *coff = B.cell_off + T.cell0;
-  const int nc = T.nc, rows = T.nrows + 2;
-  const uint32_t mb = smem_u32(&mbar);
-  if (threadIdx.x < 32)
-  {
-    const int lane = threadIdx.x;
-    int left = 0, main = 0, right = 0, nl = 0, nm = 0, nr = 0;
-    if (lane < rows)
-    {
-      const int row = wrap_cell(T.row0 - 1 + lane, nc) * nc;
-      const int lx = row + wrap_cell(T.col0 - 1, nc), rx = row + wrap_cell(T.col0 + T.ncols, nc);
-      left = coff[lx];
-      main = coff[row + T.col0];
-      right = coff[rx];
-      nl = coff[lx + 1] - left;
-      nm = coff[row + T.col0 + T.ncols] - main;
-      nr = coff[rx + 1] - right;
-    }
-    const int len = nl + nm + nr;
-    int end = len, own = (lane >= 1 && lane <= T.nrows) ? nm : 0;
-#pragma unroll
-    for (int off = 1; off < 8; off <<= 1)
-    {
-      const int y = __shfl_up_sync(0xffffffffu, end, off), z = __shfl_up_sync(0xffffffffu, own, off);
-      if (lane >= off)
-      {
-        end += y;
-        own += z;
-      }
-    }
-    const int total = __shfl_sync(0xffffffffu, end, rows - 1), np = __shfl_sync(0xffffffffu, own, T.nrows);
-    const bool staged = nc >= 3 && total <= kTileCap && np > 0;
-    if (lane < rows)
-    {
-      R.base[lane] = end - len;
-      R.left[lane] = left;
-      R.main[lane] = main;
-      R.right[lane] = right;
-      R.nleft[lane] = nl;
-      R.nmain[lane] = nm;
-      R.nright[lane] = nr;
-      if (lane <= T.nrows) R.own[lane] = own;
-    }
-    if (lane == 0)
-    {
-      R.total = total;
-      staged_all = staged;
-      if (staged)
-      {
-        init_mbarrier(mb);
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mb),
-                     "r"((STEPPER == 2 ? 32u : 16u) * (uint32_t) total)
-                     : "memory");
-      }
-    }
-    __syncwarp();
-    if (staged && lane < rows)
-    {
-      // pieces that follow each other in the slot order are one copy
-      int at = end - len, from[3] = {left, main, right}, n[3] = {nl, nm, nr};
-      if (left + nl == main)
-      {
-        from[1] = left;
-        n[1] += nl;
-        n[0] = 0;
-      }
-      if (from[1] + n[1] == right)
-      {
-        n[1] += nr;
-        n[2] = 0;
-      }
-#pragma unroll
-      for (int k = 0; k < 3; ++k)
-      {
-        if (n[k] == 0) continue;
-        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                         smem_u32(&srec[at])),
-                     "l"(rin + from[k]), "r"(16u * (uint32_t) n[k]), "r"(mb)
-                     : "memory");
-        if (STEPPER == 2)
-          asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                           smem_u32(&saux[at])),
-                       "l"(ain + from[k]), "r"(16u * (uint32_t) n[k]), "r"(mb)
-                       : "memory");
-        at += n[k];
-      }
-    }
-  }
-  __syncthreads();
-  const bool staged = staged_all;
-  const int np = R.own[T.nrows];
-  if (np == 0) return;
-  const SysParams *S = MULTI ? B.sys + T.sys : nullptr;
+  const SysParams *S = MULTI ? B.sys + B.sys_of[q] : nullptr;
+  const int cell0 = MULTI ? S->cell0 : P.cell0, nc = MULTI ? S->nc : P.nc;
   const float rho2 = MULTI ? S->rho2_f : P.rho2_f, band = MULTI ? S->band_f : P.band_f;
-  // the thread's first particle and the column offsets, on their way while the records land
-  int i = threadIdx.x, r = 0, q = 0, lc = 0;
-  OwnParticle o;
-  auto take = [&](int k) {
-    r = 0;
-    while (r + 1 < T.nrows && k >= R.own[r + 1]) ++r;
-    q = R.main[r + 1] + (k - R.own[r]);
-    o = load_own<MODEL, KIND_CELLS>(B, rin, ain, q);
-    lc = B.cell_sorted[q] - T.cell0 - (T.row0 + r) * nc - T.col0;
-  };
-  if (i < np) take(i);
-  if (staged)
+  const int c = B.cell_sorted[q] - cell0;
+  const uint4 ri = rin[q];
+  const int cy = c / nc, cx = c - cy * nc;
+  const int *coff = B.cell_off + cell0;
+  CellSums<OMEGA> a{make_float2(0.f, 0.f), make_float2(0.f, 0.f), 0, 3.0e38f};
+  if (nc >= 3)
   {
-    for (int w = threadIdx.x; w < rows * (T.ncols + 3); w += kTileThreads)
+    const int lo = max(cx - 1, 0), hi = min(cx + 2, nc);
+    int s[3], e[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
     {
-      const int rr = w / (T.ncols + 3), c = w - rr * (T.ncols + 3);
-      int at = R.base[rr];
-      if (c > T.ncols + 1) at += R.nleft[rr] + R.nmain[rr] + R.nright[rr];
-      else if (c > 0) at += R.nleft[rr] + coff[wrap_cell(T.row0 - 1 + rr, nc) * nc + T.col0 + c - 1] - R.main[rr];
-      soff[rr][c] = (short) at;
+      const int row = wrap_cell(cy + k - 1, nc) * nc;
+      s[k] = coff[row + lo];
+      e[k] = coff[row + hi];
     }
-    const uint32_t done = wait_phase(mb, 0);
-    if (!__syncthreads_and(done))
+    if (cx > 0 && cx + 1 < nc)
     {
-      // the copies did not complete in time: report, give them a second
-      // bounded wait so none is in flight when the CTA exits, and stop
-      if (threadIdx.x == 0) atomicOr(&ctrl->error, 2);
-      wait_phase(mb, 0);
-      return;
-    }
-  }
-  int err = 0;
-  for (; i < np; i += kTileThreads)
-  {
-    if (i != (int) threadIdx.x) take(i);
-    Acc a{0.f, 0.f, 0.f, 0.f, 0};
-    if (staged)
-    {
-      const int self = R.base[r + 1] + R.nleft[r + 1] + (q - R.main[r + 1]);
-      float2 cs = make_float2(0.f, 0.f), w = make_float2(0.f, 0.f);
-      int card = 0;
-      float nearest = 3.0e38f;
-#pragma unroll 1
-      for (int rr = r; rr < r + 3; ++rr)
-      {
-        const int e = soff[rr][lc + 3];
-#pragma unroll 2
-        for (int idx = soff[rr][lc]; idx < e; ++idx)
-        {
-          const uint4 rj = srec[idx];
-          const float wj = STEPPER == 2 ? __uint_as_float(saux[idx].w) : 0.0f;
-          const float dx = (float) (int) (rj.x - o.r.x);
-          const float dy = (float) (int) (rj.y - o.r.y);
-          float d2 = fmaf(dx, dx, dy * dy);
-          if (idx == self) d2 = 3.0e38f;
-          nearest = fminf(nearest, fabsf(d2 - rho2));
-          if (d2 <= rho2)
-          {
-            const float2 t = make_float2(__uint_as_float(rj.z), __uint_as_float(rj.w));
-            cs = add2(cs, t);
-            if (STEPPER == 2) w = fma2(make_float2(wj, wj), t, w);
-            card += 1;
-          }
-        }
-      }
-      a = Acc{cs.y, cs.x, w.y, w.x, card};
-      if (nearest <= band)
-      {
-        Acc again;
-        cell_sums_exact<STEPPER == 2>(R, soff, srec, saux, ain, r, lc, self, o.r, o.a, rho2, band,
-                                      MULTI ? S->rho2_d : P.rho2_d, &again);
-        a = again;
-      }
+#pragma unroll
+      for (int k = 0; k < 3; ++k) cell_run<OMEGA>(rin, ain, s[k], e[k], q, ri.x, ri.y, rho2, a);
     } else
     {
-      const FastParams Q = MULTI ? with_system(P, *S) : P;
-      gather_sums<KIND_CELLS, STEPPER == 2>(Q, B, rin, ain, q, 0, nullptr, 0, o.r, join64(o.r.x, o.a.x),
-                                            join64(o.r.y, o.a.y), a);
+      for (int k = 0; k < 3; ++k)
+      {
+        const int row = wrap_cell(cy + k - 1, nc) * nc;
+        const int wx = row + (cx == 0 ? nc - 1 : 0);
+        const int ws = coff[wx], we = coff[wx + 1];
+        const int rs = coff[row + lo], re = coff[row + hi];
+        if (cx == 0) cell_run<OMEGA>(rin, ain, ws, we, q, ri.x, ri.y, rho2, a);
+        cell_run<OMEGA>(rin, ain, rs, re, q, ri.x, ri.y, rho2, a);
+        if (cx != 0) cell_run<OMEGA>(rin, ain, ws, we, q, ri.x, ri.y, rho2, a);
+      }
     }
-    const FastParams Q = MULTI ? with_system(P, *S) : P;
-    float z[6];
-    draw_noise<MODEL, STEPPER>(Q, step, o.p, z);
-    update_particle<MODEL, STEPPER, true>(Q, B, q, o.r, o.a, o.v, a, z, rout, aout, err);
   }
+  const uint4 ai = ain[q];
+  Acc t{a.cs.y, a.cs.x, a.w.y, a.w.x, a.card};
+  const FastParams Q = MULTI ? with_system(P, *S) : P;
+  if (nc < 3 || a.nearest <= band)
+  {
+    // fewer than three cells a side (the stencil meets cells more than once), or
+    // a candidate inside the guard band: candidate by candidate, with the FP64
+    // decisions
+    t = Acc{0.f, 0.f, 0.f, 0.f, 0};
+    gather_sums<KIND_CELLS, OMEGA>(Q, B, rin, ain, q, 0, nullptr, 0, ri, join64(ri.x, ai.x), join64(ri.y, ai.y), t);
+  }
+  int err = 0;
+  float z[6];
+  draw_noise<MODEL, STEPPER>(Q, ctrl->step - (unsigned long long) fresh, B.pid[q], z);
+  update_particle<MODEL, STEPPER, true>(Q, B, q, ri, ai, MODEL == 2 ? B.vel[q] : make_float2(0.f, 0.f), t, z, rout, aout,
+                                        err);
   if (err) atomicOr(&ctrl->error, 1);
 }
 
@@ -2869,7 +2726,6 @@ static FastBuffers buffers(spss_ctx *ctx)
   B.order = f->binner.members.ptr;
   B.cell_count = f->binner.count.ptr;
   B.cell_slot = f->binner.slot.ptr;
-  B.cell_tiles = f->cell_tiles.ptr;
   B.vl = f->vl.ptr;
   B.vl_cnt = f->vl_cnt.ptr;
   B.tile_maxcnt = f->tile_maxcnt.ptr;
@@ -2985,55 +2841,19 @@ static int set_tiling(spss_ctx *ctx, int tile_cells)
   f->tile_cells = tile_cells;
   int ntiles = 0;
   std::vector<int> tile_sys;
-  std::vector<CellTile> cell_tiles;
   for (int r = 0; r < f->nsys; ++r)
   {
     SysParams &S = f->h_sys[r];
     S.tile0 = ntiles;
-    if (f->kind == KIND_CELLS)
-    {
-      // as many whole rows of at most tile_cells cells as fill a CTA, no tile
-      // much smaller than the others
-      const double occupancy = (double) S.n / ((double) S.nc * S.nc);
-      const int widest = std::max(1, std::min({tile_cells, kCellCols, (int) (kCellTarget / occupancy), S.nc}));
-      const int nbx = tiles_per_row(S.nc, widest);
-      const double row = occupancy * S.nc / nbx;  // mean particles of a tile's row
-      const int high = std::max(1, std::min({kCellRows, (int) std::lround(kCellTarget / row), S.nc}));
-      const int nby = tiles_per_row(S.nc, high);
-      for (int y = 0; y < nby; ++y)
-        for (int x = 0; x < nbx; ++x)
-        {
-          CellTile T{};
-          T.sys = r;
-          T.row0 = (int) ((long) S.nc * y / nby);
-          T.nrows = (int) ((long) S.nc * (y + 1) / nby) - T.row0;
-          T.col0 = (int) ((long) S.nc * x / nbx);
-          T.ncols = (int) ((long) S.nc * (x + 1) / nbx) - T.col0;
-          T.nc = S.nc;
-          T.cell0 = S.cell0;
-          cell_tiles.push_back(T);
-        }
-      S.ntiles = nbx * nby;
-      ntiles += S.ntiles;
-      continue;
-    }
     S.ntiles = S.nc * tiles_per_row(S.nc, tile_cells);
     ntiles += S.ntiles;
     tile_sys.insert(tile_sys.end(), (size_t) S.ntiles, r);
   }
   f->ntiles = ntiles;
-  if (f->kind == KIND_CELLS)
-  {
-    SPSS_TRY(f->cell_tiles.reserve((size_t) ntiles));
-    SPSS_CUDA_TRY(cudaMemcpyAsync(f->cell_tiles.ptr, cell_tiles.data(), sizeof(CellTile) * ntiles,
-                                  cudaMemcpyHostToDevice, ctx->stream));
-  } else
-  {
-    SPSS_TRY(f->tiles.reserve(sizeof(TileLayout) * (size_t) ntiles));
-    SPSS_TRY(f->tile_sys.reserve((size_t) ntiles));
-    SPSS_CUDA_TRY(cudaMemcpyAsync(f->tile_sys.ptr, tile_sys.data(), sizeof(int) * ntiles, cudaMemcpyHostToDevice,
-                                  ctx->stream));
-  }
+  SPSS_TRY(f->tiles.reserve(sizeof(TileLayout) * (size_t) ntiles));
+  SPSS_TRY(f->tile_sys.reserve((size_t) ntiles));
+  SPSS_CUDA_TRY(cudaMemcpyAsync(f->tile_sys.ptr, tile_sys.data(), sizeof(int) * ntiles, cudaMemcpyHostToDevice,
+                                ctx->stream));
   SPSS_CUDA_TRY(cudaMemcpyAsync(f->sys.ptr, f->h_sys.data(), sizeof(SysParams) * f->nsys, cudaMemcpyHostToDevice,
                                 ctx->stream));
   if (f->kind == KIND_VERLET)
@@ -3230,7 +3050,6 @@ void fast_destroy(spss_ctx *ctx)
   f->vl_cnt.release();
   f->tile_maxcnt.release();
   f->tiles.release();
-  f->cell_tiles.release();
   f->sys.release();
   f->sys_of.release();
   f->tile_sys.release();
@@ -3311,10 +3130,11 @@ static int ensure_cells(spss_ctx *ctx, const FastParams &P)
 template<int MODEL, int STEPPER>
 static void launch_cell_tiles(spss_ctx *ctx, const FastParams &P, const FastBuffers &B, int fresh, bool chained)
 {
+  const int blocks = blocks_for(P.n, kCellThreads);
   if (P.nsys > 1)
-    launch_chained(chained, fast_cell_tile_kernel<MODEL, STEPPER, true>, P.ntiles, kTileThreads, 0, ctx->stream, P, B, fresh);
+    launch_chained(chained, fast_cell_step_kernel<MODEL, STEPPER, true>, blocks, kCellThreads, 0, ctx->stream, P, B, fresh);
   else
-    launch_chained(chained, fast_cell_tile_kernel<MODEL, STEPPER, false>, P.ntiles, kTileThreads, 0, ctx->stream, P, B, fresh);
+    launch_chained(chained, fast_cell_step_kernel<MODEL, STEPPER, false>, blocks, kCellThreads, 0, ctx->stream, P, B, fresh);
 }
 
 static int launch_cell_kernel(spss_ctx *ctx, int stepper, const FastParams &P, int fresh, bool chained)
@@ -3331,7 +3151,7 @@ static int launch_cell_kernel(spss_ctx *ctx, int stepper, const FastParams &P, i
     else launch_cell_tiles<2, 2>(ctx, P, B, fresh, chained);
   }
   ++ctx->launches;
-  SPSS_TRY(check_launch("fast_cell_tile_kernel"));
+  SPSS_TRY(check_launch("fast_cell_step_kernel"));
   if (ctx->timing) SPSS_CUDA_TRY(cudaEventRecord(ctx->ev1, ctx->stream));
   return SPSS_OK;
 }
