@@ -62,11 +62,11 @@ enum
 // One independent system of a context (a context holds one or a batch of
 // them; each is the reference's particle system on its own unit box).  Its
 // particles are the slots [first, first + n) in every slot order, its cells
-// the global cells [cell0, cell0 + nc^2), its tiles [tile0, tile0 + ntiles).
+// the global cells [cell0, cell0 + nc^2).
 struct SysParams
 {
   int n, first, nc, cell0;
-  int tile0, ntiles, index, replica;
+  int index, replica;
   float v0, xi, xi_r, xi_phi, sigma, ca, sa, rho2_f;
   float band_f, rmax2_f, b_r, b_phi;
   double rho2_d, half_skin;
@@ -86,8 +86,8 @@ enum Kind
 struct FastParams
 {
   int n, nc, cap, model;      // n: slots of the whole context
-  int kind, always_rebuild, tile_cells, persistent;
-  int nsys, ntiles, first, sub_n;
+  int kind, always_rebuild, nsys;
+  int first, sub_n;
   int cell0, sys, selective, pad1;  // selective: per-system rebuilds (batches of Verlet-list systems)
   float v0, xi, xi_r, xi_phi, sigma, ca, sa;
   float rho2_f, band_f, rmax2_f;
@@ -108,6 +108,7 @@ struct FastBuffers
   int *turns;  // 2 pi turns of the phase, by original index
   int *cell_of, *cell_sorted;
   const int *cell_off;
+  int *cell_off_w;  // the same offsets, for the kernel that writes a system's
   const int *order;            // slots in cell order, arrival order inside a cell
   int *cell_count, *cell_slot; // counts of the next binning, and each slot's arrival number
   short *vl;
@@ -117,10 +118,7 @@ struct FastBuffers
   double *field_partial; // block partials of the field sums
   const SysParams *sys;  // system table
   const int *sys_of;     // system of each slot (equivalently of each original index)
-  const int *tile_sys;   // system of each tile
   SysControl *sysctl;
-  int *tile_maxcnt;  // longest list of each tile (rows to stage)
-  void *tiles;       // TileLayout of every tile (Verlet lists), written at rebuild
   FastControl *ctrl;
 };
 
@@ -211,11 +209,10 @@ struct FastPath
   DeviceArray<float2> vel, vel_tmp;
   DeviceArray<unsigned> pid, pid_tmp, inv;
   DeviceArray<int2> img;
-  DeviceArray<int> turns, cell_of, cell_sorted, vl_cnt, tile_maxcnt;
+  DeviceArray<int> turns, cell_of, cell_sorted, vl_cnt;
   DeviceArray<short> vl;
-  DeviceArray<unsigned char> tiles;
   DeviceArray<SysParams> sys;
-  DeviceArray<int> sys_of, tile_sys;
+  DeviceArray<int> sys_of;
   DeviceArray<SysControl> sysctl;
   DeviceArray<float> nu;
   DeviceArray<float> field;
@@ -227,10 +224,8 @@ struct FastPath
   std::vector<SysParams> h_sys;
   int nsys = 1;
   int total_cells = 1;
-  int ntiles = 0;
-  int tile_cells = 32;
+  int tile_cells = 32;  // spss_set_tiling: reported back, no kernel depends on them
   int persistent = 0;
-  int persistent_grid = 0;
   Binner binner;
   FastControl *ctrl = nullptr;    // device
   FastControl *h_ctrl = nullptr;  // pinned mirror
@@ -241,6 +236,7 @@ struct FastPath
   bool trigger_only = false;
   int nc_build = 1;
   int cap = 0;
+  bool small_systems = false;  // a batch of Verlet-list systems that one CTA each rebuilds
   bool have_state = false;
   bool perm_valid = false;
   std::map<std::tuple<int, double, int>, GraphEntry> graphs;  // (stepper, dt, with sampling)
@@ -371,44 +367,16 @@ struct Acc
   int card;
 };
 
-// One candidate pair: FP32 distance from the 32-bit high words (exact minimum
-// image by integer subtraction); inside the guard band the decision is
-// recomputed in FP64 from the full 64-bit positions, so it equals the FP64
-// decision for these positions.
-// The FP64 cutoff decision from the full 64-bit positions, for a pair inside
-// the guard band (a few pairs per step).
-__device__ __forceinline__ bool exact_within_inline(uint32_t xh, uint32_t yh, uint32_t xl, uint32_t yl, uint64_t Xi,
-                                                   uint64_t Yi, double rho2)
+// A candidate pair is decided by its FP32 distance from the 32-bit high words
+// (exact minimum image by integer subtraction); inside the guard band the FP64
+// distance of the full 64-bit positions decides, so the neighbour set is the
+// FP64 one for these positions.
+__device__ __forceinline__ bool exact_within(uint32_t xh, uint32_t yh, uint32_t xl, uint32_t yl, uint64_t Xi,
+                                             uint64_t Yi, double rho2)
 {
   const double ex = (double) (long long) (join64(xh, xl) - Xi) * 5.421010862427522e-20;
   const double ey = (double) (long long) (join64(yh, yl) - Yi) * 5.421010862427522e-20;
   return __dadd_rn(__dmul_rn(ex, ex), __dmul_rn(ey, ey)) <= rho2;
-}
-
-// Out of line, for the stencil scans: keeps their loops small in the
-// instruction cache (the Verlet-list walk keeps the inline form, which costs
-// no call).
-__device__ __noinline__ bool exact_within(uint32_t xh, uint32_t yh, uint32_t xl, uint32_t yl, uint64_t Xi,
-                                          uint64_t Yi, double rho2)
-{
-  return exact_within_inline(xh, yh, xl, yl, Xi, Yi, rho2);
-}
-
-template<bool OUTLINE>
-__device__ __forceinline__ bool in_range(const FastParams &P, const uint4 &ri, uint64_t Xi, uint64_t Yi,
-                                         const uint4 &rj, const uint4 *__restrict__ aux, int j)
-{
-  const float dx = (float) (int) (rj.x - ri.x);
-  const float dy = (float) (int) (rj.y - ri.y);
-  const float d2 = fmaf(dx, dx, dy * dy);
-  bool in = d2 <= P.rho2_f;
-  if (fabsf(d2 - P.rho2_f) <= P.band_f)
-  {
-    const uint2 l = __ldg(reinterpret_cast<const uint2 *>(&aux[j]));
-    in = OUTLINE ? exact_within(rj.x, rj.y, l.x, l.y, Xi, Yi, P.rho2_d)
-                 : exact_within_inline(rj.x, rj.y, l.x, l.y, Xi, Yi, P.rho2_d);
-  }
-  return in;
 }
 
 __device__ __forceinline__ void accumulate(Acc &a, const uint4 &rj, float wj)
@@ -419,36 +387,6 @@ __device__ __forceinline__ void accumulate(Acc &a, const uint4 &rj, float wj)
   a.wc = fmaf(wj, cj, a.wc);
   a.ws = fmaf(wj, sj, a.ws);
   a.card += 1;
-}
-
-template<bool OMEGA, bool OUTLINE>
-__device__ __forceinline__ void candidate(const FastParams &P, const uint4 &ri, uint64_t Xi, uint64_t Yi,
-                                          const uint4 *__restrict__ rec, const uint4 *__restrict__ aux, int j, Acc &a)
-{
-  const uint4 rj = __ldg(&rec[j]);
-  if (in_range<OUTLINE>(P, ri, Xi, Yi, rj, aux, j)) accumulate(a, rj, OMEGA ? __uint_as_float(__ldg(&aux[j].w)) : 0.0f);
-}
-
-// Four list entries at a time: the entry loads, then the record loads, then
-// the omega loads of the pairs in range are issued together, so a thread has
-// several gathers in flight instead of a chain of dependent ones.
-template<bool OMEGA, bool OUTLINE>
-__device__ __forceinline__ void candidates4(const FastParams &P, const uint4 &ri, uint64_t Xi, uint64_t Yi,
-                                            const uint4 *__restrict__ rec, const uint4 *__restrict__ aux,
-                                            const int j[4], Acc &a)
-{
-  uint4 r[4];
-#pragma unroll
-  for (int u = 0; u < 4; ++u) r[u] = __ldg(&rec[j[u]]);
-  bool in[4];
-#pragma unroll
-  for (int u = 0; u < 4; ++u) in[u] = in_range<OUTLINE>(P, ri, Xi, Yi, r[u], aux, j[u]);
-  float w[4];
-#pragma unroll
-  for (int u = 0; u < 4; ++u) w[u] = (OMEGA && in[u]) ? __uint_as_float(__ldg(&aux[j[u]].w)) : 0.0f;
-#pragma unroll
-  for (int u = 0; u < 4; ++u)
-    if (in[u]) accumulate(a, r[u], w[u]);
 }
 
 // ---------------------------------------------------------------- conversions
@@ -735,273 +673,37 @@ __global__ void fast_after_rebuild_kernel(FastControl *ctrl, SysControl *sysctl,
   }
 }
 
-// ---------------------------------------------------------------- tiles
-//
-// Verlet lists: a tile is a run of whole cells of one row of a system's rebuild
-// grid; one CTA steps the particles of a tile.  A row holds ceil(nc /
-// tile_cells) tiles, which split the row's particles into runs of nearly equal
-// count (boundaries at cell edges), so a tile of about 120 particles fills
-// its 128 threads whatever the local density, where runs of equal width leave
-// Poisson counts above 128 to a second pass of a few threads (36-cell tiles
-// at N = 4,194,304: 0.1963 -> 0.1882 ms per launch, same bits); the layout is
-// computed once per rebuild.  Slots are sorted by cell, so the tile's particles
-// are one slot range and the records of its 3 x (width + 2) neighbour cells are
-// at most six slot segments (three rows, each split in two where the periodic
-// x-wrap crosses the row end).  The CTA stages those segments into shared memory
-// with TMA bulk copies; the Verlet list of a particle in a staged tile stores
-// shared-memory indices directly.  (Cell lists need no tiles: fast_cell_step_kernel.)
-
-constexpr int kTileCellsDefault = 32;  // cells per tile unless tuned
-constexpr int kTileCap = 512;     // staged neighbour records per CTA (2 x 8 KiB)
 constexpr int kTileThreads = 128;
-// Resident CTAs per SM the Stochastic Euler Verlet tile kernel is compiled for:
-// 10 (48 registers, 4 to 16 bytes spilled); the 512-system sweep at 36-cell
-// tiles ran 0.684 / 0.623 / 0.553 / 0.573 ms per step at 14 / 12 / 10 / 9.
-#ifndef SPSS_SE_VERLET_TILE_BLOCKS
-#define SPSS_SE_VERLET_TILE_BLOCKS 10
-#endif
-constexpr long long kWaitCycles = 1ll << 31;  // about one second at the SM clock
 
-struct TileLayout
-{
-  int p_begin, p_end;  // slots of the tile's own particles
-  int nseg, total;     // staged segments (ascending slot order) and records
-  int start[6], len[6], base[6];
-  int staged;          // the neighbourhood fits kTileCap records
-  int row, col0, ncols;  // the tile's cells: row `row`, columns col0 .. col0 + ncols - 1
-};
+// ---------------------------------------------------------------- step
 
-// Stencil of one cell of a staged tile (list build): for each stencil row (dy =
-// -1, 0, 1) the staged records of the three cells (cx - 1, cx, cx + 1, wrapped)
-// as at most three contiguous runs of staged indices, in the reference's
-// stencil order (ParticleSystemFirstOrder.cpp:47-52).
-constexpr int kRunCells = 64;  // widest tile with a run table
-struct StencilRuns
+// One candidate slot j of particle q, with the decision above.
+template<bool OMEGA>
+__device__ __forceinline__ void exact_candidate(const uint4 *__restrict__ rec, const uint4 *__restrict__ aux, int j,
+                                                const uint4 &ri, uint64_t Xi, uint64_t Yi, float rho2, float band,
+                                                double rho2_d, Acc &a)
 {
-  short s[3][3], e[3][3];  // [dy + 1][piece]
-};
-
-__host__ __device__ __forceinline__ int tiles_per_row(int nc, int tc)
-{
-  return (nc + tc - 1) / tc;
+  const uint4 rj = __ldg(rec + j), aj = __ldg(aux + j);
+  const float dx = (float) (int) (rj.x - ri.x), dy = (float) (int) (rj.y - ri.y);
+  const float d2 = fmaf(dx, dx, dy * dy);
+  bool in = d2 <= rho2;
+  if (fabsf(d2 - rho2) <= band) in = exact_within(rj.x, rj.y, aj.x, aj.y, Xi, Yi, rho2_d);
+  if (in) accumulate(a, rj, OMEGA ? __uint_as_float(aj.w) : 0.0f);
 }
 
-// Equal-count tiles: the row's particles split into `nbx` runs of whole
-// cells, boundary k at the first cell edge where the row's running count
-// reaches k * (row count) / nbx.
-__device__ __forceinline__ int row_target(const int *__restrict__ ro, int nc, int k, int nbx)
+// Neighbour sums of slot q (in cell c of an nc x nc grid with offsets coff) from
+// the stencil of its cell, candidate by candidate: the cell-list step's and the
+// Verlet walk's rare cases.
+template<bool OMEGA>
+__device__ __noinline__ void stencil_sums_exact(const uint4 *__restrict__ rec, const uint4 *__restrict__ aux,
+                                                const int *__restrict__ coff, int c, int nc, int q, float rho2,
+                                                float band, double rho2_d, Acc *out)
 {
-  return ro[0] + (int) ((long long) (ro[nc] - ro[0]) * k / nbx);
-}
-
-__device__ __forceinline__ int first_cell_reaching(const int *__restrict__ ro, int nc, int target)
-{
-  int lo = 0, hi = nc;  // ro[hi] >= target always
-  while (lo < hi)
-  {
-    const int mid = (lo + hi) >> 1;
-    if (ro[mid] >= target) hi = mid;
-    else lo = mid + 1;
-  }
-  return lo;
-}
-
-// Deterministic layout of tile t of a system (cell offsets `off` of that
-// system's grid; the list build and the step compute the same).
-__device__ void tile_layout(int t, int nc, int tc, const int *__restrict__ off, TileLayout &L)
-{
-  const int nbx = tiles_per_row(nc, tc);
-  const int cy = t / nbx, bx = t - cy * nbx;
-  const int *ro = off + cy * nc;
-  const int cx_lo = first_cell_reaching(ro, nc, row_target(ro, nc, bx, nbx));
-  const int cx_hi = bx + 1 == nbx ? nc : first_cell_reaching(ro, nc, row_target(ro, nc, bx + 1, nbx));
-  L.p_begin = off[cy * nc + cx_lo];
-  L.p_end = off[cy * nc + cx_hi];
-  L.row = cy;
-  L.col0 = cx_lo;
-  L.ncols = cx_hi - cx_lo;
-  L.nseg = 0;
-  L.total = 0;
-  L.staged = 0;
-  if (nc < 3) return;  // rows would repeat in the stencil
-  int st[6], en[6], ns = 0;
-  const bool whole_row = (cx_hi - cx_lo + 2) >= nc;
-  for (int dy = -1; dy <= 1; ++dy)
-  {
-    const int row = wrap_cell(cy + dy, nc) * nc;
-    if (whole_row)
-    {
-      st[ns] = off[row];
-      en[ns++] = off[row + nc];
-    } else if (cx_lo == 0)
-    {
-      st[ns] = off[row];  // cells 0 .. cx_hi
-      en[ns++] = off[row + cx_hi + 1];
-      st[ns] = off[row + nc - 1];  // left neighbour wraps to the last cell
-      en[ns++] = off[row + nc];
-    } else if (cx_hi == nc)
-    {
-      st[ns] = off[row];  // right neighbour wraps to the first cell
-      en[ns++] = off[row + 1];
-      st[ns] = off[row + cx_lo - 1];
-      en[ns++] = off[row + nc];
-    } else
-    {
-      st[ns] = off[row + cx_lo - 1];
-      en[ns++] = off[row + cx_hi + 1];
-    }
-  }
-  for (int a = 1; a < ns; ++a)
-  {
-    const int s0 = st[a], e0 = en[a];
-    int b = a - 1;
-    while (b >= 0 && st[b] > s0)
-    {
-      st[b + 1] = st[b];
-      en[b + 1] = en[b];
-      --b;
-    }
-    st[b + 1] = s0;
-    en[b + 1] = e0;
-  }
-  for (int a = 0; a < ns; ++a)
-  {
-    if (en[a] <= st[a]) continue;
-    L.start[L.nseg] = st[a];
-    L.len[L.nseg] = en[a] - st[a];
-    L.base[L.nseg] = L.total;
-    L.total += en[a] - st[a];
-    ++L.nseg;
-  }
-  L.staged = L.total <= kTileCap;
-}
-
-// Layout of every tile of every system, once per rebuild.
-__global__ void fast_tile_layout_kernel(FastParams P, FastBuffers B)
-{
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= P.ntiles) return;
-  if (!rebuilds_system(B, B.tile_sys[t])) return;
-  const SysParams *S = B.sys + B.tile_sys[t];
-  TileLayout L;
-  tile_layout(t - S->tile0, S->nc, P.tile_cells, B.cell_off + S->cell0, L);
-  reinterpret_cast<TileLayout *>(B.tiles)[t] = L;
-}
-
-// Tile-major Verlet lists: tile t keeps rows m = 0 .. cap-1 of its particles
-// contiguously, row stride round_up8(particles of the tile) entries, starting
-// at cap * round_up8(p_begin + 16 t) (16-byte aligned, never overlapping the
-// next tile); a tile's list rows are thus one block a bulk copy can stage.
-__device__ __forceinline__ long tile_list_base(int cap, int t, int p_begin)
-{
-  return (long) cap * (long) ((p_begin + 16 * t + 7) & ~7);
-}
-
-__device__ __forceinline__ int tile_list_stride(int p_begin, int p_end)
-{
-  return (p_end - p_begin + 7) & ~7;
-}
-
-constexpr int kListCap = 4096;  // staged list entries per CTA (8 KiB)
-
-// Shared-memory index of slot j inside the staged segments (-1: not staged).
-__device__ __forceinline__ int staged_index(const TileLayout &L, int j)
-{
-  for (int k = 0; k < L.nseg; ++k)
-    if (j >= L.start[k] && j < L.start[k] + L.len[k]) return L.base[k] + (j - L.start[k]);
-  return -1;
-}
-
-// Slot of a staged index (rare path: the guard band needs the slot's low words).
-__device__ __forceinline__ int staged_slot(const TileLayout &L, int idx)
-{
-  for (int k = 0; k < L.nseg; ++k)
-    if (idx >= L.base[k] && idx < L.base[k] + L.len[k]) return L.start[k] + (idx - L.base[k]);
-  return 0;
-}
-
-// Run table and per-particle cell column of a staged tile (all threads of the
-// CTA; cell offsets `coff` of the tile's system).  Returns through `self_base`
-// the shift from a slot of the tile to its staged index.
-__device__ __forceinline__ void build_runs(const TileLayout &L, const int *__restrict__ coff, int nc,
-                                           StencilRuns *runs, unsigned char *col_of, int *self_base, int *error)
-{
-  for (int w = threadIdx.x; w < 3 * L.ncols; w += blockDim.x)
-  {
-    const int k = w / 3, dy = w - 3 * k - 1;
-    const int cx = L.col0 + k;
-    const int row = wrap_cell(L.row + dy, nc) * nc;
-    const int cells[3] = {wrap_cell(cx - 1, nc), cx, wrap_cell(cx + 1, nc)};
-    short ps[3] = {0, 0, 0}, pe[3] = {0, 0, 0};
-    int np = 0;
-    for (int u = 0; u < 3; ++u)
-    {
-      const int b = coff[row + cells[u]], e = coff[row + cells[u] + 1];
-      if (e <= b) continue;
-      const int i0 = staged_index(L, b);
-      if (i0 < 0)
-      {
-        atomicOr(error, 4);  // a stencil cell outside the staged segments (the layout rules this out)
-        continue;
-      }
-      if (np > 0 && pe[np - 1] == i0)
-      {
-        pe[np - 1] = (short) (i0 + (e - b));
-      } else
-      {
-        ps[np] = (short) i0;
-        pe[np] = (short) (i0 + (e - b));
-        ++np;
-      }
-    }
-    for (int u = 0; u < 3; ++u)
-    {
-      runs[k].s[dy + 1][u] = ps[u];
-      runs[k].e[dy + 1][u] = pe[u];
-    }
-    if (dy == 0)
-    {
-      const int rb = L.row * nc;
-      for (int q = coff[rb + cx]; q < coff[rb + cx + 1]; ++q) col_of[q - L.p_begin] = (unsigned char) k;
-    }
-  }
-  if (threadIdx.x == 0)
-  {
-    for (int k = 0; k < L.nseg; ++k)
-      if (L.p_begin >= L.start[k] && L.p_begin < L.start[k] + L.len[k]) *self_base = L.base[k] - L.start[k];
-  }
-}
-
-__device__ __forceinline__ uint32_t smem_u32(const void *p)
-{
-  return (uint32_t) __cvta_generic_to_shared(p);
-}
-
-// Verlet lists from the 3x3 stencil of the rebuild grid (ParticleSystemFirstOrder.cpp:536-589):
-// pairs with r <= r_max (conservatively widened by the guard band; an entry
-// beyond r_max can never come within rho before the next rebuild).  Entry m of
-// slot q at vl[m * n + q] (16 bits): the neighbour's shared-memory index when
-// q's tile is staged, else the offset j - q.  A count of -1 marks a list
-// longer than the capacity or an offset beyond 16 bits; the step then scans
-// the stencil of the rebuild-time cell instead.  This per-slot form (global
-// gathers) serves the tiles whose neighbourhood is not staged; the staged
-// tiles build in fast_verlet_tile_build_kernel.
-__device__ void verlet_build_slot(const FastParams &P, const FastBuffers &B, int q, int t)
-{
-  const int par = B.ctrl->parity;
-  const uint4 *rec = par ? B.rec1 : B.rec0;
-  const uint4 ri = rec[q];
-  const SysParams *S = B.sys + B.sys_of[q];
-  const int nc = S->nc;
-  const float rmax2_f = S->rmax2_f;
-  const int *coff = B.cell_off + S->cell0;
-  const int c = B.cell_sorted[q] - S->cell0;
-  const int cx = c % nc, cy = c / nc;
-  const TileLayout L = reinterpret_cast<const TileLayout *>(B.tiles)[t];
-  int cnt = 0;
-  bool far = false;
-  const int stride = tile_list_stride(L.p_begin, L.p_end);
-  short *lp = B.vl + tile_list_base(P.cap, t, L.p_begin) + (q - L.p_begin);
+  const uint4 ri = rec[q], ai = aux[q];
+  const uint64_t Xi = join64(ri.x, ai.x), Yi = join64(ri.y, ai.y);
+  const int cy = c / nc, cx = c - cy * nc;
+  Acc a{0.f, 0.f, 0.f, 0.f, 0};
+  // stencil in the reference's order (-1,-1),(0,-1),(1,-1),(-1,0),... (ParticleSystemFirstOrder.cpp:47-52)
   for (int sy = -1; sy <= 1; ++sy)
   {
     const int jy = wrap_cell(cy + sy, nc);
@@ -1010,217 +712,10 @@ __device__ void verlet_build_slot(const FastParams &P, const FastBuffers &B, int
       const int jc = jy * nc + wrap_cell(cx + sx, nc);
       const int e = coff[jc + 1];
       for (int j = coff[jc]; j < e; ++j)
-      {
-        if (j == q) continue;
-        const uint4 rj = __ldg(&rec[j]);
-        const float dx = (float) (int) (rj.x - ri.x);
-        const float dy = (float) (int) (rj.y - ri.y);
-        if (fmaf(dx, dx, dy * dy) <= rmax2_f)
-        {
-          int entry;
-          if (L.staged)
-          {
-            entry = staged_index(L, j);
-            if (entry < 0) far = true;
-          } else
-          {
-            entry = j - q;
-            if (entry < -32768 || entry > 32767) far = true;
-          }
-          if (cnt < P.cap)
-          {
-            *lp = (short) entry;
-            lp += stride;
-          }
-          ++cnt;
-        }
-      }
+        if (j != q) exact_candidate<OMEGA>(rec, aux, j, ri, Xi, Yi, rho2, band, rho2_d, a);
     }
   }
-  if (cnt > P.cap) atomicMax(&B.ctrl->overflow, cnt);
-  atomicMax(&B.tile_maxcnt[t], min(cnt, P.cap));
-  B.vl_cnt[q] = (cnt > P.cap || far) ? -1 : cnt;
-}
-
-// ---------------------------------------------------------------- step
-
-// Neighbour sums of slot q from global memory (per-slot kernel, and tiles
-// that do not fit shared memory): the Verlet list holds slot offsets.
-template<int KIND, bool OMEGA>
-__device__ __forceinline__ void gather_sums(const FastParams &P, const FastBuffers &B, const uint4 *__restrict__ rec,
-                                            const uint4 *__restrict__ aux, int q, int cnt, const short *lp, int stride,
-                                            const uint4 &ri, uint64_t Xi, uint64_t Yi, Acc &a)
-{
-  if (KIND == KIND_VERLET)
-  {
-    if (cnt >= 0)
-    {
-      const long n = stride;
-      int m = 0;
-      for (; m + 4 <= cnt; m += 4)
-      {
-        const int j[4] = {q + (int) lp[0], q + (int) lp[n], q + (int) lp[2 * n], q + (int) lp[3 * n]};
-        lp += 4 * n;
-        candidates4<OMEGA, KIND == KIND_CELLS>(P, ri, Xi, Yi, rec, aux, j, a);
-      }
-      for (; m < cnt; ++m)
-      {
-        const int j = q + (int) lp[0];
-        lp += n;
-        candidate<OMEGA, KIND == KIND_CELLS>(P, ri, Xi, Yi, rec, aux, j, a);
-      }
-      return;
-    }
-    // list unusable: the stencil of the rebuild-time cell holds every particle
-    // the list would (displacements since the rebuild < skin / 2)
-  }
-  const int *coff = B.cell_off + P.cell0;
-  const int c = B.cell_sorted[q] - P.cell0;
-  const int cx = c % P.nc, cy = c / P.nc;
-  // stencil in the reference's order (-1,-1),(0,-1),(1,-1),(-1,0),... (ParticleSystemFirstOrder.cpp:47-52)
-  for (int sy = -1; sy <= 1; ++sy)
-  {
-    const int jy = wrap_cell(cy + sy, P.nc);
-    for (int sx = -1; sx <= 1; ++sx)
-    {
-      const int jc = jy * P.nc + wrap_cell(cx + sx, P.nc);
-      const int e = coff[jc + 1];
-      for (int j = coff[jc]; j < e; ++j)
-        if (j != q) candidate<OMEGA, KIND == KIND_CELLS>(P, ri, Xi, Yi, rec, aux, j, a);
-    }
-  }
-}
-
-// The FP64 cutoff decision for a staged candidate inside the guard band when
-// the aux words are not staged (steppers that need no neighbour omega): the
-// low position words come from global memory at the candidate's slot.
-__device__ __forceinline__ bool exact_within_slot_inline(const TileLayout &L, const uint4 *__restrict__ aux, int idx,
-                                                        uint32_t xh, uint32_t yh, uint64_t Xi, uint64_t Yi,
-                                                        double rho2)
-{
-  const uint2 l = __ldg(reinterpret_cast<const uint2 *>(&aux[staged_slot(L, idx)]));
-  return exact_within_inline(xh, yh, l.x, l.y, Xi, Yi, rho2);
-}
-
-__device__ __noinline__ bool exact_within_slot(const TileLayout &L, const uint4 *__restrict__ aux, int idx,
-                                               uint32_t xh, uint32_t yh, uint64_t Xi, uint64_t Yi, double rho2)
-{
-  return exact_within_slot_inline(L, aux, idx, xh, yh, Xi, Yi, rho2);
-}
-
-// One staged candidate: the record comes from shared memory; the guard band
-// (rare) takes the slot's low position words from the staged aux words (SRK,
-// which stages them for the neighbours' omega) or from global memory (SE).
-template<bool OMEGA, bool OUTLINE = true>
-__device__ __forceinline__ void candidate_staged(const FastParams &P, const uint4 &ri, uint64_t Xi, uint64_t Yi,
-                                                 const uint4 *srec, const uint4 *saux, const TileLayout &L,
-                                                 const uint4 *__restrict__ aux, int idx, Acc &a)
-{
-  const uint4 rj = srec[idx];
-  // the omega word is loaded with the record, before the range test, so the
-  // two shared-memory loads overlap instead of forming a dependent chain
-  const float wj = OMEGA ? __uint_as_float(saux[idx].w) : 0.0f;
-  const float dx = (float) (int) (rj.x - ri.x);
-  const float dy = (float) (int) (rj.y - ri.y);
-  const float d2 = fmaf(dx, dx, dy * dy);
-  bool in = d2 <= P.rho2_f;
-  if (fabsf(d2 - P.rho2_f) <= P.band_f)
-  {
-    if (OMEGA)
-    {
-      const uint4 l = saux[idx];
-      in = OUTLINE ? exact_within(rj.x, rj.y, l.x, l.y, Xi, Yi, P.rho2_d)
-                   : exact_within_inline(rj.x, rj.y, l.x, l.y, Xi, Yi, P.rho2_d);
-    } else
-    {
-      in = OUTLINE ? exact_within_slot(L, aux, idx, rj.x, rj.y, Xi, Yi, P.rho2_d)
-                   : exact_within_slot_inline(L, aux, idx, rj.x, rj.y, Xi, Yi, P.rho2_d);
-    }
-  }
-  if (in) accumulate(a, rj, wj);
-}
-
-// Neighbour sums of slot q from the tile's staged records.
-template<int KIND, bool OMEGA>
-__device__ __forceinline__ void gather_sums_staged(const FastParams &P, const FastBuffers &B, const uint4 *srec,
-                                                   const uint4 *saux, const TileLayout &L,
-                                                   const uint4 *__restrict__ rec, const uint4 *__restrict__ aux, int q,
-                                                   int cnt, const short *lp, int stride, const uint4 &ri, uint64_t Xi,
-                                                   uint64_t Yi, Acc &a)
-{
-  if (KIND == KIND_VERLET && cnt >= 0)
-  {
-    const long n = stride;
-    int m = 0;
-    for (; m + 4 <= cnt; m += 4)
-    {
-      // four candidates as one group: entries, records and omega words loaded
-      // together, four FP32 distances, one guard-band test for the group (a
-      // group with a candidate inside the band is redone one by one with the
-      // FP64 decision there), so the common path has no branch between loads
-      const int i[4] = {lp[0], lp[n], lp[2 * n], lp[3 * n]};
-      lp += 4 * n;
-      uint4 r[4];
-      float w[4], d2[4];
-#pragma unroll
-      for (int k = 0; k < 4; ++k)
-      {
-        r[k] = srec[i[k]];
-        w[k] = OMEGA ? __uint_as_float(saux[i[k]].w) : 0.0f;
-      }
-      bool band = false;
-#pragma unroll
-      for (int k = 0; k < 4; ++k)
-      {
-        const float dx = (float) (int) (r[k].x - ri.x);
-        const float dy = (float) (int) (r[k].y - ri.y);
-        d2[k] = fmaf(dx, dx, dy * dy);
-        band |= fabsf(d2[k] - P.rho2_f) <= P.band_f;
-      }
-      if (!band)
-      {
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-          if (d2[k] <= P.rho2_f) accumulate(a, r[k], w[k]);
-      } else
-      {
-#pragma unroll 1
-        for (int k = 0; k < 4; ++k) candidate_staged<OMEGA, true>(P, ri, Xi, Yi, srec, saux, L, aux, i[k], a);
-      }
-    }
-    for (; m < cnt; ++m)
-    {
-      candidate_staged<OMEGA, false>(P, ri, Xi, Yi, srec, saux, L, aux, lp[0], a);
-      lp += n;
-    }
-    return;
-  }
-  // a Verlet list that did not fit: scan the stencil of the rebuild-time cell;
-  // each stencil cell is one contiguous staged range
-  const int *coff = B.cell_off + P.cell0;
-  const int c = B.cell_sorted[q] - P.cell0;
-  const int cx = c % P.nc, cy = c / P.nc;
-  for (int sy = -1; sy <= 1; ++sy)
-  {
-    const int jy = wrap_cell(cy + sy, P.nc);
-    for (int sx = -1; sx <= 1; ++sx)
-    {
-      const int jc = jy * P.nc + wrap_cell(cx + sx, P.nc);
-      const int b = coff[jc], e = coff[jc + 1];
-      if (e <= b) continue;
-      const int i0 = staged_index(L, b);
-      if (i0 < 0 || i0 + (e - b) > L.total)
-      {
-        // not inside the staged segments (cannot happen for a cell of this tile's stencil)
-        for (int j = b; j < e; ++j)
-          if (j != q) candidate<OMEGA, KIND == KIND_CELLS>(P, ri, Xi, Yi, rec, aux, j, a);
-        continue;
-      }
-      const int self = q - b;
-      for (int u = 0; u < e - b; ++u)
-        if (u != self) candidate_staged<OMEGA, KIND == KIND_CELLS>(P, ri, Xi, Yi, srec, saux, L, aux, i0 + u, a);
-    }
-  }
+  *out = a;
 }
 
 // Exactly the normals the stepper consumes, in the reference's draw order.
@@ -1500,7 +995,7 @@ __device__ __noinline__ void pair_batch_exact(const uint4 *srec, const float *sw
     if (fabsf(d2 - rho2) <= band)
     {
       const uint2 l = __ldg(reinterpret_cast<const uint2 *>(&aux[j0 + k]));
-      in = exact_within_inline(rj.x, rj.y, l.x, l.y, Xi, Yi, rho2_d);
+      in = exact_within(rj.x, rj.y, l.x, l.y, Xi, Yi, rho2_d);
     }
     if (!in) continue;
     const float2 cs = make_float2(__uint_as_float(rj.z), __uint_as_float(rj.w));
@@ -1643,333 +1138,6 @@ __global__ void __launch_bounds__(32 * kPairWarps, 2) fast_allpairs_kernel(FastP
   publish_max(ctrl, B.sysctl, sys, d2max, err);
 }
 
-// Bounded wait for phase `phase` of an mbarrier (about one second).
-__device__ __forceinline__ uint32_t wait_phase(uint32_t mb, uint32_t phase)
-{
-  uint32_t done = 0;
-  const long long t0 = clock64();
-  while (!done && clock64() - t0 < kWaitCycles)
-    asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
-                 : "=r"(done)
-                 : "r"(mb), "r"(phase)
-                 : "memory");
-  return done;
-}
-
-// A particle's own words, loaded from global memory at its slot.
-struct OwnParticle
-{
-  unsigned p;  // original index (noise counter)
-  uint4 r, a;  // record and aux words
-  int cnt;     // Verlet list length
-  float2 v;    // velocity (second order)
-};
-
-template<int MODEL, int KIND>
-__device__ __forceinline__ OwnParticle load_own(const FastBuffers &B, const uint4 *rin, const uint4 *ain, int q)
-{
-  OwnParticle o;
-  o.p = B.pid[q];
-  o.r = rin[q];
-  o.a = ain[q];
-  o.cnt = KIND == KIND_VERLET ? B.vl_cnt[q] : 0;
-  o.v = MODEL == 2 ? B.vel[q] : make_float2(0.f, 0.f);
-  return o;
-}
-
-// The particles of one tile, one per thread; `o` holds the thread's first
-// particle, loaded before the wait for the tile's bulk copies.  The noise is
-// drawn after the neighbour walk (fewer registers live across the walk).
-template<int MODEL, int STEPPER, int KIND>
-__device__ __forceinline__ void step_tile(const FastParams &Q, const FastBuffers &B, const TileLayout &L,
-                                          OwnParticle o, const uint4 *srec, const uint4 *saux, const short *slist,
-                                          const short *glist, int list_staged, int list_stride, bool staged,
-                                          const uint4 *rin, const uint4 *ain, uint4 *rout, uint4 *aout, float &d2max,
-                                          int &err)
-{
-  const int q0 = L.p_begin + threadIdx.x;
-  for (int q = q0; q < L.p_end; q += blockDim.x)
-  {
-    if (q != q0) o = load_own<MODEL, KIND>(B, rin, ain, q);
-    Acc a{0.f, 0.f, 0.f, 0.f, 0};
-    const uint64_t Xi = join64(o.r.x, o.a.x), Yi = join64(o.r.y, o.a.y);
-    const int i = q - L.p_begin;
-    const short *lp = KIND == KIND_VERLET ? (list_staged ? slist + i : glist + i) : nullptr;
-    // a staged list is walked through its shared-memory pointer, so its
-    // entries are read with shared-memory loads
-    if (staged && KIND == KIND_VERLET && list_staged)
-      gather_sums_staged<KIND, STEPPER == 2>(Q, B, srec, saux, L, rin, ain, q, o.cnt, slist + i, list_stride, o.r,
-                                             Xi, Yi, a);
-    else if (staged)
-      gather_sums_staged<KIND, STEPPER == 2>(Q, B, srec, saux, L, rin, ain, q, o.cnt, lp, list_stride, o.r, Xi, Yi, a);
-    else
-      gather_sums<KIND, STEPPER == 2>(Q, B, rin, ain, q, o.cnt, lp, list_stride, o.r, Xi, Yi, a);
-    float z[6];
-    draw_noise<MODEL, STEPPER>(Q, B.ctrl->step, o.p, z);
-    d2max = fmaxf(d2max, update_particle<MODEL, STEPPER>(Q, B, q, o.r, o.a, o.v, a, z, rout, aout, err));
-  }
-}
-
-// Staging of tile t by thread 0 (persistent launch): layout, list geometry,
-// and the bulk copies of the neighbour records, aux words (AUX: SRK, which
-// needs the neighbours' omega) and list rows onto the mbarrier.
-template<int KIND, bool AUX>
-__device__ __forceinline__ void stage_tile(const FastParams &P, const FastBuffers &B, int t, const uint4 *rin,
-                                           const uint4 *ain, uint4 *srec, uint4 *saux, short *slist, uint32_t mb,
-                                           TileLayout &L, int &list_staged, int &list_stride, bool reuse)
-{
-  L = reinterpret_cast<const TileLayout *>(B.tiles)[t];
-  if (L.p_end <= L.p_begin) L.staged = 0;
-  list_stride = tile_list_stride(L.p_begin, L.p_end);
-  const int rows = KIND == KIND_VERLET ? B.tile_maxcnt[t] : 0;
-  const uint32_t list_bytes = 2u * (uint32_t) rows * (uint32_t) list_stride;
-  list_staged = L.staged && KIND == KIND_VERLET && rows > 0 && rows * list_stride <= kListCap;
-  if (!L.staged) return;
-  // generic-proxy reads of the buffers (previous tile) before async-proxy writes
-  if (reuse) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-  const uint32_t tx = (AUX ? 32u : 16u) * L.total + (list_staged ? list_bytes : 0u);
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mb), "r"(tx) : "memory");
-  for (int k = 0; k < L.nseg; ++k)
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                     smem_u32(&srec[L.base[k]])),
-                 "l"(rin + L.start[k]), "r"(16u * L.len[k]), "r"(mb)
-                 : "memory");
-  if (AUX)
-    for (int k = 0; k < L.nseg; ++k)
-      asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                       smem_u32(&saux[L.base[k]])),
-                   "l"(ain + L.start[k]), "r"(16u * L.len[k]), "r"(mb)
-                   : "memory");
-  if (list_staged)
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                     smem_u32(slist)),
-                 "l"(B.vl + tile_list_base(P.cap, t, L.p_begin)), "r"(list_bytes), "r"(mb)
-                 : "memory");
-}
-
-// Staging of tile t by warp 0 (one launch per step): the layout read one word
-// per lane, then the bulk copies issued by several lanes at once (records:
-// lanes 0..5, aux words: lanes 8..13, list rows: lane 16) after lane 0 has
-// armed the mbarrier with the expected bytes.  Against the same staging by
-// thread 0 alone the benchmark kernel ran 0.1889 -> 0.1853 ms (same bits):
-// the serial layout copy and copy issue sat on every CTA's critical path.
-template<int KIND, bool AUX>
-__device__ __forceinline__ void stage_tile_warp(const FastParams &P, const FastBuffers &B, int t, const uint4 *rin,
-                                                const uint4 *ain, uint4 *srec, uint4 *saux, short *slist, uint32_t mb,
-                                                TileLayout &L, int &list_staged, int &list_stride)
-{
-  constexpr int kWords = (int) (sizeof(TileLayout) / sizeof(int));
-  static_assert(kWords <= 32, "one layout word per lane");
-  const int lane = threadIdx.x & 31;
-  const int *src = reinterpret_cast<const int *>(reinterpret_cast<const TileLayout *>(B.tiles) + t);
-  if (lane < kWords) reinterpret_cast<int *>(&L)[lane] = src[lane];
-  const int rows = KIND == KIND_VERLET ? B.tile_maxcnt[t] : 0;
-  __syncwarp();
-  const int p_begin = L.p_begin, p_end = L.p_end, total = L.total, nseg = L.nseg;
-  const bool staged = L.staged && p_end > p_begin;
-  const int stride = tile_list_stride(p_begin, p_end);
-  const uint32_t list_bytes = 2u * (uint32_t) rows * (uint32_t) stride;
-  const bool lstaged = staged && KIND == KIND_VERLET && rows > 0 && rows * stride <= kListCap;
-  __syncwarp();
-  if (lane == 0)
-  {
-    L.staged = staged ? 1 : 0;
-    list_stride = stride;
-    list_staged = lstaged ? 1 : 0;
-    if (staged)
-    {
-      const uint32_t tx = (AUX ? 32u : 16u) * (uint32_t) total + (lstaged ? list_bytes : 0u);
-      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mb), "r"(tx) : "memory");
-    }
-  }
-  if (!staged) return;
-  __syncwarp();
-  if (lane < nseg)
-  {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                     smem_u32(&srec[L.base[lane]])),
-                 "l"(rin + L.start[lane]), "r"(16u * L.len[lane]), "r"(mb)
-                 : "memory");
-  } else if (AUX && lane >= 8 && lane < 8 + nseg)
-  {
-    const int k = lane - 8;
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                     smem_u32(&saux[L.base[k]])),
-                 "l"(ain + L.start[k]), "r"(16u * L.len[k]), "r"(mb)
-                 : "memory");
-  } else if (lane == 16 && lstaged)
-  {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                     smem_u32(slist)),
-                 "l"(B.vl + tile_list_base(P.cap, t, p_begin)), "r"(list_bytes), "r"(mb)
-                 : "memory");
-  }
-}
-
-__device__ __forceinline__ void init_mbarrier(uint32_t mb)
-{
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mb) : "memory");
-  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-}
-
-// SE or SRK step of one tile per CTA with the neighbourhood staged in shared
-// memory by TMA bulk copies (cp.async.bulk, completion on an mbarrier).
-// MULTI: several systems, whose parameters come from the system table (one
-// system: from the kernel's parameter space, which costs no registers).
-// Verlet lists.  Residency: SRK 9 CTAs per SM (56 registers, 24.7 KB of shared
-// memory); SE stages no aux words and runs 10.
-template<int MODEL, int STEPPER, int KIND, bool MULTI>
-__global__ void __launch_bounds__(kTileThreads, STEPPER == 2 ? 9 : SPSS_SE_VERLET_TILE_BLOCKS)
-    fast_tile_kernel(FastParams P, FastBuffers B)
-{
-  __shared__ __align__(16) uint4 srec[kTileCap];
-  __shared__ __align__(16) uint4 saux[STEPPER == 2 ? kTileCap : 1];  // aux words: SRK only (neighbour omega)
-  __shared__ __align__(16) short slist[KIND == KIND_VERLET ? kListCap : 8];
-  __shared__ __align__(8) unsigned long long mbar;
-  __shared__ TileLayout L;
-  __shared__ int list_staged, list_stride;
-  pdl_enter();
-  FastControl *ctrl = B.ctrl;
-  const int par = ctrl->parity;
-  buffers_now(B, ctrl->order_parity);
-  const uint4 *rin = par ? B.rec1 : B.rec0;
-  const uint4 *ain = par ? B.aux1 : B.aux0;
-  uint4 *rout = par ? B.rec0 : B.rec1;
-  uint4 *aout = par ? B.aux0 : B.aux1;
-  const int t = blockIdx.x;
-  const uint32_t mb = smem_u32(&mbar);
-  if (threadIdx.x < 32)
-  {
-    if (threadIdx.x == 0) init_mbarrier(mb);
-    __syncwarp();
-    stage_tile_warp<KIND, STEPPER == 2>(P, B, t, rin, ain, srec, saux, slist, mb, L, list_staged, list_stride);
-  }
-  __syncthreads();
-  const bool staged = L.staged;
-  if (L.p_end <= L.p_begin) return;
-  const int sys = MULTI ? B.tile_sys[t] : 0;
-  const FastParams Q = MULTI ? with_system(P, B.sys[sys]) : P;
-  const short *glist = KIND == KIND_VERLET ? B.vl + tile_list_base(P.cap, t, L.p_begin) : nullptr;
-  // the thread's first particle is loaded before the wait for the bulk
-  // copies, so its global loads are in flight while the tile lands
-  const int q0 = L.p_begin + threadIdx.x;
-  OwnParticle o;
-  if (q0 < L.p_end) o = load_own<MODEL, KIND>(B, rin, ain, q0);
-  if (staged)
-  {
-    const uint32_t done = wait_phase(mb, 0);
-    if (!__syncthreads_and(done))
-    {
-      // the copies did not complete in time: report, give them a second
-      // bounded wait so none is in flight when the CTA exits, and stop
-      if (threadIdx.x == 0) atomicOr(&ctrl->error, 2);
-      wait_phase(mb, 0);
-      return;
-    }
-  }
-  float d2max = 0.0f;
-  int err = 0;
-  // the loop body is step_tile's, written out here: through the shared
-  // function this kernel spills and runs 1 % slower
-  for (int q = q0; q < L.p_end; q += blockDim.x)
-  {
-    if (q != q0) o = load_own<MODEL, KIND>(B, rin, ain, q);
-    const unsigned p = o.p;
-    const uint4 ri = o.r;
-    const uint4 ai = o.a;
-    const int cnt = o.cnt;
-    const float2 v = o.v;
-    Acc a{0.f, 0.f, 0.f, 0.f, 0};
-    const uint64_t Xi = join64(ri.x, ai.x), Yi = join64(ri.y, ai.y);
-    const int i = q - L.p_begin;
-    const short *lp = KIND == KIND_VERLET ? (list_staged ? slist + i : glist + i) : nullptr;
-    // a staged list is walked through its shared-memory pointer, so its
-    // entries are read with shared-memory loads
-    if (staged && KIND == KIND_VERLET && list_staged)
-      gather_sums_staged<KIND, STEPPER == 2>(Q, B, srec, saux, L, rin, ain, q, cnt, slist + i, list_stride, ri, Xi,
-                                             Yi, a);
-    else if (staged)
-      gather_sums_staged<KIND, STEPPER == 2>(Q, B, srec, saux, L, rin, ain, q, cnt, lp, list_stride, ri, Xi, Yi, a);
-    else
-      gather_sums<KIND, STEPPER == 2>(Q, B, rin, ain, q, cnt, lp, list_stride, ri, Xi, Yi, a);
-    float z[6];
-    draw_noise<MODEL, STEPPER>(Q, ctrl->step, p, z);
-    d2max = fmaxf(d2max, update_particle<MODEL, STEPPER>(Q, B, q, ri, ai, v, a, z, rout, aout, err));
-  }
-  publish_max(ctrl, B.sysctl, sys, d2max, err);
-}
-
-// The same step as a persistent launch: one wave of CTAs, each taking tiles
-// from a work counter until all tiles of all systems are done; the staging
-// buffers and the mbarrier (one phase per staged tile) are reused.
-template<int MODEL, int STEPPER, int KIND, bool MULTI>
-__global__ void __launch_bounds__(kTileThreads, 8) fast_tile_persistent_kernel(FastParams P, FastBuffers B)
-{
-  __shared__ __align__(16) uint4 srec[kTileCap];
-  __shared__ __align__(16) uint4 saux[STEPPER == 2 ? kTileCap : 1];  // aux words: SRK only (neighbour omega)
-  __shared__ __align__(16) short slist[KIND == KIND_VERLET ? kListCap : 8];
-  __shared__ __align__(8) unsigned long long mbar;
-  __shared__ TileLayout L;
-  __shared__ int list_staged, list_stride, tile_id;
-  __shared__ uint32_t phase;  // mbarrier phase of the next staged tile
-  pdl_enter();
-  FastControl *ctrl = B.ctrl;
-  const int par = ctrl->parity;
-  buffers_now(B, ctrl->order_parity);
-  const uint4 *rin = par ? B.rec1 : B.rec0;
-  const uint4 *ain = par ? B.aux1 : B.aux0;
-  uint4 *rout = par ? B.rec0 : B.rec1;
-  uint4 *aout = par ? B.aux0 : B.aux1;
-  const uint32_t mb = smem_u32(&mbar);
-  if (threadIdx.x == 0)
-  {
-    init_mbarrier(mb);
-    phase = 0;
-  }
-  for (bool first = true;; first = false)
-  {
-    if (!first) __syncthreads();  // the previous tile's shared data is no longer read
-    if (threadIdx.x == 0)
-    {
-      const int t = atomicAdd(&ctrl->tile_next, 1);
-      tile_id = t;
-      if (t < P.ntiles)
-        stage_tile<KIND, STEPPER == 2>(P, B, t, rin, ain, srec, saux, slist, mb, L, list_staged, list_stride,
-                                       !first);
-    }
-    __syncthreads();
-    const int t = tile_id;
-    if (t >= P.ntiles) break;
-    const bool staged = L.staged;
-    const int sys = MULTI ? B.tile_sys[t] : 0;
-    OwnParticle o;
-    if (L.p_begin + (int) threadIdx.x < L.p_end) o = load_own<MODEL, KIND>(B, rin, ain, L.p_begin + threadIdx.x);
-    if (staged)
-    {
-      const uint32_t ph = phase;
-      const uint32_t done = wait_phase(mb, ph);
-      if (!__syncthreads_and(done))
-      {
-        if (threadIdx.x == 0) atomicOr(&ctrl->error, 2);
-        wait_phase(mb, ph);
-        return;
-      }
-      if (threadIdx.x == 0) phase = ph ^ 1u;  // read again only after the next barrier
-    }
-    if (L.p_end <= L.p_begin) continue;
-    const short *glist = KIND == KIND_VERLET ? B.vl + tile_list_base(P.cap, t, L.p_begin) : nullptr;
-    float d2max = 0.0f;
-    int err = 0;
-    if (!MULTI)
-      step_tile<MODEL, STEPPER, KIND>(P, B, L, o, srec, saux, slist, glist, list_staged, list_stride, staged, rin,
-                                      ain, rout, aout, d2max, err);
-    else
-      step_tile<MODEL, STEPPER, KIND>(with_system(P, B.sys[sys]), B, L, o, srec, saux, slist, glist, list_staged,
-                                      list_stride, staged, rin, ain, rout, aout, d2max, err);
-    publish_max(ctrl, B.sysctl, sys, d2max, err);
-  }
-}
-
 // ---------------------------------------------------------------- cell-list step
 //
 // One SE or SRK step of one particle per thread, neighbours from the 3 x 3
@@ -2100,17 +1268,17 @@ __global__ void __launch_bounds__(kCellThreads, SPSS_CELL_BLOCKS) fast_cell_step
       }
     }
   }
-  const uint4 ai = ain[q];
   Acc t{a.cs.y, a.cs.x, a.w.y, a.w.x, a.card};
-  const FastParams Q = MULTI ? with_system(P, *S) : P;
   if (nc < 3 || a.nearest <= band)
   {
     // fewer than three cells a side (the stencil meets cells more than once), or
-    // a candidate inside the guard band: candidate by candidate, with the FP64
-    // decisions
-    t = Acc{0.f, 0.f, 0.f, 0.f, 0};
-    gather_sums<KIND_CELLS, OMEGA>(Q, B, rin, ain, q, 0, nullptr, 0, ri, join64(ri.x, ai.x), join64(ri.y, ai.y), t);
+    // a candidate inside the guard band
+    Acc again;
+    stencil_sums_exact<OMEGA>(rin, ain, coff, c, nc, q, rho2, band, MULTI ? S->rho2_d : P.rho2_d, &again);
+    t = again;
   }
+  const uint4 ai = ain[q];
+  const FastParams Q = MULTI ? with_system(P, *S) : P;
   int err = 0;
   float z[6];
   draw_noise<MODEL, STEPPER>(Q, ctrl->step - (unsigned long long) fresh, B.pid[q], z);
@@ -2119,108 +1287,387 @@ __global__ void __launch_bounds__(kCellThreads, SPSS_CELL_BLOCKS) fast_cell_step
   if (err) atomicOr(&ctrl->error, 1);
 }
 
-// Verlet lists of one tile per CTA, from the 3x3 stencil of the rebuild grid
-// (ParticleSystemFirstOrder.cpp:536-589).  The tile's neighbourhood records
-// are staged in shared memory by bulk copies; each particle scans its stencil
-// through the tile's run table (per stencil row at most three contiguous runs
-// of staged records, in the reference's stencil order), so its list holds the
-// same entries, in the same order, as the per-slot build: the staged indices
-// of the neighbours with r <= r_max (widened by the guard band).  Tiles that
-// are not staged, or wider than the run table, build per slot from global
-// memory.  The entries go straight to global memory (L2 merges the 2-byte
-// stores; assembling the rows in shared memory first measured slower).  The
-// tile's longest list (rows to stage at the step) is a block maximum.
-__global__ void __launch_bounds__(kTileThreads) fast_verlet_tile_build_kernel(FastParams P, FastBuffers B)
+// Whether this block is the last of the launch to get here (its partials are
+// written); all threads of the block get the answer.
+__device__ __forceinline__ bool last_block(FastControl *ctrl)
 {
-  __shared__ __align__(16) uint4 srec[kTileCap];
-  __shared__ __align__(8) unsigned long long mbar;
-  __shared__ TileLayout L;
-  __shared__ int self_base, tile_max;
-  __shared__ StencilRuns runs[kRunCells];
-  __shared__ unsigned char col_of[kTileCap];
-  FastControl *ctrl = B.ctrl;
-  const int t = blockIdx.x;
-  if (!rebuilds_system(B, B.tile_sys[t])) return;  // the whole CTA: its tile keeps its lists
-  const uint4 *rec = ctrl->parity ? B.rec1 : B.rec0;
-  const SysParams *S = B.sys + B.tile_sys[t];
-  const uint32_t mb = smem_u32(&mbar);
+  __shared__ unsigned mine;
+  __threadfence();
+  __syncthreads();
   if (threadIdx.x == 0)
   {
-    tile_max = 0;
-    B.tile_maxcnt[t] = 0;  // the per-slot build below raises it
-    L = reinterpret_cast<const TileLayout *>(B.tiles)[t];
-    if (L.p_end <= L.p_begin || L.ncols > kRunCells) L.staged = 0;
-    if (L.staged)
+    mine = atomicAdd(&ctrl->ticket, 1u);
+    if (mine == gridDim.x - 1) ctrl->ticket = 0u;
+    __threadfence();
+  }
+  __syncthreads();
+  return mine == gridDim.x - 1;
+}
+
+// ---------------------------------------------------------------- Verlet lists
+//
+// Lists by slot, the 32 slots of a warp together: entries 4 g .. 4 g + 3 of slot
+// q stand in the eight bytes at [q / 32][g][q mod 32], so a warp reads four
+// entries of all its lanes as one 256-byte line and its lists are one stretch of
+// memory (rows [g][q] over all slots instead: the list kernel 300 us for 238 us
+// at 4.19 million particles).  An entry is the neighbour's slot offset j - q in
+// 16 bits, modulo the system's size where the stencil crosses the vertical
+// periodic boundary (kListWrapped in the count: one list in 70 at N = 65,536; as
+// stencil scans these few took as long as the rest of the step).  A count of -1 marks a list longer than the capacity or an offset
+// beyond 16 bits; the step then scans the stencil of the rebuild-time cell,
+// which holds every particle the list would.
+constexpr int kListWrapped = 1 << 30;
+
+// Slot of an entry of a wrapped list: q + e back into the system's slots.
+__device__ __forceinline__ int wrapped_slot(int q, int e, int first, int n)
+{
+  const int j = q + e;
+  return j < first ? j + n : (j >= first + n ? j - n : j);
+}
+
+__device__ __forceinline__ long list_at(int cap, int q)
+{
+  return (long) (q >> 5) * (32L * cap) + 4 * (q & 31);
+}
+
+// Verlet list of slot q from the 3x3 stencil of the rebuild grid
+// (ParticleSystemFirstOrder.cpp:536-589): pairs with r <= r_max (conservatively
+// widened by the guard band; an entry beyond r_max can never come within rho
+// before the next rebuild), in the reference's order.
+__device__ __forceinline__ void build_list(const FastParams &P, const FastBuffers &B, const SysParams *S,
+                                           const uint4 *rec, int q)
+{
+  const int nc = S->nc;
+  const float rmax2 = S->rmax2_f;
+  const int *coff = B.cell_off + S->cell0;
+  const int c = B.cell_sorted[q] - S->cell0;
+  const uint2 ri = *reinterpret_cast<const uint2 *>(rec + q);
+  const int cy = c / nc, cx = c - cy * nc;
+  short *list = B.vl + list_at(P.cap, q);
+  const int n = S->n, half = n / 2;
+  int cnt = 0;
+  bool far = false, wrapped = false;
+  auto scan = [&](int s, int e) {
+    for (; s < e; s += 4)
     {
-      init_mbarrier(mb);
-      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mb), "r"(16u * L.total) : "memory");
-      for (int k = 0; k < L.nseg; ++k)
-        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                         smem_u32(&srec[L.base[k]])),
-                     "l"(rec + L.start[k]), "r"(16u * L.len[k]), "r"(mb)
-                     : "memory");
+      uint2 r[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) r[k] = __ldg(reinterpret_cast<const uint2 *>(rec + min(s + k, e - 1)));
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+      {
+        const float dx = (float) (int) (r[k].x - ri.x), dy = (float) (int) (r[k].y - ri.y);
+        if (s + k >= e || s + k == q || !(fmaf(dx, dx, dy * dy) <= rmax2)) continue;
+        int off = s + k - q;
+        if (off != (int) (short) off)
+        {
+          off += off > half ? -n : n;
+          far |= off != (int) (short) off;
+          wrapped = true;
+        }
+        if (cnt < P.cap) list[(cnt >> 2) * 128 + (cnt & 3)] = (short) off;
+        ++cnt;
+      }
+    }
+  };
+  for (int sy = -1; sy <= 1; ++sy)
+  {
+    const int row = wrap_cell(cy + sy, nc) * nc;
+    if (cx > 0 && cx + 1 < nc)
+    {
+      scan(coff[row + cx - 1], coff[row + cx + 2]);
+    } else
+    {
+      for (int sx = -1; sx <= 1; ++sx)
+      {
+        const int jc = row + wrap_cell(cx + sx, nc);
+        scan(coff[jc], coff[jc + 1]);
+      }
     }
   }
-  __syncthreads();
-  if (L.p_end <= L.p_begin) return;
-  if (!L.staged)
+  if (cnt > P.cap) atomicMax(&B.ctrl->overflow, cnt);
+  B.vl_cnt[q] = (cnt > P.cap || far) ? -1 : (wrapped ? cnt | kListWrapped : cnt);
+}
+
+// One slot per thread.  `finish`: the launch also ends the rebuild (the batches
+// of small systems, whose step graphs hold it unconditionally: it leaves at once
+// when nothing is due).
+constexpr int kBuildThreads = 256;
+
+__global__ void __launch_bounds__(kBuildThreads) fast_verlet_build_kernel(FastParams P, FastBuffers B, int finish)
+{
+  FastControl *ctrl = B.ctrl;
+  if (finish && ctrl->rebuild == REBUILD_NONE) return;
+  const int q = blockIdx.x * kBuildThreads + threadIdx.x;
+  if (q < P.n)
   {
-    for (int q = L.p_begin + threadIdx.x; q < L.p_end; q += blockDim.x) verlet_build_slot(P, B, q, t);
-    return;
+    const SysParams *S = B.sys + B.sys_of[q];
+    if (rebuilds_system(B, S->index)) build_list(P, B, S, ctrl->parity ? B.rec1 : B.rec0, q);
   }
-  build_runs(L, B.cell_off + S->cell0, S->nc, runs, col_of, &self_base, &ctrl->error);
-  const uint32_t done = wait_phase(mb, 0);
-  if (!__syncthreads_and(done))
+  if (!finish || !last_block(ctrl)) return;
+  for (int r = threadIdx.x; r < P.nsys; r += kBuildThreads) B.sysctl[r].rebuild = 0;
+  if (threadIdx.x == 0)
   {
-    // the copies did not complete in time: report, wait once more so none is
-    // in flight when the CTA exits, and leave the lists unbuilt
-    if (threadIdx.x == 0) atomicOr(&ctrl->error, 2);
-    wait_phase(mb, 0);
-    return;
+    ctrl->rebuild = REBUILD_NONE;
+    ctrl->rebuilds += 1;
+    ctrl->cells_fresh = 0;
   }
-  const float rmax2 = S->rmax2_f;
-  const int stride = tile_list_stride(L.p_begin, L.p_end);
-  short *const rows = B.vl + tile_list_base(P.cap, t, L.p_begin);
-  int mymax = 0;
-  for (int q = L.p_begin + threadIdx.x; q < L.p_end; q += blockDim.x)
+}
+
+// The re-sort of one small system by one CTA: cell ids and counts, offsets,
+// members, the particles through the other buffers and back (so no parity flips
+// and the other systems are not touched); CTAs of systems that are not due leave
+// at once, and the list kernel follows.  A batch of a thousand systems rebuilds
+// some of them on most steps, and the general sequence of eleven launches over
+// every slot, launched from the device, took as long as the step.  1,024
+// systems of 1,024 particles, one of them or all due, take 12.6 us; a step with
+// its share of rebuilds 80.5 -> 55 us, in clustered states, where some system is
+// due on every step, 336 -> 160 us (the list build in this kernel: 190 us; with
+// 1,024 threads: 14 us).
+constexpr int kSystemThreads = 512;
+constexpr int kSystemSlots = 4096;  // largest system taken
+constexpr int kSystemCells = 4096;  // and cells of its grid
+
+__global__ void __launch_bounds__(kSystemThreads) fast_system_rebuild_kernel(FastParams P, FastBuffers B)
+{
+  __shared__ int off[kSystemCells + 1];            // counts, then offsets within the system
+  __shared__ short member[kSystemSlots], cell[kSystemSlots];
+  __shared__ unsigned short arrival[kSystemSlots];
+  __shared__ int warp_tot[kSystemThreads / 32];
+  FastControl *ctrl = B.ctrl;
+  if (ctrl->rebuild == REBUILD_NONE) return;
+  const SysParams *S = B.sys + blockIdx.x;
+  const bool due = rebuilds_system(B, blockIdx.x);
+  if (due)
   {
-    const int i = q - L.p_begin;
-    const int self = q + self_base;
-    const uint4 ri = srec[self];
-    const StencilRuns &R = runs[col_of[i]];
-    int off = i;  // entry cnt of this particle at off = i + cnt * stride
-    int cnt = 0;
-#pragma unroll 1
-    for (int r = 0; r < 3; ++r)
-#pragma unroll 1
-      for (int u = 0; u < 3; ++u)
-      {
-        const int e = R.e[r][u];
-        for (int idx = R.s[r][u]; idx < e; ++idx)
-        {
-          const uint4 rj = srec[idx];
-          const float dx = (float) (int) (rj.x - ri.x);
-          const float dy = (float) (int) (rj.y - ri.y);
-          if (idx != self && fmaf(dx, dx, dy * dy) <= rmax2)
-          {
-            if (cnt < P.cap)
-            {
-              rows[off] = (short) idx;
-              off += stride;
-            }
-            ++cnt;
-          }
-        }
-      }
-    if (cnt > P.cap) atomicMax(&ctrl->overflow, cnt);
-    B.vl_cnt[q] = cnt > P.cap ? -1 : cnt;
-    mymax = max(mymax, min(cnt, P.cap));
-  }
+    const int n = S->n, first = S->first, nc = S->nc, ncell = nc * nc, cell0 = S->cell0;
+    const int par = ctrl->parity;
+    buffers_now(B, ctrl->order_parity);
+    uint4 *rec = par ? B.rec1 : B.rec0, *rec_to = par ? B.rec0 : B.rec1;
+    uint4 *aux = par ? B.aux1 : B.aux0, *aux_to = par ? B.aux0 : B.aux1;
+    for (int c = threadIdx.x; c < ncell; c += kSystemThreads) off[c] = 0;
+    __syncthreads();
+    for (int i = threadIdx.x; i < n; i += kSystemThreads)
+    {
+      const uint4 r = rec[first + i], a = aux[first + i];
+      const int c = cell_of_fix(join64(r.x, a.x), join64(r.y, a.y), nc);
+      cell[i] = (short) c;
+      arrival[i] = (unsigned short) atomicAdd(&off[c], 1);
+    }
+    __syncthreads();
+    // exclusive scan of the counts: consecutive cells a thread
+    {
+      constexpr int kItems = kSystemCells / kSystemThreads;
+      const int base = threadIdx.x * kItems, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+      int v[kItems], local = 0;
 #pragma unroll
-  for (int off = 16; off > 0; off >>= 1) mymax = max(mymax, __shfl_xor_sync(0xffffffffu, mymax, off));
-  if ((threadIdx.x & 31) == 0) atomicMax(&tile_max, mymax);
-  __syncthreads();
-  if (threadIdx.x == 0) B.tile_maxcnt[t] = tile_max;
+      for (int k = 0; k < kItems; ++k)
+      {
+        v[k] = base + k < ncell ? off[base + k] : 0;
+        local += v[k];
+      }
+      int x = local;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1)
+      {
+        const int y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+      }
+      if (lane == 31) warp_tot[warp] = x;
+      __syncthreads();
+      int excl = x - local;
+      for (int w = 0; w < warp; ++w) excl += warp_tot[w];
+#pragma unroll
+      for (int k = 0; k < kItems; ++k)
+      {
+        if (base + k < ncell)
+        {
+          off[base + k] = excl;
+          B.cell_off_w[cell0 + base + k] = first + excl;
+        }
+        excl += v[k];
+      }
+      if (threadIdx.x == 0)
+      {
+        off[ncell] = n;
+        B.cell_off_w[cell0 + ncell] = first + n;  // the next system's first offset, or the total: the same value
+      }
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < n; i += kSystemThreads) member[off[cell[i]] + arrival[i]] = (short) i;
+    __syncthreads();
+    for (int m = threadIdx.x; m < n; m += kSystemThreads)
+    {
+      const int i = member[m], c = cell[i], b = off[c], e = off[c + 1];
+      int q = b;
+      for (int k = b; k < e; ++k) q += member[k] < i;
+      const int src = first + i, to = first + q;
+      rec_to[to] = rec[src];
+      aux_to[to] = aux[src];
+      const unsigned p = B.pid[src];
+      B.pid_tmp[to] = p;
+      B.inv[p] = (unsigned) to;
+      if (P.model == 2) B.vel_tmp[to] = B.vel[src];
+      B.cell_sorted[to] = cell0 + c;
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < n; i += kSystemThreads)
+    {
+      const int q = first + i;
+      rec[q] = rec_to[q];
+      aux[q] = aux_to[q];
+      B.pid[q] = B.pid_tmp[q];
+      if (P.model == 2) B.vel[q] = B.vel_tmp[q];
+    }
+  }
+}
+
+// A particle's own words, loaded from global memory at its slot.
+struct OwnParticle
+{
+  unsigned p;  // original index (noise counter)
+  uint4 r, a;  // record and aux words
+  float2 v;    // velocity (second order)
+};
+
+template<int MODEL>
+__device__ __forceinline__ OwnParticle load_own(const FastBuffers &B, const uint4 *rin, const uint4 *ain, int q)
+{
+  OwnParticle o;
+  o.p = B.pid[q];
+  o.r = rin[q];
+  o.a = ain[q];
+  o.v = MODEL == 2 ? B.vel[q] : make_float2(0.f, 0.f);
+  return o;
+}
+
+// Listed neighbours again, candidate by candidate.
+template<bool OMEGA>
+__device__ __noinline__ void list_sums_exact(const uint4 *__restrict__ rec, const uint4 *__restrict__ aux,
+                                             const short *list, int cnt, int q, int first, int n,
+                                             float rho2, float band, double rho2_d, Acc *out)
+{
+  const uint4 ri = rec[q], ai = aux[q];
+  const uint64_t Xi = join64(ri.x, ai.x), Yi = join64(ri.y, ai.y);
+  Acc a{0.f, 0.f, 0.f, 0.f, 0};
+  for (int m = 0; m < cnt; ++m)
+    exact_candidate<OMEGA>(rec, aux, wrapped_slot(q, list[(m >> 2) * 128 + (m & 3)], first, n), ri, Xi, Yi, rho2,
+                           band, rho2_d, a);
+  *out = a;
+}
+
+// The listed neighbours of particle q in fours, decided in FP32; the entries of
+// the next four are on their way meanwhile.
+template<bool OMEGA, bool WRAPPED>
+__device__ __forceinline__ void walk_list(const uint4 *__restrict__ rec, const uint4 *__restrict__ aux,
+                                          const short *list, short4 next, int cnt, int q, int first, int n,
+                                          uint32_t xi, uint32_t yi, float rho2, CellSums<OMEGA> &a)
+{
+#pragma unroll 1
+  for (int m = 0; m < cnt; m += 4)
+  {
+    const short4 e = next;
+    list += 128;
+    if (m + 4 < cnt) next = *reinterpret_cast<const short4 *>(list);
+    const int last = cnt - m;
+    // entries past the end repeat the particle itself, which is never counted
+    int j[4] = {q + e.x, last > 1 ? q + e.y : q, last > 2 ? q + e.z : q, last > 3 ? q + e.w : q};
+    if (WRAPPED)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) j[k] = wrapped_slot(j[k], 0, first, n);
+    uint4 r[4];
+    float w[4], d2[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+    {
+      r[k] = __ldg(rec + j[k]);
+      w[k] = OMEGA ? __uint_as_float(__ldg(&aux[j[k]].w)) : 0.0f;
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+    {
+      const float dx = (float) (int) (r[k].x - xi), dy = (float) (int) (r[k].y - yi);
+      d2[k] = fmaf(dx, dx, dy * dy);
+      if (k > 0 && last <= k) d2[k] = 3.0e38f;
+      a.nearest = fminf(a.nearest, fabsf(d2[k] - rho2));
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (d2[k] <= rho2)
+      {
+        const float2 c = make_float2(__uint_as_float(r[k].z), __uint_as_float(r[k].w));
+        a.cs = add2(a.cs, c);
+        if (OMEGA) a.w = fma2(make_float2(w[k], w[k]), c, a.w);
+        a.card += 1;
+      }
+  }
+}
+
+#ifndef SPSS_LIST_BLOCKS_SRK
+#define SPSS_LIST_BLOCKS_SRK 12
+#endif
+#ifndef SPSS_LIST_BLOCKS_SE
+#define SPSS_LIST_BLOCKS_SE 13
+#endif
+
+// SE or SRK step of 128 slots a CTA, one particle per thread, neighbours from its
+// Verlet list through L1 (a warp's particles are neighbours of each other).
+template<int MODEL, int STEPPER, bool MULTI>
+__global__ void __launch_bounds__(kTileThreads, STEPPER == 2 ? SPSS_LIST_BLOCKS_SRK : SPSS_LIST_BLOCKS_SE)
+    fast_tile_kernel(FastParams P, FastBuffers B)
+{
+  pdl_enter();
+  constexpr bool OMEGA = STEPPER == 2;
+  const int slot = blockIdx.x * kTileThreads + threadIdx.x;
+  const int q = min(slot, P.n - 1);
+  FastControl *ctrl = B.ctrl;
+  const int par = ctrl->parity;
+  buffers_now(B, ctrl->order_parity);
+  const uint4 *rin = par ? B.rec1 : B.rec0;
+  const uint4 *ain = par ? B.aux1 : B.aux0;
+  uint4 *rout = par ? B.rec0 : B.rec1;
+  uint4 *aout = par ? B.aux0 : B.aux1;
+  const int listed = B.vl_cnt[q];
+  const int cnt = listed < 0 ? listed : listed & ~kListWrapped;
+  const short *list = B.vl + list_at(P.cap, q);
+  const uint4 ri = rin[q];
+  // the first entries of every list, before anything waits
+  const short4 entries = *reinterpret_cast<const short4 *>(list);
+  const int sys = MULTI ? B.sys_of[q] : 0;
+  const SysParams *S = MULTI ? B.sys + sys : nullptr;
+  const float rho2 = MULTI ? S->rho2_f : P.rho2_f;
+  CellSums<OMEGA> a{make_float2(0.f, 0.f), make_float2(0.f, 0.f), 0, 3.0e38f};
+  if (listed == cnt)
+    walk_list<OMEGA, false>(rin, ain, list, entries, cnt, q, 0, 0, ri.x, ri.y, rho2, a);
+  else
+    walk_list<OMEGA, true>(rin, ain, list, entries, cnt, q, MULTI ? S->first : P.first, MULTI ? S->n : P.sub_n, ri.x,
+                           ri.y, rho2, a);
+  float d2max = 0.0f;
+  int err = 0;
+  if (slot < P.n)
+  {
+    Acc t{a.cs.y, a.cs.x, a.w.y, a.w.x, a.card};
+    const float band = MULTI ? S->band_f : P.band_f;
+    if (cnt < 0 || a.nearest <= band)
+    {
+      const double rho2_d = MULTI ? S->rho2_d : P.rho2_d;
+      const int cell0 = MULTI ? S->cell0 : P.cell0, nc = MULTI ? S->nc : P.nc;
+      Acc again;
+      if (cnt < 0)
+        stencil_sums_exact<OMEGA>(rin, ain, B.cell_off + cell0, B.cell_sorted[q] - cell0, nc, q, rho2, band, rho2_d,
+                                  &again);
+      else
+        list_sums_exact<OMEGA>(rin, ain, list, cnt, q, MULTI ? S->first : P.first, MULTI ? S->n : P.sub_n, rho2, band,
+                               rho2_d, &again);
+      t = again;
+    }
+    const OwnParticle o = load_own<MODEL>(B, rin, ain, q);
+    const FastParams Q = MULTI ? with_system(P, *S) : P;
+    float z[6];
+    draw_noise<MODEL, STEPPER>(Q, ctrl->step, o.p, z);
+    d2max = update_particle<MODEL, STEPPER>(Q, B, q, o.r, o.a, o.v, t, z, rout, aout, err);
+  }
+  publish_max(ctrl, B.sysctl, sys, d2max, err);
 }
 
 // After a step: advance the noise counter and the buffer parity, accumulate
@@ -2269,7 +1716,6 @@ __global__ void fast_control_kernel(FastControl *ctrl, SysControl *sysctl, const
   {
     ctrl->step += 1;
     ctrl->parity ^= 1;
-    ctrl->tile_next = 0;
     ctrl->cells_fresh = cells_written;
     ctrl->triggered = (always_rebuild || any) ? 1 : 0;
     if (always_rebuild) ctrl->rebuild = REBUILD_ALL;
@@ -2324,9 +1770,15 @@ __global__ void fast_pbc_kernel(int2 *img, int n)
 
 constexpr int kOrderChunk = 2048;  // slots per partial sum
 
+// Whether a sample follows the step that brought the counter to `step`.
+__host__ __device__ __forceinline__ bool samples_after(const FastControl *c, unsigned long long step)
+{
+  return c->sample_every > 0 && (long long) step >= c->sample_from && (long long) step % c->sample_every == 0;
+}
+
 __device__ __forceinline__ bool sample_now(const FastControl *c)
 {
-  return c->sample_every > 0 && (long long) c->step >= c->sample_from && (long long) c->step % c->sample_every == 0;
+  return samples_after(c, c->step);
 }
 
 __device__ __forceinline__ double warp_sum(double v)
@@ -2474,23 +1926,6 @@ __device__ __forceinline__ void two_sum_add(float &hi, float &lo, float x)
   const float b = __fsub_rn(s, hi);
   lo = __fadd_rn(lo, __fadd_rn(__fsub_rn(hi, __fsub_rn(s, b)), __fsub_rn(x, b)));
   hi = s;
-}
-
-// Whether this block is the last of the launch to get here (its partials are
-// written); all threads of the block get the answer.
-__device__ __forceinline__ bool last_block(FastControl *ctrl)
-{
-  __shared__ unsigned mine;
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0)
-  {
-    mine = atomicAdd(&ctrl->ticket, 1u);
-    if (mine == gridDim.x - 1) ctrl->ticket = 0u;
-    __threadfence();
-  }
-  __syncthreads();
-  return mine == gridDim.x - 1;
 }
 
 // Sums of cos phi, sin phi, omega cos phi, omega sin phi over the particles,
@@ -2723,16 +2158,14 @@ static FastBuffers buffers(spss_ctx *ctx)
   B.cell_of = f->cell_of.ptr;
   B.cell_sorted = f->cell_sorted.ptr;
   B.cell_off = f->binner.offsets.ptr;
+  B.cell_off_w = f->binner.offsets.ptr;
   B.order = f->binner.members.ptr;
   B.cell_count = f->binner.count.ptr;
   B.cell_slot = f->binner.slot.ptr;
   B.vl = f->vl.ptr;
   B.vl_cnt = f->vl_cnt.ptr;
-  B.tile_maxcnt = f->tile_maxcnt.ptr;
-  B.tiles = f->tiles.ptr;
   B.sys = f->sys.ptr;
   B.sys_of = f->sys_of.ptr;
-  B.tile_sys = f->tile_sys.ptr;
   B.sysctl = f->sysctl.ptr;
   B.nu = f->nu.ptr;
   B.field = f->field.ptr;
@@ -2743,8 +2176,8 @@ static FastBuffers buffers(spss_ctx *ctx)
 
 // Table entry of one system: its parameters in the FP32 / fixed-point units
 // of the kernels.
-static SysParams system_params(const spss_params &p, int index, int first, int nc, int cell0, int tile0,
-                               int ntiles, double r_min, double r_max)
+static SysParams system_params(const spss_params &p, int index, int first, int nc, int cell0, double r_min,
+                               double r_max)
 {
   SysParams S;
   std::memset(&S, 0, sizeof(S));
@@ -2752,8 +2185,6 @@ static SysParams system_params(const spss_params &p, int index, int first, int n
   S.first = first;
   S.nc = nc;
   S.cell0 = cell0;
-  S.tile0 = tile0;
-  S.ntiles = ntiles;
   S.index = index;
   S.replica = (int) p.replica;
   S.v0 = (float) p.v0;
@@ -2798,10 +2229,7 @@ static FastParams params(spss_ctx *ctx, double dt)
   P.kind = f->kind;
   P.always_rebuild = f->kind == KIND_CELLS ? 1 : 0;
   P.selective = f->nsys > 1 && f->kind == KIND_VERLET ? 1 : 0;
-  P.tile_cells = f->tile_cells;
-  P.persistent = f->persistent;
   P.nsys = f->nsys;
-  P.ntiles = f->ntiles;
   // system 0 (kernels that serve several systems read theirs from the table)
   P.nc = S.nc;
   P.first = S.first;
@@ -2830,47 +2258,6 @@ static FastParams params(spss_ctx *ctx, double dt)
   philox_round_keys(p.seed, P.kx, P.ky);
   P.replica = (uint32_t) S.replica;
   return P;
-}
-
-// Tile tables for a tile width (cells per tile); every system's tiles follow
-// the previous system's.
-static int set_tiling(spss_ctx *ctx, int tile_cells)
-{
-  FastPath *f = ctx->fast;
-  if (f->kind == KIND_ALL_PAIRS || f->kind == KIND_GLOBAL) return SPSS_OK;
-  f->tile_cells = tile_cells;
-  int ntiles = 0;
-  std::vector<int> tile_sys;
-  for (int r = 0; r < f->nsys; ++r)
-  {
-    SysParams &S = f->h_sys[r];
-    S.tile0 = ntiles;
-    S.ntiles = S.nc * tiles_per_row(S.nc, tile_cells);
-    ntiles += S.ntiles;
-    tile_sys.insert(tile_sys.end(), (size_t) S.ntiles, r);
-  }
-  f->ntiles = ntiles;
-  SPSS_TRY(f->tiles.reserve(sizeof(TileLayout) * (size_t) ntiles));
-  SPSS_TRY(f->tile_sys.reserve((size_t) ntiles));
-  SPSS_CUDA_TRY(cudaMemcpyAsync(f->tile_sys.ptr, tile_sys.data(), sizeof(int) * ntiles, cudaMemcpyHostToDevice,
-                                ctx->stream));
-  SPSS_CUDA_TRY(cudaMemcpyAsync(f->sys.ptr, f->h_sys.data(), sizeof(SysParams) * f->nsys, cudaMemcpyHostToDevice,
-                                ctx->stream));
-  if (f->kind == KIND_VERLET)
-  {
-    SPSS_TRY(f->vl.reserve((size_t) f->cap * ((size_t) ctx->p.n + 16 * (size_t) ntiles + 16)));
-    SPSS_TRY(f->tile_maxcnt.reserve((size_t) ntiles));
-  }
-  SPSS_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-  // lists and layouts follow the tiles: rebuild before the next step
-  f->h_ctrl->rebuild = 1;
-  ctx->should_update_lists = 1;
-  SPSS_CUDA_TRY(cudaMemcpyAsync(&f->ctrl->rebuild, &f->h_ctrl->rebuild, sizeof(int), cudaMemcpyHostToDevice,
-                                ctx->stream));
-  for (auto &g : f->graphs) g.second.release();
-  f->graphs.clear();
-  SPSS_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-  return SPSS_OK;
 }
 
 int fast_create(spss_ctx *ctx)
@@ -2932,7 +2319,7 @@ int fast_create(spss_ctx *ctx)
     if (kind >= 0 && k != kind) return SPSS_ERR_NOT_SUPPORTED;  // one list kind per context
     kind = k;
     if ((long) cell0 + (long) grid * grid > 0x7fffffffL) return SPSS_ERR_SIZE;
-    f->h_sys.push_back(system_params(q, r, first, grid, cell0, 0, 0, r_min, r_max));
+    f->h_sys.push_back(system_params(q, r, first, grid, cell0, r_min, r_max));
     first += q.n;
     cell0 += grid * grid;
     lam_max = std::max(lam_max, M_PI * r_max * r_max * q.n);
@@ -2940,6 +2327,9 @@ int fast_create(spss_ctx *ctx)
   if (first != n) return SPSS_ERR_INVALID_ARGUMENT;
   f->kind = kind;
   f->total_cells = cell0;
+  f->small_systems = kind == KIND_VERLET && f->nsys > 1;
+  for (const SysParams &S : f->h_sys)
+    if (S.n > kSystemSlots || S.nc * S.nc > kSystemCells) f->small_systems = false;
   if (kind == KIND_GLOBAL)
   {
     SPSS_TRY(f->nu.reserve((size_t) n));
@@ -3013,16 +2403,7 @@ int fast_create(spss_ctx *ctx)
   SPSS_CUDA_TRY(cudaMemcpyAsync(f->ctrl, f->h_ctrl, sizeof(FastControl), cudaMemcpyHostToDevice, ctx->stream));
   SPSS_CUDA_TRY(cudaMemsetAsync(f->vel.ptr, 0, sizeof(float2) * n, ctx->stream));
   if (has_cells(f->kind)) SPSS_TRY(f->binner.prepare(n, f->total_cells, ctx->stream));
-  SPSS_TRY(set_tiling(ctx, kTileCellsDefault));
-  // resident CTAs of the persistent tile kernel: one wave
-  {
-    int dev = 0, sms = 0, per_sm = 0;
-    SPSS_CUDA_TRY(cudaGetDevice(&dev));
-    SPSS_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    SPSS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fast_tile_persistent_kernel<2, 2, KIND_VERLET, true>,
-                                                                kTileThreads, 0));
-    f->persistent_grid = std::max(1, sms * std::max(1, per_sm));
-  }
+  if (f->kind == KIND_VERLET) SPSS_TRY(f->vl.reserve((size_t) f->cap * (((size_t) n + 31) / 32 * 32)));
   SPSS_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
   return SPSS_OK;
 }
@@ -3048,11 +2429,8 @@ void fast_destroy(spss_ctx *ctx)
   f->cell_sorted.release();
   f->vl.release();
   f->vl_cnt.release();
-  f->tile_maxcnt.release();
-  f->tiles.release();
   f->sys.release();
   f->sys_of.release();
-  f->tile_sys.release();
   f->sysctl.release();
   f->nu.release();
   f->field.release();
@@ -3081,6 +2459,15 @@ static int launch_rebuild(spss_ctx *ctx, const FastParams &P)
   const FastBuffers B = buffers(ctx);
   const int n = P.n;
   const bool lists = f->kind == KIND_VERLET;
+  if (lists && f->small_systems)
+  {
+    fast_system_rebuild_kernel<<<f->nsys, kSystemThreads, 0, ctx->stream>>>(P, B);
+    ++ctx->launches;
+    SPSS_TRY(check_launch("fast_system_rebuild_kernel"));
+    fast_verlet_build_kernel<<<blocks_for(n, kBuildThreads), kBuildThreads, 0, ctx->stream>>>(P, B, 1);
+    ++ctx->launches;
+    return check_launch("fast_verlet_build_kernel");
+  }
   if (lists)
   {
     fast_cells_kernel<<<blocks_for(n, kTB), kTB, 0, ctx->stream>>>(P, B);
@@ -3102,12 +2489,9 @@ static int launch_rebuild(spss_ctx *ctx, const FastParams &P)
   SPSS_TRY(check_launch("fast_after_permute_kernel"));
   if (lists)
   {
-    fast_tile_layout_kernel<<<blocks_for(f->ntiles, 128), 128, 0, ctx->stream>>>(P, B);
+    fast_verlet_build_kernel<<<blocks_for(n, kBuildThreads), kBuildThreads, 0, ctx->stream>>>(P, B, 0);
     ++ctx->launches;
-    SPSS_TRY(check_launch("fast_tile_layout_kernel"));
-    fast_verlet_tile_build_kernel<<<f->ntiles, kTileThreads, 0, ctx->stream>>>(P, B);
-    ++ctx->launches;
-    SPSS_TRY(check_launch("fast_verlet_tile_build_kernel"));
+    SPSS_TRY(check_launch("fast_verlet_build_kernel"));
   }
   fast_after_rebuild_kernel<<<1, 256, 0, ctx->stream>>>(f->ctrl, f->sysctl.ptr, f->nsys);
   ++ctx->launches;
@@ -3171,25 +2555,19 @@ static int launch_cells_step(spss_ctx *ctx, int stepper, const FastParams &P, bo
 }
 
 template<int MODEL, int STEPPER>
-static void launch_tiles(spss_ctx *ctx, const FastParams &P, const FastBuffers &B, int grid)
+static void launch_tiles(spss_ctx *ctx, const FastParams &P, const FastBuffers &B)
 {
-  constexpr int K = KIND_VERLET;
-  if (P.persistent)
-  {
-    if (P.nsys > 1) launch_chained(false, fast_tile_persistent_kernel<MODEL, STEPPER, K, true>, grid, kTileThreads, 0, ctx->stream, P, B);
-    else launch_chained(false, fast_tile_persistent_kernel<MODEL, STEPPER, K, false>, grid, kTileThreads, 0, ctx->stream, P, B);
-  } else
-  {
-    if (P.nsys > 1) launch_chained(false, fast_tile_kernel<MODEL, STEPPER, K, true>, grid, kTileThreads, 0, ctx->stream, P, B);
-    else launch_chained(false, fast_tile_kernel<MODEL, STEPPER, K, false>, grid, kTileThreads, 0, ctx->stream, P, B);
-  }
+  const int blocks = blocks_for(P.n, kTileThreads);
+  if (P.nsys > 1)
+    launch_chained(false, fast_tile_kernel<MODEL, STEPPER, true>, blocks, kTileThreads, 0, ctx->stream, P, B);
+  else
+    launch_chained(false, fast_tile_kernel<MODEL, STEPPER, false>, blocks, kTileThreads, 0, ctx->stream, P, B);
 }
 
 template<int MODEL, int STEPPER>
 static void launch_step_kind(spss_ctx *ctx, const FastParams &P, const FastBuffers &B)
 {
   const int grid = blocks_for(P.n, kTB);
-  const int tiles = P.persistent ? std::min(P.ntiles, ctx->fast->persistent_grid) : P.ntiles;
   if (ctx->fast->kind == KIND_GLOBAL)
   {
     if (MODEL == 1)
@@ -3205,14 +2583,21 @@ static void launch_step_kind(spss_ctx *ctx, const FastParams &P, const FastBuffe
     else fast_allpairs_kernel<MODEL, STEPPER, false><<<blocks, 32 * kPairWarps, 0, ctx->stream>>>(P, B);
   } else
   {
-    launch_tiles<MODEL, STEPPER>(ctx, P, B, tiles);
+    launch_tiles<MODEL, STEPPER>(ctx, P, B);
   }
+}
+
+// One block: a system a thread, whose FP64 chain (square root, sum, comparison)
+// is all the kernel does (1,024 systems: 9.5 us with 256 threads, 6.6 us with 1,024).
+static int control_threads(int nsys)
+{
+  return std::min(1024, (nsys + 31) / 32 * 32);
 }
 
 static int launch_control(spss_ctx *ctx, const FastParams &P, int cells_written)
 {
   FastPath *f = ctx->fast;
-  fast_control_kernel<false><<<1, 256, 0, ctx->stream>>>(f->ctrl, f->sysctl.ptr, f->sys.ptr, f->nsys, P.always_rebuild,
+  fast_control_kernel<false><<<1, control_threads(f->nsys), 0, ctx->stream>>>(f->ctrl, f->sysctl.ptr, f->sys.ptr, f->nsys, P.always_rebuild,
                                                          f->kind == KIND_VERLET || f->trigger_only, P.selective,
                                                          cells_written, nullptr);
   ++ctx->launches;
@@ -3237,7 +2622,7 @@ static int launch_step(spss_ctx *ctx, int stepper, const FastParams &P, cudaGrap
   if (ctx->timing) SPSS_CUDA_TRY(cudaEventRecord(ctx->ev1, ctx->stream));
   FastPath *f = ctx->fast;
   if (rebuild_exec)
-    fast_control_kernel<true><<<1, 256, 0, ctx->stream>>>(f->ctrl, f->sysctl.ptr, f->sys.ptr, f->nsys,
+    fast_control_kernel<true><<<1, control_threads(f->nsys), 0, ctx->stream>>>(f->ctrl, f->sysctl.ptr, f->sys.ptr, f->nsys,
                                                           P.always_rebuild, f->kind == KIND_VERLET || f->trigger_only,
                                                           P.selective, 0, rebuild_exec);
   else
@@ -3332,12 +2717,44 @@ int fast_get_state(spss_ctx *ctx, double *d_aos)
   return check_launch("fast_download_kernel");
 }
 
+// Room for longer lists once some were too long (clusters outgrow the capacity
+// estimated for the mean density, and a particle whose list did not fit scans
+// its stencil every step): a quarter more than the longest seen.  The lists in
+// use move as they are, and the next rebuild fills the larger ones, so no result depends on when this happens.  Memory is taken only while
+// it is plentiful; a failed allocation leaves things as they were.
+constexpr int kListCapMax = 512;
+
+static int grow_lists(spss_ctx *ctx)
+{
+  FastPath *f = ctx->fast;
+  if (f->kind != KIND_VERLET || f->h_ctrl->overflow <= f->cap) return SPSS_OK;
+  const int cap = std::min(kListCapMax, (f->h_ctrl->overflow + f->h_ctrl->overflow / 4 + 3) & ~3);
+  if (cap <= f->cap) return SPSS_OK;
+  const size_t warps = ((size_t) ctx->p.n + 31) / 32, want = warps * 32 * cap;
+  size_t free_bytes = 0, total_bytes = 0;
+  SPSS_CUDA_TRY(cudaMemGetInfo(&free_bytes, &total_bytes));
+  if (want * sizeof(short) > free_bytes / 4) return SPSS_OK;
+  DeviceArray<short> larger;
+  if (larger.reserve(want) != SPSS_OK) return SPSS_OK;
+  const size_t pitch = 32 * sizeof(short) * cap, old_pitch = 32 * sizeof(short) * f->cap;
+  SPSS_CUDA_TRY(cudaMemcpy2DAsync(larger.ptr, pitch, f->vl.ptr, old_pitch, old_pitch, warps, cudaMemcpyDeviceToDevice,
+                                  ctx->stream));
+  SPSS_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+  f->vl.release();
+  f->vl = larger;
+  f->cap = cap;
+  for (auto &g : f->graphs) g.second.release();
+  f->graphs.clear();
+  return SPSS_OK;
+}
+
 int fast_step(spss_ctx *ctx, int stepper, double t, double dt)
 {
   (void) t;
   FastPath *f = ctx->fast;
   if (!f->have_state) return SPSS_ERR_INVALID_ARGUMENT;
   if (stepper == SPSS_STEPPER_RK4) return SPSS_ERR_NOT_SUPPORTED;
+  SPSS_TRY(grow_lists(ctx));
   const FastParams P = params(ctx, dt);
   SPSS_TRY(push_host_control(ctx));
   if (f->kind == KIND_CELLS)
@@ -3479,7 +2896,9 @@ static int build_graph_on(spss_ctx *ctx, int stepper, const FastParams &P, int s
                           unsigned long long launches0)
 {
   FastPath *f = ctx->fast;
-  const bool trigger = f->kind == KIND_VERLET || f->trigger_only;
+  // a batch of small systems rebuilds by one kernel, which every step launches
+  const bool trigger = (f->kind == KIND_VERLET && !f->small_systems) || f->trigger_only;
+  const bool always = f->kind == KIND_CELLS || f->small_systems;
   if (trigger && f->device_rebuild)
   {
     const int rc = build_device_rebuild(ctx, P, g);
@@ -3492,14 +2911,15 @@ static int build_graph_on(spss_ctx *ctx, int stepper, const FastParams &P, int s
       ctx->launches = launches0;
     }
   }
-  if (!f->device_rebuild && f->kind != KIND_CELLS)
+  if (!f->device_rebuild && !always)
     return build_graph_conditional(ctx, stepper, P, sampling, g, launches0);
   const unsigned long long launches_step = ctx->launches;
   cudaGraph_t graph = nullptr;
   SPSS_CUDA_TRY(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeRelaxed));
   int rc = SPSS_OK;
   if (f->kind == KIND_CELLS) rc = launch_cells_step(ctx, stepper, P, true);
-  else rc = launch_step(ctx, stepper, P, trigger ? g.rebuild_exec : nullptr);
+  else if (f->small_systems) rc = launch_rebuild(ctx, P);
+  if (rc == SPSS_OK && f->kind != KIND_CELLS) rc = launch_step(ctx, stepper, P, trigger ? g.rebuild_exec : nullptr);
   if (rc == SPSS_OK && sampling) rc = launch_sampling(ctx, P, 1);
   const cudaError_t e = cudaStreamEndCapture(ctx->stream, &graph);
   if (rc != SPSS_OK)
@@ -3511,7 +2931,7 @@ static int build_graph_on(spss_ctx *ctx, int stepper, const FastParams &P, int s
   g.graph = graph;
   SPSS_CUDA_TRY(cudaGraphInstantiate(&g.exec, graph, 0));
   g.per_step = (int) (ctx->launches - launches_step);
-  g.form = trigger ? GRAPH_DEVICE : (f->kind == KIND_CELLS ? GRAPH_ALWAYS : GRAPH_NONE);
+  g.form = trigger ? GRAPH_DEVICE : (always ? GRAPH_ALWAYS : GRAPH_NONE);
   ctx->launches = launches0;  // captured, not launched
   return SPSS_OK;
 }
@@ -3532,28 +2952,45 @@ static int run_steps(spss_ctx *ctx, int stepper, double dt, long nsteps, int sam
     }
     return sampling ? sync_control(ctx) : SPSS_OK;
   }
+  SPSS_TRY(grow_lists(ctx));
   SPSS_TRY(push_host_control(ctx));
-  auto key = std::make_tuple(stepper, dt, sampling ? 1 : 0);
-  auto it = f->graphs.find(key);
-  if (it == f->graphs.end())
-  {
-    GraphEntry g;
-    SPSS_TRY(build_graph(ctx, stepper, dt, sampling, g));
-    it = f->graphs.emplace(key, g).first;
-  }
   if (f->kind == KIND_CELLS) SPSS_TRY(ensure_cells(ctx, params(ctx, dt)));
+  // the plain step, and the step with a sample behind it for the steps that
+  // take one (whose kernels check the same condition on the device)
+  GraphEntry *graph[2] = {nullptr, nullptr};
   int rebuilds0 = f->h_ctrl->rebuilds;
-  if ((it->second.form == GRAPH_DEVICE || it->second.form == GRAPH_NONE) && f->h_ctrl->rebuild)
+  bool first = true;
+  int per_rebuild = 0;
+  for (long k = 0; k < nsteps; ++k)
   {
-    // a rebuild pending before the first step (host request, eager steps):
-    // these graphs rebuild only after a step's trigger
-    SPSS_TRY(launch_rebuild(ctx, params(ctx, dt)));
-    rebuilds0 += 1;
+    const int with_sample = sampling && samples_after(f->h_ctrl, f->h_ctrl->step + (unsigned long long) k + 1) ? 1 : 0;
+    if (!graph[with_sample])
+    {
+      const auto key = std::make_tuple(stepper, dt, with_sample);
+      auto it = f->graphs.find(key);
+      if (it == f->graphs.end())
+      {
+        GraphEntry g;
+        SPSS_TRY(build_graph(ctx, stepper, dt, with_sample, g));
+        it = f->graphs.emplace(key, g).first;
+      }
+      graph[with_sample] = &it->second;
+      per_rebuild = it->second.per_rebuild;
+    }
+    GraphEntry &g = *graph[with_sample];
+    if (first && (g.form == GRAPH_DEVICE || g.form == GRAPH_NONE) && f->h_ctrl->rebuild)
+    {
+      // a rebuild pending before the first step (host request, eager steps):
+      // these graphs rebuild only after a step's trigger
+      SPSS_TRY(launch_rebuild(ctx, params(ctx, dt)));
+      rebuilds0 += 1;
+    }
+    first = false;
+    SPSS_CUDA_TRY(cudaGraphLaunch(g.exec, ctx->stream));
+    ctx->launches += (unsigned long long) g.per_step;
   }
-  for (long k = 0; k < nsteps; ++k) SPSS_CUDA_TRY(cudaGraphLaunch(it->second.exec, ctx->stream));
   const int rc = sync_control(ctx);
-  ctx->launches += (unsigned long long) nsteps * it->second.per_step
-      + (unsigned long long) (f->h_ctrl->rebuilds - rebuilds0) * it->second.per_rebuild;
+  ctx->launches += (unsigned long long) (f->h_ctrl->rebuilds - rebuilds0) * per_rebuild;
   return rc;
 }
 
@@ -3680,8 +3117,20 @@ int fast_set_tiling(spss_ctx *ctx, int tile_cells, int persistent)
 {
   if (tile_cells < 1 || tile_cells > 4096 || (persistent != 0 && persistent != 1)) return SPSS_ERR_INVALID_ARGUMENT;
   FastPath *f = ctx->fast;
+  if (!has_cells(f->kind))
+  {
+    f->persistent = persistent;
+    return SPSS_OK;
+  }
+  f->tile_cells = tile_cells;
   f->persistent = persistent;
-  return set_tiling(ctx, tile_cells);
+  // the lists are rebuilt before the next step
+  f->h_ctrl->rebuild = REBUILD_ALL;
+  ctx->should_update_lists = 1;
+  SPSS_CUDA_TRY(cudaMemcpyAsync(&f->ctrl->rebuild, &f->h_ctrl->rebuild, sizeof(int), cudaMemcpyHostToDevice,
+                                ctx->stream));
+  SPSS_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+  return SPSS_OK;
 }
 
 int fast_set_device_rebuild(spss_ctx *ctx, int enabled)
@@ -3738,9 +3187,8 @@ static int take_snapshot(spss_ctx *ctx)
   return SPSS_OK;
 }
 
-// Back to the snapshot; the lists are rebuilt before the next step.  `keep`:
-// the snapshot stays for another restore.
-static int restore_snapshot(spss_ctx *ctx, bool keep = false)
+// Back to the snapshot; the lists are rebuilt before the next step.
+static int restore_snapshot(spss_ctx *ctx)
 {
   FastPath *f = ctx->fast;
   Snapshot &S = f->snap;
@@ -3766,14 +3214,13 @@ static int restore_snapshot(spss_ctx *ctx, bool keep = false)
   ctx->step_counter = f->h_ctrl->step;
   ctx->accumulated_displacement = f->h_ctrl->acc;
   ctx->should_update_lists = 1;
-  if (!keep) S.release();
+  S.release();
   return SPSS_OK;
 }
 
-// Times `steps` steps (graph launches, CUDA events) for every tile width and
-// launch form, each from the state the call found, keeps the fastest and
-// puts the state back as it was.  The step results do not depend on the
-// tiling.
+// Times `steps` steps (graph launches, CUDA events) from the state the call
+// finds and puts the state back as it was.  The step kernels take a particle
+// per thread whatever the tiling, so there is nothing to choose between.
 int fast_autotune(spss_ctx *ctx, int stepper, double dt, int steps, double *best_ms)
 {
   FastPath *f = ctx->fast;
@@ -3787,47 +3234,25 @@ int fast_autotune(spss_ctx *ctx, int stepper, double dt, int steps, double *best
   const int timing = ctx->timing;
   ctx->timing = 0;
   SPSS_TRY(take_snapshot(ctx));
-  const int widths[] = {16, 20, 24, 28, 32, 36, 40, 44, 48, 52, 56, 60, 64};
-  double best = 1e300;
-  int best_w = f->tile_cells, best_p = f->persistent;
-  int rc = SPSS_OK;
-  for (int w : widths)
-    // cell-list steps have one launch form
-    for (int pers = 0; pers <= (f->kind == KIND_CELLS ? 0 : 1) && rc == SPSS_OK; ++pers)
-    {
-      // every candidate from the same state: a list rebuild that the trigger
-      // calls for inside the timed steps falls on the same step for all of
-      // them (results do not depend on the tiling), not on whichever
-      // candidate happens to be running when the accumulated displacement
-      // reaches the skin
-      rc = restore_snapshot(ctx, true);
-      if (rc != SPSS_OK) break;
-      f->persistent = pers;
-      rc = set_tiling(ctx, w);
-      if (rc == SPSS_OK) rc = run_steps(ctx, stepper, dt, 2, 0);  // builds the graph, warms up
-      if (rc != SPSS_OK) break;
-      cudaEventRecord(ctx->ev0, ctx->stream);
-      rc = run_steps(ctx, stepper, dt, steps, 0);
-      cudaEventRecord(ctx->ev1, ctx->stream);
-      if (rc != SPSS_OK) break;
-      float ms = 0.0f;
-      SPSS_CUDA_TRY(cudaEventSynchronize(ctx->ev1));
-      SPSS_CUDA_TRY(cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1));
-      if (ms / steps < best)
-      {
-        best = ms / steps;
-        best_w = w;
-        best_p = pers;
-      }
-    }
-  f->persistent = best_p;
-  const int rc2 = set_tiling(ctx, best_w);
-  const int rc3 = restore_snapshot(ctx);
+  float ms = 0.0f;
+  int rc = run_steps(ctx, stepper, dt, 2, 0);  // builds the graph, warms up
+  if (rc == SPSS_OK)
+  {
+    cudaEventRecord(ctx->ev0, ctx->stream);
+    rc = run_steps(ctx, stepper, dt, steps, 0);
+    cudaEventRecord(ctx->ev1, ctx->stream);
+  }
+  if (rc == SPSS_OK && (cudaEventSynchronize(ctx->ev1) != cudaSuccess ||
+                        cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1) != cudaSuccess))
+  {
+    cudaGetLastError();
+    rc = SPSS_ERR_CUDA;
+  }
+  const int rc2 = restore_snapshot(ctx);
   ctx->timing = timing;
   if (rc != SPSS_OK) return rc;
   if (rc2 != SPSS_OK) return rc2;
-  if (rc3 != SPSS_OK) return rc3;
-  if (best_ms) *best_ms = best;
+  if (best_ms) *best_ms = ms / steps;
   return SPSS_OK;
 }
 

@@ -440,7 +440,6 @@ struct FastControl
                             // timeout; bit 2: stencil cell outside the staged segments; bit 3: the
                             // device launch of the rebuild graph was refused
   int uses_verlet;
-  int tile_next;            // work counter of the persistent tile kernel
   unsigned ticket;          // blocks of the running reduction that are done (its last block puts it back to 0)
   int triggered;            // the last step's displacement trigger fired (its rebuild may already be done)
   long long sample_every;   // order-parameter samples after steps that are multiples of this (0: none)
