@@ -350,15 +350,45 @@ __device__ __forceinline__ void normals_f64(const double2 *__restrict__ table, c
 
 // ------------------------------------------------------------------ reductions
 
-// Sums of `nparts` partials of four values each, in a fixed order, by one
-// block of 256 threads (the result is valid in thread 0): thread t adds
-// partials t, t + 256, ..., the warps' lanes combine by a shuffle tree, thread
-// 0 adds the warps.
-__device__ __forceinline__ void block_sum_partials(const double *__restrict__ partials, int nparts, double t[4])
+// Sums of four values over a warp: lane l gets that of value l >> 3.  The first
+// two exchanges halve what a lane carries, so six additions an FP64 warp sum
+// costs, not 20 (16 cycles each: the chip has two FP64 lanes an SM).
+__device__ __forceinline__ double warp_sum4(const double a[4])
 {
-  __shared__ double sh[8][4];
+  const int lane = threadIdx.x & 31;
+  const bool up = lane & 16, odd = lane & 8;
+  const double k0 = (up ? a[2] : a[0]) + __shfl_xor_sync(0xffffffffu, up ? a[0] : a[2], 16);
+  const double k1 = (up ? a[3] : a[1]) + __shfl_xor_sync(0xffffffffu, up ? a[1] : a[3], 16);
+  double k = (odd ? k1 : k0) + __shfl_xor_sync(0xffffffffu, odd ? k0 : k1, 8);
 #pragma unroll
-  for (int c = 0; c < 4; ++c) t[c] = 0.0;
+  for (int off = 4; off > 0; off >>= 1) k += __shfl_xor_sync(0xffffffffu, k, off);
+  return k;
+}
+
+// Sums of four values over a block of 256 threads, `mine` as warp_sum4 returns
+// it: lane l of warp 0 gets that of value l >> 3.
+__device__ __forceinline__ double block_sum4(double mine)
+{
+  __shared__ double sh[4][8];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  if ((lane & 7) == 0) sh[lane >> 3][wid] = mine;
+  __syncthreads();
+  double k = 0.0;
+  if (wid == 0)
+  {
+    k = sh[lane >> 3][lane & 7];
+#pragma unroll
+    for (int off = 4; off > 0; off >>= 1) k += __shfl_xor_sync(0xffffffffu, k, off);
+  }
+  __syncthreads();
+  return k;
+}
+
+// Sums of `nparts` partials of four values each, in a fixed order, by one
+// block of 256 threads: lane l of warp 0 gets that of value l >> 3.
+__device__ __forceinline__ double block_sum_partials4(const double *__restrict__ partials, int nparts)
+{
+  double t[4] = {0.0, 0.0, 0.0, 0.0};
   for (int b = threadIdx.x; b < nparts; b += 256)
   {
     // __ldcg: the partials may have been written by other blocks of the same launch
@@ -369,18 +399,16 @@ __device__ __forceinline__ void block_sum_partials(const double *__restrict__ pa
     t[2] += hi.x;
     t[3] += hi.y;
   }
+  return block_sum4(warp_sum4(t));
+}
+
+// The same with all four sums in thread 0.
+__device__ __forceinline__ void block_sum_partials(const double *__restrict__ partials, int nparts, double t[4])
+{
+  const double k = block_sum_partials4(partials, nparts);
+  if (threadIdx.x < 32)
 #pragma unroll
-  for (int off = 16; off > 0; off >>= 1)
-#pragma unroll
-    for (int c = 0; c < 4; ++c) t[c] += __shfl_xor_sync(0xffffffffu, t[c], off);
-  if ((threadIdx.x & 31) == 0)
-#pragma unroll
-    for (int c = 0; c < 4; ++c) sh[threadIdx.x >> 5][c] = t[c];
-  __syncthreads();
-  if (threadIdx.x == 0)
-    for (int w = 1; w < 8; ++w)
-#pragma unroll
-      for (int c = 0; c < 4; ++c) t[c] += sh[w][c];
+    for (int c = 0; c < 4; ++c) t[c] = __shfl_sync(0xffffffffu, k, 8 * c);
 }
 
 // {|R|, arg R, |R_v|, arg R_v} from the sums of cos phi, sin phi, v_x/|v|, v_y/|v|.
@@ -433,7 +461,8 @@ struct FastControl
   int parity;               // current rec/aux buffer
   int order_parity;         // current vel/pid buffer (they change places only when the slots are re-sorted)
   int rebuild;              // lists (and slot order) rebuilt before the next evaluation
-  int cells_fresh;          // cell ids and counts of the current slots were written by the last cell-list step
+  int cells_fresh;          // the last step left what the next one begins with: cell ids and counts of the
+                            // current slots (cell lists), the field of the current state (global field)
   int overflow;             // largest Verlet count seen beyond capacity (0: none)
   int rebuilds;             // number of rebuilds performed
   int error;                // bit 0: displacement too large for the fixed-point increment; bit 1: staging
