@@ -1722,7 +1722,10 @@ __global__ void __launch_bounds__(kTileThreads, STEPPER == 2 ? SPSS_LIST_BLOCKS_
   publish_max(ctrl, B.sysctl, sys, d2max, err);
 }
 
-// end_step as a launch of its own.
+// end_step as a launch of its own, resident before the step kernel ends (a step
+// of 2,000 to 65,536 particles on Verlet lists 0.5 us shorter; as the last block
+// of the step kernel, whose barrier and registers every block then pays for,
+// 1 to 2 us longer, 25 % at 4,194,304).
 // TAIL (steps run as graphs): `rebuild_exec`, the rebuild as a device graph,
 // is tail-launched here when a rebuild is due, so it runs right after this
 // step's graph and before the next one, and a step without a rebuild needs
@@ -1733,6 +1736,7 @@ __global__ void fast_control_kernel(FastControl *ctrl, SysControl *sysctl, const
                                     int always_rebuild, int verlet, int selective, int cells_written,
                                     cudaGraphExec_t rebuild_exec)
 {
+  pdl_enter();
   end_step(ctrl, sysctl, sys, nsys, always_rebuild, verlet, selective, cells_written);
   if (threadIdx.x == 0 && TAIL && ctrl->rebuild)
     if (cudaGraphLaunch(rebuild_exec, cudaStreamGraphTailLaunch) != cudaSuccess) atomicOr(&ctrl->error, 8);
@@ -2671,9 +2675,10 @@ static int control_threads(int nsys)
 static int launch_control(spss_ctx *ctx, const FastParams &P, int cells_written)
 {
   FastPath *f = ctx->fast;
-  fast_control_kernel<false><<<1, control_threads(f->nsys), 0, ctx->stream>>>(f->ctrl, f->sysctl.ptr, f->sys.ptr, f->nsys, P.always_rebuild,
-                                                         f->kind == KIND_VERLET || f->trigger_only, P.selective,
-                                                         cells_written, nullptr);
+  SPSS_CUDA_TRY(launch_chained(true, fast_control_kernel<false>, 1, control_threads(f->nsys), 0, ctx->stream, f->ctrl,
+                               f->sysctl.ptr, (const SysParams *) f->sys.ptr, f->nsys, P.always_rebuild,
+                               (int) (f->kind == KIND_VERLET || f->trigger_only), P.selective, cells_written,
+                               (cudaGraphExec_t) nullptr));
   ++ctx->launches;
   return check_launch("fast_control_kernel");
 }
@@ -2697,9 +2702,9 @@ static int launch_step(spss_ctx *ctx, int stepper, const FastParams &P, cudaGrap
   FastPath *f = ctx->fast;
   if (f->kind == KIND_GLOBAL) return SPSS_OK;  // its step kernel ends the step
   if (rebuild_exec)
-    fast_control_kernel<true><<<1, control_threads(f->nsys), 0, ctx->stream>>>(f->ctrl, f->sysctl.ptr, f->sys.ptr, f->nsys,
-                                                          P.always_rebuild, f->kind == KIND_VERLET || f->trigger_only,
-                                                          P.selective, 0, rebuild_exec);
+    SPSS_CUDA_TRY(launch_chained(true, fast_control_kernel<true>, 1, control_threads(f->nsys), 0, ctx->stream, f->ctrl,
+                                 f->sysctl.ptr, (const SysParams *) f->sys.ptr, f->nsys, P.always_rebuild,
+                                 (int) (f->kind == KIND_VERLET || f->trigger_only), P.selective, 0, rebuild_exec));
   else
     SPSS_TRY(launch_control(ctx, P, 0));
   if (rebuild_exec) ++ctx->launches;
