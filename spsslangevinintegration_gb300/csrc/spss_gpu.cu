@@ -509,6 +509,7 @@ int spss_step_host(spss_ctx *ctx, int stepper, double *state, long len, double t
   // host link and the download kernel writes it back, each in one pass that
   // also converts the layout.  Otherwise stage through device memory.
   double *io = ctx->registered_device;
+  if (io && !is_f64(ctx)) return fast_step_state(ctx, stepper, dt, io);
   if (!io)
   {
     SPSS_TRY(ctx->scratch_a.reserve(len));

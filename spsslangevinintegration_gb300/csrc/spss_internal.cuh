@@ -595,6 +595,7 @@ int fast_set_state(spss_ctx *ctx, const double *d_aos);
 int fast_get_state(spss_ctx *ctx, double *d_aos);
 int fast_evaluate(spss_ctx *ctx, int variant, const double *d_state, const double *d_kprev, double *d_knext,
                   double k_coef, double dt);
+int fast_step_state(spss_ctx *ctx, int stepper, double dt, double *io);
 int fast_step(spss_ctx *ctx, int stepper, double t, double dt);
 int fast_steps(spss_ctx *ctx, int stepper, double t0, double dt, int nsteps);
 int fast_noise(spss_ctx *ctx, int stepper, unsigned long long step, double *d_out);
