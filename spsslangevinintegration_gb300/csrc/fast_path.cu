@@ -495,8 +495,8 @@ __global__ void fast_upload_kernel(const double *__restrict__ x, int n, int s, i
 __global__ void fast_download_kernel(double *__restrict__ x, int n, int s, int model, FastBuffers B,
                                      FastControl *__restrict__ host_ctrl)
 {
-  extern __shared__ double rows[];
   pdl_enter();
+  extern __shared__ double rows[];
   if (host_ctrl)
   {
     if (blockIdx.x == 0 && threadIdx.x == 0) *host_ctrl = *B.ctrl;
