@@ -328,6 +328,17 @@ int Binner::place(const int *cell_of, int n, cudaStream_t stream, unsigned long 
   return check_launch("bin_scatter_kernel");
 }
 
+// From the counts to the sorted members.
+int Binner::finish(const int *cell_of, int n, cudaStream_t stream, unsigned long long &launches, bool chained)
+{
+  const int tb = 256;
+  SPSS_TRY(place(cell_of, n, stream, launches, chained));
+  SPSS_CUDA_TRY(launch_chained(chained, bin_sort_kernel, (ncell + tb - 1) / tb, tb, 0, stream,
+                               (const int *) offsets.ptr, ncell, members.ptr));
+  ++launches;
+  return check_launch("bin_sort_kernel");
+}
+
 int Binner::run(const int *cell_of, int n, int ncell_in, cudaStream_t stream, unsigned long long &launches)
 {
   SPSS_TRY(prepare(n, ncell_in, stream));
@@ -335,10 +346,7 @@ int Binner::run(const int *cell_of, int n, int ncell_in, cudaStream_t stream, un
   bin_count_kernel<<<(n + tb - 1) / tb, tb, 0, stream>>>(cell_of, n, count.ptr, slot.ptr);
   ++launches;
   SPSS_TRY(check_launch("bin_count_kernel"));
-  SPSS_TRY(place(cell_of, n, stream, launches));
-  bin_sort_kernel<<<(ncell + tb - 1) / tb, tb, 0, stream>>>(offsets.ptr, ncell, members.ptr);
-  ++launches;
-  return check_launch("bin_sort_kernel");
+  return finish(cell_of, n, stream, launches, false);
 }
 
 }  // namespace spss

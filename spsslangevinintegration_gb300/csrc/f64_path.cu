@@ -239,11 +239,29 @@ __device__ __forceinline__ void write_k(const K64 &k, int i, const double *st, S
 
 // ------------------------------------------------------------ kernels
 
+// The binning that a stage kernel starts (nc cells a side, 0: none).
+struct StageCells
+{
+  int nc, *cell_of, *count, *slot;
+};
+
+// Cell of a stage position, and its place among the cell's members by arrival.
+__device__ __forceinline__ int stage_cell(const K64 &k, const double *rk, int i, int nc)
+{
+  double x, y;
+  pos_for_cells(k, rk, i, x, y);
+  return cell_coord(y, nc) * nc + cell_coord(x, nc);
+}
+
 // rk_system_state = system_state + k_coef * dt * k_prev (ParticleSystemFirstOrder.cpp:175-184),
 // and (posf not null) the stage positions wrapped into the unit box as floats
-// for the range pre-test; one particle per thread.
+// for the range pre-test; one particle per thread.  kp null: k_prev is zero.
+// det (not null): its torque components are cleared, which the derivative
+// leaves as they are where a particle has no neighbour.  Cells: counted on the
+// way, which as two kernels behind this one took 9 us of a step of N = 65,536.
 __global__ void f64_stage_kernel(K64 k, const double *__restrict__ st, const double *__restrict__ kp,
-                                 double *__restrict__ rk, float2 *__restrict__ posf, double k_coef, double dt)
+                                 double *__restrict__ rk, float2 *__restrict__ posf, double k_coef, double dt,
+                                 double *__restrict__ det, StageCells cells)
 {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= k.n) return;
@@ -252,10 +270,17 @@ __global__ void f64_stage_kernel(K64 k, const double *__restrict__ st, const dou
   double2 *r2 = reinterpret_cast<double2 *>(rk + (long) k.s * i);
   for (int q = 0; q < k.s / 2; ++q)
   {
-    const double2 a = s2[q], b = k2[q];
+    const double2 a = s2[q], b = kp ? k2[q] : make_double2(0.0, 0.0);
     const double2 r = make_double2(a.x + k_coef * dt * b.x, a.y + k_coef * dt * b.y);
     r2[q] = r;
     if (q == 0 && posf) posf[i] = make_float2((float) (r.x - floor(r.x)), (float) (r.y - floor(r.y)));
+  }
+  if (det) det[(long) k.s * i + k.s - 1] = 0.0;
+  if (cells.nc)
+  {
+    const int c = stage_cell(k, rk, i, cells.nc);
+    cells.cell_of[i] = c;
+    cells.slot[i] = atomicAdd(cells.count + c, 1);
   }
 }
 
@@ -263,9 +288,7 @@ __global__ void f64_cell_kernel(K64 k, const double *__restrict__ rk, int nc, in
 {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= k.n) return;
-  double x, y;
-  pos_for_cells(k, rk, i, x, y);
-  cell_of[i] = cell_coord(y, nc) * nc + cell_coord(x, nc);
+  cell_of[i] = stage_cell(k, rk, i, nc);
 }
 
 // The stage state of one particle per thread (the same expression as
@@ -682,6 +705,7 @@ __global__ void __launch_bounds__(kPairThreads) f64_linked_list_kernel(K64 k, co
                                                                        double *__restrict__ k_next,
                                                                        double *__restrict__ caf)
 {
+  pdl_enter();
   __shared__ PairBuffers buf[kPairThreads / 32];
   PairBuffers &Q = buf[threadIdx.x >> 5];
   const int t = blockIdx.x * kPairThreads + threadIdx.x;
@@ -801,6 +825,7 @@ __global__ void __launch_bounds__(kPairThreads) f64_verlet_pairs_kernel(K64 k, c
                                                                         double *__restrict__ k_next,
                                                                         double *__restrict__ caf)
 {
+  pdl_enter();
   __shared__ PairBuffers buf[kPairThreads / 32];
   PairBuffers &Q = buf[threadIdx.x >> 5];
   const int t = blockIdx.x * kPairThreads + threadIdx.x;
@@ -898,14 +923,41 @@ __global__ void f64_rk4_combine_kernel(double *__restrict__ x, const double *__r
   x[q] += d;
 }
 
+// Where a stepper leaves the largest squared displacement of its step for the
+// Verlet trigger (ParticleSystemFirstOrder.cpp:672-684): `host` is page-locked,
+// `max2` and `ticket` are zero between launches.  max2 null: not asked for.
+struct MaxOut
+{
+  unsigned long long *max2, *host;
+  unsigned *ticket;
+};
+
+// Non-negative doubles order like their bit patterns; NaN counts as 0.  All
+// threads of all blocks; the last block hands the maximum to the host (a kernel
+// over the displacements, a copy and two clears, as it was, took 6 us a step).
+__device__ __forceinline__ void publish_max2(const MaxOut &m, double2 d)
+{
+  if (!m.max2) return;
+  const double d2 = d.x * d.x + d.y * d.y;
+  unsigned long long v = d2 > 0.0 ? (unsigned long long) __double_as_longlong(d2) : 0ull;
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, off));
+  if ((threadIdx.x & 31) == 0 && v > *(volatile unsigned long long *) m.max2) atomicMax(m.max2, v);
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x != 0 || atomicAdd(m.ticket, 1u) != gridDim.x - 1) return;
+  __threadfence();
+  *m.ticket = 0u;
+  *m.host = atomicExch(m.max2, 0ull);
+}
+
 // Second-order stochastic Euler (StochasticEulerStepper.hpp:33-51 with
 // ParticleSystemSecondOrder::AddNoise, ParticleSystemSecondOrder.cpp:439-451).
-__global__ void f64_se2_kernel(double *__restrict__ x, const double *__restrict__ det, double *__restrict__ td,
-                               int n, double dt, double sqrt_dt, double intensity_r, double intensity_phi,
-                               NoiseKey nk, const double2 *__restrict__ table)
+__device__ __forceinline__ double2 se2_particle(int i, double *__restrict__ x, const double *__restrict__ det,
+                                                double *__restrict__ td, double dt, double sqrt_dt,
+                                                double intensity_r, double intensity_phi, NoiseKey nk,
+                                                const double2 *__restrict__ table)
 {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
   const uint4 u = philox_block(nk, (uint32_t) i, 0);
   // without translational noise (intensity_r = 0) its two normals multiply 0
   double z[4] = {0.0, 0.0, 0.0, 0.0};
@@ -925,15 +977,26 @@ __global__ void f64_se2_kernel(double *__restrict__ x, const double *__restrict_
   x2[0] = make_double2(a.x + tr.x, a.y + tr.y);
   x2[1] = make_double2(b.x + tv.x, b.y + tv.y);
   x2[2] = make_double2(c.x + tp.x, c.y + tp.y);
+  return tr;
+}
+
+__global__ void f64_se2_kernel(double *__restrict__ x, const double *__restrict__ det, double *__restrict__ td,
+                               int n, double dt, double sqrt_dt, double intensity_r, double intensity_phi,
+                               NoiseKey nk, const double2 *__restrict__ table, MaxOut m)
+{
+  pdl_enter();
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  double2 moved = make_double2(0.0, 0.0);
+  if (i < n) moved = se2_particle(i, x, det, td, dt, sqrt_dt, intensity_r, intensity_phi, nk, table);
+  publish_max2(m, moved);
 }
 
 // First-order stochastic Euler (StochasticEulerStepperPtr.hpp:40-73).
-__global__ void f64_se1_kernel(double *__restrict__ x, const double *__restrict__ d, double *__restrict__ td, int n,
-                               double dt, double sqrt_dt, double intensity_phi, NoiseKey nk,
-                               const double2 *__restrict__ table)
+__device__ __forceinline__ double2 se1_particle(int i, double *__restrict__ x, const double *__restrict__ d,
+                                                double *__restrict__ td, double dt, double sqrt_dt,
+                                                double intensity_phi, NoiseKey nk,
+                                                const double2 *__restrict__ table)
 {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
   double z[2];
   normals_f64<1>(table, nk, (uint32_t) i, 0, z);
   const double delta_W_phi = sqrt_dt * z[0];
@@ -943,16 +1006,27 @@ __global__ void f64_se1_kernel(double *__restrict__ x, const double *__restrict_
   td[ii + 2] = d[ii + 2] * dt;
   td[ii + 3] = d[ii + 3] * dt + intensity_phi * delta_W_phi;
   for (int s = 0; s < 4; ++s) x[ii + s] += td[ii + s];
+  return make_double2(td[ii], td[ii + 1]);
+}
+
+__global__ void f64_se1_kernel(double *__restrict__ x, const double *__restrict__ d, double *__restrict__ td,
+                               int n, double dt, double sqrt_dt, double intensity_phi, NoiseKey nk,
+                               const double2 *__restrict__ table, MaxOut m)
+{
+  pdl_enter();
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  double2 moved = make_double2(0.0, 0.0);
+  if (i < n) moved = se1_particle(i, x, d, td, dt, sqrt_dt, intensity_phi, nk, table);
+  publish_max2(m, moved);
 }
 
 // First-order strong order 1.5 Taylor scheme (StochasticRungeKuttaStepperPtr.hpp:40-76).
-__global__ void f64_srk1_kernel(double *__restrict__ x, const double *__restrict__ d, const double *__restrict__ caf,
-                                double *__restrict__ td, int n, double dt, double sqrt_dt, double dt15,
-                                double inv_sqrt3, double sqrt_2noise, double friction, NoiseKey nk,
-                                const double2 *__restrict__ table)
+__device__ __forceinline__ double2 srk1_particle(int i, double *__restrict__ x, const double *__restrict__ d,
+                                                 const double *__restrict__ caf, double *__restrict__ td,
+                                                 double dt, double sqrt_dt, double dt15, double inv_sqrt3,
+                                                 double sqrt_2noise, double friction, NoiseKey nk,
+                                                 const double2 *__restrict__ table)
 {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
   double z[2];
   normals_f64<1>(table, nk, (uint32_t) i, 0, z);
   const double U_1 = z[0], U_2 = z[1];
@@ -965,18 +1039,30 @@ __global__ void f64_srk1_kernel(double *__restrict__ x, const double *__restrict
   td[ii + 3] = d[ii + 3] * dt + 0.5 * (caf[i] - friction * d[ii + 3]) * dt * dt
       + sqrt_2noise * (delta_W_i - friction * delta_Z_i);
   for (int s = 0; s < 4; ++s) x[ii + s] += td[ii + s];
+  return make_double2(td[ii], td[ii + 1]);
+}
+
+__global__ void f64_srk1_kernel(double *__restrict__ x, const double *__restrict__ d,
+                                const double *__restrict__ caf, double *__restrict__ td, int n, double dt,
+                                double sqrt_dt, double dt15, double inv_sqrt3, double sqrt_2noise, double friction,
+                                NoiseKey nk, const double2 *__restrict__ table, MaxOut m)
+{
+  pdl_enter();
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  double2 moved = make_double2(0.0, 0.0);
+  if (i < n) moved = srk1_particle(i, x, d, caf, td, dt, sqrt_dt, dt15, inv_sqrt3, sqrt_2noise, friction, nk, table);
+  publish_max2(m, moved);
 }
 
 // Second-order strong order 1.5 Taylor scheme (no reference code): the
 // first-order scheme's construction applied to the second-order drift with
 // additive noise on v_x, v_y (b_r) and omega (b_phi); see spss_oracle.c.
-__global__ void f64_srk2_kernel(double *__restrict__ x, const double *__restrict__ d, const double *__restrict__ caf,
-                                double *__restrict__ td, int n, double dt, double sqdt, double dt15, double inv_sqrt3,
-                                double b_r, double b_phi, double xi_r, double xi_phi, double v0, NoiseKey nk,
-                                const double2 *__restrict__ table)
+__device__ __forceinline__ double2 srk2_particle(int i, double *__restrict__ x, const double *__restrict__ d,
+                                                 const double *__restrict__ caf, double *__restrict__ td,
+                                                 double dt, double sqdt, double dt15, double inv_sqrt3, double b_r,
+                                                 double b_phi, double xi_r, double xi_phi, double v0, NoiseKey nk,
+                                                 const double2 *__restrict__ table)
 {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
   double u[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
   if (b_r != 0.0) normals_f64<2>(table, nk, (uint32_t) i, 0, u);  // b_r = 0 multiplies them
   normals_f64<1>(table, nk, (uint32_t) i, 1, u + 4);
@@ -993,6 +1079,21 @@ __global__ void f64_srk2_kernel(double *__restrict__ x, const double *__restrict
   td[ii + 4] = d[ii + 4] * dt + 0.5 * d[ii + 5] * dt * dt + b_phi * dZw;
   td[ii + 5] = d[ii + 5] * dt + 0.5 * (caf[i] - xi_phi * d[ii + 5]) * dt * dt + b_phi * (dWw - xi_phi * dZw);
   for (int s = 0; s < 6; ++s) x[ii + s] += td[ii + s];
+  return make_double2(td[ii], td[ii + 1]);
+}
+
+__global__ void f64_srk2_kernel(double *__restrict__ x, const double *__restrict__ d,
+                                const double *__restrict__ caf, double *__restrict__ td, int n, double dt,
+                                double sqdt, double dt15, double inv_sqrt3, double b_r, double b_phi, double xi_r,
+                                double xi_phi, double v0, NoiseKey nk, const double2 *__restrict__ table,
+                                MaxOut m)
+{
+  pdl_enter();
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  double2 moved = make_double2(0.0, 0.0);
+  if (i < n) moved = srk2_particle(i, x, d, caf, td, dt, sqdt, dt15, inv_sqrt3, b_r, b_phi, xi_r, xi_phi, v0, nk,
+                               table);
+  publish_max2(m, moved);
 }
 
 // max_i (dx^2 + dy^2) of a displacement array (ParticleSystemFirstOrder.cpp:672-684);
@@ -1062,7 +1163,8 @@ int f64_create(spss_ctx *ctx)
   SPSS_TRY(f->csphi.reserve(ctx->p.n));
   SPSS_TRY(f->vl_count.reserve(ctx->p.n));
   SPSS_TRY(f->vl_off.reserve(ctx->p.n + 1));
-  SPSS_TRY(f->max2.reserve(1));
+  SPSS_TRY(f->max2.reserve(3));  // of an array of displacements; a stepper's, and its count of finished blocks
+  SPSS_CUDA_TRY(cudaMemsetAsync(f->max2.ptr, 0, 3 * sizeof(unsigned long long), ctx->stream));
   SPSS_TRY(f->partials.reserve(4 * 1024));
   SPSS_TRY(make_f64_tables(f->table, ctx->stream));
   SPSS_CUDA_TRY(cudaMallocHost((void **) &f->h_max2, sizeof(unsigned long long)));
@@ -1180,8 +1282,9 @@ static int build_verlet(spss_ctx *ctx, const K64 &k, bool from_cells)
   return SPSS_OK;
 }
 
-int f64_evaluate(spss_ctx *ctx, int variant, const double *d_state, const double *d_kprev, double *d_knext,
-                 double k_coef, double dt)
+// `det` (not null): cleared as a derivative whose torque components nothing adds to.
+static int evaluate(spss_ctx *ctx, int variant, const double *d_state, const double *d_kprev, double *d_knext,
+                    double k_coef, double dt, double *det)
 {
   F64Path *f = ctx->f64;
   variant = variant_for(ctx, variant);
@@ -1193,11 +1296,21 @@ int f64_evaluate(spss_ctx *ctx, int variant, const double *d_state, const double
     f64_stage_posf_kernel<<<blocks_for(k.n, tb), tb, 0, ctx->stream>>>(k, d_state, d_kprev, f->rk.ptr, f->posf.ptr,
                                                                        f->csphi.ptr, k_coef, dt);
   else
+  {
+    StageCells cells{0, nullptr, nullptr, nullptr};
+    if (variant == SPSS_VARIANT_LINKED_LIST)
+    {
+      SPSS_TRY(f->binner.prepare(k.n, ctx->nc * ctx->nc, ctx->stream));
+      cells = StageCells{ctx->nc, f->cell_of.ptr, f->binner.count.ptr, f->binner.slot.ptr};
+    }
     f64_stage_kernel<<<blocks_for(k.n, tb), tb, 0, ctx->stream>>>(
-        k, d_state, d_kprev, f->rk.ptr, variant == SPSS_VARIANT_GLOBAL_FIELD ? nullptr : f->posf.ptr, k_coef, dt);
+        k, d_state, d_kprev, f->rk.ptr, variant == SPSS_VARIANT_GLOBAL_FIELD ? nullptr : f->posf.ptr, k_coef, dt, det,
+        cells);
+  }
   ++ctx->launches;
   SPSS_TRY(check_launch("f64_stage_kernel"));
-  if (k.higher_order) SPSS_CUDA_TRY(cudaMemsetAsync(f->caf.ptr, 0, sizeof(double) * k.n, ctx->stream));
+  // the pair kernels write every complementary force
+  if (k.higher_order && variant == SPSS_VARIANT_GLOBAL_FIELD) SPSS_CUDA_TRY(cudaMemsetAsync(f->caf.ptr, 0, sizeof(double) * k.n, ctx->stream));
   switch (variant)
   {
     case SPSS_VARIANT_ALL_PAIRS:
@@ -1206,25 +1319,32 @@ int f64_evaluate(spss_ctx *ctx, int variant, const double *d_state, const double
       ++ctx->launches;
       return check_launch("f64_allpairs_kernel");
     case SPSS_VARIANT_LINKED_LIST:
-      SPSS_TRY(build_cells(ctx, k, ctx->nc));
-      f64_linked_list_kernel<<<blocks_for(k.n, kPairThreads), kPairThreads, 0, ctx->stream>>>(
-          k, f->rk.ptr, f->posf.ptr, ctx->nc, f->binner.offsets.ptr, f->binner.members.ptr, d_knext, f->caf.ptr);
+      SPSS_TRY(f->binner.finish(f->cell_of.ptr, k.n, ctx->stream, ctx->launches, true));
+      f->cells_nc = ctx->nc;
+      SPSS_CUDA_TRY(launch_chained(true, f64_linked_list_kernel, blocks_for(k.n, kPairThreads), kPairThreads, 0,
+                                   ctx->stream, k, (const double *) f->rk.ptr, (const float2 *) f->posf.ptr, ctx->nc,
+                                   (const int *) f->binner.offsets.ptr, (const int *) f->binner.members.ptr, d_knext,
+                                   f->caf.ptr));
       ++ctx->launches;
       return check_launch("f64_linked_list_kernel");
     case SPSS_VARIANT_VERLET:
     case SPSS_VARIANT_LINKED_LIST_VERLET:
-      if (ctx->should_update_lists)
+    {
+      const bool build = ctx->should_update_lists;
+      if (build)
       {
         SPSS_TRY(build_verlet(ctx, k, variant == SPSS_VARIANT_LINKED_LIST_VERLET));
         ctx->should_update_lists = 0;
         ++ctx->list_builds;
       }
       ctx->uses_verlet_list = 1;
-      f64_verlet_pairs_kernel<<<blocks_for(k.n, kPairThreads), kPairThreads, 0, ctx->stream>>>(
-          k, f->rk.ptr, f->posf.ptr, f->cells_nc ? f->binner.members.ptr : nullptr, f->vl_off.ptr, f->vl_ent.ptr,
-          d_knext, f->caf.ptr);
+      SPSS_CUDA_TRY(launch_chained(!build, f64_verlet_pairs_kernel, blocks_for(k.n, kPairThreads), kPairThreads, 0,
+                                   ctx->stream, k, (const double *) f->rk.ptr, (const float2 *) f->posf.ptr,
+                                   (const int *) (f->cells_nc ? f->binner.members.ptr : nullptr),
+                                   (const int *) f->vl_off.ptr, (const int *) f->vl_ent.ptr, d_knext, f->caf.ptr));
       ++ctx->launches;
       return check_launch("f64_verlet_pairs_kernel");
+    }
     case SPSS_VARIANT_GLOBAL_FIELD:
     {
       const int nparts = std::min(1024, blocks_for(k.n, 256));
@@ -1238,6 +1358,12 @@ int f64_evaluate(spss_ctx *ctx, int variant, const double *d_state, const double
     }
   }
   return SPSS_ERR_INVALID_ARGUMENT;
+}
+
+int f64_evaluate(spss_ctx *ctx, int variant, const double *d_state, const double *d_kprev, double *d_knext,
+                 double k_coef, double dt)
+{
+  return evaluate(ctx, variant, d_state, d_kprev, d_knext, k_coef, dt, nullptr);
 }
 
 int f64_max_displacement(spss_ctx *ctx, const double *d_td, double *max2_out)
@@ -1332,32 +1458,37 @@ int f64_step(spss_ctx *ctx, int stepper, double t, double dt)
   } else
   {
     const NoiseKey nk = noise_key(ctx, ctx->step_counter);
-    SPSS_CUDA_TRY(cudaMemsetAsync(f->det.ptr, 0, sizeof(double) * len, ctx->stream));
+    if (variant_for(ctx, variant) == SPSS_VARIANT_ALL_PAIRS)
+      SPSS_CUDA_TRY(cudaMemsetAsync(f->det.ptr, 0, sizeof(double) * len, ctx->stream));
     if (stepper == SPSS_STEPPER_STOCHASTIC_RUNGE_KUTTA) ctx->higher_order = 1;
-    SPSS_TRY(f64_evaluate(ctx, variant, f->state.ptr, f->det.ptr, f->det.ptr, 0.0, dt));
-    const double sqrt_dt = std::sqrt(dt);
+    if (variant_for(ctx, variant) == SPSS_VARIANT_ALL_PAIRS)
+      SPSS_TRY(evaluate(ctx, variant, f->state.ptr, f->det.ptr, f->det.ptr, 0.0, dt, nullptr));
+    else
+      SPSS_TRY(evaluate(ctx, variant, f->state.ptr, nullptr, f->det.ptr, 0.0, dt, f->det.ptr));
+    const double sqrt_dt = std::sqrt(dt), dt15 = std::pow(dt, 1.5), inv_sqrt3 = 1.0 / std::sqrt(3.0);
+    const double b_r = std::sqrt(2.0 * ctx->p.D_r), b_phi = std::sqrt(2.0 * ctx->p.D_phi);
+    const double *det = f->det.ptr, *caf = f->caf.ptr;
+    const double2 *table = f->table.ptr;
+    const int blocks = blocks_for(n, tb);
+    MaxOut m{nullptr, nullptr, nullptr};
+    if (ctx->uses_verlet_list) m = MaxOut{f->max2.ptr + 1, f->h_max2, reinterpret_cast<unsigned *>(f->max2.ptr + 2)};
     if (stepper == SPSS_STEPPER_STOCHASTIC_EULER)
     {
       if (ctx->p.model == 2)
-        f64_se2_kernel<<<blocks_for(n, tb), tb, 0, ctx->stream>>>(f->state.ptr, f->det.ptr, f->td.ptr, n, dt,
-                                                                  sqrt_dt, std::sqrt(2.0 * ctx->p.D_r),
-                                                                  std::sqrt(2.0 * ctx->p.D_phi), nk, f->table.ptr);
+        SPSS_CUDA_TRY(launch_chained(true, f64_se2_kernel, blocks, tb, 0, ctx->stream, f->state.ptr, det, f->td.ptr, n,
+                                     dt, sqrt_dt, b_r, b_phi, nk, table, m));
       else
-        f64_se1_kernel<<<blocks_for(n, tb), tb, 0, ctx->stream>>>(f->state.ptr, f->det.ptr, f->td.ptr, n, dt,
-                                                                  sqrt_dt, std::sqrt(2.0 * ctx->p.D_phi), nk, f->table.ptr);
+        SPSS_CUDA_TRY(launch_chained(true, f64_se1_kernel, blocks, tb, 0, ctx->stream, f->state.ptr, det, f->td.ptr, n,
+                                     dt, sqrt_dt, b_phi, nk, table, m));
     } else if (stepper == SPSS_STEPPER_STOCHASTIC_RUNGE_KUTTA)
     {
-      const double dt15 = std::pow(dt, 1.5), inv_sqrt3 = 1.0 / std::sqrt(3.0);
       if (ctx->p.model == 1)
-        f64_srk1_kernel<<<blocks_for(n, tb), tb, 0, ctx->stream>>>(f->state.ptr, f->det.ptr, f->caf.ptr, f->td.ptr,
-                                                                   n, dt, sqrt_dt, dt15, inv_sqrt3,
-                                                                   std::sqrt(2.0 * ctx->p.D_phi), ctx->p.xi, nk,
-                                                                   f->table.ptr);
+        SPSS_CUDA_TRY(launch_chained(true, f64_srk1_kernel, blocks, tb, 0, ctx->stream, f->state.ptr, det, caf,
+                                     f->td.ptr, n, dt, sqrt_dt, dt15, inv_sqrt3, b_phi, ctx->p.xi, nk, table, m));
       else
-        f64_srk2_kernel<<<blocks_for(n, tb), tb, 0, ctx->stream>>>(
-            f->state.ptr, f->det.ptr, f->caf.ptr, f->td.ptr, n, dt, sqrt_dt, dt15, inv_sqrt3,
-            std::sqrt(2.0 * ctx->p.D_r), std::sqrt(2.0 * ctx->p.D_phi), ctx->p.xi_r, ctx->p.xi_phi, ctx->p.v0, nk,
-            f->table.ptr);
+        SPSS_CUDA_TRY(launch_chained(true, f64_srk2_kernel, blocks, tb, 0, ctx->stream, f->state.ptr, det, caf,
+                                     f->td.ptr, n, dt, sqrt_dt, dt15, inv_sqrt3, b_r, b_phi, ctx->p.xi_r,
+                                     ctx->p.xi_phi, ctx->p.v0, nk, table, m));
     } else
     {
       return SPSS_ERR_INVALID_ARGUMENT;
@@ -1369,7 +1500,14 @@ int f64_step(spss_ctx *ctx, int stepper, double t, double dt)
   if (ctx->uses_verlet_list)
   {
     double max2 = 0.0;
-    SPSS_TRY(f64_max_displacement(ctx, f->td.ptr, &max2));
+    if (stepper == SPSS_STEPPER_RK4)
+    {
+      SPSS_TRY(f64_max_displacement(ctx, f->td.ptr, &max2));
+    } else
+    {
+      SPSS_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+      std::memcpy(&max2, f->h_max2, sizeof(double));
+    }
     SPSS_TRY(host_calculate_max_displacement(ctx, max2));
   }
   return SPSS_OK;

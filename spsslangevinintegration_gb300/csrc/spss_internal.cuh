@@ -510,7 +510,9 @@ struct Binner
   // in arrival order; the counts are zero again.
   int place(const int *cell_of, int n, cudaStream_t stream, unsigned long long &launches, bool chained = false,
             FastControl *ctrl = nullptr);
-  // all of it, members in ascending order
+  // the same with members in ascending order
+  int finish(const int *cell_of, int n, cudaStream_t stream, unsigned long long &launches, bool chained);
+  // all of it
   int run(const int *cell_of, int n, int ncell, cudaStream_t stream, unsigned long long &launches);
   void release()
   {
