@@ -1,4 +1,6 @@
 // Shared device utilities: prefix sum, stable cell binning, error recording.
+#include <sys/mman.h>
+#include <unistd.h>
 #include <climits>
 #include <cstdio>
 #include <cstring>
@@ -7,6 +9,16 @@
 
 namespace spss
 {
+
+void prefault(void *p, size_t bytes)
+{
+#ifdef __linux__
+  const uintptr_t page = (uintptr_t) sysconf(_SC_PAGESIZE);
+  const uintptr_t first = (uintptr_t) p & ~(page - 1), end = ((uintptr_t) p + bytes + page - 1) & ~(page - 1);
+  constexpr int kPopulateWrite = 23;  // MADV_POPULATE_WRITE, Linux 5.14
+  if (bytes >= 2 * page) madvise((void *) first, end - first, kPopulateWrite);
+#endif
+}
 
 static thread_local char g_last_error[512];
 

@@ -297,6 +297,7 @@ int spss_get_state(spss_ctx *ctx, double *state, long len)
   if (len != state_len(ctx)) return SPSS_ERR_SIZE;
   SPSS_TRY(ctx->scratch_a.reserve(len));
   SPSS_TRY(is_f64(ctx) ? f64_get_state(ctx, ctx->scratch_a.ptr) : fast_get_state(ctx, ctx->scratch_a.ptr));
+  prefault(state, sizeof(double) * len);
   SPSS_CUDA_TRY(cudaMemcpyAsync(state, ctx->scratch_a.ptr, sizeof(double) * len, cudaMemcpyDeviceToHost, ctx->stream));
   SPSS_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
   return SPSS_OK;

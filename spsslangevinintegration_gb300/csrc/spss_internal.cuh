@@ -72,6 +72,14 @@ inline cudaError_t launch_chained(bool chained, void (*kernel)(Params...), dim3 
   return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
+// ------------------------------------------------------------------ host memory
+
+// Maps the pages of a caller's result array by one system call in place of a
+// fault on each as the copy reaches it (a new 3.1 MB array: 380 -> 231 us for
+// the whole call; pages that are there already: within the noise).  Contents
+// stay as they are, and where the system refuses, the faults come as before.
+void prefault(void *p, size_t bytes);
+
 // ------------------------------------------------------------------ device memory
 
 template<class T>
