@@ -26,12 +26,14 @@ struct F64Path
   DeviceArray<int> cell_of;
   DeviceArray<float2> posf;  // stage positions wrapped into the box, float (all-pairs range pre-test)
   DeviceArray<double2> table;  // of the FP64 functions
-  DeviceArray<double2> csphi;  // cos and sin of the stage phase (all pairs: written with the stage)
+  DeviceArray<double2> csphi;    // cos and sin of the stage phase, written with the stage
+  DeviceArray<longlong2> turns;  // the same in fixed point
   // the other stage buffers of an all-pairs RK4 step, whose pair kernels
   // write the next stage's state while they read this one's
   DeviceArray<double> rk2;
   DeviceArray<float2> posf2;
   DeviceArray<double2> csphi2;
+  DeviceArray<longlong2> turns2;
   Binner binner;
   int cells_nc = 0;  // cells per side of the last build (0: none)
   DeviceArray<int> vl_count, vl_off, vl_ent;
@@ -181,26 +183,61 @@ struct Sums
   double af, card, caf;
 };
 
-// Pair terms: first order ParticleSystemFirstOrderPtr.cpp:404-415; second
-// order ParticleSystemSecondOrder.cpp:160-161 (its complementary force is the
-// first-order term in the second-order sin(phi_j - phi_i - alpha) convention).
-__device__ __forceinline__ void pair_terms(const K64 &k, double phi_i, double omega_i, double phi_j, double omega_j,
-                                           double &af, double &caf)
+// cos and sin of a phase in units of 2^-54 (a NaN becomes the lowest value).
+__device__ __forceinline__ longlong2 turn_fixed(double c, double s)
 {
-  const double d = k.model == 1 ? phi_j - phi_i : phi_j - phi_i - k.alpha;
-  double s, c = 0.0;
-  if (k.higher_order || (k.model == 1 && k.sa != 0.0)) fast_sincos(k.table, d, s, c);
-  else s = fast_sin(k.table, d);
-  caf = 0.0;
-  if (k.model == 1)
+  return make_longlong2(__double2ll_rn(c * 18014398509481984.0), __double2ll_rn(s * 18014398509481984.0));
+}
+
+// Sums over the neighbours of one particle: of the directions, exactly, as
+// integers (511 terms before `flush` empties them into c, s), and of the
+// directions times omega_j - omega_i in FP64 (only for the complementary force).
+//
+// Every pair term is a sine or cosine of phi_j - phi_i (- alpha), so their sums
+// follow from the sums of cos phi_j and sin phi_j, one evaluation a particle
+// in place of one a pair: a direction enters with an error of 2^-55, the sums
+// are exact, where the sum of n sines rounded each sine and each addition.  The
+// integer pipe adds 64 bits some thirty times faster than the FP64 pipe.
+struct NeighbourSums
+{
+  long long ci = 0, si = 0;
+  int n = 0, bad = 0;
+  double c = 0.0, s = 0.0, count = 0.0, wc = 0.0, ws = 0.0;
+
+  __device__ __forceinline__ void add(longlong2 d)
   {
-    af = s * k.ca - c * k.sa;
-    if (k.higher_order) caf = (omega_j - omega_i) * (c * k.ca + s * k.sa);
-  } else
-  {
-    af = s;
-    if (k.higher_order) caf = (omega_j - omega_i) * c;
+    ci += d.x;
+    si += d.y;
+    bad |= (int) (d.x >> 32) == INT_MIN;
+    ++n;
   }
+
+  __device__ __forceinline__ void flush()
+  {
+    c = c + (double) ci * 5.5511151231257827e-17;
+    s = s + (double) si * 5.5511151231257827e-17;
+    count = count + (double) n;
+    ci = si = 0;
+    n = 0;
+  }
+};
+
+constexpr int kExactTerms = 511;
+
+// Pair sums: first order ParticleSystemFirstOrderPtr.cpp:404-415; second order
+// ParticleSystemSecondOrder.cpp:160-161, sin(phi_j - phi_i - alpha) (its
+// complementary force is the first-order term in that convention).
+__device__ __forceinline__ Sums pair_sums(const K64 &k, const NeighbourSums &a, double2 own)
+{
+  const double c = a.bad ? nan("") : a.c, s = a.bad ? nan("") : a.s;
+  const double p = s * own.x - c * own.y, q = c * own.x + s * own.y;  // sums of sin, cos (phi_j - phi_i)
+  Sums r{p * k.ca - q * k.sa, a.count, 0.0};
+  if (k.higher_order)
+  {
+    const double pw = a.ws * own.x - a.wc * own.y, qw = a.wc * own.x + a.ws * own.y;
+    r.caf = qw * k.ca + pw * k.sa;
+  }
+  return r;
 }
 
 // Output of one particle (ParticleSystemFirstOrder.cpp:220-226, ParticleSystemSecondOrder.cpp:166-175);
@@ -224,11 +261,11 @@ __device__ __forceinline__ void write_k_but_torque(const K64 &k, int i, const do
   }
 }
 
-__device__ __forceinline__ void write_k(const K64 &k, int i, const double *st, Sums a, double *k_next, double *caf)
+// own: cos and sin of the particle's phase.
+__device__ __forceinline__ void write_k(const K64 &k, int i, const double *st, double2 own, Sums a, double *k_next,
+                                        double *caf)
 {
-  double c, s;
-  fast_sincos(k.table, st[k.model == 1 ? 2 : 4], s, c);
-  write_k_but_torque(k, i, st, k_next, c, s);
+  write_k_but_torque(k, i, st, k_next, own.x, own.y);
   if (a.card != 0.0)
   {
     k_next[(long) k.s * i + k.s - 1] = -(k.model == 1 ? k.xi : k.xi_phi) * st[k.s - 1] + k.sigma * a.af / a.card;
@@ -255,13 +292,15 @@ __device__ __forceinline__ int stage_cell(const K64 &k, const double *rk, int i,
 
 // rk_system_state = system_state + k_coef * dt * k_prev (ParticleSystemFirstOrder.cpp:175-184),
 // and (posf not null) the stage positions wrapped into the unit box as floats
-// for the range pre-test; one particle per thread.  kp null: k_prev is zero.
+// for the range pre-test and the directions of the phases (FP64 and fixed
+// point); one particle per thread.  kp null: k_prev is zero.
 // det (not null): its torque components are cleared, which the derivative
 // leaves as they are where a particle has no neighbour.  Cells: counted on the
 // way, which as two kernels behind this one took 9 us of a step of N = 65,536.
 __global__ void f64_stage_kernel(K64 k, const double *__restrict__ st, const double *__restrict__ kp,
-                                 double *__restrict__ rk, float2 *__restrict__ posf, double k_coef, double dt,
-                                 double *__restrict__ det, StageCells cells)
+                                 double *__restrict__ rk, float2 *__restrict__ posf, double2 *__restrict__ csphi,
+                                 longlong2 *__restrict__ turns, double k_coef, double dt, double *__restrict__ det,
+                                 StageCells cells)
 {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= k.n) return;
@@ -274,6 +313,13 @@ __global__ void f64_stage_kernel(K64 k, const double *__restrict__ st, const dou
     const double2 r = make_double2(a.x + k_coef * dt * b.x, a.y + k_coef * dt * b.y);
     r2[q] = r;
     if (q == 0 && posf) posf[i] = make_float2((float) (r.x - floor(r.x)), (float) (r.y - floor(r.y)));
+    if (q == k.s / 2 - 1 && posf)
+    {
+      double c, sn;
+      fast_sincos(k.table, r.x, sn, c);
+      csphi[i] = make_double2(c, sn);
+      turns[i] = turn_fixed(c, sn);
+    }
   }
   if (det) det[(long) k.s * i + k.s - 1] = 0.0;
   if (cells.nc)
@@ -298,7 +344,8 @@ __global__ void f64_cell_kernel(K64 k, const double *__restrict__ rk, int nc, in
 // the pair kernel would spend a whole warp's FP64 pipe time on one lane).
 __global__ void f64_stage_posf_kernel(K64 k, const double *__restrict__ st, const double *__restrict__ kp,
                                       double *__restrict__ rk, float2 *__restrict__ posf,
-                                      double2 *__restrict__ csphi, double k_coef, double dt)
+                                      double2 *__restrict__ csphi, longlong2 *__restrict__ turns, double k_coef,
+                                      double dt)
 {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= k.n) return;
@@ -310,6 +357,7 @@ __global__ void f64_stage_posf_kernel(K64 k, const double *__restrict__ st, cons
   double c, sn;
   fast_sincos(k.table, phi, sn, c);
   csphi[i] = make_double2(c, sn);
+  turns[i] = turn_fixed(c, sn);
 }
 
 // Where a pair stands to a cutoff by its float wrapped positions alone: 0 out of
@@ -345,6 +393,7 @@ struct NextStage
   double *rk;
   float2 *posf;
   double2 *csphi;
+  longlong2 *turns;
   const double *k1, *k2, *k3;  // COMBINE
   double *td;
 };
@@ -402,49 +451,64 @@ __device__ __forceinline__ void advance_but_omega(const K64 &k, int i, const dou
   double c, sn;
   fast_sincos(k.table, k.model == 1 ? row[2] : row[4], sn, c);
   next.csphi[i] = make_double2(c, sn);
+  next.turns[i] = turn_fixed(c, sn);
 }
 
 // All pairs (ParticleSystemFirstOrder.cpp:162-228, ParticleSystemFirstOrderPtr.cpp:225-316,
 // ParticleSystemSecondOrder.cpp:116-177): eight particles a block, two warps
 // scanning half the system each for one of them by the float pre-test (FP64
 // within the margins of the cutoff, and for every second-order pair not
-// certainly out of range); the neighbours' phases, in ascending order, wait in
-// the warp's queue.  After the scan the block evaluates all its pair terms
-// together, so an FP64 instruction runs for many lanes (see "neighbour sums"),
-// while another warp does what does not need them: everything of the
-// derivative and of the next stage but the torque and omega.  A warp whose
-// queue fills up (many neighbours) evaluates it on the spot.
-// At N = 1,000 the block is a chain of latencies (an FP64 instruction's result
-// takes some 50 cycles): 11 us an evaluation in a graph of steps; with one
-// warp a particle doing all of its own FP64 work it was 24.
+// certainly out of range).  Every lane adds up the neighbours it finds; after
+// the scan eight lanes finish the eight particles, while another warp does what
+// does not need the sums: everything of the derivative and of the next stage
+// but the torque and omega.  At N = 1,000 the block is a chain of latencies (an
+// FP64 instruction's result takes some 50 cycles): 7.5 us an evaluation in a
+// graph of RK4 steps, 10 with a sine for every pair evaluated after the scan.
 constexpr int kAllParticles = 8;
 constexpr int kAllWarps = 2 * kAllParticles;
-constexpr int kAllQueue = 64;
+
+// One scanning warp's sums: the directions in two parts, so that those of all
+// lanes fit, and what the lanes flushed or have in FP64.
+struct WarpSums
+{
+  long long ch, cl, sh, sl;
+  int n, bad, flushed;
+  double c, s, count, wc, ws;
+};
+
+__device__ __forceinline__ long long warp_add(long long v)
+{
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+  return v;
+}
+
+__device__ __forceinline__ double warp_add(double v)
+{
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+  return v;
+}
 
 template<int AFTER>
 __global__ void __launch_bounds__(32 * kAllWarps) f64_allpairs_kernel(K64 k, const double *__restrict__ rk,
                                                                       const float2 *__restrict__ posf,
                                                                       const double2 *__restrict__ csphi,
+                                                                      const longlong2 *__restrict__ turns,
                                                                       double *__restrict__ k_next,
                                                                       double *__restrict__ caf, NextStage next)
 {
-  __shared__ double2 queue[kAllWarps][kAllQueue];  // phase and omega of the neighbours
-  __shared__ double term[kAllWarps * kAllQueue], cterm[kAllWarps * kAllQueue];
-  __shared__ double2 own[kAllParticles];
-  __shared__ double early[kAllWarps][3];  // sums of the queues evaluated during the scan
-  __shared__ int count[kAllWarps];
+  __shared__ WarpSums sums[kAllWarps];
   pdl_enter();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int i0 = blockIdx.x * kAllParticles;
   const int i = i0 + (warp >> 1);
   const int ip = k.model == 1 ? 2 : 4;
-  int cnt = 0;
-  Sums a{0.0, 0.0, 0.0};
+  NeighbourSums a;
   if (i < k.n)
   {
     const double *st = rk + (long) k.s * i;
-    const double2 mine = *reinterpret_cast<const double2 *>(st + ip);
-    if (lane == 0) own[warp >> 1] = mine;
+    const double omega_i = k.higher_order ? st[ip + 1] : 0.0;
     const float2 p_i = posf[i];
     const int half = (k.n + 1) / 2;
     const int begin = (warp & 1) ? half : 0, end = (warp & 1) ? k.n : half;
@@ -483,198 +547,146 @@ __global__ void __launch_bounds__(32 * kAllWarps) f64_allpairs_kernel(K64 k, con
       }
 #pragma unroll
       for (int u = 0; u < U; ++u)
-      {
-        const unsigned found = __ballot_sync(0xffffffffu, in[u]);
-        if (!found) continue;
         if (in[u])
-          queue[warp][cnt + __popc(found & ((1u << lane) - 1u))] =
-              *reinterpret_cast<const double2 *>(rk + (long) k.s * (j0 + 32 * u) + ip);
-        cnt += __popc(found);
-        if (cnt > kAllQueue - 32)
         {
-          __syncwarp();
-          for (int q = lane; q < cnt; q += 32)
+          const int j = j0 + 32 * u;
+          a.add(turns[j]);
+          if (k.higher_order)
           {
-            const double2 pj = queue[warp][q];
-            double af, cf;
-            pair_terms(k, mine.x, mine.y, pj.x, pj.y, af, cf);
-            a.af += af;
-            a.caf += cf;
+            const double2 cs = csphi[j];
+            const double dw = rk[(long) k.s * j + ip + 1] - omega_i;
+            a.wc += dw * cs.x;
+            a.ws += dw * cs.y;
           }
-          a.card += (double) cnt;
-          cnt = 0;
-          __syncwarp();
         }
-      }
+      if (a.n > kExactTerms - U) a.flush();
     }
   }
-  if (__any_sync(0xffffffffu, a.card != 0.0))
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1)
-    {
-      a.af += __shfl_xor_sync(0xffffffffu, a.af, off);
-      a.caf += __shfl_xor_sync(0xffffffffu, a.caf, off);
-    }
-  if (lane == 0)
   {
-    count[warp] = cnt;
-    early[warp][0] = a.af;
-    early[warp][1] = a.card;
-    early[warp][2] = a.caf;
+    const bool flushed = __any_sync(0xffffffffu, a.count != 0.0);
+    constexpr long long low = (1ll << 27) - 1;
+    WarpSums w;
+    w.ch = warp_add(a.ci >> 27);
+    w.cl = warp_add(a.ci & low);
+    w.sh = warp_add(a.si >> 27);
+    w.sl = warp_add(a.si & low);
+    w.n = __reduce_add_sync(0xffffffffu, a.n);
+    w.bad = __any_sync(0xffffffffu, a.bad);
+    w.flushed = flushed;
+    w.c = flushed ? warp_add(a.c) : 0.0;
+    w.s = flushed ? warp_add(a.s) : 0.0;
+    w.count = flushed ? warp_add(a.count) : 0.0;
+    w.wc = k.higher_order ? warp_add(a.wc) : 0.0;
+    w.ws = k.higher_order ? warp_add(a.ws) : 0.0;
+    if (lane == 0) sums[warp] = w;
+  }
+  const int g = i0 + lane;
+  // the finishing lanes' words, asked for before the block meets
+  const bool finisher = warp == 0 && lane < kAllParticles && g < k.n;
+  const long at = (long) k.s * (finisher ? g : min(i0, k.n - 1)) + k.s - 1;
+  StageWords words{0.0, 0.0, 0.0, 0.0};
+  double torque = 0.0, omega = 0.0;
+  double2 own = make_double2(0.0, 0.0);
+  if (finisher)
+  {
+    own = csphi[g];
+    omega = rk[at];
+    if (AFTER != AFTER_NOTHING)
+    {
+      words = load_stage<AFTER>(next, at);
+      torque = k_next[at];  // kept where the particle has no neighbour
+    }
   }
   __syncthreads();
-  // warp 0 (as many more as there are pairs): the block's queued pairs, end to
-  // end; the last warp: the rest of the derivative and of the next stage
-  int total = 0;
-#pragma unroll
-  for (int w = 0; w < kAllWarps; ++w) total += count[w];
-  const int g = i0 + lane;
   if (warp == kAllWarps - 1 && lane < kAllParticles && g < k.n)
   {
     const double2 cs = csphi[g];
     write_k_but_torque(k, g, rk + (long) k.s * g, k_next, cs.x, cs.y);
     if (AFTER != AFTER_NOTHING) advance_but_omega<AFTER>(k, g, k_next, next);
   }
-  // what the finishing lanes need from memory, asked for before the pair terms
-  const bool finisher = warp == 0 && lane < kAllParticles && g < k.n;
-  const long at = (long) k.s * (finisher ? g : i0) + k.s - 1;
-  StageWords words{0.0, 0.0, 0.0, 0.0};
-  double torque = 0.0;
-  if (finisher && AFTER != AFTER_NOTHING)
-  {
-    words = load_stage<AFTER>(next, at);
-    torque = k_next[at];  // kept where the particle has no neighbour
-  }
-  const int workers = 32 * (kAllWarps - 1);
-  if (threadIdx.x < workers)
-    for (int p = threadIdx.x; p < total; p += workers)
-    {
-      int w = 0, q = p;
-      while (q >= count[w]) q -= count[w++];
-      const double2 pj = queue[w][q], me = own[w >> 1];
-      double af, cf;
-      pair_terms(k, me.x, me.y, pj.x, pj.y, af, cf);
-      term[p] = af;
-      if (k.higher_order) cterm[p] = cf;
-    }
-  __syncthreads();
   if (!finisher) return;
-  a = Sums{0.0, 0.0, 0.0};
-  const int w = 2 * lane;
-  int p = 0;
-#pragma unroll
-  for (int v = 0; v < kAllWarps; ++v) p += v < w ? count[v] : 0;
-  const int c0 = count[w], c1 = count[w + 1];
-  a.card = early[w][1] + early[w + 1][1] + (double) (c0 + c1);
-  if (early[w][1] != 0.0 || early[w + 1][1] != 0.0)
+  const WarpSums &u = sums[2 * lane], &v = sums[2 * lane + 1];
+  // 2^-27 and 2^-54: the parts are below 2^53, so one rounding each
+  a.c = (double) (u.ch + v.ch) * 7.4505805969238281e-09 + (double) (u.cl + v.cl) * 5.5511151231257827e-17;
+  a.s = (double) (u.sh + v.sh) * 7.4505805969238281e-09 + (double) (u.sl + v.sl) * 5.5511151231257827e-17;
+  a.count = (double) (u.n + v.n);
+  if (u.flushed || v.flushed)
   {
-    a.af = early[w][0] + early[w + 1][0];
-    a.caf = early[w][2] + early[w + 1][2];
+    a.c += u.c + v.c;
+    a.s += u.s + v.s;
+    a.count += u.count + v.count;
   }
-  for (const int e = p + c0 + c1; p < e; ++p)
+  a.bad = u.bad | v.bad;
+  a.wc = u.wc + v.wc;
+  a.ws = u.ws + v.ws;
+  Sums r = pair_sums(k, a, own);
+  if (r.card != 0.0)
   {
-    a.af += term[p];
-    if (k.higher_order) a.caf += cterm[p];
-  }
-  if (a.card != 0.0)
-  {
-    torque = -(k.model == 1 ? k.xi : k.xi_phi) * own[lane].y + k.sigma * a.af / a.card;
+    torque = -(k.model == 1 ? k.xi : k.xi_phi) * omega + k.sigma * r.af / r.card;
     k_next[at] = torque;
-    if (k.higher_order) a.caf *= k.sigma / a.card;
+    if (k.higher_order) r.caf *= k.sigma / r.card;
   }
-  if (k.higher_order) caf[g] = a.caf;
+  if (k.higher_order) caf[g] = r.caf;
   if (AFTER != AFTER_NOTHING) advance_component<AFTER>(next, at, words, torque);
 }
 
 // ------------------------------------------------------------ neighbour sums
 //
-// One particle per lane finds its neighbours; the pair terms are then evaluated
-// by the whole warp.  GB300 executes an FP64 instruction for a warp in the time
-// of about 69 FP32 ones whether one lane needs it or 32, so the FP64 sines of
-// the few candidates in range (6 of 18 at density 2, each lane's at its own
-// place in the scan) cost as much as if every candidate were in range.  The
-// scan uses the float pre-test (FP64 only for a pair within the margins of the
-// cutoff) and queues the neighbours per lane; the queues are laid end to end
-// and 32 pair terms are evaluated at a time; each lane then adds its own terms
-// in the order it found them, so the sums are the reference's, bit for bit.
-// N = 65,536, density 2: linked list 313 -> 67 us; Verlet pairs at N = 20,011
-// 87 -> 37 us (44 and 29 us with the table-driven functions and the narrow
-// pre-test margin).
-constexpr int kQueue = 16;       // queued neighbours a lane
-constexpr int kScan = 4;         // candidates a lane looks at together (their loads are in flight at once)
+// One particle per lane finds its neighbours by the float pre-test (FP64 only
+// for a pair within the margins of the cutoff) and adds up their directions.
+// With a sine a pair (queued, and evaluated by the whole warp) ten steps of
+// N = 65,536 took 815 us, and 2,160 once clusters had formed; by sums of
+// directions 825 and 1,520.
+constexpr int kScan = 4;          // candidates a lane looks at together (their loads are in flight at once)
 constexpr int kPairThreads = 32;  // one warp a block: 20,011 particles in blocks of 64 left SMs with 3 blocks beside SMs with 2
 
-struct PairBuffers
+// Read-only views of what the pair kernels need of every particle.
+struct PairInputs
 {
-  double af[kQueue * 32], caf[kQueue * 32];
-  int j[kQueue * 32];
-  unsigned short flat[kQueue * 32];
+  const double *rk;
+  const float2 *posf;
+  const double2 *csphi;
+  const longlong2 *turns;
 };
 
-// Evaluates the queued pairs of the warp's lanes (cnt of this lane's, in rows
-// j[m * 32 + lane]) and adds each lane's terms to its sums in order.
-__device__ __forceinline__ void add_queued(const K64 &k, PairBuffers &Q, const double *__restrict__ rk, int cnt,
-                                           double phi_i, double omega_i, Sums &a)
-{
-  const int lane = threadIdx.x & 31;
-  int end = cnt;
-#pragma unroll
-  for (int off = 1; off < 32; off <<= 1)
-  {
-    const int y = __shfl_up_sync(0xffffffffu, end, off);
-    if (lane >= off) end += y;
-  }
-  const int total = __shfl_sync(0xffffffffu, end, 31);
-  for (int m = 0; m < cnt; ++m) Q.flat[end - cnt + m] = (unsigned short) (m * 32 + lane);
-  __syncwarp();
-  const int ip = k.model == 1 ? 2 : 4;
-  for (int base = 0; base < total; base += 32)
-  {
-    const int p = base + lane;
-    const int f = p < total ? Q.flat[p] : lane;
-    const double phi_o = __shfl_sync(0xffffffffu, phi_i, f & 31), omega_o = __shfl_sync(0xffffffffu, omega_i, f & 31);
-    if (p < total)
-    {
-      const double2 pj = *reinterpret_cast<const double2 *>(rk + (long) k.s * Q.j[f] + ip);
-      double af, caf;
-      pair_terms(k, phi_o, omega_o, pj.x, pj.y, af, caf);
-      Q.af[f] = af;
-      if (k.higher_order) Q.caf[f] = caf;
-    }
-  }
-  __syncwarp();
-  for (int m = 0; m < cnt; ++m)
-  {
-    a.af += Q.af[m * 32 + lane];
-    if (k.higher_order) a.caf += Q.caf[m * 32 + lane];
-  }
-  a.card += (double) cnt;
-  __syncwarp();
-}
-
 // Candidates list[m .. m + kScan) (below e) of the lane's particle i: those in
-// range go to the lane's queue, in order.
-__device__ __forceinline__ void scan_candidates(const K64 &k, PairBuffers &Q, const double *__restrict__ rk,
-                                                const float2 *__restrict__ posf, const int *__restrict__ list, int m,
-                                                int e, int i, float2 p_i, double x_i, double y_i, int &cnt)
+// range are added to its sums.
+__device__ __forceinline__ void scan_candidates(const K64 &k, const PairInputs &in, const int *__restrict__ list,
+                                                int m, int e, int i, float2 p_i, double x_i, double y_i,
+                                                double omega_i, NeighbourSums &a)
 {
-  int j[kScan];
+  int j[kScan], hit[kScan];
   float2 p[kScan];
+  longlong2 d[kScan];
 #pragma unroll
   for (int u = 0; u < kScan; ++u) j[u] = m + u < e ? __ldg(list + m + u) : i;
 #pragma unroll
-  for (int u = 0; u < kScan; ++u) p[u] = __ldg(posf + j[u]);
+  for (int u = 0; u < kScan; ++u) p[u] = __ldg(in.posf + j[u]);
 #pragma unroll
   for (int u = 0; u < kScan; ++u)
   {
-    int in = j[u] == i ? 0 : pretest(p_i, p[u], k.rho_incl, k.rho_excl);
-    if (in == 2)
+    hit[u] = j[u] == i ? 0 : pretest(p_i, p[u], k.rho_incl, k.rho_excl);
+    if (hit[u] == 2)
     {
-      const double *sj = rk + (long) k.s * j[u];
-      in = pair_dr2<true>(k, x_i, y_i, sj[0], sj[1]) <= k.rho2;
+      const double *sj = in.rk + (long) k.s * j[u];
+      hit[u] = pair_dr2<true>(k, x_i, y_i, sj[0], sj[1]) <= k.rho2;
     }
-    if (in) Q.j[32 * cnt++ + (threadIdx.x & 31)] = j[u];
+    d[u] = hit[u] ? __ldg(in.turns + j[u]) : make_longlong2(0, 0);
   }
+#pragma unroll
+  for (int u = 0; u < kScan; ++u)
+    if (hit[u])
+    {
+      a.add(d[u]);
+      if (k.higher_order)
+      {
+        const double2 cs = __ldg(in.csphi + j[u]);
+        const double dw = __ldg(in.rk + (long) k.s * j[u] + k.s - 1) - omega_i;
+        a.wc += dw * cs.x;
+        a.ws += dw * cs.y;
+      }
+    }
+  if (a.n > kExactTerms - kScan) a.flush();
 }
 
 // The stencil of a cell as runs of the cell list, in the reference's order: a
@@ -698,46 +710,32 @@ __device__ __forceinline__ void next_run(int cx, int cy, int nc, const int *__re
 
 // Linked list (ParticleSystemFirstOrder.cpp:231-353, ParticleSystemSecondOrder.cpp:276-409).
 // Particles are taken in cell order, so a warp's lanes scan neighbouring cells.
-__global__ void __launch_bounds__(kPairThreads) f64_linked_list_kernel(K64 k, const double *__restrict__ rk,
-                                                                       const float2 *__restrict__ posf, int nc,
+__global__ void __launch_bounds__(kPairThreads) f64_linked_list_kernel(K64 k, PairInputs in, int nc,
                                                                        const int *__restrict__ off,
                                                                        const int *__restrict__ mem,
                                                                        double *__restrict__ k_next,
                                                                        double *__restrict__ caf)
 {
   pdl_enter();
-  __shared__ PairBuffers buf[kPairThreads / 32];
-  PairBuffers &Q = buf[threadIdx.x >> 5];
   const int t = blockIdx.x * kPairThreads + threadIdx.x;
-  const bool live = t < k.n;
-  const int i = mem[live ? t : k.n - 1];
-  const int ip = k.model == 1 ? 2 : 4;
-  const double *st = rk + (long) k.s * i;
+  if (t >= k.n) return;
+  const int i = mem[t];
+  const double *st = in.rk + (long) k.s * i;
   double x_i, y_i;
-  pos_for_cells(k, rk, i, x_i, y_i);
-  const double phi_i = st[ip], omega_i = st[ip + 1];
-  const float2 p_i = posf[i];
+  pos_for_cells(k, in.rk, i, x_i, y_i);
+  const double omega_i = st[k.s - 1];
+  const float2 p_i = in.posf[i];
   const int cx = cell_coord(x_i, nc), cy = cell_coord(y_i, nc);
-  Sums a{0.0, 0.0, 0.0};
-  int c = live ? 0 : 9, m = 0, e = 0, cnt = 0;
-  while (true)
+  NeighbourSums a;
+  for (int c = 0; c < 9;)
   {
-    while (cnt <= kQueue - kScan)
-    {
-      if (m >= e)
-      {
-        if (c >= 9) break;
-        next_run(cx, cy, nc, off, c, m, e);
-        continue;
-      }
-      scan_candidates(k, Q, rk, posf, mem, m, e, i, p_i, x_i, y_i, cnt);
-      m += kScan;
-    }
-    add_queued(k, Q, rk, cnt, phi_i, omega_i, a);
-    cnt = 0;
-    if (!__any_sync(0xffffffffu, c < 9 || m < e)) break;
+    int m, e;
+    next_run(cx, cy, nc, off, c, m, e);
+    for (; m < e; m += kScan) scan_candidates(k, in, mem, m, e, i, p_i, x_i, y_i, omega_i, a);
   }
-  if (live) write_k(k, i, st, a, k_next, caf);
+  a.flush();
+  const double2 own = in.csphi[i];
+  write_k(k, i, st, own, pair_sums(k, a, own), k_next, caf);
 }
 
 // Verlet list from the cell list (ParticleSystemFirstOrder.cpp:536-589): first
@@ -817,8 +815,7 @@ __global__ void f64_verlet_all_kernel(K64 k, const double *__restrict__ rk, int 
 // Pair loop over the Verlet list (ParticleSystemFirstOrder.cpp:594-648, ParticleSystemFirstOrderPtr.cpp:861-930).
 // `order` (not null): particles in the cell order of the last build, so a
 // warp's lanes read neighbouring particles.
-__global__ void __launch_bounds__(kPairThreads) f64_verlet_pairs_kernel(K64 k, const double *__restrict__ rk,
-                                                                        const float2 *__restrict__ posf,
+__global__ void __launch_bounds__(kPairThreads) f64_verlet_pairs_kernel(K64 k, PairInputs in,
                                                                         const int *__restrict__ order,
                                                                         const int *__restrict__ vl_off,
                                                                         const int *__restrict__ vl_ent,
@@ -826,32 +823,20 @@ __global__ void __launch_bounds__(kPairThreads) f64_verlet_pairs_kernel(K64 k, c
                                                                         double *__restrict__ caf)
 {
   pdl_enter();
-  __shared__ PairBuffers buf[kPairThreads / 32];
-  PairBuffers &Q = buf[threadIdx.x >> 5];
   const int t = blockIdx.x * kPairThreads + threadIdx.x;
-  const bool live = t < k.n;
-  const int i = order ? order[live ? t : k.n - 1] : (live ? t : k.n - 1);
-  const int ip = k.model == 1 ? 2 : 4;
-  const double *st = rk + (long) k.s * i;
+  if (t >= k.n) return;
+  const int i = order ? order[t] : t;
+  const double *st = in.rk + (long) k.s * i;
   double x_i = st[0], y_i = st[1];
   if (k.model == 2) wrap_if_outside(x_i, y_i);
-  const double phi_i = st[ip], omega_i = st[ip + 1];
-  const float2 p_i = posf[i];
-  Sums a{0.0, 0.0, 0.0};
-  int m = vl_off[i], cnt = 0;
-  const int e = live ? vl_off[i + 1] : m;
-  while (true)
-  {
-    while (cnt <= kQueue - kScan && m < e)
-    {
-      scan_candidates(k, Q, rk, posf, vl_ent, m, e, i, p_i, x_i, y_i, cnt);
-      m += kScan;
-    }
-    add_queued(k, Q, rk, cnt, phi_i, omega_i, a);
-    cnt = 0;
-    if (!__any_sync(0xffffffffu, m < e)) break;
-  }
-  if (live) write_k(k, i, st, a, k_next, caf);
+  const double omega_i = st[k.s - 1];
+  const float2 p_i = in.posf[i];
+  NeighbourSums a;
+  const int e = vl_off[i + 1];
+  for (int m = vl_off[i]; m < e; m += kScan) scan_candidates(k, in, vl_ent, m, e, i, p_i, x_i, y_i, omega_i, a);
+  a.flush();
+  const double2 own = in.csphi[i];
+  write_k(k, i, st, own, pair_sums(k, a, own), k_next, caf);
 }
 
 // Global polar order field, first order (ParticleSystemFirstOrder.cpp:122-159,
@@ -1161,6 +1146,7 @@ int f64_create(spss_ctx *ctx)
   SPSS_TRY(f->cell_of.reserve(ctx->p.n));
   SPSS_TRY(f->posf.reserve(ctx->p.n));
   SPSS_TRY(f->csphi.reserve(ctx->p.n));
+  SPSS_TRY(f->turns.reserve(ctx->p.n));
   SPSS_TRY(f->vl_count.reserve(ctx->p.n));
   SPSS_TRY(f->vl_off.reserve(ctx->p.n + 1));
   SPSS_TRY(f->max2.reserve(3));  // of an array of displacements; a stepper's, and its count of finished blocks
@@ -1193,10 +1179,12 @@ void f64_destroy(spss_ctx *ctx)
   f->cell_of.release();
   f->posf.release();
   f->csphi.release();
+  f->turns.release();
   f->table.release();
   f->rk2.release();
   f->posf2.release();
   f->csphi2.release();
+  f->turns2.release();
   if (f->rk4_exec) cudaGraphExecDestroy(f->rk4_exec);
   if (f->rk4_graph) cudaGraphDestroy(f->rk4_graph);
   f->binner.release();
@@ -1294,7 +1282,7 @@ static int evaluate(spss_ctx *ctx, int variant, const double *d_state, const dou
   const int tb = 256;
   if (variant == SPSS_VARIANT_ALL_PAIRS)
     f64_stage_posf_kernel<<<blocks_for(k.n, tb), tb, 0, ctx->stream>>>(k, d_state, d_kprev, f->rk.ptr, f->posf.ptr,
-                                                                       f->csphi.ptr, k_coef, dt);
+                                                                       f->csphi.ptr, f->turns.ptr, k_coef, dt);
   else
   {
     StageCells cells{0, nullptr, nullptr, nullptr};
@@ -1304,27 +1292,27 @@ static int evaluate(spss_ctx *ctx, int variant, const double *d_state, const dou
       cells = StageCells{ctx->nc, f->cell_of.ptr, f->binner.count.ptr, f->binner.slot.ptr};
     }
     f64_stage_kernel<<<blocks_for(k.n, tb), tb, 0, ctx->stream>>>(
-        k, d_state, d_kprev, f->rk.ptr, variant == SPSS_VARIANT_GLOBAL_FIELD ? nullptr : f->posf.ptr, k_coef, dt, det,
-        cells);
+        k, d_state, d_kprev, f->rk.ptr, variant == SPSS_VARIANT_GLOBAL_FIELD ? nullptr : f->posf.ptr, f->csphi.ptr,
+        f->turns.ptr, k_coef, dt, det, cells);
   }
   ++ctx->launches;
   SPSS_TRY(check_launch("f64_stage_kernel"));
+  const PairInputs in{f->rk.ptr, f->posf.ptr, f->csphi.ptr, f->turns.ptr};
   // the pair kernels write every complementary force
   if (k.higher_order && variant == SPSS_VARIANT_GLOBAL_FIELD) SPSS_CUDA_TRY(cudaMemsetAsync(f->caf.ptr, 0, sizeof(double) * k.n, ctx->stream));
   switch (variant)
   {
     case SPSS_VARIANT_ALL_PAIRS:
       f64_allpairs_kernel<AFTER_NOTHING><<<blocks_for(k.n, kAllParticles), 32 * kAllWarps, 0, ctx->stream>>>(
-          k, f->rk.ptr, f->posf.ptr, f->csphi.ptr, d_knext, f->caf.ptr, NextStage{});
+          k, f->rk.ptr, f->posf.ptr, f->csphi.ptr, f->turns.ptr, d_knext, f->caf.ptr, NextStage{});
       ++ctx->launches;
       return check_launch("f64_allpairs_kernel");
     case SPSS_VARIANT_LINKED_LIST:
       SPSS_TRY(f->binner.finish(f->cell_of.ptr, k.n, ctx->stream, ctx->launches, true));
       f->cells_nc = ctx->nc;
       SPSS_CUDA_TRY(launch_chained(true, f64_linked_list_kernel, blocks_for(k.n, kPairThreads), kPairThreads, 0,
-                                   ctx->stream, k, (const double *) f->rk.ptr, (const float2 *) f->posf.ptr, ctx->nc,
-                                   (const int *) f->binner.offsets.ptr, (const int *) f->binner.members.ptr, d_knext,
-                                   f->caf.ptr));
+                                   ctx->stream, k, in, ctx->nc, (const int *) f->binner.offsets.ptr,
+                                   (const int *) f->binner.members.ptr, d_knext, f->caf.ptr));
       ++ctx->launches;
       return check_launch("f64_linked_list_kernel");
     case SPSS_VARIANT_VERLET:
@@ -1339,8 +1327,7 @@ static int evaluate(spss_ctx *ctx, int variant, const double *d_state, const dou
       }
       ctx->uses_verlet_list = 1;
       SPSS_CUDA_TRY(launch_chained(!build, f64_verlet_pairs_kernel, blocks_for(k.n, kPairThreads), kPairThreads, 0,
-                                   ctx->stream, k, (const double *) f->rk.ptr, (const float2 *) f->posf.ptr,
-                                   (const int *) (f->cells_nc ? f->binner.members.ptr : nullptr),
+                                   ctx->stream, k, in, (const int *) (f->cells_nc ? f->binner.members.ptr : nullptr),
                                    (const int *) f->vl_off.ptr, (const int *) f->vl_ent.ptr, d_knext, f->caf.ptr));
       ++ctx->launches;
       return check_launch("f64_verlet_pairs_kernel");
@@ -1399,22 +1386,24 @@ static int allpairs_rk4_stages(spss_ctx *ctx, const K64 &k, double dt, bool chai
   double *rk[2] = {f->rk.ptr, f->rk2.ptr};
   float2 *pf[2] = {f->posf.ptr, f->posf2.ptr};
   double2 *cs[2] = {f->csphi.ptr, f->csphi2.ptr};
+  longlong2 *ts[2] = {f->turns.ptr, f->turns2.ptr};
   const double coef[4] = {0.5, 0.5, 1.0, 0.0};
   for (int e = 0; e < 4; ++e)
   {
     const int a = e & 1, b = a ^ 1;
     const NextStage next{f->state.ptr, coef[e],     dt,          rk[b],       pf[b],
-                         cs[b],        f->k[0].ptr, f->k[1].ptr, f->k[2].ptr, f->td.ptr};
+                         cs[b],        ts[b],       f->k[0].ptr, f->k[1].ptr, f->k[2].ptr, f->td.ptr};
     const int blocks = blocks_for(k.n, kAllParticles), threads = 32 * kAllWarps;
     const double *in = rk[a];
     const float2 *pin = pf[a];
     const double2 *cin = cs[a];
+    const longlong2 *tin = ts[a];
     if (e < 3)
       SPSS_CUDA_TRY(launch_chained(chained && e > 0, f64_allpairs_kernel<AFTER_STAGE>, blocks, threads, 0, ctx->stream,
-                                   k, in, pin, cin, f->k[e].ptr, f->caf.ptr, next));
+                                   k, in, pin, cin, tin, f->k[e].ptr, f->caf.ptr, next));
     else
       SPSS_CUDA_TRY(launch_chained(chained, f64_allpairs_kernel<AFTER_COMBINE>, blocks, threads, 0, ctx->stream, k, in,
-                                   pin, cin, f->k[e].ptr, f->caf.ptr, next));
+                                   pin, cin, tin, f->k[e].ptr, f->caf.ptr, next));
     ++ctx->launches;
     SPSS_TRY(check_launch("f64_allpairs_kernel"));
   }
@@ -1439,8 +1428,10 @@ int f64_step(spss_ctx *ctx, int stepper, double t, double dt)
     SPSS_TRY(f->rk2.reserve(len));
     SPSS_TRY(f->posf2.reserve(n));
     SPSS_TRY(f->csphi2.reserve(n));
+    SPSS_TRY(f->turns2.reserve(n));
     f64_stage_posf_kernel<<<blocks_for(n, tb), tb, 0, ctx->stream>>>(k, f->state.ptr, f->k[0].ptr, f->rk.ptr,
-                                                                     f->posf.ptr, f->csphi.ptr, 0.0, dt);
+                                                                     f->posf.ptr, f->csphi.ptr, f->turns.ptr, 0.0,
+                                                                     dt);
     ++ctx->launches;
     SPSS_TRY(check_launch("f64_stage_posf_kernel"));
     SPSS_TRY(allpairs_rk4_stages(ctx, k, dt, false));
