@@ -275,14 +275,25 @@ __global__ void bin_scatter_kernel(const int *__restrict__ cell_of, const int *_
 // insertion sort in place.
 constexpr int kSortRegs = 8;
 
-__global__ void bin_sort_kernel(const int *__restrict__ offsets, int ncell, int *__restrict__ members)
+__device__ __forceinline__ void write_row(const BinRows &rows, int at, int member)
+{
+  if (!rows.pos_out) return;
+  rows.pos_out[at] = __ldg(rows.pos + member);
+  rows.turns_out[at] = __ldg(rows.turns + member);
+}
+
+__global__ void bin_sort_kernel(const int *__restrict__ offsets, int ncell, int *__restrict__ members, BinRows rows)
 {
   pdl_enter();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= ncell) return;
   const int b = offsets[c], e = offsets[c + 1];
   const int m = e - b;
-  if (m <= 1) return;
+  if (m <= 1)
+  {
+    if (m == 1) write_row(rows, b, members[b]);
+    return;
+  }
   if (m <= kSortRegs)
   {
     int v[kSortRegs];
@@ -299,7 +310,11 @@ __global__ void bin_sort_kernel(const int *__restrict__ offsets, int ncell, int 
       }
 #pragma unroll
     for (int k = 0; k < kSortRegs; ++k)
-      if (k < m) members[b + k] = v[k];
+      if (k < m)
+      {
+        members[b + k] = v[k];
+        write_row(rows, b + k, v[k]);
+      }
     return;
   }
   for (int q = b + 1; q < e; ++q)
@@ -313,6 +328,7 @@ __global__ void bin_sort_kernel(const int *__restrict__ offsets, int ncell, int 
     }
     members[r + 1] = v;
   }
+  for (int q = b; q < e; ++q) write_row(rows, q, members[q]);
 }
 
 int Binner::prepare(int n, int ncell_in, cudaStream_t stream)
@@ -341,12 +357,13 @@ int Binner::place(const int *cell_of, int n, cudaStream_t stream, unsigned long 
 }
 
 // From the counts to the sorted members.
-int Binner::finish(const int *cell_of, int n, cudaStream_t stream, unsigned long long &launches, bool chained)
+int Binner::finish(const int *cell_of, int n, cudaStream_t stream, unsigned long long &launches, bool chained,
+                   const BinRows &rows)
 {
   const int tb = 256;
   SPSS_TRY(place(cell_of, n, stream, launches, chained));
   SPSS_CUDA_TRY(launch_chained(chained, bin_sort_kernel, (ncell + tb - 1) / tb, tb, 0, stream,
-                               (const int *) offsets.ptr, ncell, members.ptr));
+                               (const int *) offsets.ptr, ncell, members.ptr, rows));
   ++launches;
   return check_launch("bin_sort_kernel");
 }
@@ -358,7 +375,7 @@ int Binner::run(const int *cell_of, int n, int ncell_in, cudaStream_t stream, un
   bin_count_kernel<<<(n + tb - 1) / tb, tb, 0, stream>>>(cell_of, n, count.ptr, slot.ptr);
   ++launches;
   SPSS_TRY(check_launch("bin_count_kernel"));
-  return finish(cell_of, n, stream, launches, false);
+  return finish(cell_of, n, stream, launches, false, BinRows{});
 }
 
 }  // namespace spss

@@ -32,6 +32,8 @@ struct F64Path
   // write the next stage's state while they read this one's
   DeviceArray<double> rk2;
   DeviceArray<float2> posf2;
+  DeviceArray<float2> posf_rows;  // posf and turns in cell order (linked list)
+  DeviceArray<longlong2> turns_rows;
   DeviceArray<double2> csphi2;
   DeviceArray<longlong2> turns2;
   Binner binner;
@@ -636,8 +638,10 @@ __global__ void __launch_bounds__(32 * kAllWarps) f64_allpairs_kernel(K64 k, con
 // for a pair within the margins of the cutoff) and adds up their directions.
 // With a sine a pair (queued, and evaluated by the whole warp) ten steps of
 // N = 65,536 took 815 us, and 2,160 once clusters had formed; by sums of
-// directions 825 and 1,520.
-constexpr int kScan = 4;          // candidates a lane looks at together (their loads are in flight at once)
+// directions 825 and 1,520, and with the linked list's positions and directions
+// copied into cell order by the sort (one load, contiguous, before a test in
+// place of two) 700 and 1,150.
+constexpr int kScan = 8;          // candidates a lane looks at together (their loads are in flight at once)
 constexpr int kPairThreads = 32;  // one warp a block: 20,011 particles in blocks of 64 left SMs with 3 blocks beside SMs with 2
 
 // Read-only views of what the pair kernels need of every particle.
@@ -647,31 +651,38 @@ struct PairInputs
   const float2 *posf;
   const double2 *csphi;
   const longlong2 *turns;
+  const float2 *posf_rows;  // posf and turns in cell order (linked list)
+  const longlong2 *turns_rows;
 };
 
-// Candidates list[m .. m + kScan) (below e) of the lane's particle i: those in
-// range are added to its sums.
+// Candidates list[m .. m + kScan) (below e) of the lane's particle: those in
+// range are added to its sums.  ROWS: a stretch of the cell list, whose
+// positions and directions stand in its order, so a lane waits for one load
+// before it tests (the member's index only where it needs more of it); `self`
+// is the particle's place there.  Else entries of a Verlet list, `self` the
+// particle.
+template<bool ROWS>
 __device__ __forceinline__ void scan_candidates(const K64 &k, const PairInputs &in, const int *__restrict__ list,
-                                                int m, int e, int i, float2 p_i, double x_i, double y_i,
+                                                int m, int e, int self, float2 p_i, double x_i, double y_i,
                                                 double omega_i, NeighbourSums &a)
 {
   int j[kScan], hit[kScan];
   float2 p[kScan];
   longlong2 d[kScan];
 #pragma unroll
-  for (int u = 0; u < kScan; ++u) j[u] = m + u < e ? __ldg(list + m + u) : i;
+  for (int u = 0; u < kScan; ++u) j[u] = m + u < e ? (ROWS ? m + u : __ldg(list + m + u)) : self;
 #pragma unroll
-  for (int u = 0; u < kScan; ++u) p[u] = __ldg(in.posf + j[u]);
+  for (int u = 0; u < kScan; ++u) p[u] = __ldg((ROWS ? in.posf_rows : in.posf) + j[u]);
 #pragma unroll
   for (int u = 0; u < kScan; ++u)
   {
-    hit[u] = j[u] == i ? 0 : pretest(p_i, p[u], k.rho_incl, k.rho_excl);
+    hit[u] = j[u] == self ? 0 : pretest(p_i, p[u], k.rho_incl, k.rho_excl);
     if (hit[u] == 2)
     {
-      const double *sj = in.rk + (long) k.s * j[u];
+      const double *sj = in.rk + (long) k.s * (ROWS ? __ldg(list + j[u]) : j[u]);
       hit[u] = pair_dr2<true>(k, x_i, y_i, sj[0], sj[1]) <= k.rho2;
     }
-    d[u] = hit[u] ? __ldg(in.turns + j[u]) : make_longlong2(0, 0);
+    d[u] = hit[u] ? __ldg((ROWS ? in.turns_rows : in.turns) + j[u]) : make_longlong2(0, 0);
   }
 #pragma unroll
   for (int u = 0; u < kScan; ++u)
@@ -680,8 +691,9 @@ __device__ __forceinline__ void scan_candidates(const K64 &k, const PairInputs &
       a.add(d[u]);
       if (k.higher_order)
       {
-        const double2 cs = __ldg(in.csphi + j[u]);
-        const double dw = __ldg(in.rk + (long) k.s * j[u] + k.s - 1) - omega_i;
+        const int o = ROWS ? __ldg(list + j[u]) : j[u];
+        const double2 cs = __ldg(in.csphi + o);
+        const double dw = __ldg(in.rk + (long) k.s * o + k.s - 1) - omega_i;
         a.wc += dw * cs.x;
         a.ws += dw * cs.y;
       }
@@ -731,7 +743,7 @@ __global__ void __launch_bounds__(kPairThreads) f64_linked_list_kernel(K64 k, Pa
   {
     int m, e;
     next_run(cx, cy, nc, off, c, m, e);
-    for (; m < e; m += kScan) scan_candidates(k, in, mem, m, e, i, p_i, x_i, y_i, omega_i, a);
+    for (; m < e; m += kScan) scan_candidates<true>(k, in, mem, m, e, t, p_i, x_i, y_i, omega_i, a);
   }
   a.flush();
   const double2 own = in.csphi[i];
@@ -833,7 +845,7 @@ __global__ void __launch_bounds__(kPairThreads) f64_verlet_pairs_kernel(K64 k, P
   const float2 p_i = in.posf[i];
   NeighbourSums a;
   const int e = vl_off[i + 1];
-  for (int m = vl_off[i]; m < e; m += kScan) scan_candidates(k, in, vl_ent, m, e, i, p_i, x_i, y_i, omega_i, a);
+  for (int m = vl_off[i]; m < e; m += kScan) scan_candidates<false>(k, in, vl_ent, m, e, i, p_i, x_i, y_i, omega_i, a);
   a.flush();
   const double2 own = in.csphi[i];
   write_k(k, i, st, own, pair_sums(k, a, own), k_next, caf);
@@ -1180,6 +1192,8 @@ void f64_destroy(spss_ctx *ctx)
   f->posf.release();
   f->csphi.release();
   f->turns.release();
+  f->posf_rows.release();
+  f->turns_rows.release();
   f->table.release();
   f->rk2.release();
   f->posf2.release();
@@ -1289,6 +1303,8 @@ static int evaluate(spss_ctx *ctx, int variant, const double *d_state, const dou
     if (variant == SPSS_VARIANT_LINKED_LIST)
     {
       SPSS_TRY(f->binner.prepare(k.n, ctx->nc * ctx->nc, ctx->stream));
+      SPSS_TRY(f->posf_rows.reserve(k.n));
+      SPSS_TRY(f->turns_rows.reserve(k.n));
       cells = StageCells{ctx->nc, f->cell_of.ptr, f->binner.count.ptr, f->binner.slot.ptr};
     }
     f64_stage_kernel<<<blocks_for(k.n, tb), tb, 0, ctx->stream>>>(
@@ -1297,7 +1313,8 @@ static int evaluate(spss_ctx *ctx, int variant, const double *d_state, const dou
   }
   ++ctx->launches;
   SPSS_TRY(check_launch("f64_stage_kernel"));
-  const PairInputs in{f->rk.ptr, f->posf.ptr, f->csphi.ptr, f->turns.ptr};
+  const PairInputs in{f->rk.ptr,    f->posf.ptr,      f->csphi.ptr,
+                      f->turns.ptr, f->posf_rows.ptr, f->turns_rows.ptr};
   // the pair kernels write every complementary force
   if (k.higher_order && variant == SPSS_VARIANT_GLOBAL_FIELD) SPSS_CUDA_TRY(cudaMemsetAsync(f->caf.ptr, 0, sizeof(double) * k.n, ctx->stream));
   switch (variant)
@@ -1308,7 +1325,8 @@ static int evaluate(spss_ctx *ctx, int variant, const double *d_state, const dou
       ++ctx->launches;
       return check_launch("f64_allpairs_kernel");
     case SPSS_VARIANT_LINKED_LIST:
-      SPSS_TRY(f->binner.finish(f->cell_of.ptr, k.n, ctx->stream, ctx->launches, true));
+      SPSS_TRY(f->binner.finish(f->cell_of.ptr, k.n, ctx->stream, ctx->launches, true,
+                                BinRows{f->posf.ptr, f->turns.ptr, f->posf_rows.ptr, f->turns_rows.ptr}));
       f->cells_nc = ctx->nc;
       SPSS_CUDA_TRY(launch_chained(true, f64_linked_list_kernel, blocks_for(k.n, kPairThreads), kPairThreads, 0,
                                    ctx->stream, k, in, ctx->nc, (const int *) f->binner.offsets.ptr,

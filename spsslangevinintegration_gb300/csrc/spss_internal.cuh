@@ -237,13 +237,6 @@ __device__ __forceinline__ void fast_sincos(const double2 *__restrict__ table, d
   sincos_at(table, k, r, s, c);
 }
 
-__device__ __forceinline__ double fast_sin(const double2 *__restrict__ table, double x)
-{
-  double s, c;
-  fast_sincos(table, x, s, c);  // the cosine is not computed where it is not used
-  return s;
-}
-
 // log((a + 0.5) 2^-32) for a 32-bit a: the mantissa m in [sqrt(1/2), sqrt(2)),
 // c = j / 128 the nearest table point (c = 1 around 1, where the result is
 // small), log(m / c) by its series to r^7 (|r| <= 1 / 180).
@@ -506,6 +499,14 @@ struct Scanner
 // Stable cell binning: cell id per element -> CSR offsets and members that list
 // each cell's elements in ascending element order (the push_back order of the
 // reference's linked_list_, ParticleSystemFirstOrder.cpp:285-288).
+struct BinRows
+{
+  const float2 *pos = nullptr;
+  const longlong2 *turns = nullptr;
+  float2 *pos_out = nullptr;
+  longlong2 *turns_out = nullptr;
+};
+
 struct Binner
 {
   DeviceArray<int> count, offsets, slot, members;
@@ -518,8 +519,10 @@ struct Binner
   // in arrival order; the counts are zero again.
   int place(const int *cell_of, int n, cudaStream_t stream, unsigned long long &launches, bool chained = false,
             FastControl *ctrl = nullptr);
-  // the same with members in ascending order
-  int finish(const int *cell_of, int n, cudaStream_t stream, unsigned long long &launches, bool chained);
+  // the same with members in ascending order, and (outputs not null) what a scan
+  // of the cells reads of each member, in members' order
+  int finish(const int *cell_of, int n, cudaStream_t stream, unsigned long long &launches, bool chained,
+             const BinRows &rows);
   // all of it
   int run(const int *cell_of, int n, int ncell, cudaStream_t stream, unsigned long long &launches);
   void release()
