@@ -1791,6 +1791,7 @@ __global__ void fast_pbc_kernel(int2 *img, int n)
 // summed in FP64 from the records of the current state.
 
 constexpr int kOrderChunk = 2048;  // slots per partial sum
+constexpr int kOrderThreads = 256;
 
 // Whether a sample follows the step that brought the counter to `step`.
 __host__ __device__ __forceinline__ bool samples_after(const FastControl *c, unsigned long long step)
@@ -1810,10 +1811,19 @@ __device__ __forceinline__ double warp_sum(double v)
   return v;
 }
 
+// The double of a float by integer instructions (a conversion takes the FP64
+// pipe); subnormal floats become 0.
+__device__ __forceinline__ double widen(float x)
+{
+  const uint32_t b = __float_as_uint(x), m = b & 0x7fffffffu;
+  const uint32_t hi = m < 0x00800000u ? 0u : (b & 0x80000000u) | ((m >> 3) + 0x38000000u);
+  return __hiloint2double((int) hi, m < 0x00800000u ? 0 : (int) (b << 29));
+}
+
 // v / |v| in FP64, added to (sx, sy); nothing for v = 0.  The reciprocal square
 // root starts from the FP32 one (relative error below 2^-22) and takes one
 // third-order step, y (1 + e/2 + 3 e^2/8) with e = 1 - |v|^2 y^2, whose
-// remainder 5 e^3 / 16 is below 1e-19: 12 FP64 instructions against about 70
+// remainder 5 e^3 / 16 is below 1e-19: nine FP64 instructions against about 70
 // for the square root and the two divisions (GB300 runs FP64 at 1/69 of its
 // FP32 rate, so the FP64 count is what these reductions cost).
 __device__ __forceinline__ void add_direction(float2 v, double &sx, double &sy)
@@ -1825,24 +1835,52 @@ __device__ __forceinline__ void add_direction(float2 v, double &sx, double &sy)
   const int ex = max(-120, min(120, 127 - (int) (__float_as_uint(big) >> 23)));
   const float scale = __uint_as_float((uint32_t) (ex + 127) << 23);
   const float fx = __fmul_rn(v.x, scale), fy = __fmul_rn(v.y, scale);
-  const double x = fx, y = fy;
+  const float f2 = fmaf(fx, fx, __fmul_rn(fy, fy));
+  if (!(f2 > 0.0f)) return;  // a NaN component: left out, as a comparison |v| > 0 leaves it out
+  if (f2 > 3.0e38f)          // an infinite one has no direction
+  {
+    sx = sy = __longlong_as_double(0x7ff8000000000000ll);
+    return;
+  }
+  const double x = widen(fx), y = widen(fy), r = widen(rsqrtf(f2));
   const double m2 = fma(x, x, y * y);
-  if (!(m2 > 0.0)) return;  // a NaN component: left out, as a comparison |v| > 0 leaves it out
-  const double r = rsqrtf(fmaf(fx, fx, __fmul_rn(fy, fy)));
   const double e = fma(-m2 * r, r, 1.0);
   const double c = fma(r * e, fma(e, 0.375, 0.5), r);
   sx = fma(x, c, sx);
   sy = fma(y, c, sy);
 }
 
+// Sum of floats of at most 1 in magnitude as integers, in units of 2^-24 and
+// 2^-48: exact down to floats of 2^-25, at a quarter of the conversion and the
+// addition in FP64.  Up to 64 terms.
+struct UnitSum
+{
+  int hi = 0, lo = 0;
+
+  __device__ __forceinline__ void add(float x)
+  {
+    const float t = x * 16777216.0f;
+    const int h = __float2int_rn(t);
+    hi += h;
+    lo += __float2int_rn((t - (float) h) * 16777216.0f);
+  }
+
+  __device__ __forceinline__ double value() const
+  {
+    return (double) (((long long) hi << 24) + lo) * 3.5527136788005009e-15;
+  }
+};
+
 // partial[k] = sums over chunk k (at most kOrderChunk slots of one system);
 // a small grid walks all chunks, so the gated launch that finds no sampling
-// step costs a few hundred CTAs.
-__global__ void fast_order_partials_kernel(FastParams P, FastBuffers B, OrderSums *__restrict__ partial,
+// step costs a few hundred CTAs.  FP64 instructions bound it (nine a particle,
+// 24 with conversions, FP64 sums of the phases' floats and a tree for each sum):
+// with the finish kernel 414 -> 229 us for 8.85 million particles in 512
+// systems, 84 -> 57 us for 1,024 systems of 1,024.
+__global__ void __launch_bounds__(kOrderThreads) fast_order_partials_kernel(FastParams P, FastBuffers B, OrderSums *__restrict__ partial,
                                            const int2 *__restrict__ items, int nitems, int gated)
 {
   if (gated && !sample_now(B.ctrl)) return;
-  __shared__ double sh[4][8];
   const uint4 *rec = B.ctrl->parity ? B.rec1 : B.rec0;
   buffers_now(B, B.ctrl->order_parity);
   for (int k = blockIdx.x; k < nitems; k += gridDim.x)
@@ -1851,43 +1889,27 @@ __global__ void fast_order_partials_kernel(FastParams P, FastBuffers B, OrderSum
     const SysParams *S = B.sys + it.x;
     const long begin = it.y;
     const long end = min((long) S->first + S->n, begin + kOrderChunk);
-    double a0 = 0.0, a1 = 0.0, a2 = 0.0, a3 = 0.0;
-    for (long q = begin + threadIdx.x; q < end; q += blockDim.x)
+    double a[4] = {0.0, 0.0, 0.0, 0.0};
+    UnitSum c, sn;
+#pragma unroll 4
+    for (long q = begin + threadIdx.x; q < end; q += kOrderThreads)
     {
       const uint4 r = rec[q];
-      a0 += (double) __uint_as_float(r.z);
-      a1 += (double) __uint_as_float(r.w);
-      if (P.model == 2)
-      {
-        add_direction(B.vel[q], a2, a3);
-      }
+      c.add(__uint_as_float(r.z));
+      sn.add(__uint_as_float(r.w));
+      if (P.model == 2) add_direction(B.vel[q], a[2], a[3]);
     }
-    a0 = warp_sum(a0);
-    a1 = warp_sum(a1);
-    a2 = warp_sum(a2);
-    a3 = warp_sum(a3);
-    const int w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    if ((threadIdx.x & 31) == 0)
-    {
-      sh[0][w] = a0;
-      sh[1][w] = a1;
-      sh[2][w] = a2;
-      sh[3][w] = a3;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0)
-    {
-      double t[4] = {0.0, 0.0, 0.0, 0.0};
-      for (int u = 0; u < nw; ++u)
-        for (int c = 0; c < 4; ++c) t[c] += sh[c][u];
-      partial[k] = OrderSums{t[0], t[1], t[2], t[3]};
-    }
-    __syncthreads();
+    a[0] = c.value();
+    a[1] = sn.value();
+    const double sum = block_sum4(warp_sum4(a));
+    if (threadIdx.x < 32 && (threadIdx.x & 7) == 0)
+      reinterpret_cast<double *>(partial + k)[threadIdx.x >> 3] = sum;
   }
 }
 
 // Per system: the order parameters (R, arg, R_v, arg_v) into out4 and, after a
 // sampling step, the running sums of R, R^2, R_v, R_v^2 and the sample count.
+// Blocks of one warp, so the arguments' FP64 work spreads over the SMs.
 __global__ void fast_order_finish_kernel(FastParams P, FastBuffers B, const OrderSums *__restrict__ partial,
                                          const int *__restrict__ first_item, double *__restrict__ out4,
                                          double *__restrict__ stats, int gated)
@@ -1896,6 +1918,7 @@ __global__ void fast_order_finish_kernel(FastParams P, FastBuffers B, const Orde
   if (r >= P.nsys) return;
   if (gated && !sample_now(B.ctrl)) return;
   double t0 = 0.0, t1 = 0.0, t2 = 0.0, t3 = 0.0;
+#pragma unroll 4
   for (int c = first_item[r]; c < first_item[r + 1]; ++c)
   {
     const OrderSums v = partial[c];
@@ -2075,9 +2098,10 @@ __global__ void fast_turn_table_kernel(double2 *__restrict__ table)
 }
 
 // FP64 instructions bound this kernel (4,194,304 particles: 8 a phase with the
-// tables, 12 a velocity, 8.4 us for each of them at the measured 0.50 T/s).
+// tables, 9 a velocity, 8.4 us for each of them at the measured 0.50 T/s).
 // Through an FP64 copy of the state, sincos, square roots and divisions it was
-// three kernels of 181 + 436 + 204 us; this one takes 179 us.
+// three kernels of 181 + 436 + 204 us; the whole call takes 146 us (181 with
+// the velocities converted on the FP64 pipe).
 template<bool TABLE>
 __global__ void __launch_bounds__(256) fast_observe_kernel(FastParams P, FastBuffers B, const double2 *__restrict__ table,
                                                            double *__restrict__ partial, double *__restrict__ sums)
@@ -2729,11 +2753,11 @@ static int launch_sampling(spss_ctx *ctx, const FastParams &P, int gated)
 {
   FastPath *f = ctx->fast;
   const FastBuffers B = buffers(ctx);
-  fast_order_partials_kernel<<<f->order_grid, 256, 0, ctx->stream>>>(P, B, f->order_partial.ptr,
+  fast_order_partials_kernel<<<f->order_grid, kOrderThreads, 0, ctx->stream>>>(P, B, f->order_partial.ptr,
                                                                        f->order_items.ptr, f->order_chunks, gated);
   ++ctx->launches;
   SPSS_TRY(check_launch("fast_order_partials_kernel"));
-  fast_order_finish_kernel<<<blocks_for(f->nsys, 128), 128, 0, ctx->stream>>>(
+  fast_order_finish_kernel<<<blocks_for(f->nsys, 32), 32, 0, ctx->stream>>>(
       P, B, f->order_partial.ptr, f->order_first.ptr, f->order_out.ptr, f->stats.ptr, gated);
   ++ctx->launches;
   return check_launch("fast_order_finish_kernel");
