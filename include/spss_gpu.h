@@ -250,24 +250,23 @@ int spss_batch_run(spss_ctx *ctx, int stepper, double t0, double dt, long nsteps
 int spss_batch_stats(spss_ctx *ctx, double *out, long len);
 int spss_batch_reset_stats(spss_ctx *ctx);
 
-/* Tiling of the pair-and-update kernel: cells per tile (each row of a
- * system's cell grid is split into ceil(nc / tile_cells) tiles of whole cells;
- * with Verlet lists the tiles of a row hold nearly equal numbers of particles,
- * with cell lists tile_cells cells each; 1 .. 4096) and launch form (0: one CTA per tile; 1: persistent,
- * one wave of CTAs taking tiles from a work counter).  Results do not depend
- * on the tiling; the lists are rebuilt before the next step.  F32 contexts. */
+/* Tiling hint (cells per tile, 1 .. 4096; launch form 0 or 1).  The step
+ * kernels take one particle per thread in slot order and need no tiling: the
+ * values are kept for spss_get_tiling, results do not depend on them, and the
+ * lists are rebuilt before the next step.  F32 contexts. */
 int spss_set_tiling(spss_ctx *ctx, int tile_cells, int persistent);
 int spss_get_tiling(spss_ctx *ctx, int *tile_cells, int *persistent);
 /* How steps run as CUDA graphs (spss_steps, spss_batch_run) rebuild Verlet
  * lists: 1 (default) the step's control kernel launches the rebuild as a
  * device graph when the trigger fires; 0 a conditional graph node holds the
  * rebuild at the start of each step (the form used where the device refuses
- * device-launched graphs; about 12 us more per step on GB300).  Results are
+ * device-launched graphs; about 12 us more per step on GB300).  Batches of
+ * systems of at most 4096 particles and cells hold a rebuild of one block a
+ * system in every step instead, which leaves at once when none is due.  Results are
  * identical.  F32 contexts.  No counterpart in the reference. */
 int spss_set_device_rebuild(spss_ctx *ctx, int enabled);
-/* Times `steps` steps of every tiling candidate (16 to 64 cells per tile in steps of 4,
- * both launch forms) on the context's current state, keeps the fastest and
- * restores the state, step counter and trigger as they were (the lists are
+/* Times `steps` steps on the context's current state (there is one form of the
+ * step to time: the tiling is a hint) and restores the state, step counter and trigger as they were (the lists are
  * rebuilt before the next step; before the first step that leaves every
  * result identical to an untuned run).  best_ms_per_step may be NULL. */
 int spss_autotune(spss_ctx *ctx, int stepper, double dt, int steps, double *best_ms_per_step);

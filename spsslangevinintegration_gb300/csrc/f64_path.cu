@@ -1,12 +1,11 @@
-// FP64 path: the reference's arithmetic, operation for operation, on the GPU.
+// FP64 path: the reference's arithmetic in 64 bits on the GPU.
 //
-// This translation unit is compiled with --fmad=false, so every expression
-// below rounds exactly like the reference built with -ffp-contract=off.  Per
-// particle the neighbour sums run in the reference's order (cell stencil
-// order, ascending members; Verlet list order), so cell ids, member lists and
-// Verlet lists are bit-identical to the reference's and floating-point
-// results differ only by the last bits of the device sin/cos/atan2/hypot and
-// by the all-pairs sum order.  Layout: AoS double[n*s], as the reference.
+// This translation unit is compiled with --fmad=false, so the stage, distance
+// and stepper expressions below round exactly like the reference built with
+// -ffp-contract=off.  Cell ids, member lists (ascending) and Verlet lists (in
+// push_back order) are bit-identical to the reference's; floating-point results
+// differ only by the last bits of sin/cos/atan2/hypot and of the torques, which
+// are formed from sums of directions instead of a sine a pair (NeighbourSums).  Layout: AoS double[n*s], as the reference.
 //
 // Reference: DynamicalSystems/ParticleSystemFirstOrder.cpp, ParticleSystemFirstOrderPtr.cpp,
 // ParticleSystemSecondOrder.cpp, BoundaryConfiguration/PeriodicBoundaryConditions.cpp,

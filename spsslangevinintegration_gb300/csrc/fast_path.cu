@@ -137,7 +137,8 @@ __device__ __forceinline__ void buffers_now(FastBuffers &B, int order_parity)
 // How a step graph does the list rebuild: under a conditional node at the
 // start of the step (GRAPH_CONDITIONAL), tail-launched as a device graph by the
 // control kernel when the trigger fires (GRAPH_DEVICE), unconditionally at the
-// start of every step (GRAPH_ALWAYS: cell lists), or not at all (GRAPH_NONE:
+// start of every step (GRAPH_ALWAYS: cell lists, and batches of small systems,
+// whose rebuild kernels leave at once when nothing is due), or not at all (GRAPH_NONE:
 // kinds without lists or trigger).  Rebuilds requested from the host run
 // before the first graph step in the last three forms.
 enum
@@ -582,7 +583,7 @@ __global__ void __launch_bounds__(256) fast_frame_kernel(float *__restrict__ out
 // ---------------------------------------------------------------- rebuild
 
 // Whether this rebuild covers system `sys`: every system, or those whose own
-// trigger fired.  A system left out keeps its slots, cells, tile layouts and
+// trigger fired.  A system left out keeps its slots, cells and
 // lists exactly as its last rebuild made them.
 __device__ __forceinline__ bool rebuilds_system(const FastBuffers &B, int sys)
 {
@@ -669,10 +670,8 @@ __global__ void fast_after_permute_kernel(FastControl *ctrl, int permuted)
   ctrl->cells_fresh = 0;  // the slots moved
 }
 
-// Lists are now current.  The flags are cleared only here, after the tile
-// layout and list kernels, so those rebuild the flagged systems alone (with
-// the flags cleared before them, every system's layouts and lists were
-// rebuilt at each flagged rebuild).  One block.
+// Lists are now current.  The flags are cleared only here, after the list
+// kernel, so that it rebuilds the lists of the flagged systems alone.  One block.
 __global__ void fast_after_rebuild_kernel(FastControl *ctrl, SysControl *sysctl, int nsys)
 {
   for (int r = threadIdx.x; r < nsys; r += blockDim.x) sysctl[r].rebuild = 0;
@@ -2847,8 +2846,9 @@ int fast_get_state(spss_ctx *ctx, double *d_aos)
 // Room for longer lists once some were too long (clusters outgrow the capacity
 // estimated for the mean density, and a particle whose list did not fit scans
 // its stencil every step): a quarter more than the longest seen.  The lists in
-// use move as they are, and the next rebuild fills the larger ones, so no result depends on when this happens.  Memory is taken only while
-// it is plentiful; a failed allocation leaves things as they were.
+// use move as they are, and the next rebuild fills the larger ones, so no result
+// depends on when this happens.  Memory is taken only while it is plentiful; a
+// failed allocation leaves things as they were.
 constexpr int kListCapMax = 512;
 
 static int grow_lists(spss_ctx *ctx)
