@@ -266,9 +266,10 @@ int spss_get_tiling(spss_ctx *ctx, int *tile_cells, int *persistent);
  * identical.  F32 contexts.  No counterpart in the reference. */
 int spss_set_device_rebuild(spss_ctx *ctx, int enabled);
 /* Times `steps` steps on the context's current state (there is one form of the
- * step to time: the tiling is a hint) and restores the state, step counter and trigger as they were (the lists are
- * rebuilt before the next step; before the first step that leaves every
- * result identical to an untuned run).  best_ms_per_step may be NULL. */
+ * step to time: the tiling is a hint) and restores the state, step counter and
+ * trigger as they were (the lists are rebuilt before the next step; before the
+ * first step that leaves every result identical to an untimed run).
+ * best_ms_per_step may be NULL. */
 int spss_autotune(spss_ctx *ctx, int stepper, double dt, int steps, double *best_ms_per_step);
 
 #ifdef __cplusplus

@@ -272,7 +272,7 @@ class Context:
                 "spss_integrate_dopri5")
         return steps.value
 
-    # -- tiling of the pair-and-update kernel (F32 contexts)
+    # -- tiling hint, kept for tiling() (F32 contexts)
     def set_tiling(self, tile_cells, persistent=False):
         N.check(self.L.spss_set_tiling(self.h, int(tile_cells), int(bool(persistent))), "spss_set_tiling")
 
@@ -287,7 +287,7 @@ class Context:
         N.check(self.L.spss_set_device_rebuild(self.h, int(bool(enabled))), "spss_set_device_rebuild")
 
     def autotune(self, stepper, dt, steps=5):
-        """Fastest tiling over trial steps; the state is restored.  Returns ms per step."""
+        """Times `steps` trial steps; the state is restored.  Returns ms per step."""
         ms = ctypes.c_double()
         N.check(self.L.spss_autotune(self.h, stepper, dt, int(steps), ctypes.byref(ms)), "spss_autotune")
         return ms.value

@@ -2778,7 +2778,7 @@ static int adopt_control(spss_ctx *ctx)
   ctx->step_counter = f->h_ctrl->step;
   ctx->accumulated_displacement = f->h_ctrl->acc;
   ctx->should_update_lists = reported_list_flag(f->h_ctrl);
-  if (f->h_ctrl->error & ~1) return SPSS_ERR_CUDA;  // a bounded wait ran out, or a device launch failed
+  if (f->h_ctrl->error & ~1) return SPSS_ERR_CUDA;  // a device launch failed
   if (f->h_ctrl->error) return SPSS_ERR_NONFINITE;
   return SPSS_OK;
 }

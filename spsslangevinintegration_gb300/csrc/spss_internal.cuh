@@ -466,8 +466,7 @@ struct FastControl
                             // current slots (cell lists), the field of the current state (global field)
   int overflow;             // largest Verlet count seen beyond capacity (0: none)
   int rebuilds;             // number of rebuilds performed
-  int error;                // bit 0: displacement too large for the fixed-point increment; bit 1: staging
-                            // timeout; bit 2: stencil cell outside the staged segments; bit 3: the
+  int error;                // bit 0: displacement too large for the fixed-point increment; bit 3: the
                             // device launch of the rebuild graph was refused
   int uses_verlet;
   unsigned ticket;          // blocks of the running reduction that are done (its last block puts it back to 0)
