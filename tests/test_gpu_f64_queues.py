@@ -1,8 +1,7 @@
-"""FP64 neighbour sums whose pair terms are queued and evaluated by the warp:
-more neighbours than a queue holds, particle numbers around the warp and block
-sizes, pairs within the pre-test's margin of the cutoff (decided in FP64), and
-coordinates several boxes away, against the oracle (the FP64 path's tolerance,
-1e-12: same operations in the same order)."""
+"""FP64 neighbour sums: many neighbours, particle numbers around the warp and
+block sizes, pairs within the pre-test's margin of the cutoff (decided in
+FP64), and coordinates several boxes away, against the oracle (the FP64 path's
+tolerance, 1e-12)."""
 import numpy as np
 import pytest
 
