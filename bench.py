@@ -770,7 +770,7 @@ def run_ours(args, rank, world, local_rank):
                    "parallelism": "replicas x%d" % world,
                    "tiling": {"tile_cells": tiling[0], "persistent": tiling[1], "autotuned_ms_per_step": tune_ms}},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                     "peak_kind": peak_kind, "kernel": "fast_tile_kernel<2,2,2> (pair sums + SRK update)",
+                     "peak_kind": peak_kind, "kernel": "fast_tile_kernel<2,2,0> (pair sums + SRK update)",
                      "kernel_ms": avg_kernel_s * 1e3,
                      "algorithmic_bytes_per_particle": algorithmic_bytes_per_particle(p),
                      "traffic": None if traffic is None else traffic * n},
