@@ -186,9 +186,11 @@ __device__ __forceinline__ uint4 philox_block(const NoiseKey &nk, uint32_t parti
 // (sin), 30 (log) and 15 (sqrt) of them.  Table-driven evaluation (the method
 // of P. T. P. Tang, "Table-driven implementation of the logarithm function in
 // IEEE floating-point arithmetic", ACM TOMS 16, 1990, and of his sine of the
-// same kind) needs 14 for a sine, 16 with the cosine, 13 for the logarithm and
-// 8 for the square root, at the same accuracy (about 1 ulp; measured against
-// the CUDA functions in tests/test_gpu_f64_functions.py).
+// same kind) needs 15 for a sine, 17 with the cosine, 13 for the logarithm and
+// 8 for the square root.  Sine and cosine carry at most 1.5 units of 2^-53 (and 2
+// ulp where one of them is small beside a multiple of pi / 2), the normals a few
+// units of 2^-53 of their radius (tests/test_gpu_f64_functions.py,
+// tests/test_gpu_f64_quarter_turns.py).
 
 constexpr int kTrigTable = 256;      // cos and sin of 2 pi k / 256
 constexpr int kLogFirst = 88, kLogLast = 184;  // j / 128 covers [sqrt(1/2), sqrt(2)] with room
@@ -209,31 +211,47 @@ __device__ __forceinline__ void sincos_at(const double2 *__restrict__ table, int
   c = fma(-T.y, sr, fma(T.x, cm, T.x));
 }
 
-// Largest |x| that the two-part reduction takes: k < 2^19 keeps k * (upper
-// part, 33 bits) exact.  Beyond it (and for infinities and NaN) the CUDA
-// functions.
-constexpr double kTrigMax = 4096.0;
+// |x| below 2^20 is reduced by hand (k < 2^26 keeps its products with the upper
+// two parts of pi / 128, 26 bits each, exact); beyond it, for infinities and
+// for NaN the CUDA functions.
+__device__ __forceinline__ bool reducible(double x)
+{
+  return (__double2hiint(x) & 0x7fffffff) < 0x41300000;
+}
 
+// x = k pi / 128 + r, |r| <= pi / 256: the first two products and differences
+// are exact, the third rounds once, and the parts' sum is pi / 128 to 2^-116, so
+// r is off by half an ulp of itself and k 2^-116.
 __device__ __forceinline__ void reduce_turn(double x, int &k, double &r)
 {
   const double t = fma(x, 40.743665431525205957, SPSS_ROUND_MAGIC);  // 128 / pi
   k = __double2loint(t);
   const double kd = t - SPSS_ROUND_MAGIC;
-  // pi / 128 = 0x1.921fb544p-6 (33 bits) + 0x1.0b4611a626331p-40
-  r = fma(kd, -0x1.921fb544p-6, x);
-  r = fma(kd, -0x1.0b4611a626331p-40, r);
+  r = fma(kd, -0x1.921fb58p-6, x);
+  r = fma(kd, 0x1.dde974p-33, r);
+  r = fma(kd, -0x1.1a62633145c07p-60, r);
 }
 
+// Whether sine or cosine is a remainder so small (below 2^-30, next to a multiple
+// of pi / 2 other than 0) that the error of the reduction shows in it.
+__device__ __forceinline__ bool near_quarter(int k, double r)
+{
+  return (k & 63) == 0 && k != 0 && (__double2hiint(r) & 0x7fffffff) < 0x3e100000;
+}
+
+// Within 1.5 units of 2^-53 of sine and cosine, and within 2 ulp of the one
+// that is small next to a multiple of pi / 2.
 __device__ __forceinline__ void fast_sincos(const double2 *__restrict__ table, double x, double &s, double &c)
 {
-  if (!(fabs(x) <= kTrigMax))
+  int k = 0;
+  double r = 0.0;
+  const bool mine = reducible(x);
+  if (mine) reduce_turn(x, k, r);
+  if (!mine || near_quarter(k, r))
   {
     sincos(x, &s, &c);
     return;
   }
-  int k;
-  double r;
-  reduce_turn(x, k, r);
   sincos_at(table, k, r, s, c);
 }
 
