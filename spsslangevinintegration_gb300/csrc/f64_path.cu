@@ -4,8 +4,10 @@
 // and stepper expressions below round exactly like the reference built with
 // -ffp-contract=off.  Cell ids, member lists (ascending) and Verlet lists (in
 // push_back order) are bit-identical to the reference's; floating-point results
-// differ only by the last bits of sin/cos/atan2/hypot and of the torques, which
-// are formed from sums of directions instead of a sine a pair (NeighbourSums).  Layout: AoS double[n*s], as the reference.
+// differ only by the last bits of sin/cos/atan2/hypot and of the torques: where
+// sums of directions are as accurate as the reference's sine a pair they are
+// formed from those, elsewhere (aligned phases) pair by pair (NeighbourSums).
+// Layout: AoS double[n*s], as the reference.
 //
 // Reference: DynamicalSystems/ParticleSystemFirstOrder.cpp, ParticleSystemFirstOrderPtr.cpp,
 // ParticleSystemSecondOrder.cpp, BoundaryConfiguration/PeriodicBoundaryConditions.cpp,
@@ -59,6 +61,8 @@ struct K64
   int higher_order;
   float rho_excl;  // a pair whose float minimum-image distance bound exceeds this is out of range
   float rho_incl, rmax_excl, rmax_incl;  // the cutoffs less (plus) two margins
+  float ca_f, sa_f;  // ca, sa
+  float least;       // mean |sin(phi_j - phi_i - alpha)| from which on sums of directions are accurate enough
 };
 
 // Margin of the range pre-test, in box units: six times what the float rounding
@@ -93,6 +97,9 @@ static K64 make_k64(const spss_ctx *ctx)
   k.rho_incl = (float) std::max(0.0, p.rho - 2.0 * kPretestMargin);
   k.rmax_excl = (float) (ctx->r_max + 2.0 * kPretestMargin);
   k.rmax_incl = (float) std::max(0.0, ctx->r_max - 2.0 * kPretestMargin);
+  k.ca_f = (float) k.ca;
+  k.sa_f = (float) k.sa;
+  k.least = p.model == 2 && p.alpha != 0.0 ? 0.25f : 0.03125f;
   return k;
 }
 
@@ -182,63 +189,178 @@ __device__ __forceinline__ double pair_dr2(const K64 &k, double x_i, double y_i,
 struct Sums
 {
   double af, card, caf;
+
+  // af and caf summed another way
+  __device__ __forceinline__ void take(double2 v)
+  {
+    af = v.x;
+    caf = v.y;
+  }
 };
 
-// cos and sin of a phase in units of 2^-54 (a NaN becomes the lowest value).
-__device__ __forceinline__ longlong2 turn_fixed(double c, double s)
-{
-  return make_longlong2(__double2ll_rn(c * 18014398509481984.0), __double2ll_rn(s * 18014398509481984.0));
-}
-
 // Sums over the neighbours of one particle: of the directions, exactly, as
-// integers (511 terms before `flush` empties them into c, s), and of the
-// directions times omega_j - omega_i in FP64 (only for the complementary force).
+// integers, and of the directions times omega_j - omega_i in FP64 (only for the
+// complementary force).
 //
 // Every pair term is a sine or cosine of phi_j - phi_i (- alpha), so their sums
 // follow from the sums of cos phi_j and sin phi_j, one evaluation a particle
-// in place of one a pair: a direction enters with an error of 2^-55, the sums
-// are exact, where the sum of n sines rounded each sine and each addition.  The
-// integer pipe adds 64 bits some thirty times faster than the FP64 pipe.
+// in place of one a pair: the integer pipe adds 64 bits some thirty times faster
+// than the FP64 pipe.  But a direction is off by some 2^-60 whatever the term, where
+// a sine is off by 2^-54 of itself.  So the sum of |sin(phi_j - phi_i - alpha)| goes
+// along in FP32, and where the terms are smaller than K64::least on average
+// (aligned or opposite neighbours) they are summed again pair by pair, as they
+// are where a phase has no fixed-point direction.  At the line, 1/32, both ways are
+// off by about the same; with alpha in the second-order model it lies at 1/4,
+// because the rotation by alpha rounds at 2^-53 of the sums of sines and cosines.
 struct NeighbourSums
 {
-  long long ci = 0, si = 0;
+  long long c = 0, s = 0;                    // of the candidates scanned together, units of 2^-59
+  long long ch = 0, cl = 0, sh = 0, sl = 0;  // units of 2^-27 and 2^-59
   int n = 0, bad = 0;
-  double c = 0.0, s = 0.0, count = 0.0, wc = 0.0, ws = 0.0;
+  float sines = 0.0f;
+  double wc = 0.0, ws = 0.0;
+  unsigned long long hits = 0;  // of the first 64 candidates
 
-  __device__ __forceinline__ void add(longlong2 d)
+  // |sin(phi_j - phi_i - alpha)|; own: own_turned of the particle
+  __device__ __forceinline__ static float sine(longlong2 d, float2 own)
   {
-    ci += d.x;
-    si += d.y;
-    bad |= (int) (d.x >> 32) == INT_MIN;
-    ++n;
+    return fabsf(fmaf((float) (int) (d.y >> 32), own.x, -((float) (int) (d.x >> 32) * own.y)));
   }
 
-  __device__ __forceinline__ void flush()
+  // A candidate's direction, zeros where it is out of range (no branch: all
+  // lanes go on together).
+  __device__ __forceinline__ void add(longlong2 d, float2 own)
   {
-    c = c + (double) ci * 5.5511151231257827e-17;
-    s = s + (double) si * 5.5511151231257827e-17;
-    count = count + (double) n;
-    ci = si = 0;
-    n = 0;
+    const int hc = (int) (d.x >> 32);
+    c += d.x;
+    s += d.y;
+    sines += sine(d, own);
+    bad |= hc ^ (hc << 1);  // negative for the lowest value alone
+  }
+
+  // After a set of eight, the `at`-th (`in`: those in range); the two sums hold
+  // fifteen at most.
+  __device__ __forceinline__ void close(unsigned in, int at)
+  {
+    ch += (int) (c >> 32);
+    cl += (unsigned) c;
+    sh += (int) (s >> 32);
+    sl += (unsigned) s;
+    c = s = 0;
+    n += __popc(in);
+    if (at < 8) hits |= (unsigned long long) in << (8 * at);
   }
 };
 
-constexpr int kExactTerms = 511;
+// cos and sin of phi_i + alpha over 2^27, from the fixed-point direction.
+__device__ __forceinline__ float2 own_turned(const K64 &k, longlong2 d)
+{
+  const float c = (float) (int) (d.x >> 32) * 5.5511151231257827e-17f;
+  const float s = (float) (int) (d.y >> 32) * 5.5511151231257827e-17f;
+  return make_float2(fmaf(c, k.ca_f, -(s * k.sa_f)), fmaf(s, k.ca_f, c * k.sa_f));
+}
+
+__device__ __forceinline__ bool lacks_direction(longlong2 d)
+{
+  return (int) (d.x >> 32) == INT_MIN;
+}
+
+__device__ __forceinline__ bool not_finite(double v)
+{
+  return (__double2hiint(v) & 0x7ff00000) == 0x7ff00000;
+}
+
+// Whether the sums of directions do not do (see above), or those with omega are
+// not finite: an infinite omega_j then meets its own cosine alone.
+__device__ __forceinline__ bool needs_pairs(const K64 &k, const NeighbourSums &a, longlong2 own)
+{
+  return a.n > 0 && (a.bad < 0 || lacks_direction(own) || a.sines < k.least * (float) a.n ||
+                     (k.higher_order && not_finite(a.wc + a.ws)));
+}
 
 // Pair sums: first order ParticleSystemFirstOrderPtr.cpp:404-415; second order
 // ParticleSystemSecondOrder.cpp:160-161, sin(phi_j - phi_i - alpha) (its
 // complementary force is the first-order term in that convention).
-__device__ __forceinline__ Sums pair_sums(const K64 &k, const NeighbourSums &a, double2 own)
+// own, turn: the particle's direction in FP64 and in fixed point.  The products of
+// the upper words are taken without a rounding between them (Kahan's ab - cd).
+__device__ __forceinline__ Sums pair_sums(const K64 &k, const NeighbourSums &a, double2 own, longlong2 turn)
 {
-  const double c = a.bad ? nan("") : a.c, s = a.bad ? nan("") : a.s;
-  const double p = s * own.x - c * own.y, q = c * own.x + s * own.y;  // sums of sin, cos (phi_j - phi_i)
-  Sums r{p * k.ca - q * k.sa, a.count, 0.0};
+  const double Ch = (double) a.ch, Sh = (double) a.sh, Cl = (double) a.cl, Sl = (double) a.sl;
+  const double ch = (double) (int) (turn.x >> 32), sh = (double) (int) (turn.y >> 32);
+  const double cl = (double) (unsigned) turn.x, sl = (double) (unsigned) turn.y;
+  constexpr double u54 = 5.5511151231257827e-17, u86 = 1.2924697071141057e-26, u59 = 1.7347234759768071e-18;
+  // sum of sin(phi_j - phi_i)
+  const double t = Ch * sh;
+  const double p = fma(fma(Sh, ch, -t) - fma(Ch, sh, -t), u54,
+                       fma(fma(Sh, cl, -(Ch * sl)), u86, fma(Sl, own.x, -(Cl * own.y)) * u59));
+  Sums r{p, (double) a.n, 0.0};
+  if (k.alpha != 0.0)
+  {
+    const double v = Sh * sh;
+    const double q = fma(fma(Ch, ch, v) + fma(Sh, sh, -v), u54,  // and of cos
+                         fma(fma(Ch, cl, Sh * sl), u86, fma(Cl, own.x, Sl * own.y) * u59));
+    r.af = p * k.ca - q * k.sa;
+  }
   if (k.higher_order)
   {
     const double pw = a.ws * own.x - a.wc * own.y, qw = a.wc * own.x + a.ws * own.y;
     r.caf = qw * k.ca + pw * k.sa;
   }
   return r;
+}
+
+// A sum with what its additions rounded off (Knuth's TwoSum).
+struct KeptSum
+{
+  double v = 0.0, e = 0.0;
+
+  __device__ __forceinline__ void add(double x)
+  {
+    const double s = v + x, b = s - v;
+    e += (v - (s - b)) + (x - b);
+    v = s;
+  }
+
+  __device__ __forceinline__ double value() const { return e == e ? v + e : v; }  // infinite terms: no rest
+};
+
+struct PairTerms
+{
+  KeptSum af, caf;
+
+  __device__ __forceinline__ double2 values() const { return make_double2(af.value(), caf.value()); }
+};
+
+// The term of one pair by its own sine and cosine, the difference of the phases
+// with what its subtractions rounded off.
+__device__ __forceinline__ void add_pair(const K64 &k, PairTerms &a, double phi_i, double omega_i, double phi_j,
+                                         double omega_j)
+{
+  double d = phi_j - phi_i, e = 0.0;
+  if (k.model == 2 && k.alpha != 0.0)
+  {
+    const double v = d - phi_j;
+    e = (phi_j - (d - v)) - (phi_i + v);
+    const double f = d - k.alpha, w = f - d;
+    e += (d - (f - w)) - (k.alpha + w);
+    d = f;
+  } else if (fabs(d) > 0.0625)  // below, what is rounded off is 2^-53 of the term at most
+  {
+    const double v = d - phi_j;
+    e = (phi_j - (d - v)) - (phi_i + v);
+  }
+  double s, c;
+  fast_sincos(k.table, d, s, c);
+  const double sd = fma(c, e, s), cd = fma(-s, e, c);
+  if (k.model == 1)
+  {
+    a.af.add(sd * k.ca - cd * k.sa);
+    if (k.higher_order) a.caf.add((omega_j - omega_i) * (cd * k.ca + sd * k.sa));
+  } else
+  {
+    a.af.add(sd);
+    if (k.higher_order) a.caf.add((omega_j - omega_i) * cd);
+  }
 }
 
 // Output of one particle (ParticleSystemFirstOrder.cpp:220-226, ParticleSystemSecondOrder.cpp:166-175);
@@ -316,10 +438,11 @@ __global__ void f64_stage_kernel(K64 k, const double *__restrict__ st, const dou
     if (q == 0 && posf) posf[i] = make_float2((float) (r.x - floor(r.x)), (float) (r.y - floor(r.y)));
     if (q == k.s / 2 - 1 && posf)
     {
-      double c, sn;
-      fast_sincos(k.table, r.x, sn, c);
-      csphi[i] = make_double2(c, sn);
-      turns[i] = turn_fixed(c, sn);
+      double2 cs;
+      longlong2 turn;
+      directions(k.table, r.x, cs, turn);
+      csphi[i] = cs;
+      turns[i] = turn;
     }
   }
   if (det) det[(long) k.s * i + k.s - 1] = 0.0;
@@ -355,10 +478,11 @@ __global__ void f64_stage_posf_kernel(K64 k, const double *__restrict__ st, cons
   const double x = rk[ii], y = rk[ii + 1];
   posf[i] = make_float2((float) (x - floor(x)), (float) (y - floor(y)));
   const double phi = rk[ii + (k.model == 1 ? 2 : 4)];
-  double c, sn;
-  fast_sincos(k.table, phi, sn, c);
-  csphi[i] = make_double2(c, sn);
-  turns[i] = turn_fixed(c, sn);
+  double2 cs;
+  longlong2 turn;
+  directions(k.table, phi, cs, turn);
+  csphi[i] = cs;
+  turns[i] = turn;
 }
 
 // Where a pair stands to a cutoff by its float wrapped positions alone: 0 out of
@@ -449,35 +573,52 @@ __device__ __forceinline__ void advance_but_omega(const K64 &k, int i, const dou
   for (int q = 0; q < 5; ++q)
     if (q < k.s - 1) row[q] = advance_component<AFTER>(next, ii + q, load_stage<AFTER>(next, ii + q), k_next[ii + q]);
   next.posf[i] = make_float2((float) (row[0] - floor(row[0])), (float) (row[1] - floor(row[1])));
-  double c, sn;
-  fast_sincos(k.table, k.model == 1 ? row[2] : row[4], sn, c);
-  next.csphi[i] = make_double2(c, sn);
-  next.turns[i] = turn_fixed(c, sn);
+  double2 cs;
+  longlong2 turn;
+  directions(k.table, k.model == 1 ? row[2] : row[4], cs, turn);
+  next.csphi[i] = cs;
+  next.turns[i] = turn;
 }
 
 // All pairs (ParticleSystemFirstOrder.cpp:162-228, ParticleSystemFirstOrderPtr.cpp:225-316,
 // ParticleSystemSecondOrder.cpp:116-177): eight particles a block, two warps
 // scanning half the system each for one of them by the float pre-test (FP64
 // within the margins of the cutoff, and for every second-order pair not
-// certainly out of range).  Every lane adds up the neighbours it finds; after
-// the scan eight lanes finish the eight particles, while another warp does what
-// does not need the sums: everything of the derivative and of the next stage
-// but the torque and omega.  At N = 1,000 the block is a chain of latencies (an
-// FP64 instruction's result takes some 50 cycles): 7.5 us an evaluation in a
-// graph of RK4 steps, 10 with a sine for every pair evaluated after the scan.
+// certainly out of range).  Every lane adds up the neighbours it finds, each warp
+// (for each 2,048 candidates) by their directions or, where NeighbourSums says so,
+// by their sines; after the scan eight lanes finish the eight particles, while
+// another warp does what does not need the sums: everything of the derivative
+// and of the next stage but the torque and omega.  At N = 1,000 the block is a
+// chain of latencies (an FP64 instruction's result takes 64 cycles): in a graph of
+// RK4 steps an evaluation takes 9.3 us with random phases, 10.3 with all aligned
+// (7.7 with directions everywhere, which aligned phases do not allow; 20.5 with a
+// library sine in each lane that finds a neighbour).  Two blocks an SM, although 64
+// registers a thread spill some: with one 8.7 us here, but 47 in place of 39 at N = 4,000.
 constexpr int kAllParticles = 8;
 constexpr int kAllWarps = 2 * kAllParticles;
 
-// One scanning warp's sums: the directions in two parts, so that those of all
-// lanes fit, and what the lanes flushed or have in FP64.
+// One scanning warp's sums: of directions and, pair by pair, of near terms and
+// forces; the phases of a few near neighbours, whose sines are taken after the
+// block meets (16 warps with one each would spend the FP64 pipe on one lane a warp),
+// and of the particle.
+constexpr int kNears = 8;
+constexpr int kNearWarps = kAllWarps * kNears / 32;
+
 struct WarpSums
 {
   long long ch, cl, sh, sl;
-  int n, bad, flushed;
-  double c, s, count, wc, ws;
+  int n, nears;
+  double wc, ws, near_sum, caf, phi, near[kNears];
 };
 
 __device__ __forceinline__ long long warp_add(long long v)
+{
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+  return v;
+}
+
+__device__ __forceinline__ float warp_add(float v)
 {
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
@@ -491,8 +632,79 @@ __device__ __forceinline__ double warp_add(double v)
   return v;
 }
 
+// sin(phi_j - phi_i - alpha), mostly of at most 1/4: the difference with what its
+// subtractions rounded off, less the nearest multiple of pi, and the series to
+// the eleventh power, in few steps one after the other (an FP64 instruction's
+// result takes 64 cycles).
+__device__ __noinline__ double near_sine(double phi_i, double phi_j, double alpha)
+{
+  double d = phi_j - phi_i;
+  const double v = d - phi_j;
+  double e = (phi_j - (d - v)) - (phi_i + v);
+  if (alpha != 0.0)
+  {
+    const double f = d - alpha, w = f - d;
+    e += (d - (f - w)) - (alpha + w);
+    d = f;
+  }
+  double r = d;
+  int odd = 0;
+  if ((__double2hiint(d) & 0x7fffffff) > 0x3fd0a3d7)  // 0.26
+  {
+    const double t = fma(d, 0.31830988618379067, SPSS_ROUND_MAGIC);  // 1 / pi
+    const double m = t - SPSS_ROUND_MAGIC;
+    odd = __double2loint(t) & 1;
+    r = fma(m, -0x1.921fb58p+1, d);  // pi in three parts, as pi / 128 in reduce_turn
+    r = fma(m, 0x1.dde974p-26, r);
+    r = fma(m, -0x1.1a62633145c07p-53, r);
+    // phases without a direction have any sine, and as in near_quarter
+    const int size = __double2hiint(r) & 0x7fffffff;
+    if (!reducible(d) || size > 0x3fd0a3d7 || size < 0x3e100000)
+    {
+      double s, c;
+      sincos(d, &s, &c);
+      return fma(c, e, s);
+    }
+  }
+  r += e;
+  const double q = r * r;
+  const double high = fma(q, -1.0 / 39916800.0, 1.0 / 362880.0), low = fma(q, 1.0 / 120.0, -1.0 / 6.0);
+  const double q2 = q * q, cube = r * q;
+  const double s = fma(cube, fma(q2, fma(q, high, -1.0 / 5040.0), low), r);
+  return odd ? -s : s;
+}
+
+// A lane's complementary force over its pairs among the slots j0, j0 + 32, ... below
+// end, each by its own cosine (a neighbour's omega is infinite).
+__device__ __noinline__ double forces_by_pairs(const K64 &k, const double *rk, const float2 *posf, int i, int j0,
+                                               int end)
+{
+  const double *st = rk + (long) k.s * i;
+  PairTerms a;
+  for (int j = j0; j < end; j += 32)
+  {
+    if (j == i) continue;
+    const double *sj = rk + (long) k.s * j;
+    int in = pretest(posf[i], posf[j], k.rho_incl, k.rho_excl);
+    if (in == 1 && k.model == 2) in = 2;
+    if (in == 2)
+    {
+      double x_i = st[0], y_i = st[1];
+      if (k.model == 1 && k.flavor == 1)
+      {
+        x_i = wrap1(x_i);
+        y_i = wrap1(y_i);
+      }
+      in = pair_dr2<false>(k, x_i, y_i, sj[0], sj[1]) <= k.rho2;
+    }
+    if (in) add_pair(k, a, st[k.s - 2], st[k.s - 1], sj[k.s - 2], sj[k.s - 1]);
+  }
+  return a.caf.value();
+}
+
 template<int AFTER>
-__global__ void __launch_bounds__(32 * kAllWarps) f64_allpairs_kernel(K64 k, const double *__restrict__ rk,
+__global__ void __launch_bounds__(32 * kAllWarps, 2) f64_allpairs_kernel(const __grid_constant__ K64 k,
+                                                                      const double *__restrict__ rk,
                                                                       const float2 *__restrict__ posf,
                                                                       const double2 *__restrict__ csphi,
                                                                       const longlong2 *__restrict__ turns,
@@ -505,30 +717,34 @@ __global__ void __launch_bounds__(32 * kAllWarps) f64_allpairs_kernel(K64 k, con
   const int i0 = blockIdx.x * kAllParticles;
   const int i = i0 + (warp >> 1);
   const int ip = k.model == 1 ? 2 : 4;
-  NeighbourSums a;
+  if (lane == 0) sums[warp] = WarpSums{};
+  __syncwarp();
   if (i < k.n)
   {
     const double *st = rk + (long) k.s * i;
-    const double omega_i = k.higher_order ? st[ip + 1] : 0.0;
-    const float2 p_i = posf[i];
+    const double phi_i = st[ip], omega_i = k.higher_order ? st[ip + 1] : 0.0;
+    const longlong2 turn = turns[i];
+    const float2 p_i = posf[i], own = own_turned(k, turn);
     const int half = (k.n + 1) / 2;
     const int begin = (warp & 1) ? half : 0, end = (warp & 1) ? k.n : half;
-    constexpr int U = 8;
-    for (int j0 = begin + lane; j0 - lane < end; j0 += 32 * U)
+    constexpr int U = 8, kStretch = 32 * 64;  // candidates whose hits a lane remembers
+    const bool one_stretch = end - begin <= kStretch;
+    NeighbourSums a;
+    for (int j0 = begin + lane, at = 0; j0 - lane < end; j0 += 32 * U, at = (at + 1) & 7)
     {
       float2 p[U];
-      int in[U];
-      bool unsure = false;
+      unsigned hits = 0, unsure = 0;
 #pragma unroll
       for (int u = 0; u < U; ++u) p[u] = posf[min(j0 + 32 * u, k.n - 1)];
 #pragma unroll
       for (int u = 0; u < U; ++u)
       {
         const int j = j0 + 32 * u;
-        in[u] = pretest(p_i, p[u], k.rho_incl, k.rho_excl);
-        if (j >= end || j == i) in[u] = 0;
-        if (in[u] == 1 && k.model == 2) in[u] = 2;
-        unsure |= in[u] == 2;
+        int in = pretest(p_i, p[u], k.rho_incl, k.rho_excl);
+        if (j >= end || j == i) in = 0;
+        if (in == 1 && k.model == 2) in = 2;
+        if (in == 1) hits |= 1u << u;
+        if (in == 2) unsure |= 1u << u;
       }
       if (unsure)
       {
@@ -538,48 +754,107 @@ __global__ void __launch_bounds__(32 * kAllWarps) f64_allpairs_kernel(K64 k, con
           x_i = wrap1(x_i);
           y_i = wrap1(y_i);
         }
+        for (; unsure; unsure &= unsure - 1)
+        {
+          const int u = __ffs(unsure) - 1;
+          const double *sj = rk + (long) k.s * (j0 + 32 * u);
+          if (pair_dr2<false>(k, x_i, y_i, sj[0], sj[1]) <= k.rho2) hits |= 1u << u;
+        }
+      }
+      if (!__any_sync(0xffffffffu, __popc(hits) > 2))
+      {
+        // few: one set of loads and sums for most
+        for (unsigned rest = hits; rest; rest &= rest - 1) a.add(turns[j0 + 32 * (__ffs(rest) - 1)], own);
+      } else
+      {
+        constexpr int V = 4;
+#pragma unroll
+        for (int v = 0; v < U; v += V)
+        {
+          longlong2 d[V];
+#pragma unroll
+          for (int u = 0; u < V; ++u) d[u] = hits & (1u << (v + u)) ? turns[j0 + 32 * (v + u)] : make_longlong2(0, 0);
+#pragma unroll
+          for (int u = 0; u < V; ++u) a.add(d[u], own);
+        }
+      }
+      a.close(hits, at);
+      if (k.higher_order)
+      {
 #pragma unroll
         for (int u = 0; u < U; ++u)
-          if (in[u] == 2)
+          if (hits & (1u << u))
           {
-            const double *sj = rk + (long) k.s * (j0 + 32 * u);
-            in[u] = pair_dr2<false>(k, x_i, y_i, sj[0], sj[1]) <= k.rho2;
-          }
-      }
-#pragma unroll
-      for (int u = 0; u < U; ++u)
-        if (in[u])
-        {
-          const int j = j0 + 32 * u;
-          a.add(turns[j]);
-          if (k.higher_order)
-          {
+            const int j = j0 + 32 * u;
             const double2 cs = csphi[j];
             const double dw = rk[(long) k.s * j + ip + 1] - omega_i;
-            a.wc += dw * cs.x;
-            a.ws += dw * cs.y;
+            a.wc = fma(dw, cs.x, a.wc);
+            a.ws = fma(dw, cs.y, a.ws);
           }
+      }
+      if (at < 7 && j0 + 32 * U - lane < end) continue;
+      // the end of a stretch: the warp's directions, or its sines one by one
+      const int first = j0 - 32 * U * at, found = __reduce_add_sync(0xffffffffu, a.n);
+      const float sines = warp_add(a.sines);
+      const bool apart = __any_sync(0xffffffffu, a.bad < 0) || lacks_direction(turn) || sines < k.least * (float) found;
+      WarpSums w{};
+      if (!apart)
+      {
+        w.ch = warp_add(a.ch);
+        w.cl = warp_add(a.cl);
+        w.sh = warp_add(a.sh);
+        w.sl = warp_add(a.sl);
+      } else if (found > 0)
+      {
+        const double *phi = rk + (long) k.s * first + ip;
+        if (one_stretch && found <= kNears)
+        {
+          for (unsigned with; (with = __ballot_sync(0xffffffffu, a.hits != 0)) != 0; w.nears += __popc(with))
+          {
+            if (!a.hits) continue;
+            sums[warp].near[w.nears + __popc(with & ((1u << lane) - 1))] = phi[(long) k.s * 32 * (__ffsll(a.hits) - 1)];
+            a.hits &= a.hits - 1;
+          }
+        } else
+        {
+          double sum = 0.0;
+          for (; a.hits; a.hits &= a.hits - 1)
+            sum += near_sine(phi_i, phi[(long) k.s * 32 * (__ffsll(a.hits) - 1)], k.alpha);
+          w.near_sum = warp_add(sum);
         }
-      if (a.n > kExactTerms - U) a.flush();
+      }
+      if (k.higher_order)
+      {
+        double force = 0.0;
+        if (not_finite(a.wc + a.ws))
+        {
+          force = forces_by_pairs(k, rk, posf, i, first, min(end, first + kStretch));
+          a.wc = a.ws = 0.0;
+        }
+        w.wc = warp_add(a.wc);
+        w.ws = warp_add(a.ws);
+        w.caf = warp_add(force);
+      }
+      if (lane == 0)
+      {
+        WarpSums &to = sums[warp];
+        to.ch += w.ch;
+        to.cl += w.cl;
+        to.sh += w.sh;
+        to.sl += w.sl;
+        to.n += found;
+        to.nears = w.nears;
+        to.near_sum += w.near_sum;
+        to.phi = phi_i;
+        if (k.higher_order)
+        {
+          to.wc += w.wc;
+          to.ws += w.ws;
+          to.caf += w.caf;
+        }
+      }
+      a = NeighbourSums();
     }
-  }
-  {
-    const bool flushed = __any_sync(0xffffffffu, a.count != 0.0);
-    constexpr long long low = (1ll << 27) - 1;
-    WarpSums w;
-    w.ch = warp_add(a.ci >> 27);
-    w.cl = warp_add(a.ci & low);
-    w.sh = warp_add(a.si >> 27);
-    w.sl = warp_add(a.si & low);
-    w.n = __reduce_add_sync(0xffffffffu, a.n);
-    w.bad = __any_sync(0xffffffffu, a.bad);
-    w.flushed = flushed;
-    w.c = flushed ? warp_add(a.c) : 0.0;
-    w.s = flushed ? warp_add(a.s) : 0.0;
-    w.count = flushed ? warp_add(a.count) : 0.0;
-    w.wc = k.higher_order ? warp_add(a.wc) : 0.0;
-    w.ws = k.higher_order ? warp_add(a.ws) : 0.0;
-    if (lane == 0) sums[warp] = w;
   }
   const int g = i0 + lane;
   // the finishing lanes' words, asked for before the block meets
@@ -588,9 +863,11 @@ __global__ void __launch_bounds__(32 * kAllWarps) f64_allpairs_kernel(K64 k, con
   StageWords words{0.0, 0.0, 0.0, 0.0};
   double torque = 0.0, omega = 0.0;
   double2 own = make_double2(0.0, 0.0);
+  longlong2 turn = make_longlong2(0, 0);
   if (finisher)
   {
     own = csphi[g];
+    turn = turns[g];
     omega = rk[at];
     if (AFTER != AFTER_NOTHING)
     {
@@ -605,22 +882,31 @@ __global__ void __launch_bounds__(32 * kAllWarps) f64_allpairs_kernel(K64 k, con
     write_k_but_torque(k, g, rk + (long) k.s * g, k_next, cs.x, cs.y);
     if (AFTER != AFTER_NOTHING) advance_but_omega<AFTER>(k, g, k_next, next);
   }
+  if (warp >= kNearWarps) return;
+  // the near sines: 32 of their places for each of a few warps
+  const bool more = __any_sync(0xffffffffu, lane < kAllWarps && sums[lane & (kAllWarps - 1)].nears > 0);
+  if (more)
+  {
+    const int at = 32 * warp + lane;
+    WarpSums &of = sums[at / kNears];
+    if (at % kNears < of.nears) of.near[at % kNears] = near_sine(of.phi, of.near[at % kNears], k.alpha);
+    asm volatile("bar.sync 1, %0;" ::"n"(32 * kNearWarps) : "memory");
+  }
   if (!finisher) return;
   const WarpSums &u = sums[2 * lane], &v = sums[2 * lane + 1];
-  // 2^-27 and 2^-54: the parts are below 2^53, so one rounding each
-  a.c = (double) (u.ch + v.ch) * 7.4505805969238281e-09 + (double) (u.cl + v.cl) * 5.5511151231257827e-17;
-  a.s = (double) (u.sh + v.sh) * 7.4505805969238281e-09 + (double) (u.sl + v.sl) * 5.5511151231257827e-17;
-  a.count = (double) (u.n + v.n);
-  if (u.flushed || v.flushed)
-  {
-    a.c += u.c + v.c;
-    a.s += u.s + v.s;
-    a.count += u.count + v.count;
-  }
-  a.bad = u.bad | v.bad;
+  NeighbourSums a;
+  a.ch = u.ch + v.ch;
+  a.cl = u.cl + v.cl;
+  a.sh = u.sh + v.sh;
+  a.sl = u.sl + v.sl;
+  a.n = u.n + v.n;
   a.wc = u.wc + v.wc;
   a.ws = u.ws + v.ws;
-  Sums r = pair_sums(k, a, own);
+  Sums r = pair_sums(k, a, own, turn);
+  r.af += u.near_sum + v.near_sum;
+  for (int t = 0; t < u.nears; ++t) r.af += u.near[t];
+  for (int t = 0; t < v.nears; ++t) r.af += v.near[t];
+  r.caf += u.caf + v.caf;
   if (r.card != 0.0)
   {
     torque = -(k.model == 1 ? k.xi : k.xi_phi) * omega + k.sigma * r.af / r.card;
@@ -637,9 +923,10 @@ __global__ void __launch_bounds__(32 * kAllWarps) f64_allpairs_kernel(K64 k, con
 // for a pair within the margins of the cutoff) and adds up their directions.
 // With a sine a pair (queued, and evaluated by the whole warp) ten steps of
 // N = 65,536 took 815 us, and 2,160 once clusters had formed; by sums of
-// directions 825 and 1,520, and with the linked list's positions and directions
+// directions 825 and 1,520, with the linked list's positions and directions
 // copied into cell order by the sort (one load, contiguous, before a test in
-// place of two) 700 and 1,150.
+// place of two) 700 and 1,150, and without branches around the sums (the few
+// lanes that need sines included) another 5 % less.
 constexpr int kScan = 8;          // candidates a lane looks at together (their loads are in flight at once)
 constexpr int kPairThreads = 32;  // one warp a block: 20,011 particles in blocks of 64 left SMs with 3 blocks beside SMs with 2
 
@@ -662,12 +949,13 @@ struct PairInputs
 // particle.
 template<bool ROWS>
 __device__ __forceinline__ void scan_candidates(const K64 &k, const PairInputs &in, const int *__restrict__ list,
-                                                int m, int e, int self, float2 p_i, double x_i, double y_i,
-                                                double omega_i, NeighbourSums &a)
+                                                int m, int e, int at, int self, float2 p_i, double x_i, double y_i,
+                                                double omega_i, float2 own, NeighbourSums &a)
 {
-  int j[kScan], hit[kScan];
+  int j[kScan];
   float2 p[kScan];
   longlong2 d[kScan];
+  unsigned hits = 0;
 #pragma unroll
   for (int u = 0; u < kScan; ++u) j[u] = m + u < e ? (ROWS ? m + u : __ldg(list + m + u)) : self;
 #pragma unroll
@@ -675,29 +963,57 @@ __device__ __forceinline__ void scan_candidates(const K64 &k, const PairInputs &
 #pragma unroll
   for (int u = 0; u < kScan; ++u)
   {
-    hit[u] = j[u] == self ? 0 : pretest(p_i, p[u], k.rho_incl, k.rho_excl);
-    if (hit[u] == 2)
+    int hit = j[u] == self ? 0 : pretest(p_i, p[u], k.rho_incl, k.rho_excl);
+    if (hit == 2)
     {
       const double *sj = in.rk + (long) k.s * (ROWS ? __ldg(list + j[u]) : j[u]);
-      hit[u] = pair_dr2<true>(k, x_i, y_i, sj[0], sj[1]) <= k.rho2;
+      hit = pair_dr2<true>(k, x_i, y_i, sj[0], sj[1]) <= k.rho2;
     }
-    d[u] = hit[u] ? __ldg((ROWS ? in.turns_rows : in.turns) + j[u]) : make_longlong2(0, 0);
+    d[u] = hit ? __ldg((ROWS ? in.turns_rows : in.turns) + j[u]) : make_longlong2(0, 0);
+    if (hit) hits |= 1u << u;
   }
 #pragma unroll
-  for (int u = 0; u < kScan; ++u)
-    if (hit[u])
-    {
-      a.add(d[u]);
-      if (k.higher_order)
+  for (int u = 0; u < kScan; ++u) a.add(d[u], own);
+  a.close(hits, at);
+  if (k.higher_order)
+  {
+    // sums of a few terms first: a long list's additions then round less
+    double wc = 0.0, ws = 0.0;
+#pragma unroll
+    for (int u = 0; u < kScan; ++u)
+      if (hits & (1u << u))
       {
         const int o = ROWS ? __ldg(list + j[u]) : j[u];
         const double2 cs = __ldg(in.csphi + o);
         const double dw = __ldg(in.rk + (long) k.s * o + k.s - 1) - omega_i;
-        a.wc += dw * cs.x;
-        a.ws += dw * cs.y;
+        wc = fma(dw, cs.x, wc);
+        ws = fma(dw, cs.y, ws);
       }
+    a.wc += wc;
+    a.ws += ws;
+  }
+}
+
+// The candidates of one such set again, those in range by their own sines: known
+// from the first scan (`hits`) or, beyond its first 64, tested again.
+template<bool ROWS>
+__device__ __forceinline__ void candidate_terms(const K64 &k, const PairInputs &in, const int *__restrict__ list, int m,
+                                                int e, int at, unsigned long long hits, int i, double x_i, double y_i,
+                                                const double *st, PairTerms &a)
+{
+  unsigned set = at < 8 ? (unsigned) (hits >> (8 * at)) & 255u : (1u << min(e - m, kScan)) - 1u;
+  for (; set; set &= set - 1)
+  {
+    const int o = list[m + __ffs(set) - 1];
+    const double *sj = in.rk + (long) k.s * o;
+    if (at >= 8)
+    {
+      int hit = o == i ? 0 : pretest(in.posf[i], in.posf[o], k.rho_incl, k.rho_excl);
+      if (hit == 2) hit = pair_dr2<true>(k, x_i, y_i, sj[0], sj[1]) <= k.rho2;
+      if (!hit) continue;
     }
-  if (a.n > kExactTerms - kScan) a.flush();
+    add_pair(k, a, st[k.s - 2], st[k.s - 1], sj[k.s - 2], sj[k.s - 1]);
+  }
 }
 
 // The stencil of a cell as runs of the cell list, in the reference's order: a
@@ -719,9 +1035,45 @@ __device__ __forceinline__ void next_run(int cx, int cy, int nc, const int *__re
   ++c;
 }
 
+// The pair sums of one particle pair by pair, in the reference's order: from the
+// cell list, and from its Verlet list.
+__device__ __noinline__ double2 linked_list_terms(const K64 &k, const PairInputs &in, int nc, const int *off,
+                                               const int *mem, int t, unsigned long long hits)
+{
+  const int i = mem[t];
+  double x_i, y_i;
+  pos_for_cells(k, in.rk, i, x_i, y_i);
+  const int cx = cell_coord(x_i, nc), cy = cell_coord(y_i, nc);
+  PairTerms a;
+  int at = 0;
+  for (int c = 0; c < 9;)
+  {
+    int m, e;
+    next_run(cx, cy, nc, off, c, m, e);
+    for (; m < e; m += kScan, ++at)
+      candidate_terms<true>(k, in, mem, m, e, at, hits, i, x_i, y_i, in.rk + (long) k.s * i, a);
+  }
+  return a.values();
+}
+
+__device__ __noinline__ double2 verlet_terms(const K64 &k, const PairInputs &in, const int *vl_off, const int *vl_ent,
+                                          int i, unsigned long long hits)
+{
+  const double *st = in.rk + (long) k.s * i;
+  double x_i = st[0], y_i = st[1];
+  if (k.model == 2) wrap_if_outside(x_i, y_i);
+  PairTerms a;
+  const int e = vl_off[i + 1];
+  int at = 0;
+  for (int m = vl_off[i]; m < e; m += kScan, ++at)
+    candidate_terms<false>(k, in, vl_ent, m, e, at, hits, i, x_i, y_i, st, a);
+  return a.values();
+}
+
 // Linked list (ParticleSystemFirstOrder.cpp:231-353, ParticleSystemSecondOrder.cpp:276-409).
 // Particles are taken in cell order, so a warp's lanes scan neighbouring cells.
-__global__ void __launch_bounds__(kPairThreads) f64_linked_list_kernel(K64 k, PairInputs in, int nc,
+__global__ void __launch_bounds__(kPairThreads) f64_linked_list_kernel(const __grid_constant__ K64 k,
+                                                                       const __grid_constant__ PairInputs in, int nc,
                                                                        const int *__restrict__ off,
                                                                        const int *__restrict__ mem,
                                                                        double *__restrict__ k_next,
@@ -737,16 +1089,20 @@ __global__ void __launch_bounds__(kPairThreads) f64_linked_list_kernel(K64 k, Pa
   const double omega_i = st[k.s - 1];
   const float2 p_i = in.posf[i];
   const int cx = cell_coord(x_i, nc), cy = cell_coord(y_i, nc);
+  const longlong2 turn = in.turns[i];
+  const float2 own_f = own_turned(k, turn);
   NeighbourSums a;
+  int at = 0;
   for (int c = 0; c < 9;)
   {
     int m, e;
     next_run(cx, cy, nc, off, c, m, e);
-    for (; m < e; m += kScan) scan_candidates<true>(k, in, mem, m, e, t, p_i, x_i, y_i, omega_i, a);
+    for (; m < e; m += kScan, ++at) scan_candidates<true>(k, in, mem, m, e, at, t, p_i, x_i, y_i, omega_i, own_f, a);
   }
-  a.flush();
   const double2 own = in.csphi[i];
-  write_k(k, i, st, own, pair_sums(k, a, own), k_next, caf);
+  Sums r = pair_sums(k, a, own, turn);
+  if (needs_pairs(k, a, turn)) r.take(linked_list_terms(k, in, nc, off, mem, t, a.hits));
+  write_k(k, i, st, own, r, k_next, caf);
 }
 
 // Verlet list from the cell list (ParticleSystemFirstOrder.cpp:536-589): first
@@ -826,7 +1182,8 @@ __global__ void f64_verlet_all_kernel(K64 k, const double *__restrict__ rk, int 
 // Pair loop over the Verlet list (ParticleSystemFirstOrder.cpp:594-648, ParticleSystemFirstOrderPtr.cpp:861-930).
 // `order` (not null): particles in the cell order of the last build, so a
 // warp's lanes read neighbouring particles.
-__global__ void __launch_bounds__(kPairThreads) f64_verlet_pairs_kernel(K64 k, PairInputs in,
+__global__ void __launch_bounds__(kPairThreads) f64_verlet_pairs_kernel(const __grid_constant__ K64 k,
+                                                                        const __grid_constant__ PairInputs in,
                                                                         const int *__restrict__ order,
                                                                         const int *__restrict__ vl_off,
                                                                         const int *__restrict__ vl_ent,
@@ -842,12 +1199,17 @@ __global__ void __launch_bounds__(kPairThreads) f64_verlet_pairs_kernel(K64 k, P
   if (k.model == 2) wrap_if_outside(x_i, y_i);
   const double omega_i = st[k.s - 1];
   const float2 p_i = in.posf[i];
+  const longlong2 turn = in.turns[i];
+  const float2 own_f = own_turned(k, turn);
   NeighbourSums a;
   const int e = vl_off[i + 1];
-  for (int m = vl_off[i]; m < e; m += kScan) scan_candidates<false>(k, in, vl_ent, m, e, i, p_i, x_i, y_i, omega_i, a);
-  a.flush();
+  int at = 0;
+  for (int m = vl_off[i]; m < e; m += kScan, ++at)
+    scan_candidates<false>(k, in, vl_ent, m, e, at, i, p_i, x_i, y_i, omega_i, own_f, a);
   const double2 own = in.csphi[i];
-  write_k(k, i, st, own, pair_sums(k, a, own), k_next, caf);
+  Sums r = pair_sums(k, a, own, turn);
+  if (needs_pairs(k, a, turn)) r.take(verlet_terms(k, in, vl_off, vl_ent, i, a.hits));
+  write_k(k, i, st, own, r, k_next, caf);
 }
 
 // Global polar order field, first order (ParticleSystemFirstOrder.cpp:122-159,

@@ -2,6 +2,7 @@
 #pragma once
 
 #include <cuda_runtime.h>
+#include <limits.h>
 #include <stdint.h>
 
 #include <cmath>
@@ -194,19 +195,26 @@ __device__ __forceinline__ uint4 philox_block(const NoiseKey &nk, uint32_t parti
 
 constexpr int kTrigTable = 256;      // cos and sin of 2 pi k / 256
 constexpr int kLogFirst = 88, kLogLast = 184;  // j / 128 covers [sqrt(1/2), sqrt(2)] with room
-constexpr int kTableEntries = kTrigTable + (kLogLast - kLogFirst + 1);
+constexpr int kTableEntries = kTrigTable + (kLogLast - kLogFirst + 1);  // then the first kTrigTable in units of 2^-59
 
 // 1.5 * 2^52: adding it rounds to an integer, which then stands in the low word.
 #define SPSS_ROUND_MAGIC 6755399441055744.0
 
-// sin and cos of 2 pi k / 256 + r, 0 <= |r| <= 2 pi / 256: Taylor polynomials
-// (remainders below 1e-20 and 4e-18) and the angle sum.
+// sin r and cos r - 1 for 0 <= |r| <= 2 pi / 256 by Taylor polynomials
+// (remainders below 1e-20 and 4e-18).
+__device__ __forceinline__ void sincos_rest(double r, double &sr, double &cm)
+{
+  const double p = r * r;
+  sr = fma(r * p, fma(p, fma(p, -1.0 / 5040.0, 1.0 / 120.0), -1.0 / 6.0), r);
+  cm = p * fma(p, fma(p, -1.0 / 720.0, 1.0 / 24.0), -0.5);
+}
+
+// sin and cos of 2 pi k / 256 + r by the angle sum.
 __device__ __forceinline__ void sincos_at(const double2 *__restrict__ table, int k, double r, double &s, double &c)
 {
   const double2 T = __ldg(table + (k & (kTrigTable - 1)));
-  const double p = r * r;
-  const double sr = fma(r * p, fma(p, fma(p, -1.0 / 5040.0, 1.0 / 120.0), -1.0 / 6.0), r);
-  const double cm = p * fma(p, fma(p, -1.0 / 720.0, 1.0 / 24.0), -0.5);
+  double sr, cm;
+  sincos_rest(r, sr, cm);
   s = fma(T.x, sr, fma(T.y, cm, T.y));
   c = fma(-T.y, sr, fma(T.x, cm, T.x));
 }
@@ -288,8 +296,32 @@ __device__ __forceinline__ double sqrt_positive(double v)
   return fma(g * e, fma(e, 0.375, 0.5), g);
 }
 
+// cos and sin of x, and in fixed point, units of 2^-59: what is added to the
+// table's point is below 2^-6, so the fixed-point pair is right to some 2^-60
+// (2^-58 at most) where the doubles are to 2^-53.  A phase that is not reduced by hand
+// (beyond 2^20, infinite, NaN) has none: the lowest value.
+__device__ __forceinline__ void directions(const double2 *__restrict__ table, double x, double2 &cs, longlong2 &turn)
+{
+  if (!reducible(x))
+  {
+    sincos(x, &cs.y, &cs.x);
+    turn = make_longlong2(LLONG_MIN, LLONG_MIN);
+    return;
+  }
+  int k;
+  double r, sr, cm;
+  reduce_turn(x, k, r);
+  const double2 T = __ldg(table + (k & (kTrigTable - 1)));
+  const longlong2 F = __ldg(reinterpret_cast<const longlong2 *>(table + kTableEntries) + (k & (kTrigTable - 1)));
+  sincos_rest(r, sr, cm);
+  const double dc = fma(T.x, cm, -(T.y * sr)), ds = fma(T.x, sr, T.y * cm);
+  cs = make_double2(T.x + dc, T.y + ds);
+  if (near_quarter(k, r)) sincos(x, &cs.y, &cs.x);
+  turn = make_longlong2(F.x + __double2ll_rn(dc * 576460752303423488.0), F.y + __double2ll_rn(ds * 576460752303423488.0));
+}
+
 // The tables of the functions above: cos, sin of 2 pi k / 256, then 128 / j and
-// -log(128 / j as rounded).
+// -log(128 / j as rounded), then the first in units of 2^-59.
 int make_f64_tables(DeviceArray<double2> &table, cudaStream_t stream);
 
 // Box-Muller on two 32-bit uniforms in (0, 1): FP64 variant for the
