@@ -1849,24 +1849,25 @@ __device__ __forceinline__ void add_direction(float2 v, double &sx, double &sy)
   sy = fma(y, c, sy);
 }
 
-// Sum of floats of at most 1 in magnitude as integers, in units of 2^-24 and
-// 2^-48: exact down to floats of 2^-25, at a quarter of the conversion and the
-// addition in FP64.  Up to 64 terms.
+// Sum of sines or cosines as integers, in units of 2^-24 and 2^-53 (the last bit of
+// the smallest one, of a phase 2^-32 turns from a multiple of a quarter): exact,
+// at a quarter of the conversion and the addition in FP64.  Up to 64 terms.
 struct UnitSum
 {
-  int hi = 0, lo = 0;
+  int hi = 0;
+  long long lo = 0;
 
   __device__ __forceinline__ void add(float x)
   {
     const float t = x * 16777216.0f;
     const int h = __float2int_rn(t);
     hi += h;
-    lo += __float2int_rn((t - (float) h) * 16777216.0f);
+    lo += __float2int_rn((t - (float) h) * 536870912.0f);
   }
 
   __device__ __forceinline__ double value() const
   {
-    return (double) (((long long) hi << 24) + lo) * 3.5527136788005009e-15;
+    return (double) (((long long) hi << 29) + lo) * 1.1102230246251565e-16;
   }
 };
 
