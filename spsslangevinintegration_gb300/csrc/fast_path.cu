@@ -1810,13 +1810,14 @@ __device__ __forceinline__ double warp_sum(double v)
   return v;
 }
 
-// The double of a float by integer instructions (a conversion takes the FP64
-// pipe); subnormal floats become 0.
-__device__ __forceinline__ double widen(float x)
+// The double x 2^ex of a finite float by integer instructions (a conversion takes
+// the FP64 pipe); subnormal ones by way of a multiple of theirs.
+__device__ __forceinline__ double widen(float x, int ex = 0)
 {
-  const uint32_t b = __float_as_uint(x), m = b & 0x7fffffffu;
-  const uint32_t hi = m < 0x00800000u ? 0u : (b & 0x80000000u) | ((m >> 3) + 0x38000000u);
-  return __hiloint2double((int) hi, m < 0x00800000u ? 0 : (int) (b << 29));
+  const bool small = fabsf(x) < 1.17549435e-38f;  // the smallest normal float
+  const uint32_t b = __float_as_uint(small ? x * 4294967296.0f : x), m = b & 0x7fffffffu;
+  const uint32_t hi = m ? (b & 0x80000000u) | ((m >> 3) + (small ? 0x36000000u : 0x38000000u) + ((uint32_t) ex << 20)) : 0u;
+  return __hiloint2double((int) hi, (int) (b << 29));
 }
 
 // v / |v| in FP64, added to (sx, sy); nothing for v = 0.  The reciprocal square
@@ -1841,7 +1842,7 @@ __device__ __forceinline__ void add_direction(float2 v, double &sx, double &sy)
     sx = sy = __longlong_as_double(0x7ff8000000000000ll);
     return;
   }
-  const double x = widen(fx), y = widen(fy), r = widen(rsqrtf(f2));
+  const double x = widen(v.x, ex), y = widen(v.y, ex), r = widen(rsqrtf(f2));
   const double m2 = fma(x, x, y * y);
   const double e = fma(-m2 * r, r, 1.0);
   const double c = fma(r * e, fma(e, 0.375, 0.5), r);
