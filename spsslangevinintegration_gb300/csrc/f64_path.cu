@@ -67,8 +67,9 @@ struct K64
 
 // Margin of the range pre-test, in box units: six times what the float rounding
 // of the wrapped positions (6e-8 a difference), of the minimum image and of
-// the squares (1e-7 together) and the FP64 wrap of positions up to 1e4 boxes
-// away (1e-12) amount to.  A pair nearer to the cutoff than this is decided in
+// the squares (1e-7 together) and the FP64 differences of positions up to 2^20
+// boxes away (2e-10) amount to; a position farther away has no float one
+// (pretest_position).  A pair nearer to the cutoff than this is decided in
 // FP64, for the whole warp's time: at N = 65,536 a margin of 2e-5 left 0.27
 // such pairs a particle and the linked-list kernel took 64 us, now 44.
 constexpr float kPretestMargin = 1e-6f;
@@ -405,6 +406,17 @@ struct StageCells
   int nc, *cell_of, *count, *slot;
 };
 
+// The position for the range pre-test: wrapped into the unit box, as floats.
+// From 2^20 boxes on, where the rounding of an FP64 difference approaches the
+// margin (and at 10^10 exceeds it), no number: every pair is then left to the
+// reference's FP64 expression.
+__device__ __forceinline__ float2 pretest_position(double x, double y)
+{
+  if (max(__double2hiint(x) & 0x7fffffff, __double2hiint(y) & 0x7fffffff) >= 0x41300000)
+    return make_float2(__int_as_float(0x7fffffff), __int_as_float(0x7fffffff));
+  return make_float2((float) (x - floor(x)), (float) (y - floor(y)));
+}
+
 // Cell of a stage position, and its place among the cell's members by arrival.
 __device__ __forceinline__ int stage_cell(const K64 &k, const double *rk, int i, int nc)
 {
@@ -435,7 +447,7 @@ __global__ void f64_stage_kernel(K64 k, const double *__restrict__ st, const dou
     const double2 a = s2[q], b = kp ? k2[q] : make_double2(0.0, 0.0);
     const double2 r = make_double2(a.x + k_coef * dt * b.x, a.y + k_coef * dt * b.y);
     r2[q] = r;
-    if (q == 0 && posf) posf[i] = make_float2((float) (r.x - floor(r.x)), (float) (r.y - floor(r.y)));
+    if (q == 0 && posf) posf[i] = pretest_position(r.x, r.y);
     if (q == k.s / 2 - 1 && posf)
     {
       double2 cs;
@@ -475,8 +487,7 @@ __global__ void f64_stage_posf_kernel(K64 k, const double *__restrict__ st, cons
   if (i >= k.n) return;
   const long ii = (long) k.s * i;
   for (int q = 0; q < k.s; ++q) rk[ii + q] = st[ii + q] + k_coef * dt * kp[ii + q];
-  const double x = rk[ii], y = rk[ii + 1];
-  posf[i] = make_float2((float) (x - floor(x)), (float) (y - floor(y)));
+  posf[i] = pretest_position(rk[ii], rk[ii + 1]);
   const double phi = rk[ii + (k.model == 1 ? 2 : 4)];
   double2 cs;
   longlong2 turn;
@@ -572,7 +583,7 @@ __device__ __forceinline__ void advance_but_omega(const K64 &k, int i, const dou
 #pragma unroll
   for (int q = 0; q < 5; ++q)
     if (q < k.s - 1) row[q] = advance_component<AFTER>(next, ii + q, load_stage<AFTER>(next, ii + q), k_next[ii + q]);
-  next.posf[i] = make_float2((float) (row[0] - floor(row[0])), (float) (row[1] - floor(row[1])));
+  next.posf[i] = pretest_position(row[0], row[1]);
   double2 cs;
   longlong2 turn;
   directions(k.table, k.model == 1 ? row[2] : row[4], cs, turn);
