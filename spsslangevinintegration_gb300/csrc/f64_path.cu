@@ -1541,6 +1541,8 @@ int f64_create(spss_ctx *ctx)
   SPSS_CUDA_TRY(cudaMemsetAsync(f->state.ptr, 0, sizeof(double) * len, ctx->stream));
   for (auto &kb : f->k) SPSS_CUDA_TRY(cudaMemsetAsync(kb.ptr, 0, sizeof(double) * len, ctx->stream));
   SPSS_CUDA_TRY(cudaMemsetAsync(f->caf.ptr, 0, sizeof(double) * ctx->p.n, ctx->stream));
+  // empty lists until the first build, as the reference's
+  SPSS_CUDA_TRY(cudaMemsetAsync(f->vl_off.ptr, 0, sizeof(int) * (ctx->p.n + 1), ctx->stream));
   SPSS_CUDA_TRY(cudaMemsetAsync(f->nat_freq.ptr, 0, sizeof(double) * ctx->p.n, ctx->stream));
   return SPSS_OK;
 }

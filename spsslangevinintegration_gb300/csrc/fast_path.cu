@@ -2502,6 +2502,9 @@ int fast_create(spss_ctx *ctx)
   f->h_ctrl->uses_verlet = f->kind == KIND_VERLET;
   SPSS_CUDA_TRY(cudaMemcpyAsync(f->ctrl, f->h_ctrl, sizeof(FastControl), cudaMemcpyHostToDevice, ctx->stream));
   SPSS_CUDA_TRY(cudaMemsetAsync(f->vel.ptr, 0, sizeof(float2) * n, ctx->stream));
+  // a download before the first state gathers slot 0; empty lists until the first build, as the reference's
+  SPSS_CUDA_TRY(cudaMemsetAsync(f->inv.ptr, 0, sizeof(unsigned) * n, ctx->stream));
+  SPSS_CUDA_TRY(cudaMemsetAsync(f->vl_cnt.ptr, 0, sizeof(int) * n, ctx->stream));
   if (has_cells(f->kind)) SPSS_TRY(f->binner.prepare(n, f->total_cells, ctx->stream));
   if (f->kind == KIND_VERLET) SPSS_TRY(f->vl.reserve((size_t) f->cap * (((size_t) n + 31) / 32 * 32)));
   SPSS_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
@@ -2888,14 +2891,14 @@ static int launch_single_step(spss_ctx *ctx, int stepper, double dt)
   SPSS_TRY(push_host_control(ctx));
   if (f->kind == KIND_CELLS)
   {
-    if (f->h_ctrl->rebuild)
+    if (f->h_ctrl->rebuild || !f->h_ctrl->rebuilds)
     {
       SPSS_TRY(ensure_cells(ctx, P));
       SPSS_TRY(launch_cells_step(ctx, stepper, P, !ctx->timing));
     } else
     {
       // the caller asked for the lists to stay (spss_set_should_update_lists):
-      // a step on the last binning, which counts the cells anew
+      // a step on the last binning (there was one), which counts the cells anew
       SPSS_CUDA_TRY(cudaMemsetAsync(f->binner.count.ptr, 0, sizeof(int) * f->binner.count.count, ctx->stream));
       SPSS_TRY(launch_cell_kernel(ctx, stepper, P, 0, false));
       SPSS_TRY(launch_control(ctx, P, 1));
