@@ -350,8 +350,6 @@ def run_cells_leg(args, rank, world, barrier, max_over_ranks):
     stream = torch.cuda.Stream()
     ctx.set_stream(stream.cuda_stream)
     ctx.set_state(initial_state(n, L, rank))
-    tune_ms = ctx.autotune(SRK, DT, steps=4)
-    tiling = ctx.tiling()
     ctx.steps(SRK, 0.0, DT, max(3, args.warmup // 4))
     steps = max(20, min(args.steps, 100))
     e0 = torch.cuda.Event(enable_timing=True)
@@ -367,9 +365,8 @@ def run_cells_leg(args, rank, world, barrier, max_over_ranks):
         return None
     value = world * n * steps / (ms * 1e-3)
     out = {"workload": "the main workload (N=%d, SRK) with cell lists of side 1/int(1/rho) rebuilt every step "
-                       "(slot re-sort and tile layout each step)" % n,
+                       "(slots re-sorted each step)" % n,
            "value": value, "unit": "particle-steps/s", "ms_per_step": ms / steps, "steps_timed": steps,
-           "tiling": {"tile_cells": tiling[0], "persistent": tiling[1], "autotuned_ms_per_step": tune_ms},
            "timing": "CUDA events around %d graph steps on the library's stream, max over ranks" % steps}
     if not args.no_cpu_baseline and world == 1:
         cpu = cpu_cells_sample(n)
@@ -409,9 +406,8 @@ def sweep_cpu_sample(points, budget_s=8.0):
 
 def run_sweep_leg(args, rank, world, barrier, max_over_ranks, verlet=False):
     """Batched parameter sweep: 512 independent systems in one batch context
-    (one CUDA graph per step for all systems), tiling picked by the autotuner;
-    phase-diagram points per hour at 20,000 steps per point.  Cell lists
-    rebuilt every step (the sweep's prescribed method), or with `verlet` the
+    (one CUDA graph per step for all systems); phase-diagram points per hour at
+    20,000 steps per point.  Cell lists rebuilt every step (the sweep's prescribed method), or with `verlet` the
     reference's linked list + Verlet routine with skin 0.3 R, each system's
     lists rebuilt when its own displacement trigger fires (the same neighbour
     sets within R)."""
@@ -425,7 +421,6 @@ def run_sweep_leg(args, rank, world, barrier, max_over_ranks, verlet=False):
     b = sweep.make_batch(mine, seed=0, first_replica=shard(len(points), world, rank)[0],
                          variant=LINKED_LIST_VERLET if verlet else LINKED_LIST, skin=SKIN if verlet else 0.0)
     b.steps(STOCHASTIC_EULER, 0.0, DT, 3)
-    tune_ms = b.autotune(STOCHASTIC_EULER, DT, steps=4)
     b.run(STOCHASTIC_EULER, 0.0, DT, 10, sample_every=SWEEP_SAMPLE_EVERY, sample_from=0)
     steps = max(20, min(args.sweep_steps, 2000))
     launches0 = b.kernel_launches
@@ -439,7 +434,6 @@ def run_sweep_leg(args, rank, world, barrier, max_over_ranks, verlet=False):
     el = max_over_ranks(time.perf_counter() - t0)
     launches = b.kernel_launches - launches0
     rebuild_steps = b.rebuild_count - rebuilds0
-    tiling = b.tiling()
     total_n = sum(p["n"] for p in points)
     b.close()
     if rank != 0:
@@ -456,7 +450,6 @@ def run_sweep_leg(args, rank, world, barrier, max_over_ranks, verlet=False):
         "steps_timed": steps, "ms_per_step": 1e3 * s_per_step, "particle_steps_per_s": total_n / s_per_step,
         "points_per_hour": len(points) * 3600.0 / (SWEEP_STEPS_PER_POINT * s_per_step),
         "points_per_hour_unit": "phase-diagram points per hour at %d steps per point" % SWEEP_STEPS_PER_POINT,
-        "tiling": {"tile_cells": tiling[0], "persistent": tiling[1], "autotuned_ms_per_step": tune_ms},
         "gpu_launches_per_step": launches / steps, "steps_with_a_rebuild": rebuild_steps,
         "timing": "wall clock around %d steps (graph launches, one host synchronisation), max over ranks" % steps,
     }
@@ -647,14 +640,7 @@ def run_ours(args, rank, world, local_rank):
             dist.barrier()
         torch.cuda.synchronize()
 
-    # tile width and launch form picked by the library's autotuner (trial
-    # steps, state restored), then warm-up (graph capture, first list build)
-    if args.tile_cells:
-        ctx.set_tiling(args.tile_cells, False)
-        tune_ms = None
-    else:
-        tune_ms = None if args.no_autotune else ctx.autotune(SRK, DT, steps=4)
-    tiling = ctx.tiling()
+    # warm-up: graph capture, first list build
     t = 0.0
     ctx.steps(SRK, t, DT, args.warmup)
     t += DT * args.warmup
@@ -767,8 +753,7 @@ def run_ours(args, rank, world, local_rank):
                                "v0=0.5, sigma=1, D=0.1; one independent replica per GPU" % n,
                    "n": n, "l2": "inputs larger than L2 (state %.0f MB + lists %.0f MB)" % (
                        n * 56 / 1e6, n * 4 * (mean_list_length(p) + 1) / 1e6),
-                   "parallelism": "replicas x%d" % world,
-                   "tiling": {"tile_cells": tiling[0], "persistent": tiling[1], "autotuned_ms_per_step": tune_ms}},
+                   "parallelism": "replicas x%d" % world},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                      "peak_kind": peak_kind, "kernel": "fast_tile_kernel<2,2,0> (pair sums + SRK update)",
                      "kernel_ms": avg_kernel_s * 1e3,
@@ -820,10 +805,8 @@ def main():
     ap.add_argument("--n", type=int, default=N_DEFAULT)
     ap.add_argument("--cpu-seconds", type=float, default=20.0)
     ap.add_argument("--no-cpu-baseline", action="store_true")
-    ap.add_argument("--no-autotune", action="store_true",
-                    help="main leg: keep the default tiling (32 cells per tile, one launch per step)")
-    ap.add_argument("--tile-cells", type=int, default=0,
-                    help="main leg: this tiling (cells per tile, one launch per step) instead of the autotuner's")
+    ap.add_argument("--no-autotune", action="store_true", help="no effect: there is one form of the step")
+    ap.add_argument("--tile-cells", type=int, default=0, help="no effect: there is one form of the step")
     ap.add_argument("--no-sweep", action="store_true")
     ap.add_argument("--sweep-steps", type=int, default=400)
     ap.add_argument("--no-surrogate", action="store_true")

@@ -115,7 +115,7 @@ def run_values(stats):
 
 
 def simulate(points, steps=2000, sample_every=10, burn_in=None, max_systems=8192, seed=0, first_replica=0,
-             variant=N.LINKED_LIST_VERLET, skin=0.3, autotune=True):
+             variant=N.LINKED_LIST_VERLET, skin=0.3, autotune=False):
     """Plain batched simulation of every point (the judge): spss_batch_stats
     rows, in the order of `points`.  Points go in batches of at most
     `max_systems` systems, each batch one context stepped as one graph per

@@ -74,11 +74,13 @@ def make_batch(points, variant=N.LINKED_LIST, seed=0, skin=0.0, state_seed=1, fi
 
 
 def run_sweep(points, steps=20000, dt=0.005, sample_every=10, burn_in=None, variant=N.LINKED_LIST, seed=0,
-              skin=0.0, autotune=True, stepper=N.STOCHASTIC_EULER, first_replica=0):
+              skin=0.0, autotune=False, stepper=N.STOCHASTIC_EULER, first_replica=0):
     """Time-averaged order parameters of every point: array (len(points), 5) =
     mean and variance of the phase order, mean and variance of the
     velocity-direction order, number of samples.  Samples every
-    `sample_every` steps after `burn_in` steps (default: half the run)."""
+    `sample_every` steps after `burn_in` steps (default: half the run).
+    `autotune`: Batch.autotune before the run, which times a few steps and
+    puts the state back."""
     if burn_in is None:
         burn_in = steps // 2
     b = make_batch(points, variant=variant, seed=seed, skin=skin, first_replica=first_replica)
