@@ -60,8 +60,8 @@ int spss_mlp_set_data(spss_mlp *m, const float *x, const float *t, long n);
  * minibatch loss of every epoch. */
 int spss_mlp_train(spss_mlp *m, int epochs, int batch, float lr, const float *w, unsigned long long shuffle_seed,
                    float *loss_per_epoch);
-/* Number of tensor-core kernels this handle launched (forward, backward and
- * weight-gradient kernels). */
+/* Number of tensor-core kernels this handle launched (forward and training
+ * kernels). */
 int spss_mlp_kernel_launches(spss_mlp *m, unsigned long long *count);
 
 #ifdef __cplusplus

@@ -86,12 +86,12 @@ enum Kind
 struct FastParams
 {
   int n, nc, cap, model;      // n: slots of the whole context
-  int kind, always_rebuild, nsys;
+  int always_rebuild, nsys;
   int first, sub_n;
-  int cell0, sys, selective, pad1;  // selective: per-system rebuilds (batches of Verlet-list systems)
+  int cell0, selective;       // selective: per-system rebuilds (batches of Verlet-list systems)
   float v0, xi, xi_r, xi_phi, sigma, ca, sa;
-  float rho2_f, band_f, rmax2_f;
-  double rho2_d, half_skin;
+  float rho2_f, band_f;
+  double rho2_d;
   float dt, sqdt, half_dt2, half_dt15, inv_sqrt3, b_r, b_phi;
   uint64_t seed;
   uint32_t replica;
@@ -235,7 +235,6 @@ struct FastPath
   // leaves fewer than three cells per side evaluates all pairs every step and
   // keeps the displacement trigger (uses_verlet_list, accumulated displacement).
   bool trigger_only = false;
-  int nc_build = 1;
   int cap = 0;
   bool small_systems = false;  // a batch of Verlet-list systems that one CTA each rebuilds
   bool have_state = false;
@@ -267,7 +266,6 @@ __device__ __forceinline__ FastParams with_system(const FastParams &P, const Sys
   Q.first = S.first;
   Q.sub_n = S.n;
   Q.cell0 = S.cell0;
-  Q.sys = S.index;
   Q.v0 = S.v0;
   Q.xi = S.xi;
   Q.xi_r = S.xi_r;
@@ -277,11 +275,9 @@ __device__ __forceinline__ FastParams with_system(const FastParams &P, const Sys
   Q.sa = S.sa;
   Q.rho2_f = S.rho2_f;
   Q.band_f = S.band_f;
-  Q.rmax2_f = S.rmax2_f;
   Q.b_r = S.b_r;
   Q.b_phi = S.b_phi;
   Q.rho2_d = S.rho2_d;
-  Q.half_skin = S.half_skin;
   Q.replica = (uint32_t) S.replica;
   return Q;
 }
@@ -659,7 +655,7 @@ __global__ void fast_copyback_kernel(FastParams P, FastBuffers B)
 
 // The permuted particles are current: a rebuild of every system flips the
 // buffer parities (the flagged-system form copied its particles back).  One
-// thread; runs before the tile layouts and list builds, which read them.
+// thread; runs before the list build, which reads them.
 __global__ void fast_after_permute_kernel(FastControl *ctrl, int permuted)
 {
   if (permuted && ctrl->rebuild != REBUILD_FLAGGED)
@@ -681,8 +677,6 @@ __global__ void fast_after_rebuild_kernel(FastControl *ctrl, SysControl *sysctl,
     ctrl->rebuilds += 1;
   }
 }
-
-constexpr int kTileThreads = 128;
 
 // ---------------------------------------------------------------- step
 
@@ -1054,7 +1048,7 @@ __device__ __forceinline__ void pair_group(const uint4 *srec, const float *sw, i
 }
 
 // The same candidates again (one of them lies inside the guard band), each
-// decided by in_range.
+// decided by exact_within where it has to be.
 template<bool OMEGA>
 __device__ __noinline__ void pair_batch_exact(const uint4 *srec, const float *sw,
                                               const uint4 *__restrict__ aux, int j0, int m, int q, const uint4 ri,
@@ -1287,16 +1281,14 @@ __device__ __forceinline__ void cell_run(const uint4 *__restrict__ rec, const ui
   for (; s < e; s += 2) cell_group<OMEGA, 2, true>(rec, aux, s, e, self, xi, yi, rho2, a);
 }
 
-#ifndef SPSS_CELL_BLOCKS
-#define SPSS_CELL_BLOCKS 12
-#endif
 constexpr int kCellThreads = 128;
+constexpr int kCellBlocks = 12;  // an SM: 40 registers a thread
 
 // `fresh`: the slots were just re-sorted (the particles stand in the other
 // rec/aux buffer, the step was counted by the scan); 0: a step on the lists of
 // an earlier binning.
 template<int MODEL, int STEPPER, bool MULTI>
-__global__ void __launch_bounds__(kCellThreads, SPSS_CELL_BLOCKS) fast_cell_step_kernel(FastParams P, FastBuffers B, int fresh)
+__global__ void __launch_bounds__(kCellThreads, kCellBlocks) fast_cell_step_kernel(FastParams P, FastBuffers B, int fresh)
 {
   pdl_enter();
   constexpr bool OMEGA = STEPPER == 2;
@@ -1664,17 +1656,13 @@ __device__ __forceinline__ void walk_list(const uint4 *__restrict__ rec, const u
   }
 }
 
-#ifndef SPSS_LIST_BLOCKS_SRK
-#define SPSS_LIST_BLOCKS_SRK 12
-#endif
-#ifndef SPSS_LIST_BLOCKS_SE
-#define SPSS_LIST_BLOCKS_SE 13
-#endif
+constexpr int kTileThreads = 128;
+constexpr int kTileBlocksSRK = 12, kTileBlocksSE = 13;  // an SM: 40 and 32 registers a thread
 
-// SE or SRK step of 128 slots a CTA, one particle per thread, neighbours from its
-// Verlet list through L1 (a warp's particles are neighbours of each other).
+// SE or SRK step of a tile of 128 slots a CTA, one particle per thread, neighbours
+// from its Verlet list through L1 (a warp's particles are neighbours of each other).
 template<int MODEL, int STEPPER, bool MULTI>
-__global__ void __launch_bounds__(kTileThreads, STEPPER == 2 ? SPSS_LIST_BLOCKS_SRK : SPSS_LIST_BLOCKS_SE)
+__global__ void __launch_bounds__(kTileThreads, STEPPER == 2 ? kTileBlocksSRK : kTileBlocksSE)
     fast_tile_kernel(FastParams P, FastBuffers B)
 {
   pdl_enter();
@@ -1959,8 +1947,10 @@ __global__ void fast_order_finish_kernel(FastParams P, FastBuffers B, const Orde
 //
 // EvaluateInteractionsWithGlobalPolarOrderField (ParticleSystemFirstOrderPtr.cpp:155-223):
 // every particle couples to Z = <e^{i phi}> (and, for the complementary force
-// of the SRK stepper, to W = <omega e^{i phi}>), both summed in FP64 over the
-// stage state; no lists.
+// of the SRK stepper, to W = <omega e^{i phi}>), both summed over the stage state
+// as error-free FP32 pairs within a warp, in FP64 beyond; no lists.  The field is
+// rounded to FP32, whose last bit is some 2^24 times what the pairs leave out.  (An
+// omega that overflows them has failed its step: |omega| dt must stay below pi.)
 
 constexpr int kFieldThreads = 256;  // as block_sum4 needs
 constexpr int kFieldBlocks = 2 * 152;
@@ -2326,7 +2316,6 @@ static FastParams params(spss_ctx *ctx, double dt)
   P.n = p.n;
   P.cap = f->cap;
   P.model = p.model;
-  P.kind = f->kind;
   P.always_rebuild = f->kind == KIND_CELLS ? 1 : 0;
   P.selective = f->nsys > 1 && f->kind == KIND_VERLET ? 1 : 0;
   P.nsys = f->nsys;
@@ -2344,9 +2333,7 @@ static FastParams params(spss_ctx *ctx, double dt)
   P.sa = S.sa;
   P.rho2_f = S.rho2_f;
   P.band_f = S.band_f;
-  P.rmax2_f = S.rmax2_f;
   P.rho2_d = S.rho2_d;
-  P.half_skin = S.half_skin;
   P.b_r = S.b_r;
   P.b_phi = S.b_phi;
   P.dt = (float) dt;
@@ -2437,7 +2424,6 @@ int fast_create(spss_ctx *ctx)
     SPSS_TRY(f->field_partial.reserve(4 * kFieldBlocks));
     SPSS_CUDA_TRY(cudaMemsetAsync(f->nu.ptr, 0, sizeof(float) * n, ctx->stream));
   }
-  f->nc_build = f->h_sys[0].nc;
   if (f->kind == KIND_VERLET || f->trigger_only) ctx->uses_verlet_list = 1;
   for (int b = 0; b < 2; ++b)
   {
@@ -2631,7 +2617,7 @@ static int ensure_field(spss_ctx *ctx, const FastParams &P)
 }
 
 template<int MODEL, int STEPPER>
-static void launch_cell_tiles(spss_ctx *ctx, const FastParams &P, const FastBuffers &B, int fresh, bool chained)
+static void launch_cell_steps(spss_ctx *ctx, const FastParams &P, const FastBuffers &B, int fresh, bool chained)
 {
   const int blocks = blocks_for(P.n, kCellThreads);
   if (P.nsys > 1)
@@ -2646,12 +2632,12 @@ static int launch_cell_kernel(spss_ctx *ctx, int stepper, const FastParams &P, i
   if (ctx->timing) SPSS_CUDA_TRY(cudaEventRecord(ctx->ev0, ctx->stream));
   if (ctx->p.model == 1)
   {
-    if (stepper == SPSS_STEPPER_STOCHASTIC_EULER) launch_cell_tiles<1, 1>(ctx, P, B, fresh, chained);
-    else launch_cell_tiles<1, 2>(ctx, P, B, fresh, chained);
+    if (stepper == SPSS_STEPPER_STOCHASTIC_EULER) launch_cell_steps<1, 1>(ctx, P, B, fresh, chained);
+    else launch_cell_steps<1, 2>(ctx, P, B, fresh, chained);
   } else
   {
-    if (stepper == SPSS_STEPPER_STOCHASTIC_EULER) launch_cell_tiles<2, 1>(ctx, P, B, fresh, chained);
-    else launch_cell_tiles<2, 2>(ctx, P, B, fresh, chained);
+    if (stepper == SPSS_STEPPER_STOCHASTIC_EULER) launch_cell_steps<2, 1>(ctx, P, B, fresh, chained);
+    else launch_cell_steps<2, 2>(ctx, P, B, fresh, chained);
   }
   ++ctx->launches;
   SPSS_TRY(check_launch("fast_cell_step_kernel"));
@@ -3047,9 +3033,10 @@ static int build_device_rebuild(spss_ctx *ctx, const FastParams &P, GraphEntry &
 // graph when the trigger fires, so a step without a rebuild is two kernels
 // and no conditional node (a conditional node and its set-condition kernel
 // cost about 12 us per step on this GB300); the conditional form where this
-// device refuses device-launched graphs (or when spss_set_device_rebuild
-// asks for it, for every kind).  Cell lists: the rebuild and the step, every
-// step.  Kinds without lists: the step alone.
+// device refuses device-launched graphs or spss_set_device_rebuild asks for it
+// (then for the kinds without lists too).  Cell lists and batches of small
+// systems: the rebuild and the step, every step.  Kinds without lists: the step
+// alone.
 static int build_graph_on(spss_ctx *ctx, int stepper, const FastParams &P, int sampling, GraphEntry &g,
                           unsigned long long launches0)
 {

@@ -45,7 +45,7 @@ constexpr int oW1 = 0, ob1 = oW1 + H * IN, oW2 = ob1 + H, ob2 = oW2 + H * H, oW3
               oW4 = ob3 + H, ob4 = oW4 + OUT * H, oEnd = ob4 + OUT;
 static_assert(oEnd == NP, "parameter count");
 constexpr long long kWaitCycles = 1ll << 31;  // about one second at the SM clock
-constexpr int kMaxPartials = 2 * 152;         // CTAs of the weight-gradient kernel
+constexpr int kMaxPartials = 2 * 152;         // CTAs of the training kernel
 
 typedef __nv_bfloat16 bf16;
 

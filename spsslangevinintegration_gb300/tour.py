@@ -5,8 +5,8 @@ usage tour of the Python handles and a quick check that every path runs.
 
 * GB300 path, second-order model, Verlet skin 0.3 R, StochasticRungeKutta,
   N = 2,097,152 at density 2: upload, list rebuild (cells, binning, slot
-  permutation, tile layout, tile list build), three steps, the order
-  parameters, one trajectory frame, download;
+  permutation, list build), three steps, the order parameters, one trajectory
+  frame, download;
 * GB300 path, a batch of 64 independent second-order systems with cell lists,
   StochasticEuler: two steps with the per-system order-parameter sample;
 * GB300 path, first-order model in the global polar order field with natural
