@@ -64,29 +64,37 @@ __global__ void f64_tables_kernel(double2 *__restrict__ table)
   table[i] = make_double2(inv, log((double) j / 128.0) - delta);
 }
 
+// cos and sin of 2 pi k / 256 in units of 2^-59, from the first eighth of a turn.
+struct FixedTable
+{
+  longlong2 at[kTrigTable];
+
+  FixedTable()
+  {
+    constexpr int quarter = kTrigTable / 4, eighth = kTrigTable / 8;
+    const long double angle = 3.14159265358979323846264338327950288L / 128.0L, unit = 576460752303423488.0L;
+    long long c[quarter + 1];  // cosines of the first quarter
+    for (int k = 0; k <= eighth; ++k)
+    {
+      c[k] = std::llroundl(std::cos(angle * k) * unit);
+      c[quarter - k] = std::llroundl(std::sin(angle * k) * unit);
+    }
+    auto cosine = [&](int k) {
+      k &= kTrigTable - 1;
+      if (k > 2 * quarter) k = kTrigTable - k;
+      return k <= quarter ? c[k] : -c[2 * quarter - k];
+    };
+    for (int k = 0; k < kTrigTable; ++k) at[k] = make_longlong2(cosine(k), cosine(k - quarter));
+  }
+};
+
 int make_f64_tables(DeviceArray<double2> &table, cudaStream_t stream)
 {
+  static const FixedTable fixed;  // constants, the same for every context
   SPSS_TRY(table.reserve(kTableEntries + kTrigTable));
   f64_tables_kernel<<<(kTableEntries + 127) / 128, 128, 0, stream>>>(table.ptr);
   SPSS_TRY(check_launch("f64_tables_kernel"));
-  // cos and sin of 2 pi k / 256 in units of 2^-59, from the first eighth of a turn
-  constexpr int quarter = kTrigTable / 4, eighth = kTrigTable / 8;
-  const long double angle = 3.14159265358979323846264338327950288L / 128.0L, unit = 576460752303423488.0L;
-  long long c[quarter + 1];  // cosines of the first quarter
-  for (int k = 0; k <= eighth; ++k)
-  {
-    c[k] = std::llroundl(std::cos(angle * k) * unit);
-    c[quarter - k] = std::llroundl(std::sin(angle * k) * unit);
-  }
-  auto cosine = [&](int k) {
-    k &= kTrigTable - 1;
-    if (k > 2 * quarter) k = kTrigTable - k;
-    return k <= quarter ? c[k] : -c[2 * quarter - k];
-  };
-  longlong2 fixed[kTrigTable];
-  for (int k = 0; k < kTrigTable; ++k) fixed[k] = make_longlong2(cosine(k), cosine(k - quarter));
-  SPSS_CUDA_TRY(cudaMemcpyAsync(table.ptr + kTableEntries, fixed, sizeof(fixed), cudaMemcpyHostToDevice, stream));
-  SPSS_CUDA_TRY(cudaStreamSynchronize(stream));
+  SPSS_CUDA_TRY(cudaMemcpyAsync(table.ptr + kTableEntries, fixed.at, sizeof(fixed.at), cudaMemcpyHostToDevice, stream));
   return SPSS_OK;
 }
 
