@@ -124,3 +124,17 @@ def test_an_infinite_frequency_meets_its_own_cosine(variant):
     np.testing.assert_array_equal(force[near], np.inf * np.cos(x[7, 2] - x[near, 2]))
     near[7] = True
     assert np.isfinite(force[~near]).all()
+
+
+@pytest.mark.parametrize("model", [1, 2])
+@pytest.mark.parametrize("kind", ["aligned", "clusters"])
+@pytest.mark.parametrize("spread", [0.3, 1e-6])
+@pytest.mark.parametrize("n,rho", [(4097, 0.06), (9001, 0.03), (9001, 0.2)])
+def test_all_pairs_in_several_stretches(n, rho, spread, kind, model):
+    """More candidates a warp than a lane remembers the hits of (2,048)."""
+    if np.finfo(np.longdouble).precision <= 18:
+        pytest.skip("no quadruple precision here")
+    rng = np.random.default_rng(n)
+    phi = phases(kind, spread, 0.4, n, rng)
+    x, torque, force = run(1, n, rho, model, 0.0, phi, True)
+    check(x, model, rho, 0.0, rng.choice(n, 60, replace=False), torque, force)
